@@ -2,67 +2,179 @@
 //
 // This is the matrix product of the true 32-bit path (float32 inputs; no tensor-core mode of
 // reduced precision), and with bfloat16 inputs it is the plain reference of the tcgen05 kernel.
-// Every output element is one sequential chain of FMAs over k = 0..K-1, so a row's result does
-// not depend on which other rows share the launch. The reference's equivalent is its 64x64x16
-// float32 tile (crates/kir/src/cuda/prelude.cu:213-276).
+// Every output element is the sum (c0 + c1) + (c2 + c3) of four sequential chains of FMAs, chain g over the
+// k's with (k / 16) % 4 == g in ascending order, whatever the tile: a row's result does not depend on which
+// other rows share the launch. The reference's equivalent is its 64x64x16 float32 tile
+// (crates/kir/src/cuda/prelude.cu:213-276).
+//
+// What bounds it is the FMA units and the shared-memory reads that feed them where the product is large (128 lanes an SM; 73 TFLOP/s measured
+// for FMAs on two registers, 49 on three), and too few threads where it is not: one chain an output left a product of 777 x 1,024 x 2,048 with
+// three warps an SM. Hence four groups of 64 threads a tile, each with its own chain; their sums meet in shared memory at the end. A thread
+// holds TM x TN outputs and reads four k's of a row in one 16-byte access (rows are 68 values apart, so eight neighbouring rows meet every
+// bank once); three stages of 64 k's arrive by cp.async.
 #include "common.cuh"
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
+constexpr int GROUPS = 4, GROUP_THREADS = 64, THREADS = GROUPS * GROUP_THREADS, GK = 16, BK = GROUPS * GK, STAGES = 3;
 
-template <typename X, typename W>
-__global__ void __launch_bounds__(256) gemm_simt_kernel(const X* __restrict__ x, const W* __restrict__ w, float* __restrict__ out, int T,
-                                                        int N, int K) {
-  __shared__ float xs[BK][BM + 1];
+__device__ __forceinline__ float4 read4(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ float4 read4(const __nv_bfloat16* p) {
+  const uint2 v = *(const uint2*)p;
+  return make_float4(__uint_as_float(v.x << 16), __uint_as_float(v.x & 0xffff0000u), __uint_as_float(v.y << 16), __uint_as_float(v.y & 0xffff0000u));
+}
+
+template <typename E>
+struct Row {   // a staged row's length: 68 float32 or 72 bfloat16 (eight rows of 16 or 8 bytes meet different banks)
+  static constexpr int LEN = sizeof(E) == 4 ? BK + 4 : BK + 8;
+};
+
+// rows r0 .. r0 + R - 1 of src [n][K], columns k0 .. k0 + BK - 1, into dst [R][LEN]; what lies outside is zero. VEC: rows start on 16
+// bytes, so 16-byte asynchronous copies are used (a copy that crosses the row's end brings zeros behind it).
+template <typename E, int R, bool VEC>
+__device__ __forceinline__ void stage_rows(E* dst, const E* __restrict__ src, int r0, int n, int k0, int K, int tid) {
+  constexpr int LEN = Row<E>::LEN;
+  if constexpr (VEC) {
+    constexpr int PER = 16 / sizeof(E), QUADS = BK / PER, STEP = THREADS / QUADS;   // rows a pass of all threads brings
+    const int r = tid / QUADS, q = tid % QUADS, k = k0 + q * PER, left = max(0, min(16, (K - k) * (int)sizeof(E)));
+    const E* from = src + (size_t)(r0 + r) * K + k;
+    const uint32_t to = (uint32_t)__cvta_generic_to_shared(dst + r * LEN + q * PER);
+#pragma unroll
+    for (int u = 0; u < (R + STEP - 1) / STEP; u++) {
+      const bool in = r0 + r + u * STEP < n && left > 0;
+      if (R % STEP == 0 || r + u * STEP < R)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(to + u * STEP * LEN * (int)sizeof(E)), "l"(in ? from + (size_t)u * STEP * K : src), "r"(in ? left : 0)
+                     : "memory");
+    }
+  } else {
+    for (int e = tid; e < R * BK; e += THREADS) {
+      const int r = e / BK, k = e % BK;
+      dst[r * LEN + k] = r0 + r < n && k0 + k < K ? src[(size_t)(r0 + r) * K + k0 + k] : (E)0.f;
+    }
+  }
+}
+
+template <typename X, typename W, int BM, int BN>
+constexpr size_t smem_bytes() {
+  const size_t stages = STAGES * (BM * Row<X>::LEN * sizeof(X) + BN * Row<W>::LEN * sizeof(W)), sums = (size_t)GROUPS * BM * (BN + 4) * 4;
+  return stages > sums ? stages : sums;
+}
+
+template <typename X, typename W, int BM, int BN, int TM, int TN, bool VEC, int MINB>
+__global__ void __launch_bounds__(THREADS, MINB) gemm_simt_kernel(const X* __restrict__ x, const W* __restrict__ w, float* __restrict__ out, int T, int N, int K) {
+  static_assert((BM / TM) * (BN / TN) == GROUP_THREADS, "a group of 64 threads covers the tile");
+  constexpr int COLS = BN / TN, ROWS = BM / TM;   // thread (ty, tx) holds rows ty + ROWS i and columns tx + COLS j
+  constexpr int XL = Row<X>::LEN, WL = Row<W>::LEN;
+  extern __shared__ __align__(16) unsigned char smem[];
+  X* xs = (X*)smem;
+  W* ws = (W*)(smem + STAGES * BM * XL * sizeof(X));
   ib::pdl_launch_dependents();
   ib::pdl_wait();
-  __shared__ float ws[BK][BN + 1];
+  const int tid = threadIdx.x, group = tid / GROUP_THREADS, lane = tid % GROUP_THREADS, ty = lane / COLS, tx = lane % COLS;
   const int t0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-  const int tid = threadIdx.x;
-  const int ty = tid / 16, tx = tid % 16;  // thread's 4x4 micro tile: rows ty*4.., cols tx*4..
   float acc[TM][TN];
 #pragma unroll
   for (int i = 0; i < TM; i++)
 #pragma unroll
     for (int j = 0; j < TN; j++) acc[i][j] = 0.f;
 
-  for (int k0 = 0; k0 < K; k0 += BK) {
-    // 64 rows x 16 k = 1024 elements per operand, 4 per thread.
-#pragma unroll
-    for (int e = 0; e < 4; e++) {
-      int idx = tid + e * 256;
-      int r = idx / BK, kk = idx % BK;
-      int k = k0 + kk;
-      int t = t0 + r, n = n0 + r;
-      xs[kk][r] = (t < T && k < K) ? ib::to_f32<X>(x[(size_t)t * K + k]) : 0.f;
-      ws[kk][r] = (n < N && k < K) ? ib::to_f32<W>(w[(size_t)n * K + k]) : 0.f;
+  const int steps = (K + BK - 1) / BK;
+  auto fill = [&](int s) {
+    if (s < steps) {
+      stage_rows<X, BM, VEC>(xs + (s % STAGES) * BM * XL, x, t0, T, s * BK, K, tid);
+      stage_rows<W, BN, VEC>(ws + (s % STAGES) * BN * WL, w, n0, N, s * BK, K, tid);
     }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < STAGES - 1; s++) fill(s);
+  for (int s = 0; s < steps; s++) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(STAGES - 2) : "memory");
     __syncthreads();
+    fill(s + STAGES - 1);   // into the buffer whose readers passed the barrier
+    const X* xa = xs + (s % STAGES) * BM * XL + ty * XL + group * GK;
+    const W* wb = ws + (s % STAGES) * BN * WL + tx * WL + group * GK;
+    // (k's past the end are zeros in both operands: an FMA with them leaves a sum as it is)
 #pragma unroll
-    for (int kk = 0; kk < BK; kk++) {
-      float a[TM], b[TN];
+    for (int q = 0; q < GK; q += 4) {
+      float4 a[TM];
 #pragma unroll
-      for (int i = 0; i < TM; i++) a[i] = xs[kk][ty * TM + i];
+      for (int i = 0; i < TM; i++) a[i] = read4(xa + i * ROWS * XL + q);
 #pragma unroll
-      for (int j = 0; j < TN; j++) b[j] = ws[kk][tx * TN + j];
+      for (int j = 0; j < TN; j++) {
+        const float4 b = read4(wb + j * COLS * WL + q);
 #pragma unroll
-      for (int i = 0; i < TM; i++)
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(a[i].x, b.x, acc[i][j]);
 #pragma unroll
-        for (int j = 0; j < TN; j++) acc[i][j] = fmaf(a[i], b[j], acc[i][j]);
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(a[i].y, b.y, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(a[i].z, b.z, acc[i][j]);
+#pragma unroll
+        for (int i = 0; i < TM; i++) acc[i][j] = fmaf(a[i].w, b.w, acc[i][j]);
+      }
     }
-    __syncthreads();
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");
+  __syncthreads();
+  float* sums = (float*)smem;   // [GROUPS][BM][BN + 4]
+  constexpr int SL = BN + 4;
 #pragma unroll
-  for (int i = 0; i < TM; i++) {
-    int t = t0 + ty * TM + i;
-    if (t >= T) continue;
+  for (int i = 0; i < TM; i++)
 #pragma unroll
-    for (int j = 0; j < TN; j++) {
-      int n = n0 + tx * TN + j;
-      if (n < N) out[(size_t)t * N + n] = acc[i][j];
+    for (int j = 0; j < TN; j++) sums[(group * BM + ty + ROWS * i) * SL + tx + COLS * j] = acc[i][j];
+  __syncthreads();
+  const bool wide = N % 4 == 0 && (uintptr_t)out % 16 == 0;
+#pragma unroll
+  for (int e = tid; e < BM * BN / 4; e += THREADS) {
+    const int r = e / (BN / 4), c = e % (BN / 4) * 4, t = t0 + r, n = n0 + c;
+    if (t >= T || n >= N) continue;
+    float4 v[GROUPS];
+#pragma unroll
+    for (int g = 0; g < GROUPS; g++) v[g] = *(const float4*)&sums[(g * BM + r) * SL + c];
+    const float4 o = make_float4((v[0].x + v[1].x) + (v[2].x + v[3].x), (v[0].y + v[1].y) + (v[2].y + v[3].y), (v[0].z + v[1].z) + (v[2].z + v[3].z),
+                                 (v[0].w + v[1].w) + (v[2].w + v[3].w));
+    float* to = out + (size_t)t * N + n;
+    if (wide) {
+      *(float4*)to = o;
+    } else {
+      to[0] = o.x;
+      if (n + 1 < N) to[1] = o.y;
+      if (n + 2 < N) to[2] = o.z;
+      if (n + 3 < N) to[3] = o.w;
     }
   }
+}
+
+template <typename X, typename W, int BM, int BN, int TM, int TN, int MINB = 2>
+int run(const X* x, const W* w, float* out, int T, int N, int K, cudaStream_t stream) {
+  const bool vec = (size_t)K * sizeof(X) % 16 == 0 && (size_t)K * sizeof(W) % 16 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)w % 16 == 0;
+  dim3 grid((N + BN - 1) / BN, (T + BM - 1) / BM);
+  IB_CHECK_ARG(grid.y <= 65535, "gemm_simt: T=%d rows exceed the grid limit", T);
+  constexpr size_t bytes = smem_bytes<X, W, BM, BN>();
+  auto kernel = vec ? gemm_simt_kernel<X, W, BM, BN, TM, TN, true, MINB> : gemm_simt_kernel<X, W, BM, BN, TM, TN, false, MINB>;
+  if (bytes > 48 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    IB_CHECK_ARG(e == cudaSuccess, "gemm_simt: %s", cudaGetErrorString(e));
+  }
+  ib::launch(kernel, grid, THREADS, bytes, stream, x, w, out, T, N, K);
+  return 0;
+}
+
+// The larger the tile, the fewer shared-memory reads an FMA costs, and the fewer CTAs share the work. Measured (us, tiles of 64 x 64 | 32 x 64 |
+// 32 x 32; the form before, one chain an output on 64 x 64 tiles of 4 x 4, took 3,058, 498, 414, 208 and 155): 2,048 x 4,096 x 4,096 rows, columns
+// and k's 1,679 | 1,816 | 2,030 (41 TFLOP/s); 777 x 6,144 x 1,024 280 | 293 | 316; 777 x 1,024 x 2,048 123 | 108 | 113; 300 x 1,024 x 2,048
+// 63 | 69 | 61; 96 x 4,096 x 1,024 34 | 37 | 32. Hence 64 x 64 from four CTAs an SM on, 32 x 64 from two, 32 x 32 from one, 16 x 16 below. Up to
+// 16 rows a tile has 16, and as many columns as leave every SM a CTA (2 x 32,768 x 1,024: 50 us against 230; 8 x 1,024 x 3,072: 26 against 236).
+template <typename X, typename W>
+int go(const X* x, const W* w, float* out, int T, int N, int K, cudaStream_t stream) {
+  auto tiles = [&](int bm, int bn) { return (long long)((N + bn - 1) / bn) * ((T + bm - 1) / bm); };
+  constexpr int SMS = 148;
+  if (T <= 16 && tiles(16, 64) >= SMS) return run<X, W, 16, 64, 2, 8>(x, w, out, T, N, K, stream);
+  if (T <= 16) return run<X, W, 16, 16, 2, 2>(x, w, out, T, N, K, stream);
+  if (tiles(64, 64) >= 4 * SMS) return run<X, W, 64, 64, 8, 8, 1>(x, w, out, T, N, K, stream);   // (one CTA an SM: 64 sums and 32 operands a thread do not fit 128 registers)
+  if (tiles(32, 64) >= 2 * SMS) return run<X, W, 32, 64, 4, 8>(x, w, out, T, N, K, stream);
+  if (tiles(32, 32) >= SMS) return run<X, W, 32, 32, 4, 4>(x, w, out, T, N, K, stream);
+  return run<X, W, 16, 16, 2, 2>(x, w, out, T, N, K, stream);
 }
 
 }  // namespace
@@ -70,16 +182,16 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const X* __restrict__ x,
 extern "C" int ib_gemm_simt(const void* x, int x_dtype, const void* w, int w_dtype, float* out, int T, int N, int K, cudaStream_t stream) {
   if (T == 0 || N == 0) return 0;
   IB_CHECK_ARG(T > 0 && N > 0 && K > 0, "gemm_simt: bad sizes T=%d N=%d K=%d", T, N, K);
-  dim3 grid((N + BN - 1) / BN, (T + BM - 1) / BM);
-  IB_CHECK_ARG(grid.y <= 65535, "gemm_simt: T=%d rows exceed the grid limit", T);
+  int bad;
   if (x_dtype == IB_F32 && w_dtype == IB_F32)
-    ib::launch(gemm_simt_kernel<float, float>, grid, 256, 0, stream, (const float*)x, (const float*)w, out, T, N, K);
+    bad = go((const float*)x, (const float*)w, out, T, N, K, stream);
   else if (x_dtype == IB_BF16 && w_dtype == IB_BF16)
-    ib::launch(gemm_simt_kernel<__nv_bfloat16, __nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, T, N, K);
+    bad = go((const __nv_bfloat16*)x, (const __nv_bfloat16*)w, out, T, N, K, stream);
   else if (x_dtype == IB_F32 && w_dtype == IB_BF16)
-    ib::launch(gemm_simt_kernel<float, __nv_bfloat16>, grid, 256, 0, stream, (const float*)x, (const __nv_bfloat16*)w, out, T, N, K);
+    bad = go((const float*)x, (const __nv_bfloat16*)w, out, T, N, K, stream);
   else
     return ib_set_error("gemm_simt: unsupported dtypes x=%d w=%d", x_dtype, w_dtype);
+  if (bad) return bad;
   IB_CHECK_LAUNCH("gemm_simt");
   return 0;
 }
