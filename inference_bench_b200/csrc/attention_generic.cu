@@ -218,7 +218,8 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, IbKvView kv, c
                                          const int* __restrict__ seg_of_token, int window, float scale, A* __restrict__ out, int T,
                                          int heads, unsigned* __restrict__ status, int qk_dim, int v_dim, float softcap, int sink, int chunk,
                                          const float* __restrict__ sink_values, const float* __restrict__ gate, int gate_P, size_t gate_stride, int gate_row,
-                                         float out_scale, int out_row, int keep) {
+                                         float out_scale, int out_row, int keep, const int* __restrict__ tokens) {
+  // tokens: null, or the T rows of q and out that are computed (the others are left as they are).
   // keep > 0 (with a window): the first `keep` positions are seen as well, whatever the window.
   // qk_dim, v_dim: a query/key head's and a value head's size (at most the cache's row). softcap > 0: s <- softcap * tanh(s / softcap).
   // sink: the softmax has one more term whose score is 0 and which has no value (its denominator is 1 + sum exp(s)); with sink_values
@@ -233,7 +234,7 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, IbKvView kv, c
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   long long item = (long long)blockIdx.x * kWarps + warp;
   if (item >= (long long)T * heads) return;
-  const int t = (int)(item / heads), h = (int)(item % heads);
+  const int t = tokens ? tokens[item / heads] : (int)(item / heads), h = (int)(item % heads);
   const int kvhead = h / (heads / kv.kv_heads);
   const int pos = positions[t], seg = seg_of_token[t];
   const int lo = chunk > 0 ? pos - pos % chunk : (window > 0 ? max(0, pos - window + 1) : 0);
@@ -373,7 +374,8 @@ extern "C" int ib_qk_norm_rope_kv(const float* qkv, int P, long long stride_p, c
 extern "C" int ib_attention_generic(const void* q, int act_dtype, const IbKvView* kv, const int* positions, const int* seg_of_token,
                                     int window, float scale, void* out, int T, int heads, unsigned* status, int qk_dim, int v_dim, float softcap, int sink,
                                     int chunk, const float* sink_values, const float* gate, int gate_P, long long gate_stride, int gate_row, float out_scale,
-                                    int out_row, int keep, cudaStream_t stream) {
+                                    int out_row, int keep, const int* tokens, cudaStream_t stream) {
+  // tokens: null, or the T rows that are computed.
   // keep: the first positions that are seen beside the window. chunk, sink_values, gate, out_scale, out_row: see the kernel; out_row = 0 stands for heads * v_dim, gate = null for no gate.
   // qk_dim, v_dim: 0 = the cache's row size; softcap: 0 = scores as they are; sink: 1 = one added to the softmax's denominator.
   if (T == 0) return 0;
@@ -391,11 +393,11 @@ extern "C" int ib_attention_generic(const void* q, int act_dtype, const IbKvView
   if (act_dtype == IB_F32)
     ib::launch(attention_generic_kernel<float, float>, blocks, kWarps * 32, 0, stream, (const float*)q, *kv, positions, seg_of_token, window, scale,
                                                                               (float*)out, T, heads, status, qk_dim, v_dim, softcap, sink, chunk, sink_values, gate,
-                                                                              gate_P, (size_t)gate_stride, gate_row, out_scale, out_row, keep);
+                                                                              gate_P, (size_t)gate_stride, gate_row, out_scale, out_row, keep, tokens);
   else
     ib::launch(attention_generic_kernel<__nv_bfloat16, __nv_bfloat16>, blocks, kWarps * 32, 0, stream, 
         (const __nv_bfloat16*)q, *kv, positions, seg_of_token, window, scale, (__nv_bfloat16*)out, T, heads, status, qk_dim, v_dim, softcap, sink, chunk,
-        sink_values, gate, gate_P, (size_t)gate_stride, gate_row, out_scale, out_row, keep);
+        sink_values, gate, gate_P, (size_t)gate_stride, gate_row, out_scale, out_row, keep, tokens);
   IB_CHECK_LAUNCH("attention_generic");
   return 0;
 }

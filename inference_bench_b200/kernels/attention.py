@@ -63,6 +63,7 @@ L.register("ib_attention_decode_stream_capped", [L._p, C.POINTER(L.KvView), L._p
                                                  C.POINTER(L.AttnTail), L._i, L._p, L._p])
 L.register("ib_attention_prefill_ws_capped", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._ll, L._f, L._i, C.POINTER(L.AttnTail),
                                               L._i, L._p, L._p])
+L.register("ib_attention_prompt_f32", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._f, L._i, C.POINTER(L.AttnTail), L._i, L._p, L._p])
 L.KERNELS_PER_CALL["ib_attention_decode_capped"] = 2
 L.KERNELS_PER_CALL["ib_attention_decode_stream_capped"] = 2
 
@@ -170,6 +171,13 @@ def decode_fused(ctx, qkv: torch.Tensor, q_norm_w, k_norm_w, eps: float, cos, si
     return out
 
 
+def _prompt_f32_fits(ctx, q: torch.Tensor, view: L.KvView, heads: int, qk_dim: int, v_dim: int, out: torch.Tensor) -> bool:
+    """Whether a step's float32 prompt portions can go through the tile kernel (csrc/attention_prompt_f32.cu): heads of 64 or 128 with keys as
+    large as values, and rows that start on 16 bytes."""
+    return (not ctx.fixed_shape and q.dtype == torch.float32 and qk_dim == v_dim == view.head_dim and view.head_dim in (64, 128) and out.shape[1] % 4 == 0
+            and heads <= 65535 and (q.data_ptr() | out.data_ptr() | view.base) % 16 == 0)
+
+
 def paged_attention(ctx, q: torch.Tensor, cache: ops.KvLayerView, heads: int, window: Optional[int], scale: float, qk_dim: Optional[int] = None,
                     v_dim: Optional[int] = None, softcap: float = 0.0, sink: bool = False, chunk: int = 0, sink_values: Optional[torch.Tensor] = None,
                     gate: Optional[tuple] = None, out_scale: float = 1.0, out: Optional[torch.Tensor] = None, keep_first: int = 0,
@@ -211,10 +219,15 @@ def paged_attention(ctx, q: torch.Tensor, cache: ops.KvLayerView, heads: int, wi
     work = None if generic else _work_lists(ctx)
     if capped and not generic and work["n_tiles"] and (rt.options.prefill_attention == "tcgen05" or not cache.tma()[0]):
         generic = True    # prompt portions with capped scores run on the kernel that TMA feeds, or on the generic one
-    if generic:
-        ops.attention_generic(q, cache, ctx.positions, ctx.seg_of_token, window, scale, out, heads, rt.status, qk_dim, v_dim, softcap, sink, chunk=chunk,
-                              sink_values=sink_values, gate=gate, out_scale=out_scale, keep_first=keep_first)
-        return out
+    if generic:   # float32 portions as tiles where that kernel takes them, everything else one row at a time
+        tiles = out_scale != 0.0 and (sink or sink_values is None) and _prompt_f32_fits(ctx, q, view, heads, qk_dim, v_dim, out) and _work_lists(ctx)["n_tiles"] > 0
+        rows = _work_lists(ctx)["dec_tokens"] if tiles else None
+        if not tiles or rows is not None:
+            ops.attention_generic(q, cache, ctx.positions, ctx.seg_of_token, window, scale, out, heads, rt.status, qk_dim, v_dim, softcap, sink, chunk=chunk,
+                                  sink_values=sink_values, gate=gate, out_scale=out_scale, keep_first=keep_first, tokens=rows)
+        if not tiles:
+            return out
+        work = _work_lists(ctx)
     tail_ref = None
     if tailed:
         t = L.AttnTail(sink_values=ops._ptr(sink_values), gate=None, gate_parts=0, gate_row=0, gate_stride=0, out_scale=float(out_scale), out_row=out.shape[1], diff=0,
@@ -231,6 +244,12 @@ def paged_attention(ctx, q: torch.Tensor, cache: ops.KvLayerView, heads: int, wi
             t.gate, t.gate_parts, t.gate_row, t.gate_stride = g.data_ptr() + 4 * col, g.shape[0], g.shape[2], T * g.shape[2]
         tail_ref = C.byref(t)
     window = -int(chunk) if chunk else window   # the kernels take blocks of positions as a negative window
+    if generic:
+        ops._check("q", q, torch.float32, (T, heads * qk_dim))
+        L.call("ib_attention_prompt_f32", q.data_ptr(), C.byref(view), work["tile_seg"].data_ptr(), work["tile_row0"].data_ptr(), work["n_tiles"], ctx.seg_start.data_ptr(),
+               ctx.seg_pos0.data_ptr(), int(window or 0), float(scale), out.data_ptr(), heads, float(softcap or 0.0), 1 if sink else 0, tail_ref, keep_first,
+               rt.status.data_ptr(), ops._stream())
+        return out
     extra = (float(softcap), 1 if sink else 0, tail_ref, keep_first) if capped else ()
     tail = "_capped" if capped else ""
     stream = ops._stream()

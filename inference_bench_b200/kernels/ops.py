@@ -266,8 +266,8 @@ def qk_norm_rope_kv(qkv: torch.Tensor, q_norm_w: Optional[torch.Tensor], k_norm_
 def attention_generic(q: torch.Tensor, kv: KvLayerView, positions: torch.Tensor, seg_of_token: torch.Tensor, window: Optional[int],
                       scale: float, out: torch.Tensor, heads: int, status: torch.Tensor, qk_dim: Optional[int] = None, v_dim: Optional[int] = None,
                       softcap: float = 0.0, sink: bool = False, chunk: int = 0, sink_values: Optional[torch.Tensor] = None,
-                      gate: Optional[tuple] = None, out_scale: float = 1.0, keep_first: int = 0) -> None:
-    """keep_first > 0 (with a window): the first positions of the request are seen as well. softcap > 0: scores become softcap * tanh(score / softcap); sink: the softmax's denominator has one added (a key of score 0
+                      gate: Optional[tuple] = None, out_scale: float = 1.0, keep_first: int = 0, tokens: Optional[torch.Tensor] = None) -> None:
+    """tokens: None, or the rows of q and out (int32) that are computed, the others staying as they are. keep_first > 0 (with a window): the first positions of the request are seen as well. softcap > 0: scores become softcap * tanh(score / softcap); sink: the softmax's denominator has one added (a key of score 0
     without a value; with sink_values, float32 [heads], a key of that score per head); qk_dim, v_dim: a query/key head's and a value
     head's size (default: the cache's row). chunk > 0: a position sees the earlier positions of its own block of `chunk` positions
     (counted from 0) instead of a window. gate = (float32 partial sums [P, T, row], column of the first head): head h's output is
@@ -292,10 +292,12 @@ def attention_generic(q: torch.Tensor, kv: KvLayerView, positions: torch.Tensor,
         g_ptr, g_stride = g.data_ptr() + 4 * col, T * g_row
     _check("positions", positions, torch.int32, (T,))
     _check("seg_of_token", seg_of_token, torch.int32, (T,))
+    if tokens is not None:
+        _check("tokens", tokens, torch.int32)
     L.call("ib_attention_generic", q.data_ptr(), dtype_code(q.dtype), C.byref(view), positions.data_ptr(), seg_of_token.data_ptr(),
-           int(window or 0), float(scale), out.data_ptr(), T, heads, status.data_ptr(), qk_dim, v_dim, float(softcap or 0.0), 1 if sink else 0,
-           int(chunk or 0), _ptr(sink_values), g_ptr, g_P, g_stride, g_row, float(out_scale), out.shape[1],
-           int(keep_first), _stream())
+           int(window or 0), float(scale), out.data_ptr(), T if tokens is None else tokens.shape[0], heads, status.data_ptr(), qk_dim, v_dim, float(softcap or 0.0),
+           1 if sink else 0, int(chunk or 0), _ptr(sink_values), g_ptr, g_P, g_stride, g_row, float(out_scale), out.shape[1],
+           int(keep_first), _ptr(tokens), _stream())
 
 
 def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:

@@ -1,10 +1,12 @@
-"""The float32 path's product at the edges of their tiles."""
+"""The float32 path's product and prompt attention at the edges of their tiles."""
 from __future__ import annotations
+
+import math
 
 import pytest
 import torch
 
-from test_kernels_gpu import DEV, _g
+from test_kernels_gpu import DEV, _attention_case, _g, status  # noqa: F401  (the fixture)
 
 pytestmark = pytest.mark.gpu
 
@@ -26,3 +28,44 @@ def test_product_at_tile_edges(T, N, K, x_dtype, w_dtype):
     alone = torch.empty(1, N, device=DEV)
     ops.gemm_simt(x[-1:].contiguous(), w, alone)
     assert torch.equal(alone[0], out[-1])
+
+
+@pytest.mark.parametrize("hd,heads,kvh,page", [(128, 4, 2, 16), (64, 6, 1, 8), (128, 3, 3, 64)])
+@pytest.mark.parametrize("variant", ["plain", "window", "window_keep", "chunk", "cap_sink", "tail"])
+def test_prompt_attention_matches_the_row_kernel(status, hd, heads, kvh, page, variant):  # noqa: F811
+    """Portions around the tiles' 64 rows and 64 keys beside decoded tokens, against the kernel that takes a row a warp and (plain, window) the
+    plain reference; every portion alone gives the same bits."""
+    from inference_bench_b200.engine.context import Segment, build_context
+    from inference_bench_b200.engine.runtime import Runtime
+    from inference_bench_b200.kernels import attention, ops
+    window = 45 if variant.startswith("window") else None
+    shapes = [(300, 300), (200, 70), (97, 1), (64, 64), (65, 65), (33, 2), (129, 128), (31, 31)]
+    q, view, pos, seg, ref, _ = _attention_case(torch.float32, heads, kvh, hd, page, window, shapes, 21)
+    T, scale, g = q.shape[0], 1 / math.sqrt(hd), _g(22)
+    kw = {"plain": {}, "window": {}, "window_keep": dict(keep_first=37), "chunk": dict(chunk=50),
+          "cap_sink": dict(softcap=2.0, sink=True, sink_values=torch.randn(heads, generator=g).to(DEV)),
+          "tail": dict(sink=True, out_scale=0.5, gate=(torch.randn(2, T, heads + 3, generator=g).to(DEV), 3))}[variant]
+    rt = Runtime(DEV, "float32")
+
+    def run(rows, segments):
+        ctx = build_context(rt, segments)
+        sub = ops.KvLayerView(view.pool, view.entry, view.block_table[[s.request for s in segments]].contiguous())
+        more = dict(kw, gate=(kw["gate"][0][:, rows].contiguous(), 3)) if "gate" in kw else kw
+        wide = torch.full((ctx.n_tokens, heads * hd + 8), 7.0, device=DEV)
+        attention.paged_attention(ctx, q[rows].contiguous(), sub, heads, window, scale, out=wide, **more)
+        assert (wide[:, heads * hd:] == 7.0).all()
+        return wide[:, :heads * hd]
+
+    segs = [Segment(i, i, L - n, [0] * n) for i, (L, n) in enumerate(shapes)]
+    out = run(slice(0, T), segs)
+    rt.check_status()
+    want = torch.empty_like(q)
+    ops.attention_generic(q, view, pos, seg, window, scale, want, heads, status, **kw)
+    # both sum up to 300 weighted values in float32: a few tens of roundings of values up to the largest output
+    assert (out - want).abs().max() <= 64 * 2.0 ** -24 * want.abs().max().clamp(min=1.0)
+    if variant in ("plain", "window"):
+        assert (out.cpu().double() - ref).abs().max() <= 1e-5 * ref.abs().max()
+    at = 0
+    for s, (_, n) in zip(segs, shapes):
+        assert torch.equal(run(slice(at, at + n), [s]), out[at:at + n])
+        at += n
