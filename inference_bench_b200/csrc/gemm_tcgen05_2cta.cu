@@ -31,6 +31,7 @@ constexpr int EPI_QKV = 3;   // the q/k/v projection finished in the epilogue: p
 constexpr int EPI_CLAMPED = 6;   // EPI_SWIGLU with clamped halves (ib::clamped_glu): the limit in QkvEpi::act_pq[0], the slope in QkvEpi::act_slope
 constexpr bool epi_gated(int epi) { return epi == EPI_SWIGLU || epi == EPI_CLAMPED; }
 constexpr int EPI_RELU2 = 5;   // bfloat16 max(product, 0)^2
+constexpr int EPI_BF16 = 7;    // the product rounded to bfloat16, tokens and matrix rows exchanged as for EPI_QKV (a thread writes a token's row piece by piece)
 constexpr int EPI_XIELU = 4;   // bfloat16 xielu(product) with the activation's two numbers (QkvEpi::act_pq)
 constexpr int kQkvHead = 128;   // head size of the EPI_QKV form: a head is 128 accumulator columns
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;   // clears the bit that tells the two CTAs of a pair apart in a shared::cluster address
@@ -196,7 +197,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           }
           uint8_t* a = tiles + s * TL::kStageBytes;
           if (rank == 0) sm100::mbar_arrive_expect_tx(&full[s], 2 * TL::kStageBytes);   // the leader counts both CTAs' bytes
-          if (EPI == EPI_QKV && !waited) {   // there the rows are the tokens, which the kernel before wrote
+          if ((EPI == EPI_QKV || EPI == EPI_BF16) && !waited) {   // there the rows are the tokens, which the kernel before wrote
             ib::pdl_wait();
             waited = true;
           }
@@ -346,6 +347,22 @@ __global__ void __launch_bounds__(kThreads, 1)
             }
           }
         }
+      } else if constexpr (EPI == EPI_BF16) {
+        const int tok = n_pair + (int)rank * BM + q * 32 + lane;
+        __nv_bfloat16* dst = (__nv_bfloat16*)out_ + (size_t)tok * T + t0;
+#pragma unroll 1
+        for (int c0 = 0; c0 < BN; c0 += 32) {
+          uint32_t r[32];
+          sm100::tmem_ld_32x32b_x32(lane_addr + b * MT * BN + c0, r);
+          sm100::tmem_ld_wait();
+          if (tok < N) {
+#pragma unroll
+            for (int c = 0; c < 32; c += 8)
+              if (t0 + c0 + c < T)   // (T is a multiple of 8)
+                *(uint4*)(dst + c0 + c) = make_uint4(pack_bf16x2(__uint_as_float(r[c]), __uint_as_float(r[c + 1])), pack_bf16x2(__uint_as_float(r[c + 2]), __uint_as_float(r[c + 3])),
+                                                     pack_bf16x2(__uint_as_float(r[c + 4]), __uint_as_float(r[c + 5])), pack_bf16x2(__uint_as_float(r[c + 6]), __uint_as_float(r[c + 7])));
+          }
+        }
       } else if constexpr (EPI == EPI_STORE || EPI == EPI_ADD || EPI == EPI_XIELU || EPI == EPI_RELU2) {
         float* dst = (float*)out_;
         __nv_bfloat16* dst_act = (__nv_bfloat16*)out_;
@@ -488,6 +505,14 @@ extern "C" int ib_gemm_tcgen05_2cta(const void* x, const void* w, float* out, in
 extern "C" int ib_gemm_tcgen05_2cta_add(const void* x, const void* w, float* out, int T, int N, int K, unsigned* status, cudaStream_t stream) {
   if (T == 0 || N == 0) return 0;
   return launch<1, EPI_ADD, 256>(x, w, out, T, N, K, N, 0, status, stream);
+}
+
+// x [T, K], w [N, K] bfloat16 -> out [T, N] bfloat16: the product, rounded once (N a multiple of 8). The tokens are the rows of the MMA, so that
+// a thread of the epilogue owns a token and stores 16 bytes at a time.
+extern "C" int ib_gemm_bf16_2cta(const void* x, const void* w, void* out, int T, int N, int K, unsigned* status, cudaStream_t stream) {
+  if (T == 0 || N == 0) return 0;
+  IB_CHECK_ARG(N % 8 == 0 && ((uintptr_t)out & 15) == 0, "gemm_bf16_2cta: rows of %d values must start on 16 bytes", N);
+  return launch<1, EPI_BF16, 256>(w, x, out, N, T, K, T, 0, status, stream);
 }
 
 // x [T, K], w [N, K] bfloat16 -> act [T, N] bfloat16 = max(x w^T, 0)^2, with the activation in the epilogue.

@@ -525,6 +525,62 @@ def latent_attention_mma(q_full: torch.Tensor, kv: KvLayerView, positions: torch
            out.data_ptr(), _ptr(part_o), _ptr(part_ml), T, heads, rank, n_slices, slice_keys, status.data_ptr(), int(window or 0), _ptr(sink), _stream())
 
 
+# ---------------------------------------------------------------- latent attention of prompt portions, keys and values made per head (csrc/latent_prefill.cu)
+L.register("ib_latent_gather", [C.POINTER(L.KvView), L._p, L._i, L._p, L._p, L._i, L._i, L._i, L._p, L._p, L._p, L._p])
+L.register("ib_gemm_bf16_2cta", [L._p, L._p, L._p, L._i, L._i, L._i, L._p, L._p])
+L.register("ib_latent_prefill", [L._p, L._p, L._i, L._p, L._i, L._p, L._p, L._ll, L._i, L._f, L._p, C.POINTER(L.AttnTail), L._p, L._i, L._i, L._i, L._i, L._p, L._p])
+
+
+def latent_prefill_supports(dim: int, rot: int, vdim: int, rank: int) -> bool:
+    return bool(L.load().ib_latent_prefill_supports(int(dim), int(rot), int(vdim), int(rank)))
+
+
+def latent_keys_values(kv: KvLayerView, blocks: torch.Tensor, seg_start: torch.Tensor, seg_pos0: torch.Tensor, w_kv: torch.Tensor, rank: int, rot: int,
+                       status: torch.Tensor, window: Optional[int] = None) -> tuple:
+    """(keys and values [64 n, heads (dim + vdim)], key part [64 n, 64] or None), bfloat16: the cached latents of `blocks` (int32 [n, 2]: segment and
+    first position, 64 positions each) through w_kv [heads dim + heads vdim, rank], and their key parts with zeros behind. Positions past a
+    segment's last one of the step, and with a window those that its first token does not see, are zero rows and not read."""
+    n, N = blocks.shape[0], w_kv.shape[0]
+    _check("blocks", blocks, torch.int32, (n, 2))
+    _check("w_kv", w_kv, torch.bfloat16, (N, rank))
+    view = kv.c_view()
+    rows = 64 * n
+    x = torch.empty((rows, rank), dtype=torch.bfloat16, device=w_kv.device)
+    part = torch.empty((rows, 64), dtype=torch.bfloat16, device=w_kv.device) if rot else None
+    out = torch.empty((rows, N), dtype=torch.bfloat16, device=w_kv.device)
+    L.call("ib_latent_gather", C.byref(view), blocks.data_ptr(), n, seg_start.data_ptr(), seg_pos0.data_ptr(), int(window or 0), int(rank), int(rot), x.data_ptr(), _ptr(part), status.data_ptr(),
+           _stream())
+    L.call("ib_gemm_bf16_2cta", x.data_ptr(), w_kv.data_ptr(), out.data_ptr(), rows, N, int(rank), status.data_ptr(), _stream())
+    return out, part
+
+
+def latent_prefill(q_nope: torch.Tensor, q_full: torch.Tensor, rank: int, tiles: torch.Tensor, keys_values: torch.Tensor, key_part: Optional[torch.Tensor], scale: float,
+                   out: torch.Tensor, status: torch.Tensor, window: Optional[int] = None, sink: Optional[torch.Tensor] = None, gate: Optional[tuple] = None) -> None:
+    """Causal attention of the tokens in `tiles` (int32 [n, 4]: first token, tokens (up to 128), first position, row of keys_values at which the
+    request's position 0 would lie), q_nope [T, heads, dim] and the turned parts q_full[..., rank:] (float32): out [T, heads, vdim], those
+    tokens' rows. window, sink: as for `latent_attention`; gate: as for `gemm_heads`."""
+    T, heads, dim = q_nope.shape
+    vdim, rot = out.shape[2], q_full.shape[2] - rank
+    _check("q_nope", q_nope, torch.bfloat16)
+    _check("q_full", q_full, torch.float32, (T, heads, rank + rot))
+    _check("tiles", tiles, torch.int32, (tiles.shape[0], 4))
+    _check("keys_values", keys_values, torch.bfloat16, (keys_values.shape[0], heads * (dim + vdim)))
+    if rot:
+        _check("key_part", key_part, torch.bfloat16, (keys_values.shape[0], 64))
+    _check("out", out, torch.bfloat16, (T, heads, vdim))
+    if sink is not None:
+        _check("sink", sink, torch.float32, (heads,))
+    tail = L.AttnTail()
+    if gate is not None:
+        g, col = gate
+        _check("gate", g, torch.float32)
+        if g.dim() != 3 or g.shape[1] != T or col + heads > g.shape[2]:
+            raise L.KernelError(f"latent_prefill: the gate's partial sums {tuple(g.shape)} do not hold {heads} columns from {col} for {T} tokens")
+        tail.gate, tail.gate_parts, tail.gate_row, tail.gate_stride = g.data_ptr() + 4 * col, g.shape[0], g.shape[2], T * g.shape[2]
+    L.call("ib_latent_prefill", q_nope.data_ptr(), q_full.data_ptr() + 4 * rank if rot else None, rank + rot, tiles.data_ptr(), tiles.shape[0], keys_values.data_ptr(),
+           _ptr(key_part), keys_values.shape[0], int(window or 0), float(scale), _ptr(sink), C.byref(tail), out.data_ptr(), heads, dim, rot, vdim, status.data_ptr(), _stream())
+
+
 # ---------------------------------------------------------------- routed experts (csrc/moe.cu)
 L.register("ib_moe_route", [L._p, L._i, L._ll, L._i, L._i, L._i, L._i, L._i, L._f, L._i, L._p, L._p, L._i, L._p, L._i, L._i, L._p, L._i, L._i, L._p])
 L.register("ib_moe_route_sort", [L._p, L._i, L._ll, L._i, L._i, L._i, L._i, L._i, L._f, L._i, L._p, L._p, L._i, L._p, L._i, L._i, L._p, L._i, L._i, L._i, L._p, L._p, L._p, L._p, L._p])

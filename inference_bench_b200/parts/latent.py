@@ -9,7 +9,9 @@ With h the layer's input, per token:
 The cache row of a token is [c | r]. The kernels never build k and v: q_n . (Wuk_a c) = (Wuk_a^T q_n) . c and
 sum_j p_j Wuv_a c_j = Wuv_a (sum_j p_j c_j), so a head's query becomes [Wuk_a^T q_n | q_r] against the cached rows, and the
 weighted sum of latents goes through Wuv_a afterwards (two small per-head products around one attention kernel that reads
-kv_rank + rot_dim values a key for all heads together). A layer with own_kv=False has no Wdkv and reads the rows another
+kv_rank + rot_dim values a key for all heads together). That is the form for decoded tokens. A prompt portion has many queries a key: its
+requests' k and v are made once a step (one product over the rows that the portion sees) and a kernel with the shape of grouped attention
+reads them (csrc/latent_prefill.cu); which way a request's tokens go is decided by `_expanded`. A layer with own_kv=False has no Wdkv and reads the rows another
 layer cached.
 
 Variants, each a constructor parameter. `q_rank` n: the queries go through a latent of their own, c_q = w_q * rms_unit(Wdq h) (n values),
@@ -31,6 +33,12 @@ from . import base
 from .base import PagedRows, WeightSpec
 
 
+# A request's tokens of a step go through keys and values made per head from this many tokens on, while its context is at most so many times
+# as long (making a key's heads costs as much as about a dozen of its pairs with a query), and while the step's rows keep the keys and
+# values of one layer below this many bytes.
+EXPAND_MIN_TOKENS, EXPAND_MAX_CONTEXT, EXPAND_MAX_BYTES = 32, 64, 1 << 29
+
+
 @base.register_mixer("latent_attention")
 class LatentAttention(base.Mixer):
     def __init__(self, prefix: str, hidden: int, heads: int, dim: int, rot_dim: int, vdim: int, kv_rank: int, scale: float, norm_eps: float,
@@ -48,6 +56,7 @@ class LatentAttention(base.Mixer):
         self.sink, self.sink_dev = bool(sink), None
         self.prefix, self.hidden, self.heads, self.dim, self.rot_dim, self.vdim, self.kv_rank = prefix, hidden, heads, dim, rot_dim, vdim, kv_rank
         self.scale, self.norm_eps, self.position, self.own_kv, self.names = scale, norm_eps, position, own_kv, tuple(names)
+        self.w_kv = None      # [k rows of all heads | v rows of all heads] over the latent, where portions go through keys and values per head
         self.w_in = self.wuk_t = self.wuv = self.wo = self.c_norm = None
 
     def cache_need(self):
@@ -85,6 +94,9 @@ class LatentAttention(base.Mixer):
             self.w_uq, self.q_norm = rt.matrix(weights[self._name(8)]), rt.vector(weights[self._name(7)])
         self.wuk_t = rt.upload(weights[self._name(3)].view(H, self.dim, r).transpose(1, 2), rt.act_dtype)   # [H, rank, dim]: q_n -> rank values
         self.wuv = rt.upload(weights[self._name(4)].view(H, self.vdim, r), rt.act_dtype)                    # [H, vdim, rank]
+        if (rt.options.latent_attention == "auto" and rt.options.expert_gemm != "simt" and rt.act_dtype == torch.bfloat16 and rt.gemm != "simt" and self.scale > 0
+                and self._tensor_cores(rt) and ops.latent_prefill_supports(self.dim, self.rot_dim, self.vdim, r)):
+            self.w_kv = rt.upload(torch.cat([weights[self._name(3)], weights[self._name(4)]], dim=0), rt.act_dtype)
         self.wo = rt.matrix(weights[self._name(5)])
         if self.sink:
             self.sink_dev = rt.vector(weights[self._name(10)])
@@ -119,6 +131,38 @@ class LatentAttention(base.Mixer):
         if per <= 1 or longest == 1:
             return rows, None
         return rows, self._units(ctx, per)
+
+    def _expanded(self, ctx):
+        """None, or how the step's longer segments go through keys and values per head: (blocks [n, 2] and tiles [m, 4] on the device, see
+        `ops.latent_keys_values` and `ops.latent_prefill`; query rows a CTA holds and runs of the other segments' tokens like `_rows_and_units`,
+        None if there are no others)."""
+        if self.w_kv is None or ctx.fixed_shape or ctx.max_segment_len < EXPAND_MIN_TOKENS:
+            return None
+        key = ("latent expanded", self.window, self.heads, self.dim + self.vdim, self.kv_rank, self.rot_dim)
+        if key not in ctx.memo:
+            room = EXPAND_MAX_BYTES // (2 * self.heads * (self.dim + self.vdim)) // 64
+            blocks, tiles, rest = [], [], []
+            for s, (a, b, pos0) in enumerate(zip(ctx.h_seg_start[:-1].tolist(), ctx.h_seg_start[1:].tolist(), ctx.h_seg_pos0.tolist())):
+                first = 0 if self.window is None else max(0, pos0 - self.window + 1) // 64 * 64
+                keys = range(first, pos0 + b - a, 64)
+                if b - a < EXPAND_MIN_TOKENS or 64 * len(keys) > EXPAND_MAX_CONTEXT * (b - a) or len(blocks) + len(keys) > room:
+                    rest.append((a, b))
+                    continue
+                base = 64 * len(blocks) - first
+                blocks += [(s, k) for k in keys]
+                tiles += [(t, min(128, b - t), pos0 + t - a, base) for t in range(a, b, 128)]
+            plan = None
+            if tiles:
+                tiles.sort(key=lambda t: -(t[2] + t[1] if self.window is None else min(t[2], self.window) + t[1]))   # the tiles that see the most keys first
+                rows = ops.latent_attention_mma_rows(self.kv_rank, self.kv_rank + self.rot_dim, self.heads * max((b - a for a, b in rest), default=1))
+                per = max(1, rows // self.heads)
+                runs = [(t, min(per, b - t)) for a, b in rest for t in range(a, b, per)]
+                flat = np.concatenate([np.asarray(v, np.int32).ravel() for v in (tiles, blocks, runs)]).astype(np.int32)
+                dev = torch.from_numpy(flat).pin_memory().to(ctx.rt.device, non_blocking=True)
+                m, n = 4 * len(tiles), 4 * len(tiles) + 2 * len(blocks)
+                plan = (dev[m:n].view(-1, 2), dev[:m].view(-1, 4), (rows, dev[n:].view(-1, 2)) if rest else None)
+            ctx.memo[key] = plan
+        return ctx.memo[key]
 
     def _units(self, ctx, per):
         key = ("latent units", per)
@@ -159,21 +203,26 @@ class LatentAttention(base.Mixer):
             ops.latent_down(qd, self.q_rank, self.q_norm, cq, self.c_norm, self.norm_eps, cos, sin, ctx.positions, ctx.seg_of_token, cache, r, rot, rt.status)
             ops.latent_prepare(rt.linear(cq, self.w_uq), None, self.norm_eps, cos, sin, ctx.positions, ctx.seg_of_token, q_nope, q_full, cache, H, self.dim, rot, r,
                                False, rt.status)
-        tc = rt.options.expert_gemm != "simt"   # (the per-head maps have the m16n8k16 kernel and the FMA kernel)
-        ops.gemm_heads(q_nope, self.wuk_t, q_full, r, tensor_cores=tc and ops.rows_mma_fits(q_nope, self.wuk_t))
-        n_slices, slice_keys = self._slices(ctx, cache.c_view())
-        scratch = None
-        if n_slices > 1:
-            skey = ("latent scratch", H, r, n_slices)
-            if skey not in ctx.memo:
-                ctx.memo[skey] = (rt.empty((T * H * n_slices * r,), torch.float32), rt.empty((T * H * n_slices * 2,), torch.float32))
-            scratch = ctx.memo[skey]
-        u = rt.empty((T, H, r))
-        if self._tensor_cores(rt):
-            rows, units = self._rows_and_units(ctx)
-            ops.latent_attention_mma(q_full, cache, ctx.positions, ctx.seg_of_token, units, self.scale, u, r, n_slices, slice_keys, scratch, rt.status, rows, window=self.window, sink=self.sink_dev)
-        else:
-            ops.latent_attention(q_full, cache, ctx.positions, ctx.seg_of_token, self.scale, u, r, n_slices, slice_keys, scratch, rt.status, window=self.window, sink=self.sink_dev)
+        plan = self._expanded(ctx)
         v = rt.empty((T, H, self.vdim))
-        ops.gemm_heads(u, self.wuv, v, self.vdim, tensor_cores=tc and ops.rows_mma_fits(u, self.wuv), gate=gate)
+        if plan is None or plan[2] is not None:   # the tokens whose queries go to the latents' space
+            tc = rt.options.expert_gemm != "simt"   # (the per-head maps have the m16n8k16 kernel and the FMA kernel)
+            ops.gemm_heads(q_nope, self.wuk_t, q_full, r, tensor_cores=tc and ops.rows_mma_fits(q_nope, self.wuk_t))
+            n_slices, slice_keys = self._slices(ctx, cache.c_view())
+            scratch = None
+            if n_slices > 1:
+                skey = ("latent scratch", H, r, n_slices)
+                if skey not in ctx.memo:
+                    ctx.memo[skey] = (rt.empty((T * H * n_slices * r,), torch.float32), rt.empty((T * H * n_slices * 2,), torch.float32))
+                scratch = ctx.memo[skey]
+            u = rt.empty((T, H, r))
+            if self._tensor_cores(rt):
+                rows, units = self._rows_and_units(ctx) if plan is None else plan[2]
+                ops.latent_attention_mma(q_full, cache, ctx.positions, ctx.seg_of_token, units, self.scale, u, r, n_slices, slice_keys, scratch, rt.status, rows, window=self.window, sink=self.sink_dev)
+            else:
+                ops.latent_attention(q_full, cache, ctx.positions, ctx.seg_of_token, self.scale, u, r, n_slices, slice_keys, scratch, rt.status, window=self.window, sink=self.sink_dev)
+            ops.gemm_heads(u, self.wuv, v, self.vdim, tensor_cores=tc and ops.rows_mma_fits(u, self.wuv), gate=gate)
+        if plan is not None:   # and those that see keys and values per head (their rows of v hold nothing yet)
+            kv, part = ops.latent_keys_values(cache, plan[0], ctx.seg_start, ctx.seg_pos0, self.w_kv, r, rot, rt.status, self.window)
+            ops.latent_prefill(q_nope, q_full, r, plan[1], kv, part, self.scale, v, rt.status, window=self.window, sink=self.sink_dev, gate=gate)
         return rt.linear(v.view(T, H * self.vdim), self.wo, add_to=residual)
