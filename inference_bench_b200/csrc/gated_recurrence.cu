@@ -3,11 +3,12 @@
 // where z_q, z_f, v are the rows [q | f | v] of one fused projection (float32 partial sums, added in order). The state S [D, V] is
 // float32, lives in the request's state slot, starts at zero and is carried from token to token; everything here is float32.
 //
-//  * gated_recurrence: one CTA per (segment, head, 32 or 16 value columns). A thread owns two neighbouring columns and RPT neighbouring rows of
+//  * gated_recurrence: one CTA per (segment, head, 64, 32 or 16 value columns). A thread owns two (or four) neighbouring columns and RPT rows of
 //    S in registers; the tokens of the segment are walked in order, sixteen at a time: the CTA first turns the sixteen tokens' projections
 //    into q, f and 1 - f in shared memory, then every thread updates its rows (the gates and queries of its rows come as 16-byte reads
-//    and serve both columns) and adds its share of o, which a shuffle sums over the DS threads of the column pair. The kernel is bound by
-//    instruction issue, not by memory: what counts is instructions per FMA. A decoded token is a segment of one: the cost is then the state's trip from memory and back.
+//    and serve all its columns; two rows advance in one two-wide instruction) and adds its share of o, which a shuffle sums over the DS threads
+//    of the same columns. The kernel is bound by instruction issue and the latency of shared-memory reads, not by memory: what counts is
+//    instructions per FMA. A decoded token is a segment of one: the cost is then the state's trip from memory and back.
 //    With `chunks` the same kernel walks chunks of a long segment instead, each from a zero state: it leaves the chunk's own
 //    outputs, its closing state and decay, and q_t times the decay from the chunk's start to t; `chunk_carry` then walks a segment's
 //    chunks in order (S_in of the next = decay * S_in + the chunk's closing state, elementwise, ending in the request's state) and
@@ -60,7 +61,7 @@ __device__ __forceinline__ float2 log_gates(const IbMemoryGates& g, int t, int a
   return make_float2(zi, fminf(zf, 0.f) - log1pf(expf(-fabsf(zf))));
 }
 
-// RPT: rows of S a thread holds (for each of its two columns); kCols: value columns per CTA (32, or 16 where a thread holds sixteen rows)
+// RPT: rows of S a thread holds (for each of its NC columns); kCols: value columns per CTA (16 NC, or 16 where a thread holds sixteen rows)
 struct RecurrenceExtras {
   const float* cos_t;   // form 2: float32 [T][rot_half], the angles of the first 2 * rot_half entries of q and k (entry i with i + rot_half), or null
   const float* sin_t;
@@ -72,8 +73,8 @@ struct RecurrenceExtras {
 };
 
 // FIXED: forms 1 and 2 (one decay a head, kept in a register), BONUS: form 3, both: form 4 (one decay a head and token, in shared memory)
-template <int RPT, int kCols, bool FIXED_, bool BONUS_, int MAXT>
-__global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? 3 : 1) gated_recurrence_kernel(const float* __restrict__ q_src, const float* __restrict__ f_src, const float* __restrict__ v_src,
+template <int RPT, int kCols, int NC, bool FIXED_, bool BONUS_, int MAXT>
+__global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? (NC == 2 ? 3 : 2) : 1) gated_recurrence_kernel(const float* __restrict__ q_src, const float* __restrict__ f_src, const float* __restrict__ v_src,
                                         int P, size_t stride_p, int R, const float* __restrict__ f_bias,
                                         const float* __restrict__ lower, float* __restrict__ state, size_t slot_stride, const int* __restrict__ seg_start,
                                         const int* __restrict__ seg_slot, float* __restrict__ o_out, int heads, int D, int V, int DS,
@@ -88,6 +89,7 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? 3 : 1) gated_r
   // seg_list: the segments this launch walks (null: all). chunks != null: blockIdx.x is a chunk (first row, rows) that starts from a zero
   // state and leaves its closing state in chunk_state[chunk][head], its decay in chunk_decay[chunk][head] and q * decay in qa_out[row][head].
   constexpr bool GATED = FIXED_ && BONUS_, FIXED = FIXED_, BONUS = BONUS_ && !FIXED_;
+  constexpr int kSums = NC * kGroup;
   __shared__ float s_keep[GATED ? kChunk : 1], s_take[GATED ? kChunk : 1];
   extern __shared__ float sm[];   // q[kChunk][D], f[kChunk][D], g[kChunk][D], v[kChunk][kCols], running decay [D]
   float* sq = sm;
@@ -98,9 +100,11 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? 3 : 1) gated_r
   ib::pdl_launch_dependents();
   ib::pdl_wait();
   const int a = blockIdx.y, j0 = blockIdx.z * kCols;
-  const int tid = threadIdx.x, ds = tid % DS, col = 2 * (tid / DS), j = j0 + col;   // columns j and j + 1, rows ds * RPT .. ds * RPT + RPT - 1
-  const int d0 = ds * RPT;
-  const bool live = j0 + 2 * ((tid & ~31) / DS) < V;   // (a warp whose columns all lie beyond V only helps to prepare the tokens)
+  const int tid = threadIdx.x, ds = tid % DS, col = NC * (tid / DS), j = j0 + col;   // columns j .. j + NC - 1
+  // A thread's rows: groups of four, 4 DS apart, so that the 16-byte reads of neighbouring threads lie side by side (rows in one run of RPT met every
+  // bank twice, half of the kernel's shared-memory cycles).
+  auto row = [&](int r) { return (r >> 2) * 4 * DS + 4 * ds + (r & 3); };
+  const bool live = j0 + NC * ((tid & ~31) / DS) < V;   // (a warp whose columns all lie beyond V only helps to prepare the tokens)
   const bool d4 = D % 4 == 0;
   int t0, t1;
   float* S;
@@ -114,20 +118,20 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? 3 : 1) gated_r
     t0 = seg_start[s], t1 = seg_start[s + 1];
     S = state + (size_t)seg_slot[s] * slot_stride + (size_t)a * D * V;
   }
-  float st[RPT][2];
+  float2 st[RPT / 2][NC];   // rows 2 r and 2 r + 1 of a column side by side: one two-wide instruction advances both
+  auto load = [&](int d, int c) { return (!chunks && d < D && j + c < V) ? S[(size_t)d * V + j + c] : 0.f; };
 #pragma unroll
-  for (int r = 0; r < RPT; r++) {
-    const int d = d0 + r;
-    st[r][0] = (!chunks && d < D && j < V) ? S[(size_t)d * V + j] : 0.f;
-    st[r][1] = (!chunks && d < D && j + 1 < V) ? S[(size_t)d * V + j + 1] : 0.f;
-  }
+  for (int r = 0; r < RPT / 2; r++)
+#pragma unroll
+    for (int c = 0; c < NC; c++) st[r][c] = make_float2(load(row(2 * r), c), load(row(2 * r + 1), c));
   const int v_cols = GATED ? V - 1 : V;   // columns the values' source has
   const int q_off = a * D, v_off = a * v_cols + j0;
   const float fixed = FIXED && !GATED ? lower[a] : 0.f;
-  float u[BONUS ? RPT : 1];
+  float2 u[BONUS ? RPT / 2 : 1];
   if constexpr (BONUS) {
+    auto bonus = [&](int d) { return d < D ? lower[a * D + d] : 0.f; };
 #pragma unroll
-    for (int r = 0; r < RPT; r++) u[r] = d0 + r < D ? lower[a * D + d0 + r] : 0.f;
+    for (int r = 0; r < RPT / 2; r++) u[r] = make_float2(bonus(row(2 * r)), bonus(row(2 * r + 1)));
   }
   for (int c0 = t0; c0 < t1; c0 += kChunk) {
     const int n = min(kChunk, t1 - c0);
@@ -145,102 +149,106 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? 3 : 1) gated_r
         }
       }
     }
-    // The sixteen tokens' rows into shared memory: every thread requests its values of kLoads items before it uses the first.
-    const int step = kLoads * blockDim.x;
+    // The sixteen tokens' rows into shared memory. A thread stays at its entry of the head and goes through the tokens, kLoads at a time, every value
+    // requested before the first is used (an item's token and entry by division took a third of the kernel's instructions).
     if (FIXED && form == 2) {   // an item is a pair of entries that are turned together, or one that is not
-      const int half = ex.rot_half, per = D - half, items = n * per;
-      for (int i0 = tid; i0 < items; i0 += step) {
-        float zq[kLoads], zk[kLoads], yq[kLoads], yk[kLoads], c[kLoads], sn[kLoads];
-#pragma unroll
-        for (int e = 0; e < kLoads; e++) {
-          const int i = i0 + e * (int)blockDim.x;
-          zq[e] = zk[e] = yq[e] = yk[e] = c[e] = sn[e] = 0.f;
-          if (i >= items) continue;
-          const int tt = i / per, w = i % per;
-          const size_t at = (size_t)(c0 + tt) * R + q_off + (w < half ? w : w + half);
-          zq[e] = q_src[at], zk[e] = f_src[at];
-          if (w < half) {
-            yq[e] = q_src[at + half], yk[e] = f_src[at + half];
-            c[e] = ex.cos_t[(size_t)(c0 + tt) * half + w], sn[e] = ex.sin_t[(size_t)(c0 + tt) * half + w];
-          }
-        }
-        for (int p = 1; p < P; p++) {
+      const int half = ex.rot_half, per = D - half, lanes = max(1, (int)blockDim.x / per), first = tid / per;
+      for (int w = tid % per; w < per && first < lanes; w += blockDim.x) {
+        const int d = w < half ? w : w + half;
+        const bool pair = w < half;
+        for (int tb = first; tb < n; tb += kLoads * lanes) {
+          float zq[kLoads], zk[kLoads], yq[kLoads], yk[kLoads], c[kLoads], sn[kLoads];
 #pragma unroll
           for (int e = 0; e < kLoads; e++) {
-            const int i = i0 + e * (int)blockDim.x;
-            if (i >= items) continue;
-            const int tt = i / per, w = i % per;
-            const size_t at = p * stride_p + (size_t)(c0 + tt) * R + q_off + (w < half ? w : w + half);
-            zq[e] += q_src[at], zk[e] += f_src[at];
-            if (w < half) yq[e] += q_src[at + half], yk[e] += f_src[at + half];
+            const int tt = tb + e * lanes;
+            zq[e] = zk[e] = yq[e] = yk[e] = c[e] = sn[e] = 0.f;
+            if (tt >= n) continue;
+            const size_t at = (size_t)(c0 + tt) * R + q_off + d;
+            zq[e] = q_src[at], zk[e] = f_src[at];
+            if (pair) {
+              yq[e] = q_src[at + half], yk[e] = f_src[at + half];
+              c[e] = ex.cos_t[(size_t)(c0 + tt) * half + w], sn[e] = ex.sin_t[(size_t)(c0 + tt) * half + w];
+            }
           }
-        }
+#pragma unroll 2
+          for (int p = 1; p < P; p++) {
 #pragma unroll
-        for (int e = 0; e < kLoads; e++) {
-          const int i = i0 + e * (int)blockDim.x;
-          if (i >= items) continue;
-          const int tt = i / per, w = i % per;
-          float q = zq[e], k = zk[e];
-          if (w < half) {
-            sq[tt * D + w + half] = yq[e] * c[e] + zq[e] * sn[e];
-            sg[tt * D + w + half] = (yk[e] * c[e] + zk[e] * sn[e]) * ex.k_scale;
-            q = zq[e] * c[e] - yq[e] * sn[e], k = zk[e] * c[e] - yk[e] * sn[e];
+            for (int e = 0; e < kLoads; e++) {
+              const int tt = tb + e * lanes;
+              if (tt >= n) continue;
+              const size_t at = p * stride_p + (size_t)(c0 + tt) * R + q_off + d;
+              zq[e] += q_src[at], zk[e] += f_src[at];
+              if (pair) yq[e] += q_src[at + half], yk[e] += f_src[at + half];
+            }
           }
-          const int d = w < half ? w : w + half;
-          sq[tt * D + d] = q;
-          sg[tt * D + d] = k * ex.k_scale;
+#pragma unroll
+          for (int e = 0; e < kLoads; e++) {
+            const int tt = tb + e * lanes;
+            if (tt >= n) continue;
+            float q = zq[e], k = zk[e];
+            if (pair) {
+              sq[tt * D + w + half] = yq[e] * c[e] + zq[e] * sn[e];
+              sg[tt * D + w + half] = (yk[e] * c[e] + zk[e] * sn[e]) * ex.k_scale;
+              q = zq[e] * c[e] - yq[e] * sn[e], k = zk[e] * c[e] - yk[e] * sn[e];
+            }
+            sq[tt * D + d] = q;
+            sg[tt * D + d] = k * ex.k_scale;
+          }
         }
       }
     } else {
-      const int items = n * D;
-      for (int i0 = tid; i0 < items; i0 += step) {
-        float zq[kLoads], zf[kLoads], dc[kLoads];
-#pragma unroll
-        for (int e = 0; e < kLoads; e++) {
-          const int i = i0 + e * (int)blockDim.x;
-          zq[e] = zf[e] = dc[e] = 0.f;
-          if (i >= items) continue;
-          const int tt = i / D, d = i % D;
-          const size_t at = (size_t)(c0 + tt) * R + q_off + d;
-          zq[e] = q_src[at], zf[e] = f_src[at];
-          if (BONUS) dc[e] = ex.decay[(size_t)(c0 + tt) * heads * D + q_off + d];
-        }
-        for (int p = 1; p < P; p++) {
+      const int lanes = max(1, (int)blockDim.x / D), first = tid / D;
+      for (int d = tid % D; d < D && first < lanes; d += blockDim.x) {
+        float bias = 0.f, lo = 0.f;
+        if constexpr (!FIXED && !BONUS) bias = f_bias[a * D + d], lo = lower[a * D + d];
+        for (int tb = first; tb < n; tb += kLoads * lanes) {
+          float zq[kLoads], zf[kLoads], dc[kLoads];
 #pragma unroll
           for (int e = 0; e < kLoads; e++) {
-            const int i = i0 + e * (int)blockDim.x;
-            if (i >= items) continue;
-            const size_t at = p * stride_p + (size_t)(c0 + i / D) * R + q_off + i % D;
-            zq[e] += q_src[at], zf[e] += f_src[at];
+            const int tt = tb + e * lanes;
+            zq[e] = zf[e] = dc[e] = 0.f;
+            if (tt >= n) continue;
+            const size_t at = (size_t)(c0 + tt) * R + q_off + d;
+            zq[e] = q_src[at], zf[e] = f_src[at];
+            if (BONUS) dc[e] = ex.decay[(size_t)(c0 + tt) * heads * D + q_off + d];
           }
-        }
+#pragma unroll 2
+          for (int p = 1; p < P; p++) {
 #pragma unroll
-        for (int e = 0; e < kLoads; e++) {
-          const int i = i0 + e * (int)blockDim.x;
-          if (i >= items) continue;
-          if constexpr (BONUS) {
-            sq[i] = zq[e];
-            sg[i] = zf[e];
-            sf[i] = dc[e];
-          } else if constexpr (GATED) {
-            sq[i] = zq[e] * ex.k_scale;
-            sg[i] = zf[e];
-          } else if constexpr (FIXED) {
-            sq[i] = zq[e] / (1.f + expf(-zq[e]));
-            sg[i] = zf[e] / (1.f + expf(-zf[e]));
-          } else {
-            sq[i] = zq[e] / (1.f + expf(-zq[e]));
-            const int d = i % D;
-            const float z = zf[e] + f_bias[a * D + d];
-            const float lo = lower[a * D + d];
-            const float sig = 1.f / (1.f + expf(-z));
-            const float f = __fmaf_rn(1.f - lo, sig, lo);
-            sf[i] = f;
-            sg[i] = 1.f - f;
+            for (int e = 0; e < kLoads; e++) {
+              const int tt = tb + e * lanes;
+              if (tt >= n) continue;
+              const size_t at = p * stride_p + (size_t)(c0 + tt) * R + q_off + d;
+              zq[e] += q_src[at], zf[e] += f_src[at];
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < kLoads; e++) {
+            const int tt = tb + e * lanes, i = tt * D + d;
+            if (tt >= n) continue;
+            if constexpr (BONUS) {
+              sq[i] = zq[e];
+              sg[i] = zf[e];
+              sf[i] = dc[e];
+            } else if constexpr (GATED) {
+              sq[i] = zq[e] * ex.k_scale;
+              sg[i] = zf[e];
+            } else if constexpr (FIXED) {
+              sq[i] = zq[e] / (1.f + expf(-zq[e]));
+              sg[i] = zf[e] / (1.f + expf(-zf[e]));
+            } else {
+              sq[i] = zq[e] / (1.f + expf(-zq[e]));
+              const float z = zf[e] + bias;
+              const float sig = 1.f / (1.f + expf(-z));
+              const float f = __fmaf_rn(1.f - lo, sig, lo);
+              sf[i] = f;
+              sg[i] = 1.f - f;
+            }
           }
         }
       }
     }
+    const int step = kLoads * blockDim.x;
     for (int i0 = tid; i0 < n * kCols; i0 += step) {
       float z[kLoads];
 #pragma unroll
@@ -273,62 +281,78 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? 3 : 1) gated_r
         run[d] = r;
       }
     }
-    // one token: the thread's rows of the state advance, acc0 and acc1 receive its share of o for its two columns
-    auto advance = [&](int tt, float& acc0, float& acc1) {
+    // one token: the thread's rows of the state advance, acc[c] receives its share of o for its column c (even rows and odd rows, then both)
+    auto advance = [&](int tt, float* acc) {
       const float take = GATED ? s_take[GATED ? tt : 0] : 1.f, keep = GATED ? s_keep[GATED ? tt : 0] : fixed;
-      const float v0 = GATED ? take * sv[tt * kCols + col] : sv[tt * kCols + col], v1 = GATED ? take * sv[tt * kCols + col + 1] : sv[tt * kCols + col + 1];
-      float f[RPT], g[RPT], q[RPT];
-      if (d4 && d0 + RPT <= D) {   // this thread's rows are whole groups of four: 16-byte reads
+      float v[NC];
+      if constexpr (NC == 4) {
+        const float4 w = *(const float4*)(sv + tt * kCols + col);
+        v[0] = w.x, v[1] = w.y, v[2] = w.z, v[3] = w.w;
+      } else {
+        const float2 w = *(const float2*)(sv + tt * kCols + col);
+        v[0] = w.x, v[1] = w.y;
+      }
+#pragma unroll
+      for (int c = 0; c < NC; c++) v[c] = GATED ? take * v[c] : v[c];
+      float2 f[RPT / 2], g[RPT / 2], q[RPT / 2];
+      if (d4 && row(RPT - 1) < D) {   // this thread's rows are whole groups of four: 16-byte reads
 #pragma unroll
         for (int r = 0; r < RPT; r += 4) {
-          const float4 b = *(const float4*)(sg + tt * D + d0 + r), c = *(const float4*)(sq + tt * D + d0 + r);
-          const float4 a = FIXED ? make_float4(keep, keep, keep, keep) : *(const float4*)(sf + tt * D + d0 + r);
-          f[r] = a.x, f[r + 1] = a.y, f[r + 2] = a.z, f[r + 3] = a.w;
-          g[r] = b.x, g[r + 1] = b.y, g[r + 2] = b.z, g[r + 3] = b.w;
-          q[r] = c.x, q[r + 1] = c.y, q[r + 2] = c.z, q[r + 3] = c.w;
+          const float4 b = *(const float4*)(sg + tt * D + row(r)), c = *(const float4*)(sq + tt * D + row(r));
+          const float4 a = FIXED ? make_float4(keep, keep, keep, keep) : *(const float4*)(sf + tt * D + row(r));
+          f[r / 2] = make_float2(a.x, a.y), f[r / 2 + 1] = make_float2(a.z, a.w);
+          g[r / 2] = make_float2(b.x, b.y), g[r / 2 + 1] = make_float2(b.z, b.w);
+          q[r / 2] = make_float2(c.x, c.y), q[r / 2 + 1] = make_float2(c.z, c.w);
         }
       } else {
+        auto at = [&](const float* entries, int d) { return d < D ? entries[tt * D + d] : 0.f; };
 #pragma unroll
-        for (int r = 0; r < RPT; r++) {
-          const int d = d0 + r;
-          const bool in = d < D;
-          f[r] = FIXED ? keep : in ? sf[tt * D + d] : 0.f, g[r] = in ? sg[tt * D + d] : 0.f, q[r] = in ? sq[tt * D + d] : 0.f;
+        for (int r = 0; r < RPT / 2; r++) {
+          const int d = row(2 * r);   // (and d + 1)
+          f[r] = FIXED ? make_float2(keep, keep) : make_float2(at(sf, d), at(sf, d + 1));
+          g[r] = make_float2(at(sg, d), at(sg, d + 1)), q[r] = make_float2(at(sq, d), at(sq, d + 1));
         }
       }
-      acc0 = acc1 = 0.f;
-      if constexpr (BONUS) {
-        float own = 0.f;   // this thread's rows of r . (u k)
+      float2 sum[NC];
 #pragma unroll
-        for (int r = 0; r < RPT; r++) {
-          own = __fmaf_rn(q[r], u[r] * g[r], own);
-          acc0 = __fmaf_rn(st[r][0], q[r], acc0);
-          acc1 = __fmaf_rn(st[r][1], q[r], acc1);
-          st[r][0] = __fmaf_rn(f[r], st[r][0], g[r] * v0);
-          st[r][1] = __fmaf_rn(f[r], st[r][1], g[r] * v1);
+      for (int c = 0; c < NC; c++) sum[c] = make_float2(0.f, 0.f);
+      if constexpr (BONUS) {
+        float2 own = make_float2(0.f, 0.f);   // this thread's rows of r . (u k)
+#pragma unroll
+        for (int r = 0; r < RPT / 2; r++) {
+          own = __ffma2_rn(q[r], __fmul2_rn(u[r], g[r]), own);
+#pragma unroll
+          for (int c = 0; c < NC; c++) {
+            sum[c] = __ffma2_rn(st[r][c], q[r], sum[c]);
+            st[r][c] = __ffma2_rn(f[r], st[r][c], __fmul2_rn(g[r], make_float2(v[c], v[c])));
+          }
         }
-        acc0 = __fmaf_rn(own, v0, acc0);
-        acc1 = __fmaf_rn(own, v1, acc1);
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc[c] = __fmaf_rn(own.x + own.y, v[c], sum[c].x + sum[c].y);
       } else {
 #pragma unroll
-        for (int r = 0; r < RPT; r++) {   // rows beyond D have f = g = q = 0: their state stays zero
-          st[r][0] = __fmaf_rn(f[r], st[r][0], g[r] * v0);
-          st[r][1] = __fmaf_rn(f[r], st[r][1], g[r] * v1);
-          acc0 = __fmaf_rn(st[r][0], q[r], acc0);
-          acc1 = __fmaf_rn(st[r][1], q[r], acc1);
+        for (int r = 0; r < RPT / 2; r++) {   // rows beyond D have f = g = q = 0: their state stays zero
+#pragma unroll
+          for (int c = 0; c < NC; c++) {
+            st[r][c] = __ffma2_rn(f[r], st[r][c], __fmul2_rn(g[r], make_float2(v[c], v[c])));
+            sum[c] = __ffma2_rn(st[r][c], q[r], sum[c]);
+          }
         }
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc[c] = sum[c].x + sum[c].y;
       }
     };
     int tt = 0;
-    // Eight tokens at a time: their sixteen sums per thread are reduced over the DS threads of the column pair together, each exchange halving
-    // what a lane still holds (15 shuffles for eight tokens and DS = 16 instead of 64; the pairs that are added, and so the bits, are those of
+    // Eight tokens at a time: their 8 NC sums per thread are reduced over the DS threads of the columns together, each exchange halving
+    // what a lane still holds (15 shuffles for eight tokens of two columns and DS = 16 instead of 64; the pairs that are added, and so the bits, are those of
     // the token-by-token reduction).
     for (; live && tt + kGroup <= n; tt += kGroup) {
-      float acc[2 * kGroup];
+      float acc[kSums];
 #pragma unroll
-      for (int k = 0; k < kGroup; k++) advance(tt + k, acc[2 * k], acc[2 * k + 1]);
+      for (int k = 0; k < kGroup; k++) advance(tt + k, acc + NC * k);
       int o = DS >> 1, first = 0;   // first: number of the sum that acc[0] ends up with
 #pragma unroll
-      for (int half = kGroup; half >= 1; half >>= 1) {
+      for (int half = kSums / 2; half >= 1; half >>= 1) {
         if (o > 0) {
           const bool up = ds & o;
 #pragma unroll
@@ -341,34 +365,38 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? 3 : 1) gated_r
         }
       }
       for (; o > 0; o >>= 1) acc[0] += __shfl_xor_sync(0xffffffffu, acc[0], o);   // more lanes than sums
-      if (DS <= 2 * kGroup || (ds & (DS / (2 * kGroup) - 1)) == 0) {
-        const int held = DS >= 2 * kGroup ? 1 : 2 * kGroup / DS;
+      if (DS <= kSums || (ds & (DS / kSums - 1)) == 0) {
+        const int held = DS >= kSums ? 1 : kSums / DS;
 #pragma unroll
-        for (int i = 0; i < kGroup; i++) {   // DS >= 2: at most kGroup sums a lane
-          const int m = first + i, c = m & 1;
-          if (i < held && j + c < V) o_out[((size_t)(c0 + tt + (m >> 1)) * heads + a) * V + j + c] = acc[i];
+        for (int i = 0; i < kSums / 2; i++) {   // DS >= 2: at most half of the sums a lane
+          const int m = first + i, c = m % NC;
+          if (i < held && j + c < V) o_out[((size_t)(c0 + tt + m / NC) * heads + a) * V + j + c] = acc[i];
         }
       }
     }
     for (; live && tt < n; tt++) {
-      float acc0, acc1;
-      advance(tt, acc0, acc1);
+      float acc[NC];
+      advance(tt, acc);
       for (int o = DS >> 1; o > 0; o >>= 1) {
-        acc0 += __shfl_xor_sync(0xffffffffu, acc0, o);
-        acc1 += __shfl_xor_sync(0xffffffffu, acc1, o);
+#pragma unroll
+        for (int c = 0; c < NC; c++) acc[c] += __shfl_xor_sync(0xffffffffu, acc[c], o);
       }
       if (ds == 0) {
         float* dst = o_out + ((size_t)(c0 + tt) * heads + a) * V + j;
-        if (j < V) dst[0] = acc0;
-        if (j + 1 < V) dst[1] = acc1;
+#pragma unroll
+        for (int c = 0; c < NC; c++)
+          if (j + c < V) dst[c] = acc[c];
       }
     }
   }
 #pragma unroll
-  for (int r = 0; r < RPT; r++) {
-    const int d = d0 + r;
-    if (d < D && j < V) S[(size_t)d * V + j] = st[r][0];
-    if (d < D && j + 1 < V) S[(size_t)d * V + j + 1] = st[r][1];
+  for (int r = 0; r < RPT / 2; r++) {
+    const int d = row(2 * r);
+#pragma unroll
+    for (int c = 0; c < NC; c++) {
+      if (d < D && j + c < V) S[(size_t)d * V + j + c] = st[r][c].x;
+      if (d + 1 < D && j + c < V) S[(size_t)(d + 1) * V + j + c] = st[r][c].y;
+    }
   }
   if (chunks && blockIdx.z == 0) {
     __syncthreads();
@@ -650,7 +678,13 @@ int launch_recurrence(const float* q_src, const float* f_src, const float* v_src
   IB_CHECK_ARG(n_segments > 0 && P >= 1 && heads > 0 && D > 0 && V > 0, "recurrence: bad sizes segments=%d P=%d heads=%d D=%d V=%d", n_segments, P, heads, D, V);
   IB_CHECK_ARG(D <= 512, "recurrence: a head's key size %d is above 512", D);
   IB_CHECK_ARG(R >= heads * D && R >= heads * V, "recurrence: rows of %d entries do not hold %d heads of %d and %d", R, heads, D, V);
-  const int rpt = D <= 256 ? 8 : 16, kCols = D <= 256 ? 32 : 16;
+  // Four columns a thread halve the work of preparing tokens, which every CTA of a head repeats, and the shared-memory reads a state entry costs;
+  // two leave twice the CTAs. Chunk walks of 16 heads of 128 x 128 (us, the form before: one row and column an instruction, items by division):
+  // 2,048 tokens 318 to 187 with four; 8 heads 172 to 105; 130 tokens 80 to 51 and 300 of 8 heads 70 to 46 with two. Which one runs changes no
+  // bit of a column's sums.
+  constexpr int kSms = 148;
+  const int rpt = D <= 256 ? 8 : 16;
+  const int nc = chunks && D <= 128 && (long long)n_segments * heads * ((V + 63) / 64) >= 2 * kSms ? 4 : 2, kCols = D <= 256 ? 16 * nc : 16;
   IB_CHECK_ARG(heads <= 65535 && (V + kCols - 1) / kCols <= 65535, "recurrence: the grid is too large");
   int DS = 1;
   while (DS * rpt < D) DS *= 2;
@@ -659,14 +693,15 @@ int launch_recurrence(const float* q_src, const float* f_src, const float* v_src
   const dim3 grid((unsigned)n_segments, (unsigned)heads, (unsigned)((V + kCols - 1) / kCols));
   auto go = [&](auto kernel) {
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    ib::launch(kernel, grid, kCols / 2 * DS, smem, stream, q_src, f_src, v_src, P, (size_t)stride_p, R, f_bias, lower, state, (size_t)slot_stride, seg_start, seg_slot, o_out,
+    ib::launch(kernel, grid, kCols / nc * DS, smem, stream, q_src, f_src, v_src, P, (size_t)stride_p, R, f_bias, lower, state, (size_t)slot_stride, seg_start, seg_slot, o_out,
                heads, D, V, DS, seg_list, chunks, chunk_state, chunk_decay, qa, form, ex);
   };
   auto pick = [&](auto fixed, auto bonus) {
     constexpr bool F = decltype(fixed)::value, B = decltype(bonus)::value;
-    if (rpt == 8 && DS <= 16) go(gated_recurrence_kernel<8, 32, F, B, 256>);
-    else if (rpt == 8) go(gated_recurrence_kernel<8, 32, F, B, 512>);
-    else go(gated_recurrence_kernel<16, 16, F, B, 256>);
+    if (nc == 4) go(gated_recurrence_kernel<8, 64, 4, F, B, 256>);
+    else if (rpt == 8 && DS <= 16) go(gated_recurrence_kernel<8, 32, 2, F, B, 256>);
+    else if (rpt == 8) go(gated_recurrence_kernel<8, 32, 2, F, B, 512>);
+    else go(gated_recurrence_kernel<16, 16, 2, F, B, 256>);
   };
   if (form == 3) pick(std::false_type(), std::true_type());
   else if (form == 4) pick(std::true_type(), std::true_type());
