@@ -55,6 +55,43 @@ __global__ void embed_kernel(const W* __restrict__ table, const int* __restrict_
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H; i += gridDim.x * blockDim.x) dst[i] = ib::to_f32<W>(src[i]);
 }
 
+// The same with 16-byte accesses (rows of a multiple of 16 bytes): a CTA per token, four chunks requested a thread before the first is used. With one
+// value a thread and 256 a CTA the launch of the CTAs was the bound: 2,048 tokens of 4,096 48 us, now 26; 4,152 tokens 86 us, now 39; 64 tokens 17 us, now 12.
+template <typename W>
+__global__ void __launch_bounds__(128) embed_vec_kernel(const W* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ x, int H, int V,
+                                                        unsigned* __restrict__ status) {
+  constexpr int PER = 16 / sizeof(W), U = 4;
+  ib::pdl_launch_dependents();
+  ib::pdl_wait();
+  const int t = blockIdx.x, chunks = H / PER;
+  int tok = tokens[t];
+  if (tok < 0 || tok >= V) {
+    if (threadIdx.x == 0) atomicOr(status, IB_ERR_BAD_TOKEN);
+    tok = 0;
+  }
+  const uint4* src = (const uint4*)(table + (size_t)tok * H);
+  float4* dst = (float4*)(x + (size_t)t * H);
+  for (int c0 = threadIdx.x; c0 < chunks; c0 += U * 128) {
+    uint4 v[U];
+#pragma unroll
+    for (int u = 0; u < U; u++)
+      if (c0 + u * 128 < chunks) v[u] = src[c0 + u * 128];
+#pragma unroll
+    for (int u = 0; u < U; u++) {
+      const int c = c0 + u * 128;
+      if (c >= chunks) continue;
+      if constexpr (sizeof(W) == 4) {
+        dst[c] = make_float4(__uint_as_float(v[u].x), __uint_as_float(v[u].y), __uint_as_float(v[u].z), __uint_as_float(v[u].w));
+      } else {
+        auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
+        auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
+        dst[2 * c] = make_float4(lo(v[u].x), hi(v[u].x), lo(v[u].y), hi(v[u].y));
+        dst[2 * c + 1] = make_float4(lo(v[u].z), hi(v[u].z), lo(v[u].w), hi(v[u].w));
+      }
+    }
+  }
+}
+
 // x[t] = table[token] * scale + pos_table[position]: an embedding with a constant on the token's vector and a learned vector per position
 // (not scaled). A position outside the table counts as a bad token (its vector is left out).
 template <typename W>
@@ -403,7 +440,12 @@ extern "C" int ib_embed(const void* table, int table_dtype, const int* tokens, f
   IB_CHECK_ARG(T > 0 && H > 0 && V > 0, "embed: bad sizes T=%d H=%d V=%d", T, H, V);
   IB_CHECK_ARG(T <= 65535, "embed: T=%d rows exceed the grid limit 65535", T);
   dim3 grid((H + 255) / 256, T);
-  if (table_dtype == IB_F32)
+  const bool vec = (uintptr_t)table % 16 == 0 && (uintptr_t)x % 16 == 0 && H % (table_dtype == IB_F32 ? 4 : 8) == 0;
+  if (vec && table_dtype == IB_F32)
+    ib::launch(embed_vec_kernel<float>, T, 128, 0, stream, (const float*)table, tokens, x, H, V, status);
+  else if (vec && table_dtype == IB_BF16)
+    ib::launch(embed_vec_kernel<__nv_bfloat16>, T, 128, 0, stream, (const __nv_bfloat16*)table, tokens, x, H, V, status);
+  else if (table_dtype == IB_F32)
     ib::launch(embed_kernel<float>, grid, 256, 0, stream, (const float*)table, tokens, x, H, V, status);
   else if (table_dtype == IB_BF16)
     ib::launch(embed_kernel<__nv_bfloat16>, grid, 256, 0, stream, (const __nv_bfloat16*)table, tokens, x, H, V, status);
