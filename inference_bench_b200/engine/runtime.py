@@ -51,6 +51,7 @@ class Runtime:
         self.act_dtype = MODES[self.mode]
         self.gemm = self.options.gemm  # "auto" | "simt" | "tcgen05"
         self._side: Optional[torch.cuda.Stream] = None
+        self.held: Optional[list] = None   # while a layer's calls are noted (parts/repeat.py): the buffers it asks for
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.activate()
 
@@ -81,7 +82,10 @@ class Runtime:
 
     # ---------------------------------------------------------------- memory
     def empty(self, shape, dtype=None) -> torch.Tensor:
-        return torch.empty(shape, dtype=dtype or self.act_dtype, device=self.device)
+        t = torch.empty(shape, dtype=dtype or self.act_dtype, device=self.device)
+        if self.held is not None:
+            self.held.append(t)
+        return t
 
     def upload(self, t: torch.Tensor, dtype=None) -> torch.Tensor:
         t = t.to(self.device, non_blocking=False)

@@ -73,6 +73,10 @@ def kv_tensor_map(pool: torch.Tensor):
     return _KV_MAPS[key]
 
 
+class PoolRow(int):
+    """A row of a pool's tensor map: tells such an argument from any other whole number."""
+
+
 @dataclass
 class KvLayerView:
     """One layer's keys and values inside a paged pool, plus the block table of the step."""
@@ -84,7 +88,7 @@ class KvLayerView:
         """(address of the pool's tensor map or None, pool row where this view's keys of page 0, head 0 start)."""
         m = kv_tensor_map(self.pool)
         _, pages, _, kv_heads, page_size, _ = self.pool.shape
-        return (m[1] if m else None), self.entry * pages * 2 * kv_heads * page_size
+        return (m[1] if m else None), PoolRow(self.entry * pages * 2 * kv_heads * page_size)
 
     def c_view(self) -> L.KvView:
         cv = self.__dict__.get("_cv")   # made once per view: a layer asks for it several times a step

@@ -218,6 +218,10 @@ class Block:
         """What an execution of this block asks of the cache manager: its mixer's need, unless the arrangement has state of its own."""
         return self.mixer.cache_need()
 
+    def repeat_key(self, cache) -> Optional[tuple]:
+        """None, or what must be equal for a layer to repeat this one's kernel calls with its own weights and cache entry (parts/repeat.py)."""
+        return None
+
     def forward(self, ctx: "StepContext", x: torch.Tensor, pending: Optional[torch.Tensor], cache) -> Optional[torch.Tensor]:
         """Runs the block on x (in place). `pending` is a contribution not yet added to x; the
         return value is the block's own last contribution, left for the next norm to add."""

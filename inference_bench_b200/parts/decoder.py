@@ -9,8 +9,10 @@ from typing import Optional
 
 import torch
 
+from ..kernels import lib as L
 from . import base
 from .plan import ModelPlan, PartSpec
+from .repeat import Repeat
 
 
 def _build(table: dict, what: str, spec: PartSpec):
@@ -93,6 +95,19 @@ class Decoder:
                 out = out + pending[p].index_select(0, rows)
         return out
 
+    @staticmethod
+    def _noted(ctx, block, x, pending, cache, key):
+        """Run a layer and note its calls: (what it leaves for the next norm, the note or None where it cannot be repeated)."""
+        block.mixer.position.tables(ctx)   # (made once a step: not among the calls)
+        rep = Repeat(key, block, cache, pending)
+        rep.calls, ctx.rt.held = [], rep.held
+        L.notes.calls = rep.calls
+        try:
+            pending = block.forward(ctx, x, pending, cache)
+        finally:
+            L.notes.calls, ctx.rt.held = None, None
+        return pending, rep if rep.close(pending) else None
+
     def forward(self, ctx) -> Optional[torch.Tensor]:
         """Runs the step's tokens through the schedule; returns float32 logits [K, V] at the wanted
         rows, or None when no row is wanted (the caches are still filled)."""
@@ -109,12 +124,24 @@ class Decoder:
         trace = ctx.trace
         if trace is not None:
             trace.append(self._residual_rows(ctx, x, None))
+        # layers that repeat the calls of the one before (a captured step costs the host nothing, and a traced one looks between layers)
+        repeats = not ctx.fixed_shape and trace is None and not nvtx and len(self.plan.schedule) > 2
+        rep: Optional[Repeat] = None
         for i, e in enumerate(self.plan.schedule):
             if nvtx:
                 nvtx.range_push(f"entry {i} layer {e.layer}")
             if e.enter is not None:
                 pending = self.stream_parts[e.enter[0]].forward(ctx, x, pending, x0, e.enter[1])
-            pending = self.blocks[e.layer].forward(ctx, x, pending, ctx.caches[i] if ctx.caches else None)
+            block, cache = self.blocks[e.layer], ctx.caches[i] if ctx.caches else None
+            key = block.repeat_key(cache) if repeats and e.enter is None else None
+            if rep is not None and key is not None and key == rep.key:
+                pending = rep.run(block, cache)
+                continue
+            rep = None
+            if key is None:
+                pending = block.forward(ctx, x, pending, cache)
+            else:
+                pending, rep = self._noted(ctx, block, x, pending, cache, key)
             if nvtx:
                 nvtx.range_pop()
             if trace is not None:

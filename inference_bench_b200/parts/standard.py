@@ -480,6 +480,25 @@ class PreNormBlock(base.Block):
         if getattr(mixer, "bias", False):
             raise ValueError("this arrangement does not add a mixer's output bias")
 
+    def repeat_key(self, cache):
+        """What decides which kernels this layer runs and with which sizes, weights and cache entry apart (see parts/repeat.py): layers with equal keys
+        may repeat one another's calls. None for a layer that is not made of the parts this is known for."""
+        m, f, n1, n2 = self.mixer, self.feed_forward, self.mixer_norm, self.feed_forward_norm
+        if (type(self) is not PreNormBlock or type(m) is not Attention or type(f) is not SwiGLU or type(n1) is not RMSNorm or type(n2) is not RMSNorm
+                or not (m.plain and m.own_kv) or f.clamp is not None or self.residual_mult != 1.0 or type(cache) is not ops.KvLayerView
+                or type(m.position) not in (RotaryEmbedding, NoPositionEncoding)):
+            return None
+        p = m.position
+        turn = (p.rotary_dim, p.theta, p.scaling, p.yarn) if type(p) is RotaryEmbedding else ()
+        return (m.hidden, m.heads, m.kv_heads, m.head_dim, m.window, m.scale, m.norm_eps, m.q_norm is None, m.k_norm is None, turn, f.hidden, f.intermediate, n1.eps, n2.eps,
+                cache.pool.data_ptr(), tuple(cache.pool.shape), cache.block_table.data_ptr(), tuple(cache.block_table.shape))
+
+    def repeat_weights(self) -> list:
+        """The addresses of the layer's weights, in one order for all layers of a key."""
+        m, f = self.mixer, self.feed_forward
+        tensors = [self.mixer_norm.w, m.wqkv.weight, m.wo.weight, self.feed_forward_norm.w, f.wgu.weight, f.wd.weight, m.q_norm, m.k_norm]
+        return [t.data_ptr() for t in tensors if t is not None]
+
     def forward(self, ctx, x, pending, cache):
         plain = self.residual_mult == 1.0
         if self.mixer.runs_norm:
