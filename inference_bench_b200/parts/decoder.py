@@ -24,6 +24,12 @@ def _build(table: dict, what: str, spec: PartSpec):
     return base.make(table, what, spec.kind, **params)
 
 
+# Up to here the layers of a step outside a graph repeat one another's calls (parts/repeat.py): the kernels of more tokens take longer than their
+# launches anyway, and the repeated layer's buffers, all held at once, would be large (contexts of 64 requests run in portions of 8,192 tokens through
+# three layers of the 8B sizes: 142 ms, 448 with the buffers held).
+REPEAT_MAX_TOKENS = 1024
+
+
 class Decoder:
     def __init__(self, plan: ModelPlan):
         plan.validate()
@@ -125,7 +131,7 @@ class Decoder:
         if trace is not None:
             trace.append(self._residual_rows(ctx, x, None))
         # layers that repeat the calls of the one before (a captured step costs the host nothing, and a traced one looks between layers)
-        repeats = not ctx.fixed_shape and trace is None and not nvtx and len(self.plan.schedule) > 2
+        repeats = ctx.n_tokens <= REPEAT_MAX_TOKENS and not ctx.fixed_shape and trace is None and not nvtx and len(self.plan.schedule) > 2
         rep: Optional[Repeat] = None
         for i, e in enumerate(self.plan.schedule):
             if nvtx:
