@@ -60,7 +60,7 @@ class _Request:
 
     @property
     def length(self) -> int:                          # positions whose state is in the cache
-        return int(self._mgr._lib.ibh_cache_length(self._mgr._core, self.slot))
+        return self._mgr._lengths[self.slot]
 
     @property
     def tables(self) -> list[np.ndarray]:             # per group: page id per page index, -1 = none (views of the core's memory)
@@ -136,6 +136,7 @@ class CacheManager:
         base = self._lib.ibh_cache_tables(self._core)
         whole = np.ctypeslib.as_array(base, shape=(max(1, len(self.groups)), max_requests, self.table_width)) if self.groups else np.zeros((0, max_requests, self.table_width), np.int32)
         self._tables = [whole[gi] for gi in range(len(self.groups))]     # per group: int32 [max_requests, table_width], the core's own memory
+        self._lengths = self._lib.ibh_cache_lengths(self._core)          # per slot, the core's own memory
         if device is not None:
             import torch
             for g in self.groups:
@@ -225,7 +226,9 @@ class CacheManager:
     def extend(self, req: Hashable, new_length: int) -> None:
         """Allocate, in every group, the pages for positions up to new_length - 1. All or nothing."""
         r = self._get(req)
-        code = self._lib.ibh_cache_extend(self._core, r.slot, int(new_length))
+        self._extended(self._lib.ibh_cache_extend(self._core, r.slot, int(new_length)), req, new_length)
+
+    def _extended(self, code: int, req: Hashable, new_length: int) -> None:
         if code == 1:
             raise OutOfPages(f"request {req!r} {native.last_error()}")
         if code == 2:
@@ -243,6 +246,26 @@ class CacheManager:
         if self._lib.ibh_cache_commit(self._core, self._get(req).slot, int(new_length)):
             raise CacheError(native.last_error())
 
+    def rows(self, reqs: Sequence[Hashable]):
+        """The slots of a step's requests, for `extend_rows`, `fill_rows` and `commit_rows`."""
+        try:
+            return (C.c_int * max(1, len(reqs)))(*[self._requests[r].slot for r in reqs])
+        except KeyError as e:
+            raise CacheError(f"request {e.args[0]!r} is not admitted") from None
+
+    def extend_rows(self, reqs: Sequence[Hashable], rows, by: int) -> None:
+        """`extend` for every request of a step in order, each to `by` positions more than it holds, in one call into the core. Raises where the first
+        one cannot be extended; those before it stay so."""
+        stopped = C.c_int()
+        code = self._lib.ibh_cache_extend_rows(self._core, rows, len(reqs), by, C.byref(stopped))
+        if code:
+            self._extended(code, reqs[stopped.value], self._lengths[rows[stopped.value]] + by)
+
+    def commit_rows(self, reqs: Sequence[Hashable], rows, by: int) -> None:
+        """`commit` for every request of a step, each `by` positions more than it held."""
+        if self._lib.ibh_cache_commit_rows(self._core, rows, len(reqs), by):
+            raise CacheError(native.last_error())
+
     def release(self, req: Hashable) -> None:
         """The request ends: all its pages and its slot are given back."""
         if self._lib.ibh_cache_release(self._core, self._get(req).slot):
@@ -258,17 +281,16 @@ class CacheManager:
     def free_pages(self) -> list[int]:
         return [g.pool.free_pages for g in self.groups]
 
-    def fill_rows(self, reqs: Sequence[Hashable], positions: np.ndarray, tables: Sequence[np.ndarray]) -> list[int]:
+    def fill_rows(self, reqs: Sequence[Hashable], positions: np.ndarray, tables: Sequence[np.ndarray], rows=None) -> list[int]:
         """For a step of single decoded tokens: write the requests' committed lengths (their next positions)
         into positions[:n] and their block tables into tables[g][:n] (int32, contiguous; typically the pinned
         input block of a captured step), in one call into the core. Returns the requests' slots."""
         n = len(reqs)
-        slots = [self._get(r).slot for r in reqs]
-        arr = (C.c_int * max(1, n))(*slots)
+        arr = self.rows(reqs) if rows is None else rows
         ptrs = (C.POINTER(C.c_int) * max(1, len(tables)))(*[t.ctypes.data_as(C.POINTER(C.c_int)) for t in tables])
         if self._lib.ibh_cache_fill_rows(self._core, arr, n, positions.ctypes.data_as(C.POINTER(C.c_int)), ptrs):
             raise CacheError(native.last_error())
-        return slots
+        return arr[:n]
 
     # ------------------------------------------------------------------ what a step hands to the parts
     def step_tables(self, reqs: Sequence[Hashable]) -> list[np.ndarray]:

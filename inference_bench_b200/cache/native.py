@@ -17,7 +17,8 @@ _SIGNATURES = {
     "ibh_cache_admit": (_i, [_p]), "ibh_cache_length": (_i, [_p, _i]), "ibh_cache_pages_missing": (None, [_p, _i, _i, _i, C.POINTER(_i)]),
     "ibh_cache_extend": (_i, [_p, _i, _i]), "ibh_cache_shrink_to_committed": (_i, [_p, _i]), "ibh_cache_commit": (_i, [_p, _i, _i]),
     "ibh_cache_release": (_i, [_p, _i]), "ibh_cache_fill_rows": (_i, [_p, C.POINTER(_i), _i, C.POINTER(_i), C.POINTER(C.POINTER(_i))]),
-    "ibh_cache_check": (_i, [_p]),
+    "ibh_cache_check": (_i, [_p]), "ibh_cache_lengths": (C.POINTER(_i), [_p]),
+    "ibh_cache_extend_rows": (_i, [_p, C.POINTER(_i), _i, _i, C.POINTER(_i)]), "ibh_cache_commit_rows": (_i, [_p, C.POINTER(_i), _i, _i]),
     "ibh_sched_new": (_p, [_p, _i, _i, _i, _i, _i]), "ibh_sched_free": (None, [_p]), "ibh_sched_submit": (_i, [_p, _i, _i]),
     "ibh_sched_cancel": (_i, [_p, _i]), "ibh_sched_n_waiting": (_i, [_p]), "ibh_sched_n_running": (_i, [_p]), "ibh_sched_steady": (_i, [_p]),
     "ibh_sched_waiting": (None, [_p, C.POINTER(_i)]), "ibh_sched_running": (None, [_p, C.POINTER(_i)]),

@@ -137,6 +137,7 @@ void* ibh_cache_new(int n_groups, const int* windows, const int* keeps, int page
 void ibh_cache_free(void* c) { delete (Cache*)c; }
 void* ibh_cache_pool(void* c, int g) { return &((Cache*)c)->pools[g]; }
 int* ibh_cache_tables(void* c) { return ((Cache*)c)->tables.data(); }
+int* ibh_cache_lengths(void* c) { return ((Cache*)c)->length.data(); }   // per slot; 0 for one that holds no request
 int ibh_cache_table_width(void* c) { return ((Cache*)c)->table_width; }
 int ibh_cache_free_slots(void* c) { return (int)((Cache*)c)->free_slots.size(); }
 
@@ -204,6 +205,18 @@ int ibh_cache_extend(void* cp, int slot, int new_length) {
   return 0;
 }
 
+// The slots of a step's rows, in order, each `by` positions longer than committed; stops at the first that cannot be, whose number goes to *stopped
+// (those before it stay extended). Returns what ibh_cache_extend returned last.
+int ibh_cache_extend_rows(void* cp, const int* slots, int n, int by, int* stopped) {
+  Cache* c = (Cache*)cp;
+  for (int i = 0; i < n; i++) {
+    *stopped = i;
+    if (!c->is_live(slots[i])) return fail(3, "slot %d holds no request", slots[i]);
+    if (int e = ibh_cache_extend(cp, slots[i], c->length[slots[i]] + by)) return e;
+  }
+  return 0;
+}
+
 // Undo an extend that no commit followed: free the pages beyond the committed length.
 int ibh_cache_shrink_to_committed(void* cp, int slot) {
   Cache* c = (Cache*)cp;
@@ -234,6 +247,16 @@ int ibh_cache_commit(void* cp, int slot, int new_length) {
         c->pools[g].release(row[p]);
         row[p] = -1;
       }
+  }
+  return 0;
+}
+
+// The same for a step's rows, each `by` positions longer than before (shorter: by < 0).
+int ibh_cache_commit_rows(void* cp, const int* slots, int n, int by) {
+  Cache* c = (Cache*)cp;
+  for (int i = 0; i < n; i++) {
+    if (!c->is_live(slots[i])) return fail(3, "slot %d holds no request", slots[i]);
+    ibh_cache_commit(cp, slots[i], c->length[slots[i]] + by);
   }
   return 0;
 }

@@ -106,7 +106,8 @@ class _DecodeGraph:
         Returns the tokens of every step, [steps][rows]."""
         if not 1 <= steps <= RUN_AHEAD_MAX:
             raise ValueError(f"run_ahead takes 1 to {RUN_AHEAD_MAX} steps, got {steps}")
-        self._fill(entries, sampling)
+        reqs = [e.request for e in entries]
+        self._fill(entries, sampling, reqs, self.runner.cache.rows(reqs))
         self.dev.copy_(self.host, non_blocking=True)
         for _ in range(steps):
             self.graph.replay()
@@ -116,9 +117,10 @@ class _DecodeGraph:
         self.runner.rt.raise_for(int(self.h_out[self.rows]))
         return self.h_history[:steps, :len(entries)].tolist()
 
-    def run(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]]) -> list[int]:
+    def run(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], reqs: list, rows) -> list[int]:
+        """reqs, rows: the entries' requests and their slots (`CacheManager.rows`)."""
         n = len(entries)
-        self._fill(entries, sampling)
+        self._fill(entries, sampling, reqs, rows)
         self.dev.copy_(self.host, non_blocking=True)
         self.graph.replay()
         self.h_out.copy_(self.result, non_blocking=True)
@@ -126,14 +128,14 @@ class _DecodeGraph:
         self.runner.rt.raise_for(int(self.h_out[self.rows]))
         return self.h_out[:n].tolist()
 
-    def launch(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], feed: bool) -> tuple[int, int]:
+    def launch(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], feed: bool, reqs: list, rows) -> tuple[int, int]:
         """Enqueue one step and return at once. With `feed` the input tokens stay what the step before
         left on the device (its sampled tokens, row by row): everything but the tokens is copied."""
         slot = self.turn
         if self.pending[slot]:
             raise RuntimeError("two decode steps are already in flight")
         self.turn ^= 1
-        self._fill(entries, sampling, tokens=not feed)
+        self._fill(entries, sampling, reqs, rows, tokens=not feed)
         stage = self.stages[slot]
         stage.copy_(self.host)
         if feed:
@@ -153,17 +155,22 @@ class _DecodeGraph:
         self.runner.rt.raise_for(int(self.h_outs[slot][self.rows]))
         return self.h_outs[slot][:n].tolist()
 
-    def _fill(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], tokens: bool = True) -> None:
+    def _fill(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], reqs: list, rows, tokens: bool = True) -> None:
         cache = self.runner.cache
         n = len(entries)
         if n < self.rows:
             self._pad_all()
-        slots = cache.fill_rows([e.request for e in entries], self.h_pos, self.h_tables)   # positions and block tables, straight into the pinned block
+        slots = cache.fill_rows(reqs, self.h_pos, self.h_tables, rows)   # positions and block tables, straight into the pinned block
         if tokens:
             self.h_tokens[:n] = [e.tokens[0] for e in entries]
         self.h_pos0[:n] = self.h_pos[:n]
         self.h_slot[:n] = slots
-        self.h_params[:n] = [p.row(step) for p, step in sampling]
+        params, last = [], (None, None, None)
+        for p, step in sampling:   # (requests that were started together share a row)
+            if p is not last[0] or step != last[1]:
+                last = (p, step, p.row(step))
+            params.append(last[2])
+        self.h_params[:n] = params
 
 
 class GpuExecutor:
@@ -191,11 +198,11 @@ class GpuExecutor:
         """Several decode steps of the same requests in a row, tokens fed back on the device."""
         cache = self.runner.cache
         g = self.graph_for(len(entries))
-        for e in entries:
-            cache.extend(e.request, cache.length(e.request) + steps)
+        reqs = [e.request for e in entries]
+        rows = cache.rows(reqs)
+        cache.extend_rows(reqs, rows, steps)
         out = g.run_ahead(entries, sampling, steps)
-        for e in entries:
-            cache.commit(e.request, cache.length(e.request) + steps)
+        cache.commit_rows(reqs, rows, steps)
         self.steps += steps
         self.h2d_bytes += g.n_ints * 4
         self.d2h_bytes += steps * g.rows * 4 + 4
@@ -213,16 +220,16 @@ class GpuExecutor:
                 if not 0 <= e.tokens[0] < self.runner.vocab:
                     raise ValueError(f"request {e.request!r}: token id {e.tokens[0]} is outside the vocabulary of {self.runner.vocab}")
         g = self.graph_for(len(entries))
+        reqs = [e.request for e in entries]
+        rows = cache.rows(reqs)
         try:
-            for e in entries:
-                cache.extend(e.request, cache.length(e.request) + 1)
+            cache.extend_rows(reqs, rows, 1)
         except Exception:
-            for e in entries:
-                cache.shrink_to_committed(e.request)
+            for req in reqs:
+                cache.shrink_to_committed(req)
             raise
-        handle = g.launch(entries, sampling, feed)
-        for e in entries:
-            cache.commit(e.request, cache.length(e.request) + 1)
+        handle = g.launch(entries, sampling, feed, reqs, rows)
+        cache.commit_rows(reqs, rows, 1)
         self.steps += 1
         self.h2d_bytes += (g.n_ints - (g.rows if feed else 0)) * 4
         self.d2h_bytes += g.rows * 4 + 4
@@ -235,16 +242,17 @@ class GpuExecutor:
     def execute(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]]) -> list[int]:
         self.steps += 1
         cache = self.runner.cache
-        if self.use_graphs and all(len(e.tokens) == 1 and list(e.want) == [0] for e in entries) and len(entries) <= self.max_graph_rows:
+        if self.use_graphs and len(entries) <= self.max_graph_rows and all(len(e.tokens) == 1 and len(e.want) == 1 and e.want[0] == 0 for e in entries):
             g = self.graph_for(len(entries))
+            vocab = self.runner.vocab
             for e in entries:
-                tok = e.tokens[0]
-                if not 0 <= tok < self.runner.vocab:
-                    raise ValueError(f"request {e.request!r}: token id {tok} is outside the vocabulary of {self.runner.vocab}")
-                cache.extend(e.request, cache.length(e.request) + 1)
-            out = g.run(entries, sampling)
-            for e in entries:
-                cache.commit(e.request, cache.length(e.request) + 1)
+                if not 0 <= e.tokens[0] < vocab:
+                    raise ValueError(f"request {e.request!r}: token id {e.tokens[0]} is outside the vocabulary of {vocab}")
+            reqs = [e.request for e in entries]
+            rows = cache.rows(reqs)     # a step's bookkeeping is one call into the core each, not one a request
+            cache.extend_rows(reqs, rows, 1)
+            out = g.run(entries, sampling, reqs, rows)
+            cache.commit_rows(reqs, rows, 1)
             self.last_logits = g.logits
             self.h2d_bytes += g.n_ints * 4
             self.d2h_bytes += g.rows * 4 + 4
