@@ -36,13 +36,16 @@ constexpr int EPI_XIELU = 4;   // bfloat16 xielu(product) with the activation's 
 constexpr int kQkvHead = 128;   // head size of the EPI_QKV form: a head is 128 accumulator columns
 constexpr uint32_t kPeerBitMask = 0xFEFFFFFFu;   // clears the bit that tells the two CTAs of a pair apart in a shared::cluster address
 
+constexpr int kMaxGroups = 256;   // matrices of one launch of the regrouped form (PairGroups)
+
 // BN: tokens per tile = accumulator columns (each CTA loads half of them)
 template <int MT, int BN>
 struct Tile {
   static constexpr int kABytes = BM * BK * 2, kBBytes = (BN / 2) * BK * 2;
   static constexpr int kStageBytes = MT * kABytes + kBBytes;
   static constexpr int kStages = (200 * 1024) / kStageBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /* alignment slack */ + 256 /* barriers */ + 1024 /* norm scales of EPI_QKV */;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /* alignment slack */ + 256 /* barriers */ + 1024 /* norm scales of EPI_QKV */ +
+                                    2 * (kMaxGroups + 1) * 4 /* the groups' table */;
   static constexpr int kAccSets = 512 / (MT * BN);   // accumulator sets that fit tensor memory
 };
 
@@ -94,6 +97,17 @@ __device__ __forceinline__ void arrive_on_leader(uint64_t* bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(sm100::smem_u32(bar) & kPeerBitMask) : "memory");
 }
 
+// Regrouped rows (routed experts): rows offsets[e] .. offsets[e + 1] of x go through matrix e, rows e * w_rows .. of w. tiles[e] is the first token tile of
+// group e and tiles[n] their number; a tile never crosses a group's end (rows past it are multiplied and not stored). n = 0: one matrix for all.
+// The table is read into shared memory once, after the wait for the kernels before; a tile's group is a search in it. Bound by the tensor cores' operand
+// traffic at many rows a group and by the matrices' bytes at few: 12,288 rows of 64 groups, 2,816 x 2,048 each, 240 us on single CTAs, 202 here, the
+// 2,048 x 1,408 product behind it 169 and 109; 49,152 rows 696 and 501, 541 and 277 (1.1 PFLOP/s).
+struct PairGroups {
+  const int* offsets;
+  const int* tiles;
+  int n, w_rows;
+};
+
 // What the EPI_QKV epilogue works with. The product is taken the other way round there: the tokens are the
 // rows of the MMA (tensor-memory lanes: a thread of the epilogue owns a token) and the rows of the fused
 // [q | k | v] weight are its columns, so that a head's 128 values of a token sit in one thread: the norm is a
@@ -124,7 +138,7 @@ struct QkvEpi {
 template <int MT, int EPI, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
     gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, void* __restrict__ out_, int T, int N,
-                     int K, int token_tiles, int total_tiles, int second_off, unsigned long long wait_ns, unsigned* __restrict__ status, const QkvEpi qe) {
+                     int K, int token_tiles, int total_tiles, int second_off, unsigned long long wait_ns, unsigned* __restrict__ status, const QkvEpi qe, const PairGroups grp) {
   using TL = Tile<MT, BN>;
   constexpr int STAGES = TL::kStages;
   constexpr int BNH = BN / 2;
@@ -145,7 +159,13 @@ __global__ void __launch_bounds__(kThreads, 1)
   const int nkt = (K + BK - 1) / BK;
   constexpr int kColsPerPair = epi_gated(EPI) ? 2 * BM : 2 * BM * MT;
 
+  int* g_off = (int*)(tiles + STAGES * TL::kStageBytes + 256 + 1024);   // [kMaxGroups + 1]
+  int* g_tile = g_off + kMaxGroups + 1;
   ib::pdl_launch_dependents();
+  if (grp.n) {   // the table is the work of the kernels before
+    ib::pdl_wait();
+    for (int i = threadIdx.x; i <= grp.n; i += kThreads) g_off[i] = grp.offsets[i], g_tile[i] = grp.tiles[i];
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; s++) {
       sm100::mbar_init(&full[s], 1);
@@ -173,6 +193,28 @@ __global__ void __launch_bounds__(kThreads, 1)
   sm100::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
+  if (grp.n) {
+    token_tiles = g_tile[grp.n];
+    total_tiles = token_tiles * ((N + kColsPerPair - 1) / kColsPerPair);
+  }
+  // a tile: its block of rows of W, its first token, one past its last, its group and where the group's matrix begins
+  struct Place {
+    int rb, t0, t_end, group, w0;
+  };
+  auto place = [&](int tile) {
+    const int b = tile % token_tiles;
+    Place p{tile / token_tiles, b * BN, T, 0, 0};
+    if (grp.n) {
+      int lo = 0, hi = grp.n;   // the last group whose first tile is at or before b
+      while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (g_tile[mid] <= b) lo = mid;
+        else hi = mid;
+      }
+      p.t0 = g_off[lo] + (b - g_tile[lo]) * BN, p.t_end = g_off[lo + 1], p.group = lo, p.w0 = lo * grp.w_rows;
+    }
+    return p;
+  };
   // W rows of accumulator m of this CTA for the pair's row block rb: plain tiles stack 256-row pairs;
   // SwiGLU takes gate rows and, second_off on, up rows
   auto w_row = [&](int rb, int m) {
@@ -187,7 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       bool waited = false, ok = true;
       int it = 0;   // k-tiles sent so far, over all tiles: stage = it % STAGES
       for (int tile = pair; tile < total_tiles && ok; tile += n_pairs) {
-        const int t0 = (tile % token_tiles) * BN, rb = tile / token_tiles;
+        const Place at = place(tile);
         for (int i = 0; i < nkt; i++, it++) {
           const int s = it % STAGES;
           if (!sm100::mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, wait_ns)) {
@@ -202,12 +244,12 @@ __global__ void __launch_bounds__(kThreads, 1)
             waited = true;
           }
 #pragma unroll
-          for (int m = 0; m < MT; m++) tma_load_2d_pair(a + m * TL::kABytes, &tmap_w, i * BK, w_row(rb, m), &full[s]);
+          for (int m = 0; m < MT; m++) tma_load_2d_pair(a + m * TL::kABytes, &tmap_w, i * BK, at.w0 + w_row(at.rb, m), &full[s]);
           if (!waited) {   // the weights above do not depend on earlier kernels; x does
             ib::pdl_wait();
             waited = true;
           }
-          tma_load_2d_pair(a + MT * TL::kABytes, &tmap_x, i * BK, t0 + (int)rank * BNH, &full[s]);
+          tma_load_2d_pair(a + MT * TL::kABytes, &tmap_x, i * BK, at.t0 + (int)rank * BNH, &full[s]);
         }
       }
     }
@@ -252,7 +294,8 @@ __global__ void __launch_bounds__(kThreads, 1)
     int tl = 0;
     for (int tile = pair; tile < total_tiles; tile += n_pairs, tl++) {
       const int b = tl % NBUF;
-      const int t0 = (tile % token_tiles) * BN, n_pair = (tile / token_tiles) * kColsPerPair;
+      const Place at = place(tile);
+      const int t0 = at.t0, n_pair = at.rb * kColsPerPair, t_end = at.t_end;
       bool ok = sm100::mbar_wait(&acc_full[b], (tl / NBUF) & 1, wait_ns);
       if (!ok && lane == 0) atomicOr(status, IB_ERR_WAIT_TIMEOUT);
       sm100::tc_fence_after();
@@ -380,14 +423,14 @@ __global__ void __launch_bounds__(kThreads, 1)
               if constexpr (EPI == EPI_ADD) {   // every element belongs to one thread of one CTA: a plain read, add, write
                 float old[32];
 #pragma unroll
-                for (int c = 0; c < 32; c++) old[c] = t0 + c0 + c < T ? dst[(size_t)(t0 + c0 + c) * N + n] : 0.f;
+                for (int c = 0; c < 32; c++) old[c] = t0 + c0 + c < t_end ? dst[(size_t)(t0 + c0 + c) * N + n] : 0.f;
 #pragma unroll
                 for (int c = 0; c < 32; c++) r[c] = __float_as_uint(old[c] + __uint_as_float(r[c]));
               }
 #pragma unroll
               for (int c = 0; c < 32; c++) {
                 const int t = t0 + c0 + c;
-                if (t < T) {
+                if (t < t_end) {
                   if constexpr (EPI == EPI_XIELU)
                     dst_act[(size_t)t * N + n] = __float2bfloat16_rn(ib::xielu(__uint_as_float(r[c]), ap, an));
                   else if constexpr (EPI == EPI_RELU2)
@@ -401,7 +444,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       } else {
         __nv_bfloat16* dst = (__nv_bfloat16*)out_;
-        const float limit = EPI == EPI_CLAMPED ? qe.act_pq[0] : 0.f;
+        const float limit = EPI == EPI_CLAMPED ? qe.act_pq[at.group] : 0.f;
         const int n = n_pair + (int)rank * BM + q * 32 + lane;
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -414,7 +457,7 @@ __global__ void __launch_bounds__(kThreads, 1)
             for (int c = 0; c < 32; c++) {
               const int t = t0 + c0 + c;
               const float gv = __uint_as_float(g[c]), uv = __uint_as_float(u[c]);
-              if (t >= T) continue;
+              if (t >= t_end) continue;
               if constexpr (EPI == EPI_CLAMPED) dst[(size_t)t * N + n] = __float2bfloat16_rn(ib::clamped_glu<true>(gv, uv, limit, qe.act_slope));
               else dst[(size_t)t * N + n] = __float2bfloat16_rn(__fdividef(gv, 1.f + __expf(-gv)) * uv);
             }
@@ -451,7 +494,7 @@ int make_tmap(CUtensorMap* m, const void* ptr, int rows, int K, int box_rows) {
 
 template <int MT, int EPI, int BN>
 int launch(const void* x, const void* w, void* out, int T, int N, int K, int w_rows, int second_off, unsigned* status, cudaStream_t stream,
-           const QkvEpi& qe = QkvEpi{}) {
+           const QkvEpi& qe = QkvEpi{}, const PairGroups& grp = PairGroups{}) {
   using TL = Tile<MT, BN>;
   IB_CHECK_ARG(T > 0 && N > 0 && K > 0 && K % 8 == 0, "gemm_tcgen05_2cta: bad sizes T=%d N=%d K=%d (K must be a multiple of 8)", T, N, K);
   IB_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)w & 15) == 0, "gemm_tcgen05_2cta: operands must be 16-byte aligned");
@@ -465,7 +508,7 @@ int launch(const void* x, const void* w, void* out, int T, int N, int K, int w_r
   if (make_tmap(&tw, w, w_rows, K, BM)) return 1;
   if (make_tmap(&tx, x, T, K, BN / 2)) return 1;
   const int cols_per_pair = epi_gated(EPI) ? 2 * BM : 2 * BM * MT;
-  const int token_tiles = (T + BN - 1) / BN, row_blocks = (N + cols_per_pair - 1) / cols_per_pair;
+  const int token_tiles = grp.n ? T / BN + grp.n : (T + BN - 1) / BN, row_blocks = (N + cols_per_pair - 1) / cols_per_pair;
   const int total_tiles = token_tiles * row_blocks;
   static int sm_count = 0;
   if (!sm_count) {
@@ -488,7 +531,7 @@ int launch(const void* x, const void* w, void* out, int T, int N, int K, int w_r
   attr[1].val.programmaticStreamSerializationAllowed = ib_pdl_enabled();
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_2cta_kernel<MT, EPI, BN>, tw, tx, out, T, N, K, token_tiles, total_tiles, second_off, ib_wait_limit_ns(), status, qe);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_2cta_kernel<MT, EPI, BN>, tw, tx, out, T, N, K, token_tiles, total_tiles, second_off, ib_wait_limit_ns(), status, qe, grp);
   IB_CHECK_ARG(e == cudaSuccess, "gemm_tcgen05_2cta: launch failed: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -541,6 +584,31 @@ extern "C" int ib_gemm_swiglu_tcgen05_2cta(const void* x, const void* w, void* a
     return launch<2, EPI_CLAMPED, 128>(x, w, act, T, I, K, 2 * I, I, status, stream, qe);
   }
   return launch<2, EPI_SWIGLU, 128>(x, w, act, T, I, K, 2 * I, I, status, stream);
+}
+
+// The products of regrouped rows on CTA pairs, tiles of 128 rows (the table: ib_moe_sort with tile_rows = 128): x [R, K] bfloat16 and w [E, N or 2 I, K];
+// offsets, tiles [E + 1] (see PairGroups). Store: out [R, N] float32; act 2: [R, N] bfloat16 max(product, 0)^2.
+extern "C" int ib_gemm_grouped_2cta(const void* x, const void* w, void* out, int R, int N, int K, const int* offsets, const int* tiles, int E, int act, unsigned* status,
+                                    cudaStream_t stream) {
+  if (R == 0 || N == 0) return 0;
+  IB_CHECK_ARG(E > 0 && E <= kMaxGroups && offsets && tiles && (act == 0 || act == 2), "gemm_grouped_2cta: %d groups (up to %d) or activation %d", E, kMaxGroups, act);
+  IB_CHECK_ARG((long long)E * N < (1ll << 31), "gemm_grouped_2cta: %d matrices of %d rows", E, N);
+  const PairGroups grp{offsets, tiles, E, N};
+  if (act == 2) return launch<2, EPI_RELU2, 128>(x, w, out, R, N, K, E * N, BM * 2, status, stream, QkvEpi{}, grp);
+  return launch<2, EPI_STORE, 128>(x, w, out, R, N, K, E * N, BM * 2, status, stream, QkvEpi{}, grp);
+}
+
+// act [R, I] bfloat16 = silu(gate) * up per group, w [E, 2 I, K] = every group's gate rows then its up rows; limits: null, or float32 [E]: clamped halves.
+extern "C" int ib_gemm_grouped_swiglu_2cta(const void* x, const void* w, void* act, int R, int I, int K, const int* offsets, const int* tiles, int E, const float* limits,
+                                           float slope, unsigned* status, cudaStream_t stream) {
+  if (R == 0 || I == 0) return 0;
+  IB_CHECK_ARG(E > 0 && E <= kMaxGroups && offsets && tiles, "gemm_grouped_swiglu_2cta: %d groups (up to %d)", E, kMaxGroups);
+  IB_CHECK_ARG((long long)E * 2 * I < (1ll << 31), "gemm_grouped_swiglu_2cta: %d matrices of %d rows", E, 2 * I);
+  const PairGroups grp{offsets, tiles, E, 2 * I};
+  QkvEpi qe{};
+  qe.act_pq = limits, qe.act_slope = slope;
+  if (limits) return launch<2, EPI_CLAMPED, 128>(x, w, act, R, I, K, E * 2 * I, I, status, stream, qe, grp);
+  return launch<2, EPI_SWIGLU, 128>(x, w, act, R, I, K, E * 2 * I, I, status, stream, qe, grp);
 }
 
 // The q/k/v projection with its epilogue: x [T, K] bfloat16 and w [(heads + 2 kv_heads) * 128, K] bfloat16 (q rows, k rows, v rows)

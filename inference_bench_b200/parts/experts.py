@@ -137,6 +137,9 @@ class RoutedExperts(base.FeedForward):
         tcgen05 = how in ("auto", "tcgen05") and rt.act_dtype == torch.bfloat16 and rt.gemm != "simt" and G.grouped_supported(self.hidden, self.expert_ff, bn, self.gated)
         if how == "tcgen05" and not tcgen05:
             raise ValueError(f"expert_gemm = \"tcgen05\" needs bfloat16 and inner sizes that are multiples of 8 (of 64 for few tokens), got {self.hidden} and {self.expert_ff}")
+        pair = tcgen05 and G.grouped_pairs(R, n, self.expert_ff, rt.sm_count)
+        if pair:
+            bn = G.PAIR_TILE
         tile_rows = bn if tcgen05 else ops.moe_tile_rows()
         one = T <= ROUTE_SORT_TOKENS and ops.moe_route_sort_fits(T, E, self.groups, always)     # the choice and the regrouping in one kernel
         ops.moe_route(logits, self.groups, self.groups_keep, top, self.route_scale, self.renorm, idx, wt, self.score, correction=self.w_correction, group_top=self.group_top,
@@ -152,10 +155,10 @@ class RoutedExperts(base.FeedForward):
             else:
                 ops.gather_rows(h, token_of_row, xs)
             if self.gated:
-                G.gemm_grouped_swiglu(xs, w_gu, act, bn, offsets, tile_start, rt.status, clamp=self.limits)
+                G.gemm_grouped_swiglu(xs, w_gu, act, bn, offsets, tile_start, rt.status, clamp=self.limits, pair=pair)
             else:
-                G.gemm_grouped_relu2(xs, w_gu, act, bn, offsets, tile_start, rt.status)
-            G.gemm_grouped(act, w_d, y, bn, offsets, tile_start, rt.status)
+                G.gemm_grouped_relu2(xs, w_gu, act, bn, offsets, tile_start, rt.status, pair=pair)
+            G.gemm_grouped(act, w_d, y, bn, offsets, tile_start, rt.status, pair=pair)
         else:
             tc = how != "simt"
             src, rows = h, token_of_row
