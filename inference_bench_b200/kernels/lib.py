@@ -133,7 +133,11 @@ launches = 0   # kernels launched so far through `call`
 KERNELS_PER_CALL = {"ib_sample_rows": 3, "ib_attention_decode": 2, "ib_attention_decode_stream": 2, "ib_attention_decode_fused": 2}
 
 
-notes = threading.local()   # .calls: a list that every `call` of this thread is added to as (name, arguments), while somebody notes them
+class _Notes(threading.local):
+    calls = None   # a list that every `call` of this thread is added to as (name, arguments), while somebody notes them
+
+
+notes = _Notes()
 
 
 _entry: dict = {}   # name -> (function, kernels it launches)
@@ -145,7 +149,7 @@ def call(name: str, *args) -> None:
     if e is None:
         e = _entry[name] = (getattr(load(), name), KERNELS_PER_CALL.get(name, 1))
     launches += e[1]
-    noted = getattr(notes, "calls", None)
+    noted = notes.calls
     if noted is not None:
         noted.append((name, args))
     if e[0](*args) != 0:
