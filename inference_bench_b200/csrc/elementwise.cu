@@ -21,7 +21,7 @@ int ib_set_error(const char* fmt, ...) {
 }
 
 static int g_pdl = 1;
-static int g_pdl_skip = 0;
+static thread_local int g_pdl_skip = 0;   // the calling thread's own next launch: another thread's must not use it up
 extern "C" int ib_pdl_enabled() {
   if (g_pdl_skip) {
     g_pdl_skip = 0;
