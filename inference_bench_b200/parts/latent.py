@@ -225,4 +225,5 @@ class LatentAttention(base.Mixer):
         if plan is not None:   # and those that see keys and values per head (their rows of v hold nothing yet)
             kv, part = ops.latent_keys_values(cache, plan[0], ctx.seg_start, ctx.seg_pos0, self.w_kv, r, rot, rt.status, self.window)
             ops.latent_prefill(q_nope, q_full, r, plan[1], kv, part, self.scale, v, rt.status, window=self.window, sink=self.sink_dev, gate=gate)
+            rt.next_in_order(ctx)   # that kernel's CTAs hold an SM's tensor memory: no product may wait for it while the norm behind lets another one start
         return rt.linear(v.view(T, H * self.vdim), self.wo, add_to=residual)
