@@ -12,6 +12,8 @@ from __future__ import annotations
 import ctypes as C
 from typing import Optional
 
+import torch
+
 from ..kernels import lib as L
 from ..kernels import ops
 
@@ -27,10 +29,12 @@ class Repeat:
         self.plan: Optional[list] = None
 
     def close(self, pending) -> bool:
-        """The layer has run and left `pending`: whether it can be repeated."""
+        """The layer has run and left `pending`: whether it can be repeated. A contribution that is more than a tensor (behind a layer of another
+        arrangement, with a norm or a constant of its own) is not one the next layer gets."""
         self.pending = pending
         a, b = self.pending_in, pending
-        return (a is None) == (b is None) and (a is None or a.shape == b.shape) and len(set(self.weights)) == len(self.weights)
+        alike = a is b is None or isinstance(a, torch.Tensor) and isinstance(b, torch.Tensor) and a.shape == b.shape
+        return alike and len(set(self.weights)) == len(self.weights)
 
     def _places(self) -> list:
         """[(name, arguments, [(place, number of what stands there)])]: the weights by number, then the cache view, its first row, and the contribution."""

@@ -62,3 +62,20 @@ def test_a_shared_weight_is_not_repeated():
         r.cache.admit(0)
         outs.append(r.step([StepEntry(0, list(range(40)), [39])], trace=trace).clone())
     assert torch.equal(*outs)
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_layers_behind_one_of_another_arrangement(dtype):
+    """A layer that gets a contribution with a norm of its own is not repeated; those behind it are."""
+    from inference_bench_b200.engine.step import StepEntry
+    from inference_bench_b200.parts.standard import RMSNorm, SandwichBlock
+    outs = []
+    for trace in (None, []):
+        r = _runner(dtype, 64, (0, 0, 0, 0, 0), 16)
+        b, posts = r.decoder.blocks[0], [RMSNorm(f"post{i}", 256, 1e-6) for i in range(2)]
+        for i, n in enumerate(posts):
+            n.w = r.rt.vector(1 + 0.1 * torch.randn(256, generator=torch.Generator().manual_seed(i)))
+        r.decoder.blocks[0] = SandwichBlock(b.mixer_norm, b.mixer, b.feed_forward_norm, b.feed_forward, *posts)
+        r.cache.admit(0)
+        outs.append([r.step([StepEntry(0, list(range(n)), [n - 1])], trace=trace).clone() for n in (40, 1, 300)])
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
