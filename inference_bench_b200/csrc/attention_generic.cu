@@ -247,32 +247,35 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, IbKvView kv, c
   float m = sink ? (sink_values ? sink_values[h] : 0.f) : -INFINITY, l = sink ? 1.f : 0.f;   // the sink is a key of its own score: it starts the running maximum and sum
   (void)row;
   const C* base = (const C*)kv.base;
-  // the keys that are kept and lie before the window come first, then the window; `base_key` turns a place in that row into a position
-  const int kept = min(keep, lo), base_key = lo - kept, n_keys = kept + pos - lo + 1;
-  for (int k0 = 0; k0 < n_keys; k0 += 32) {
-    const int key = k0 + lane < kept ? k0 + lane : base_key + k0 + lane;
+  // Runs of 32 positions that start at multiples of 32: those that hold keys that are kept, then those of the window. Where a row's sums are cut
+  // depends on positions alone, and every multiply and add is written out, so that the kernel for tiles of rows (attention_prompt_f32.cu)
+  // gives the same bits.
+  const int kept = min(keep, lo);
+  for (int k0 = 0; k0 <= pos; k0 += 32) {
+    if (k0 >= kept && k0 + 31 < lo) k0 = lo & ~31;
+    const int key = k0 + lane;
     long long off = -1;
     float s = -INFINITY;
-    if (k0 + lane < n_keys) {
+    if (key <= pos && (key >= lo || key < kept)) {
       off = ib::kv_offset(kv, seg, key, kvhead);
       if (off < 0) {
         atomicOr(status, IB_ERR_BAD_PAGE);
       } else {
         const C* kr = base + off;
         float dot = 0.f;
-        for (int d = 0; d < hd; d++) dot += qs[warp][d] * ib::to_f32<C>(kr[d]);
-        s = dot * scale;
-        if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+        for (int d = 0; d < hd; d++) dot = __fmaf_rn(qs[warp][d], ib::to_f32<C>(kr[d]), dot);
+        s = __fmul_rn(dot, scale);
+        if (softcap > 0.f) s = __fmul_rn(softcap, tanhf(s / softcap));
       }
     }
     float m_new = fmaxf(m, ib::warp_max(s));
     if (m_new == -INFINITY) continue;  // every key of this chunk was unreadable
     float corr = expf(m - m_new);
     float p = s == -INFINITY ? 0.f : expf(s - m_new);
-    l = l * corr + ib::warp_sum(p);
+    l = __fmaf_rn(l, corr, ib::warp_sum(p));
 #pragma unroll
-    for (int r = 0; r < kMaxHeadDim / 32; r++) acc[r] *= corr;
-    int n = min(32, n_keys - k0);
+    for (int r = 0; r < kMaxHeadDim / 32; r++) acc[r] = __fmul_rn(acc[r], corr);
+    int n = min(32, pos - k0 + 1);
     for (int jj = 0; jj < n; jj++) {
       float pj = __shfl_sync(0xffffffffu, p, jj);
       long long oj = __shfl_sync(0xffffffffu, off, jj);
@@ -281,7 +284,7 @@ __global__ void attention_generic_kernel(const A* __restrict__ q, IbKvView kv, c
 #pragma unroll
       for (int r = 0; r < kMaxHeadDim / 32; r++) {
         int d = lane + 32 * r;
-        if (d < v_dim) acc[r] += pj * ib::to_f32<C>(vr[d]);
+        if (d < v_dim) acc[r] = __fmaf_rn(pj, ib::to_f32<C>(vr[d]), acc[r]);
       }
     }
     m = m_new;

@@ -4,12 +4,13 @@
 // attention_generic_kernel computes, with its window, blocks of positions, kept first positions, cap, sink, gate and factor. There a warp
 // holds one query row and every lane reads a key row of its own, so a portion reads each key once a row and the FMA units wait for it
 // (259 + 518 tokens of 16 heads of 128: 1,610 us a layer). Here a CTA holds 64 rows of one head over tiles of 64 keys in shared memory, a
-// thread 4 x 4 scores and 4 rows of 8 outputs: 132 us. What bounds it is shared-memory reads (8 of 16 bytes for 64 FMAs in the scores, 12
+// thread 4 x 4 scores and 4 rows of 8 outputs: 138 us. What bounds it is shared-memory reads (8 of 16 bytes for 64 FMAs in the scores, 12
 // for 128 in the sum) and, for few portions, the longest row tile's chain of key tiles; where the next tile's keys lie is looked up a tile
 // ahead (looked up where it is needed, the same work took 232 us with tiles of 32 keys, 169 a tile ahead).
 //
-// Key tiles start at multiples of 64 positions, so a row's sums are cut in the same places whatever the tile it lies in: its result
-// does not depend on which rows share the step. Reference: crates/kir/src/cuda/attention/flash_mma.rs:193 (the causal mask and window).
+// Key tiles start at multiples of 64 positions, and a row's maximum, sum and output advance in runs of 32 keys, each operation and its place as
+// in attention_generic_kernel: a position's bits are the same in a portion, alone and as a decoded token, however a prompt is cut. (One
+// advance for all 64 keys of a tile took 132 us.) Reference: crates/kir/src/cuda/attention/flash_mma.rs:193 (the causal mask and window).
 #include <type_traits>
 
 #include "kv_view.cuh"
@@ -120,59 +121,69 @@ attention_prompt_f32_kernel(const float* __restrict__ q, IbKvView kv, const int*
         for (int j = 0; j < 4; j++) s[i][j] = fmaf(a[i].w, b[j].w, fmaf(a[i].z, b[j].z, fmaf(a[i].y, b[j].y, fmaf(a[i].x, b[j].x, s[i][j]))));
     }
     const bool whole = k0 + BKEYS - 1 <= pos0 && (k0 >= ib::first_visible(last, va.window) || k0 + BKEYS <= keep);   // every row sees every key
+    float corr[4][2];   // what the sums so far are multiplied by before each run of 32 keys
 #pragma unroll
     for (int i = 0; i < 4; i++) {
       const int pos = pos0 + ty + 16 * i;
-      float top = -INFINITY;
+      float top[2] = {-INFINITY, -INFINITY};
 #pragma unroll
       for (int j = 0; j < 4; j++) {
         const int key = k0 + tx + 16 * j;
-        s[i][j] *= va.scale;
-        if (va.softcap > 0.f) s[i][j] = va.softcap * tanhf(s[i][j] / va.softcap);
+        s[i][j] = __fmul_rn(s[i][j], va.scale);
+        if (va.softcap > 0.f) s[i][j] = __fmul_rn(va.softcap, tanhf(s[i][j] / va.softcap));
         if (offs[buf * BKEYS + tx + 16 * j] < 0 || key > pos || (key < lo[i] && key >= keep)) s[i][j] = -INFINITY;
-        top = fmaxf(top, s[i][j]);
+        top[j >> 1] = fmaxf(top[j >> 1], s[i][j]);
       }
 #pragma unroll
-      for (int x = 8; x > 0; x >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, x));
-      const float m_new = fmaxf(m[i], top);
-      const float corr = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);   // (nothing seen so far: the sums are zero)
-      float sum = 0.f;
+      for (int x = 8; x > 0; x >>= 1) top[0] = fmaxf(top[0], __shfl_xor_sync(0xffffffffu, top[0], x)), top[1] = fmaxf(top[1], __shfl_xor_sync(0xffffffffu, top[1], x));
 #pragma unroll
-      for (int j = 0; j < 4; j++) {
-        const float p = s[i][j] == -INFINITY ? 0.f : expf(s[i][j] - m_new);
-        ps[(ty + 16 * i) * PL + tx + 16 * j] = p;
-        sum += p;
+      for (int run = 0; run < 2; run++) {
+        const float m_new = fmaxf(m[i], top[run]);
+        corr[i][run] = m_new == -INFINITY ? 1.f : expf(m[i] - m_new);   // (nothing seen so far: the sums are zero)
+        float p[2];
+#pragma unroll
+        for (int e = 0; e < 2; e++) {
+          const int j = 2 * run + e;
+          p[e] = s[i][j] == -INFINITY ? -0.f : expf(s[i][j] - m_new);   // (-0 marks a key that the row does not see)
+          ps[(ty + 16 * i) * PL + tx + 16 * j] = p[e];
+        }
+        float sum = p[0] + p[1];
+#pragma unroll
+        for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
+        l[i] = __fmaf_rn(l[i], corr[i][run], sum), m[i] = m_new;
       }
-#pragma unroll
-      for (int x = 8; x > 0; x >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, x);
-      l[i] = l[i] * corr + sum, m[i] = m_new;
-#pragma unroll
-      for (int c = 0; c < 4 * NC; c++) o[i][c] *= corr;
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
     __syncthreads();   // the values are here, and nobody reads the keys any more
     if (it + 1 < n) load(ks, QL, buf ^ 1, 0);
     auto add = [&](auto guard) {
+#pragma unroll 1
+      for (int run = 0; run < 2; run++) {
+#pragma unroll
+        for (int i = 0; i < 4; i++)
+#pragma unroll
+          for (int c = 0; c < 4 * NC; c++) o[i][c] = __fmul_rn(o[i][c], run ? corr[i][1] : corr[i][0]);
 #pragma unroll 2
-      for (int j = 0; j < BKEYS; j += 4) {
-        float4 p[4];
+        for (int j = 32 * run; j < 32 * run + 32; j += 4) {
+          float4 p[4];
 #pragma unroll
-        for (int i = 0; i < 4; i++) p[i] = *(const float4*)&ps[(ty + 16 * i) * PL + j];
+          for (int i = 0; i < 4; i++) p[i] = *(const float4*)&ps[(ty + 16 * i) * PL + j];
 #pragma unroll
-        for (int jj = 0; jj < 4; jj++)
+          for (int jj = 0; jj < 4; jj++)
 #pragma unroll
-          for (int c = 0; c < NC; c++) {
-            const float4 v = *(const float4*)&vs[(j + jj) * HD + c * 64 + tx * 4];
+            for (int c = 0; c < NC; c++) {
+              const float4 v = *(const float4*)&vs[(j + jj) * HD + c * 64 + tx * 4];
 #pragma unroll
-            for (int i = 0; i < 4; i++) {
-              const float w = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
-              // (a key that a row does not see adds nothing to it, whatever its value holds)
-              if (!decltype(guard)::value || w != 0.f) {
-                o[i][4 * c] = fmaf(w, v.x, o[i][4 * c]), o[i][4 * c + 1] = fmaf(w, v.y, o[i][4 * c + 1]);
-                o[i][4 * c + 2] = fmaf(w, v.z, o[i][4 * c + 2]), o[i][4 * c + 3] = fmaf(w, v.w, o[i][4 * c + 3]);
+              for (int i = 0; i < 4; i++) {
+                const float w = jj == 0 ? p[i].x : jj == 1 ? p[i].y : jj == 2 ? p[i].z : p[i].w;
+                // (a key that a row does not see adds nothing to it, whatever its value holds)
+                if (!decltype(guard)::value || __float_as_uint(w) != 0x80000000u) {
+                  o[i][4 * c] = fmaf(w, v.x, o[i][4 * c]), o[i][4 * c + 1] = fmaf(w, v.y, o[i][4 * c + 1]);
+                  o[i][4 * c + 2] = fmaf(w, v.z, o[i][4 * c + 2]), o[i][4 * c + 3] = fmaf(w, v.w, o[i][4 * c + 3]);
+                }
               }
             }
-          }
+        }
       }
     };
     if (whole) add(std::false_type{});

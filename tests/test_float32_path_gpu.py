@@ -69,3 +69,52 @@ def test_prompt_attention_matches_the_row_kernel(status, hd, heads, kvh, page, v
     for s, (_, n) in zip(segs, shapes):
         assert torch.equal(run(slice(at, at + n), [s]), out[at:at + n])
         at += n
+
+
+@pytest.mark.parametrize("hd,heads,kvh,page", [(128, 4, 2, 16), (64, 6, 1, 8)])
+@pytest.mark.parametrize("variant", ["plain", "window", "window_keep", "chunk", "cap_sink", "gate_sink"])
+def test_prompt_attention_gives_the_bits_of_the_row_kernel(hd, heads, kvh, page, variant):
+    """A position's result does not depend on the kernel that computes it: portions whose rows start anywhere in a tile, with windows and blocks
+    that begin anywhere in a run of 32 keys."""
+    from inference_bench_b200.engine.context import Segment, build_context
+    from inference_bench_b200.engine.runtime import Runtime
+    from inference_bench_b200.kernels import attention, lib, ops
+    window = 77 if variant.startswith("window") else None
+    shapes = [(300, 300), (200, 70), (161, 33), (64, 64), (65, 63), (33, 2), (257, 128)]
+    q, view, pos, seg, _, _ = _attention_case(torch.float32, heads, kvh, hd, page, window, shapes, 23)
+    T, scale, g = q.shape[0], 1 / math.sqrt(hd), _g(24)
+    kw = {"plain": {}, "window": {}, "window_keep": dict(keep_first=37), "chunk": dict(chunk=50), "cap_sink": dict(softcap=2.0, sink=True, sink_values=torch.randn(heads, generator=g).to(DEV)),
+          "gate_sink": dict(sink=True, out_scale=0.3, gate=(torch.randn(3, T, heads + 3, generator=g).to(DEV), 2))}[variant]
+    rt = Runtime(DEV, "float32")
+    names, real = [], lib.call
+    lib.call = lambda name, *a: (names.append(name), real(name, *a))[1]
+    try:
+        out = attention.paged_attention(build_context(rt, [Segment(i, i, L - n, [0] * n) for i, (L, n) in enumerate(shapes)]), q, view, heads, window, scale, **kw)
+    finally:
+        lib.call = real
+    want = torch.empty_like(q)
+    ops.attention_generic(q, view, pos, seg, window, scale, want, heads, rt.status, **kw)
+    rt.check_status()
+    assert names == ["ib_attention_prompt_f32"] and torch.equal(out, want)
+
+
+@pytest.mark.parametrize("head_dim", [64, 128])
+@pytest.mark.parametrize("windows", [(0, 0, 0), (1, 0, 1)])
+def test_logits_do_not_depend_on_how_a_prompt_is_cut(head_dim, windows):
+    """A prompt in one portion, with its last token alone, in odd pieces, and beside others: the same bits, in the cache too."""
+    from inference_bench_b200.engine.step import StepEntry
+    from test_repeat_gpu import _runner
+    tokens, outs = torch.randint(0, 333, (211,), generator=_g(3)).tolist(), []
+    for cuts, other in (([211], 0), ([210, 1], 0), ([1, 97, 64, 1, 48], 0), ([64, 130, 17], 9)):
+        r, at = _runner("float32", head_dim, windows, 16), 0
+        r.cache.admit(0), r.cache.admit(1)
+        for n in cuts:
+            entries = [StepEntry(1, [7 + n] * other, [])] * (other > 0) + [StepEntry(0, tokens[at:at + n], [n - 1])]
+            logits = r.step(entries)
+            at += n
+        rows = [[(gr.tensor[:, p].clone(), min(16, 211 - 16 * i)) for i, p in enumerate(r.cache.table(g, 0)[:14].tolist()) if p >= 0] for g, gr in enumerate(r.cache.groups)]
+        outs.append((logits.clone(), [[t[..., :n, :] for t, n in row] for row in rows]))
+    for logits, rows in outs[1:]:
+        assert torch.equal(logits, outs[0][0])
+        for a, b in zip(rows, outs[0][1]):
+            assert len(a) == len(b) > 0 and all(torch.equal(u, v) for u, v in zip(a, b))
