@@ -4,7 +4,8 @@
 //  * grouped: the regrouped rows of routed experts (csrc/moe.cu): rows offsets[e]..offsets[e+1] go through W[e]; a 64 x 64 tile
 //    belongs to one expert; the rows of x may be gathered through an index. With `gated`, W[e] holds gate rows then up rows
 //    and the output is silu(gate) * up (float32 arithmetic on the accumulators).
-//  * heads: out[t][b] = W[b] x[t][b] for every head b, rows and heads strided (the per-head maps around latent attention).
+//  * heads: out[t][b] = W[b] x[t][b] for every head b, rows and heads strided (the per-head maps around latent attention), for all rows t or for
+//    those of a list (the tokens of a mixed step whose queries go to the latents' space; the others' rows are neither read nor written).
 //
 // A CTA of four warps (2 x 2, 32 x 32 each) walks K in tiles of 64 values: 16-byte cp.async copies into two swizzled buffers
 // (the next tile arrives while this one is multiplied), ldmatrix fragments. Each output is one accumulation over k in a fixed
@@ -21,14 +22,14 @@ struct RowsArgs {
   const __nv_bfloat16* x;
   const __nv_bfloat16* w;
   void* out;
+  const int* src_row;   // grouped: the row of x of every regrouped row, or null; heads: the rows that are computed, or null for all
   // grouped
-  const int* src_row;
   const int* offsets;
   const int* tile_start;
   int n_groups;
   // heads
   long long x_row, x_head, o_row, o_head;
-  int rows;      // heads mode: T
+  int rows;      // heads mode: how many rows are computed
   int N, K;
   int grouped;
   // heads mode: float32 partial sums [gate_P][T][gate_row], offset to the first head's column, or null: head b's output of row t is multiplied
@@ -90,8 +91,8 @@ __global__ void __launch_bounds__(128) gemm_rows_mma_kernel(RowsArgs p) {
     const int r = (tid >> 3) + 16 * i, row = r0 + r, n = n0 + r;
     a_src[i] = nullptr;
     if (row < r1) {
-      if (p.grouped) a_src[i] = p.x + (size_t)(p.src_row ? p.src_row[row] : row) * K;
-      else a_src[i] = p.x + (size_t)row * p.x_row + (size_t)group * p.x_head;
+      const size_t t = p.src_row ? p.src_row[row] : row;
+      a_src[i] = p.grouped ? p.x + t * K : p.x + t * p.x_row + (size_t)group * p.x_head;
     }
     b_src[i] = n < N ? wg + (size_t)n * K : nullptr;
     u_src[i] = (GATED && n < N) ? wg + (size_t)(N + n) * K : nullptr;
@@ -165,10 +166,11 @@ __global__ void __launch_bounds__(128) gemm_rows_mma_kernel(RowsArgs p) {
     for (int h = 0; h < 2; h++) {
       const int row = r0 + wm * 32 + m * 16 + g + 8 * h;
       if (row >= r1) continue;
-      O* dst = p.grouped ? out + (size_t)row * N : out + (size_t)row * p.o_row + (size_t)group * p.o_head;
+      const size_t t = !p.grouped && p.src_row ? p.src_row[row] : row;
+      O* dst = p.grouped ? out + t * N : out + t * p.o_row + (size_t)group * p.o_head;
       float f = 1.f;
       if (!p.grouped && p.gate) {
-        const float* gr = p.gate + (size_t)row * p.gate_row + group;
+        const float* gr = p.gate + t * p.gate_row + group;
         float z = gr[0];
         for (int q = 1; q < p.gate_P; q++) z += gr[q * p.gate_stride];
         f = 1.f / (1.f + expf(-z));
@@ -223,13 +225,14 @@ extern "C" int ib_gemm_grouped_mma(const void* x, const int* src_row, const void
 }
 
 extern "C" int ib_gemm_heads_mma(const void* x, long long x_row, long long x_head, const void* w, void* out, int out_dtype, long long o_row, long long o_head, int T,
-                                 int heads, int N, int K, const float* gate, int gate_P, long long gate_stride, int gate_row, cudaStream_t stream) {
+                                 int heads, int N, int K, const float* gate, int gate_P, long long gate_stride, int gate_row, const int* rows, cudaStream_t stream) {
+  // rows: null, or the T rows of x, out and gate that are computed
   if (T == 0 || N == 0 || heads == 0) return 0;
   IB_CHECK_ARG(T > 0 && N > 0 && K > 0 && heads > 0, "gemm_heads_mma: bad sizes T=%d heads=%d N=%d K=%d", T, heads, N, K);
   IB_CHECK_ARG(x_row % 8 == 0 && x_head % 8 == 0, "gemm_heads_mma: row stride %lld and head stride %lld must be multiples of 8", x_row, x_head);
   RowsArgs a = {};
   a.x = (const __nv_bfloat16*)x, a.w = (const __nv_bfloat16*)w, a.out = out, a.x_row = x_row, a.x_head = x_head, a.o_row = o_row, a.o_head = o_head;
-  a.rows = T, a.N = N, a.K = K, a.grouped = 0;
+  a.rows = T, a.src_row = rows, a.N = N, a.K = K, a.grouped = 0;
   a.gate = gate, a.gate_P = gate_P, a.gate_stride = gate_stride, a.gate_row = gate_row;
   return launch_rows(a, dim3((N + TN - 1) / TN, (T + TM - 1) / TM, heads), 0, out_dtype, stream, "gemm_heads_mma");
 }

@@ -405,7 +405,7 @@ def latent_prepare(qd: torch.Tensor, c_norm_w: Optional[torch.Tensor], eps: floa
 
 
 L.register("ib_gemm_grouped_mma", [L._p, L._p, L._p, L._p, L._i, L._p, L._p, L._i, L._i, L._i, L._i, L._i, L._p, L._f, L._p])
-L.register("ib_gemm_heads_mma", [L._p, L._ll, L._ll, L._p, L._p, L._i, L._ll, L._ll, L._i, L._i, L._i, L._i, L._p, L._i, L._ll, L._i, L._p])
+L.register("ib_gemm_heads_mma", [L._p, L._ll, L._ll, L._p, L._p, L._i, L._ll, L._ll, L._i, L._i, L._i, L._i, L._p, L._i, L._ll, L._i, L._p, L._p])
 
 
 def latent_down(qd: torch.Tensor, q_rank: int, q_norm_w: torch.Tensor, cq: torch.Tensor, c_norm_w: torch.Tensor, eps: float, cos: Optional[torch.Tensor],
@@ -434,10 +434,12 @@ def rows_mma_fits(x: torch.Tensor, w: torch.Tensor) -> bool:
     return x.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and x.shape[-1] % 8 == 0 and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0
 
 
-def gemm_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n: int, tensor_cores: bool = False, gate: Optional[tuple] = None) -> None:
+def gemm_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n: int, tensor_cores: bool = False, gate: Optional[tuple] = None,
+               rows: Optional[torch.Tensor] = None) -> None:
     """out[t, b, :n] = w[b] x[t, b] for every head b: x [T, heads, K] (contiguous), w [heads, N, K], out [T, heads, >= n] whose
     first n columns of every head are written (the rest stay). tensor_cores: the m16n8k16 kernel (see `rows_mma_fits`).
-    gate = (float32 partial sums [P, T, row], column of the first head): head b's output is multiplied by the sigmoid of its column."""
+    gate = (float32 partial sums [P, T, row], column of the first head): head b's output is multiplied by the sigmoid of its column.
+    rows (tensor cores only): None, or the rows t (int32) that are computed; the others are not read and stay as they are."""
     T, heads, K = x.shape
     g_ptr, g_P, g_stride, g_row = None, 0, 0, 0
     if gate is not None:
@@ -455,9 +457,13 @@ def gemm_heads(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, n: int, tens
     if tensor_cores:
         if not rows_mma_fits(x, w):
             raise L.KernelError("gemm_heads: the tensor-core kernel needs bfloat16 operands with an inner size that is a multiple of 8")
-        L.call("ib_gemm_heads_mma", x.data_ptr(), heads * K, K, w.data_ptr(), out.data_ptr(), dtype_code(out.dtype), heads * out.shape[2], out.shape[2], T, heads, n, K,
-               g_ptr, g_P, g_stride, g_row, _stream())
+        if rows is not None:
+            _check("rows", rows, torch.int32)
+        L.call("ib_gemm_heads_mma", x.data_ptr(), heads * K, K, w.data_ptr(), out.data_ptr(), dtype_code(out.dtype), heads * out.shape[2], out.shape[2],
+               T if rows is None else rows.shape[0], heads, n, K, g_ptr, g_P, g_stride, g_row, _ptr(rows), _stream())
         return
+    if rows is not None:
+        raise L.KernelError("gemm_heads: a list of rows is for the tensor-core kernel")
     L.call("ib_gemm_heads", x.data_ptr(), dtype_code(x.dtype), heads * K, K, w.data_ptr(), dtype_code(w.dtype), out.data_ptr(), dtype_code(out.dtype),
            heads * out.shape[2], out.shape[2], T, heads, n, K, g_ptr, g_P, g_stride, g_row, _stream())
 

@@ -134,8 +134,8 @@ class LatentAttention(base.Mixer):
 
     def _expanded(self, ctx):
         """None, or how the step's longer segments go through keys and values per head: (blocks [n, 2] and tiles [m, 4] on the device, see
-        `ops.latent_keys_values` and `ops.latent_prefill`; query rows a CTA holds and runs of the other segments' tokens like `_rows_and_units`,
-        None if there are no others)."""
+        `ops.latent_keys_values` and `ops.latent_prefill`; query rows a CTA holds and runs of the other segments' tokens like `_rows_and_units` and
+        those tokens' rows, None if there are no others)."""
         if self.w_kv is None or ctx.fixed_shape or ctx.max_segment_len < EXPAND_MIN_TOKENS:
             return None
         key = ("latent expanded", self.window, self.heads, self.dim + self.vdim, self.kv_rank, self.rot_dim)
@@ -157,10 +157,12 @@ class LatentAttention(base.Mixer):
                 rows = ops.latent_attention_mma_rows(self.kv_rank, self.kv_rank + self.rot_dim, self.heads * max((b - a for a, b in rest), default=1))
                 per = max(1, rows // self.heads)
                 runs = [(t, min(per, b - t)) for a, b in rest for t in range(a, b, per)]
-                flat = np.concatenate([np.asarray(v, np.int32).ravel() for v in (tiles, blocks, runs)]).astype(np.int32)
+                tokens = [t for a, b in rest for t in range(a, b)]
+                flat = np.concatenate([np.asarray(v, np.int32).ravel() for v in (tiles, blocks, runs, tokens)]).astype(np.int32)
                 dev = torch.from_numpy(flat).pin_memory().to(ctx.rt.device, non_blocking=True)
                 m, n = 4 * len(tiles), 4 * len(tiles) + 2 * len(blocks)
-                plan = (dev[m:n].view(-1, 2), dev[:m].view(-1, 4), (rows, dev[n:].view(-1, 2)) if rest else None)
+                k = n + 2 * len(runs)
+                plan = (dev[m:n].view(-1, 2), dev[:m].view(-1, 4), (rows, dev[n:k].view(-1, 2), dev[k:]) if rest else None)
             ctx.memo[key] = plan
         return ctx.memo[key]
 
@@ -207,7 +209,8 @@ class LatentAttention(base.Mixer):
         v = rt.empty((T, H, self.vdim))
         if plan is None or plan[2] is not None:   # the tokens whose queries go to the latents' space
             tc = rt.options.expert_gemm != "simt"   # (the per-head maps have the m16n8k16 kernel and the FMA kernel)
-            ops.gemm_heads(q_nope, self.wuk_t, q_full, r, tensor_cores=tc and ops.rows_mma_fits(q_nope, self.wuk_t))
+            only = None if plan is None else plan[2][2]
+            ops.gemm_heads(q_nope, self.wuk_t, q_full, r, tensor_cores=tc and ops.rows_mma_fits(q_nope, self.wuk_t), rows=only)
             n_slices, slice_keys = self._slices(ctx, cache.c_view())
             scratch = None
             if n_slices > 1:
@@ -217,11 +220,11 @@ class LatentAttention(base.Mixer):
                 scratch = ctx.memo[skey]
             u = rt.empty((T, H, r))
             if self._tensor_cores(rt):
-                rows, units = self._rows_and_units(ctx) if plan is None else plan[2]
+                rows, units = self._rows_and_units(ctx) if plan is None else plan[2][:2]
                 ops.latent_attention_mma(q_full, cache, ctx.positions, ctx.seg_of_token, units, self.scale, u, r, n_slices, slice_keys, scratch, rt.status, rows, window=self.window, sink=self.sink_dev)
             else:
                 ops.latent_attention(q_full, cache, ctx.positions, ctx.seg_of_token, self.scale, u, r, n_slices, slice_keys, scratch, rt.status, window=self.window, sink=self.sink_dev)
-            ops.gemm_heads(u, self.wuv, v, self.vdim, tensor_cores=tc and ops.rows_mma_fits(u, self.wuv), gate=gate)
+            ops.gemm_heads(u, self.wuv, v, self.vdim, tensor_cores=tc and ops.rows_mma_fits(u, self.wuv), gate=gate, rows=only)
         if plan is not None:   # and those that see keys and values per head (their rows of v hold nothing yet)
             kv, part = ops.latent_keys_values(cache, plan[0], ctx.seg_start, ctx.seg_pos0, self.w_kv, r, rot, rt.status, self.window)
             ops.latent_prefill(q_nope, q_full, r, plan[1], kv, part, self.scale, v, rt.status, window=self.window, sink=self.sink_dev, gate=gate)

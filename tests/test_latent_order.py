@@ -16,8 +16,8 @@ def test_the_mark_for_the_next_launch_is_the_threads_own():
     assert other == [1] and core.ib_pdl_enabled() == 0 and core.ib_pdl_enabled() == 1
 
 
-def _latent_forward(monkeypatch, plan):
-    """The names of what one forward pass of latent attention asks for, in order, with nothing run."""
+def _latent_forward(monkeypatch, plan, given=None):
+    """The names of what one forward pass of latent attention asks for, in order, with nothing run; `given` collects the named arguments."""
     from types import SimpleNamespace
 
     import torch
@@ -27,7 +27,7 @@ def _latent_forward(monkeypatch, plan):
     from inference_bench_b200.parts.standard import NoPositionEncoding
     done, T = [], 40
     for name in ("latent_prepare", "gemm_heads", "latent_attention_mma", "latent_prefill"):
-        monkeypatch.setattr(ops, name, lambda *a, _name=name, **kw: done.append(_name))
+        monkeypatch.setattr(ops, name, lambda *a, _name=name, **kw: (done.append(_name), given is not None and given.append((_name, kw))))
     monkeypatch.setattr(ops, "latent_keys_values", lambda *a, **kw: (done.append("latent_keys_values"), None))
     monkeypatch.setattr(ops, "rows_mma_fits", lambda *a: True)
     rt = SimpleNamespace(act_dtype=torch.bfloat16, sm_count=148, status=None, options=SimpleNamespace(expert_gemm="auto", latent_attention="auto"),
@@ -52,3 +52,12 @@ def test_the_output_projection_follows_the_prompt_attention_in_order(monkeypatch
     done = _latent_forward(monkeypatch, (None, None, None))
     assert done[-3:] == ["latent_prefill", "next_in_order", "linear out"] and done.count("next_in_order") == 1
     assert "next_in_order" not in _latent_forward(monkeypatch, None)
+
+
+def test_the_maps_take_the_rows_that_need_them(monkeypatch):
+    """Beside portions with keys and values per head, the other tokens' queries alone go to the latents' space and back; without such portions all do."""
+    rows = object()
+    for plan, want in (((None, None, (16, None, rows)), [rows, rows]), ((None, None, None), []), (None, [None, None])):
+        given = []
+        _latent_forward(monkeypatch, plan, given)
+        assert [kw["rows"] for name, kw in given if name == "gemm_heads"] == want

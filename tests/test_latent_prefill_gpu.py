@@ -115,3 +115,23 @@ def test_a_step_of_portions_and_tokens_matches_the_other_form(q_rank, gate, sink
     for a, b in zip(outs["auto"], outs["mma"]):
         # two roundings of values and weights to bfloat16 in either form, summed over 4 heads of 64
         assert (a - b).abs().max() <= 2e-2 * b.abs().max()
+
+
+@pytest.mark.parametrize("K,n,rows", [(64, 256, [0]), (128, 512, list(range(70))), (256, 64, [3, 4, 9, 63, 64, 65, 130, 199]), (40, 33, list(range(199, 60, -1)))])
+def test_the_maps_of_a_list_of_rows(K, n, rows):
+    """Rows of a list give the bits that they have among all rows; the others are not read (they are NaN) and not written."""
+    from inference_bench_b200.kernels import ops
+    T, heads, g = 200, 3, _g(K + n)
+    x = torch.randn(T, heads, K, generator=g).to(torch.bfloat16).to(DEV)
+    w = torch.randn(heads, n, K, generator=g).to(torch.bfloat16).to(DEV)
+    gate = (torch.randn(2, T, heads + 1, generator=g).to(DEV), 1)
+    whole = torch.empty(T, heads, n + 8, device=DEV)
+    ops.gemm_heads(x, w, whole, n, tensor_cores=True, gate=gate)
+    at = torch.tensor(rows, device=DEV)
+    some, out = torch.full_like(x, float("nan")), torch.full((T, heads, n + 8), 7.0, device=DEV)
+    some[at] = x[at]
+    ops.gemm_heads(some, w, out, n, tensor_cores=True, gate=gate, rows=at.int())
+    assert torch.equal(out[at, :, :n], whole[at, :, :n])
+    rest = torch.ones(T, dtype=torch.bool, device=DEV)
+    rest[at] = False
+    assert (out[rest] == 7.0).all() and (out[..., n:] == 7.0).all()
