@@ -226,15 +226,16 @@ class CacheManager:
     def extend(self, req: Hashable, new_length: int) -> None:
         """Allocate, in every group, the pages for positions up to new_length - 1. All or nothing."""
         r = self._get(req)
-        self._extended(self._lib.ibh_cache_extend(self._core, r.slot, int(new_length)), req, new_length)
+        code = self._lib.ibh_cache_extend(self._core, r.slot, int(new_length))
+        if code:
+            self._extended(code, req, new_length)
 
     def _extended(self, code: int, req: Hashable, new_length: int) -> None:
         if code == 1:
             raise OutOfPages(f"request {req!r} {native.last_error()}")
         if code == 2:
             raise OutOfPages(f"request {req!r} would hold {new_length} tokens, more than the limit of {self.max_tokens_per_request}")
-        if code:
-            raise CacheError(native.last_error())
+        raise CacheError(native.last_error())
 
     def shrink_to_committed(self, req: Hashable) -> None:
         """Undo an `extend` that no `commit` followed: free the pages beyond the committed length."""
