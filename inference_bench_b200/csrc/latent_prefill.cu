@@ -11,7 +11,7 @@
 //   latent_prefill_kernel   a CTA per 128 query rows of one head: the roles of attention_prefill_ws.cu (four softmax warps, a warp that issues
 //                           the MMAs one score tile ahead, a warp each for the key and value tiles), with a query of dim + rot values
 // Bound by the softmax warps' chain from a score tile to the next (two CTAs an SM fill each other's gaps), then by the scores' operand reads.
-// Measured, 16 heads of 128 + 64 on a latent of 512: 2,048 tokens 8 + 19 + 47 us (gather, product, attention) where the maps to the latents'
+// Which segments of a step come here is decided in parts/latent.py. Measured, 16 heads of 128 + 64 on a latent of 512: 2,048 tokens 8 + 19 + 47 us (gather, product, attention) where the maps to the latents'
 // space and attention there took 70 + 666; 333 tokens of three requests behind 116 to 583 cached positions 8 + 19 + 25 against 31 + 80; 64
 // tokens behind 900 8 + 15 + 25 against 21 + 92; 32 tokens alone 9 + 13 + 11 against 19 + 17.
 #include <cuda.h>
@@ -250,7 +250,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
     float m_ref = -INFINITY, l = 0.f;
     for (int j = 0; j < n_kt; j++) {
-            wait(&s_full[j & 1], (j >> 1) & 1);
+      wait(&s_full[j & 1], (j >> 1) & 1);
       sm100::tc_fence_after();
       uint32_t sr[BN];
       sm100::tmem_ld_32x32b_x32(t_lane + (j & 1) * BN, sr);
@@ -411,20 +411,24 @@ extern "C" int ib_latent_prefill(const void* q_nope, const float* q_rot, int q_r
   CUtensorMap km, rm;
   if (make_map(&km, keys_values, rows, heads * (dim + vdim))) return 1;
   if (make_map(&rm, rot ? key_part : keys_values, rows, rot ? kRot : heads * (dim + vdim))) return 1;
-  auto go = [&](auto kernel, int bytes) -> int {
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    IB_CHECK_ARG(e == cudaSuccess, "latent_prefill: cannot reserve %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
-    ib::launch(kernel, dim3(heads, n_tiles), kThreads, bytes, stream, (const __nv_bfloat16*)q_nope, q_rot, q_rot_row, rot, (const int4*)tiles, km, rm, window,
+  auto sized = [&](auto d, auto r, auto v) -> int {
+    constexpr int D = decltype(d)::value, R = decltype(r)::value, V = decltype(v)::value, bytes = Smem<D, R, V>::kBytes;
+    static bool configured = false;
+    if (!configured) {
+      cudaError_t e = cudaFuncSetAttribute(latent_prefill_kernel<D, R, V>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+      IB_CHECK_ARG(e == cudaSuccess, "latent_prefill: cannot reserve %d bytes of shared memory: %s", bytes, cudaGetErrorString(e));
+      configured = true;
+    }
+    ib::launch(latent_prefill_kernel<D, R, V>, dim3(heads, n_tiles), kThreads, bytes, stream, (const __nv_bfloat16*)q_nope, q_rot, q_rot_row, rot, (const int4*)tiles, km, rm, window,
                scale * 1.4426950408889634f, sink_values, tail, (__nv_bfloat16*)out, heads, ib_wait_limit_ns(), status);
     return 0;
   };
-  auto sized = [&](auto d, auto v) -> int {
-    constexpr int D = decltype(d)::value, V = decltype(v)::value;
-    return rot ? go(latent_prefill_kernel<D, kRot, V>, Smem<D, kRot, V>::kBytes) : go(latent_prefill_kernel<D, 0, V>, Smem<D, 0, V>::kBytes);
-  };
   using std::integral_constant;
-  const int bad = dim == 128 ? (vdim == 128 ? sized(integral_constant<int, 128>{}, integral_constant<int, 128>{}) : sized(integral_constant<int, 128>{}, integral_constant<int, 64>{}))
-                             : (vdim == 128 ? sized(integral_constant<int, 64>{}, integral_constant<int, 128>{}) : sized(integral_constant<int, 64>{}, integral_constant<int, 64>{}));
+  const integral_constant<int, 64> c64{};
+  const integral_constant<int, 128> c128{};
+  auto with_values = [&](auto d, auto r) { return vdim == 128 ? sized(d, r, c128) : sized(d, r, c64); };
+  auto with_part = [&](auto d) { return rot ? with_values(d, integral_constant<int, kRot>{}) : with_values(d, integral_constant<int, 0>{}); };
+  const int bad = dim == 128 ? with_part(c128) : with_part(c64);
   if (bad) return bad;
   IB_CHECK_LAUNCH("latent_prefill");
   return 0;

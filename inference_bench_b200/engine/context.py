@@ -9,6 +9,7 @@ crates/specrt/src/runtime/fused.rs:6-11); here any number of either may share a 
 from __future__ import annotations
 
 from dataclasses import dataclass, field
+from functools import cached_property
 from typing import Any, Optional, Sequence
 
 import numpy as np
@@ -62,9 +63,9 @@ class StepContext:
     def n_segments(self) -> int:
         return len(self.segments)
 
-    @property
+    @cached_property   # (asked several times a layer)
     def max_segment_len(self) -> int:
-        return int(np.max(np.diff(self.h_seg_start))) if self.segments else 0
+        return int((self.h_seg_start[1:] - self.h_seg_start[:-1]).max()) if self.segments else 0
 
 
 def build_context(rt: Runtime, segments: list[Segment], caches: Optional[list] = None) -> StepContext:

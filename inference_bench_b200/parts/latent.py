@@ -37,6 +37,27 @@ from .base import PagedRows, WeightSpec
 # as long (making a key's heads costs as much as about a dozen of its pairs with a query), and while the step's rows keep the keys and
 # values of one layer below this many bytes.
 EXPAND_MIN_TOKENS, EXPAND_MAX_CONTEXT, EXPAND_MAX_BYTES = 32, 64, 1 << 29
+# Where all other tokens of such a step may go the same way too, they do: one form costs less than two. Where some need the form that reads the
+# latents (decoded tokens with long contexts), both forms run, three kernels more than the second alone: the portions must then save at least
+# this many microseconds by the estimate of `_saved`. Whole passes of one layer beside 8 decoded tokens, the second form alone and both, us: heads
+# of 64 + 32 on a latent of 256, 300 tokens 362 and 423, 1,000 426 and 446, 1,500 473 and 468, 2,048 531 and 488; 16 heads of 128 + 64 on 512,
+# 300 tokens 385 and 422, 600 431 and 435, 1,000 507 and 458, 2,048 858 and 552.
+EXPAND_BESIDE_SAVED_US = 60.0
+# Multiplies a microsecond, from the kernels alone at portions of 512 to 2,048 tokens of both sizes: the maps to the latents' space and back, attention
+# there, the product of keys and values, attention over them.
+MAP_RATE, LATENT_RATE, MAKE_RATE, PAIR_RATE = 60e6, 53e6, 500e6, 400e6
+
+
+def _runs(ranges, per: int) -> list:
+    """The tokens a .. b - 1 of every range in runs of up to `per`: first, how many, first, how many ... in order."""
+    out = []
+    for a, b in ranges:
+        whole = b - (b - a) % per
+        for t in range(a, whole, per):
+            out += (t, per)
+        if whole < b:
+            out += (whole, b - whole)
+    return out
 
 
 @base.register_mixer("latent_attention")
@@ -133,46 +154,99 @@ class LatentAttention(base.Mixer):
         return rows, self._units(ctx, per)
 
     def _expanded(self, ctx):
-        """None, or how the step's longer segments go through keys and values per head: (blocks [n, 2] and tiles [m, 4] on the device, see
+        """None, or how the step's segments go through keys and values per head: (blocks [n, 2] and tiles [m, 4] on the device, see
         `ops.latent_keys_values` and `ops.latent_prefill`; query rows a CTA holds and runs of the other segments' tokens like `_rows_and_units` and
         those tokens' rows, None if there are no others)."""
-        if self.w_kv is None or ctx.fixed_shape or ctx.max_segment_len < EXPAND_MIN_TOKENS:
+        if self.w_kv is None or ctx.fixed_shape:
             return None
         key = ("latent expanded", self.window, self.heads, self.dim + self.vdim, self.kv_rank, self.rot_dim)
         if key not in ctx.memo:
-            room = EXPAND_MAX_BYTES // (2 * self.heads * (self.dim + self.vdim)) // 64
-            blocks, tiles, rest = [], [], []
-            for s, (a, b, pos0) in enumerate(zip(ctx.h_seg_start[:-1].tolist(), ctx.h_seg_start[1:].tolist(), ctx.h_seg_pos0.tolist())):
-                first = 0 if self.window is None else max(0, pos0 - self.window + 1) // 64 * 64
-                keys = range(first, pos0 + b - a, 64)
-                if b - a < EXPAND_MIN_TOKENS or 64 * len(keys) > EXPAND_MAX_CONTEXT * (b - a) or len(blocks) + len(keys) > room:
-                    rest.append((a, b))
-                    continue
-                base = 64 * len(blocks) - first
-                blocks += [(s, k) for k in keys]
-                tiles += [(t, min(128, b - t), pos0 + t - a, base) for t in range(a, b, 128)]
-            plan = None
-            if tiles:
-                tiles.sort(key=lambda t: -(t[2] + t[1] if self.window is None else min(t[2], self.window) + t[1]))   # the tiles that see the most keys first
-                rows = ops.latent_attention_mma_rows(self.kv_rank, self.kv_rank + self.rot_dim, self.heads * max((b - a for a, b in rest), default=1))
-                per = max(1, rows // self.heads)
-                runs = [(t, min(per, b - t)) for a, b in rest for t in range(a, b, per)]
-                tokens = [t for a, b in rest for t in range(a, b)]
-                flat = np.concatenate([np.asarray(v, np.int32).ravel() for v in (tiles, blocks, runs, tokens)]).astype(np.int32)
-                dev = torch.from_numpy(flat).pin_memory().to(ctx.rt.device, non_blocking=True)
-                m, n = 4 * len(tiles), 4 * len(tiles) + 2 * len(blocks)
-                k = n + 2 * len(runs)
-                plan = (dev[m:n].view(-1, 2), dev[:m].view(-1, 4), (rows, dev[n:k].view(-1, 2), dev[k:]) if rest else None)
-            ctx.memo[key] = plan
+            ctx.memo[key] = self._plan_expanded(ctx)
         return ctx.memo[key]
+
+    def _saved(self, tokens, pos0, keys):
+        """About how many microseconds of kernels a portion saves through keys and values per head."""
+        seen = tokens * pos0 + tokens * (tokens + 1) // 2
+        if self.window is not None:
+            seen = min(seen, tokens * self.window)
+        make = self.heads * self.kv_rank * (self.dim + self.vdim)
+        return (tokens * make / MAP_RATE + seen * self.heads * (2 * self.kv_rank + self.rot_dim) / LATENT_RATE
+                - keys * make / MAKE_RATE - seen * self.heads * (self.dim + self.rot_dim + self.vdim) / PAIR_RATE)
+
+    def _choose(self, starts, pos0s):
+        """None, or which of a step's segments (first tokens, then the step's end; first positions) go through keys and values per head, as (segment, first
+        token, one past its last, its position, first position of its blocks, their number), and the token ranges of the others."""
+        lens = [b - a for a, b in zip(starts, starts[1:])]
+        if max(lens, default=0) < EXPAND_MIN_TOKENS:
+            return None
+        room = EXPAND_MAX_BYTES // (2 * self.heads * (self.dim + self.vdim)) // 64
+
+        def place(s, some, n):
+            """Puts segment s at the end of `some`, which holds n blocks, if it may go there; the blocks it holds then."""
+            a, b, pos0 = starts[s], starts[s + 1], pos0s[s]
+            first = 0 if self.window is None else max(0, pos0 - self.window + 1) // 64 * 64
+            own = (pos0 + b - a - first + 63) // 64
+            if 64 * own > EXPAND_MAX_CONTEXT * (b - a) or n + own > room:
+                return n
+            some.append((s, a, b, pos0, first, own))
+            return n + own
+
+        some, n = [], 0
+        for s, length in enumerate(lens):
+            if length >= EXPAND_MIN_TOKENS:
+                n = place(s, some, n)
+        if not some:
+            return None
+        taken = {c[0] for c in some}
+        rest = [s for s, length in enumerate(lens) if length and s not in taken]
+        every = []
+        for i, s in enumerate(rest):
+            n = place(s, every, n)
+            if len(every) == i:
+                break
+        if len(every) == len(rest):   # one form serves the whole step
+            return some + every, []
+        if sum(self._saved(c[2] - c[1], c[3], 64 * c[5]) for c in some) < EXPAND_BESIDE_SAVED_US:
+            return None
+        return some, [(starts[s], starts[s + 1]) for s in rest]
+
+    def _plan_expanded(self, ctx):
+        chosen = self._choose(ctx.h_seg_start.tolist(), ctx.h_seg_pos0.tolist())
+        if chosen is None:
+            return None
+        some, rest = chosen
+        tiles, spans, n_blocks = [], [], 0
+        for s, a, b, pos0, first, n in some:
+            tiles += [(t, min(128, b - t), pos0 + t - a, 64 * n_blocks - first) for t in range(a, b, 128)]
+            spans.append((s, first, n_blocks, n_blocks + n))
+            n_blocks += n
+        tiles.sort(key=lambda t: -(t[2] + t[1] if self.window is None else min(t[2], self.window) + t[1]))   # the tiles that see the most keys first
+        rows, runs, tokens = 0, [], []
+        if rest:
+            rows = ops.latent_attention_mma_rows(self.kv_rank, self.kv_rank + self.rot_dim, self.heads * max(b - a for a, b in rest))
+            runs = _runs(rest, max(1, rows // self.heads))
+            for a, b in rest:
+                tokens += range(a, b)
+        m, n = 4 * len(tiles), 4 * len(tiles) + 2 * n_blocks
+        staging = torch.empty(n + len(runs) + len(tokens), dtype=torch.int32, pin_memory=True)
+        h = staging.numpy()
+        h[:m] = [v for t in tiles for v in t]
+        blocks = h[m:n].reshape(-1, 2)
+        for s, first, i, j in spans:
+            blocks[i:j, 0], blocks[i:j, 1] = s, np.arange(first, first + 64 * (j - i), 64)
+        h[n:] = runs + tokens
+        dev = staging.to(ctx.rt.device, non_blocking=True)
+        part = lambda at, rows, cols: dev.as_strided((rows, cols), (cols, 1), at)
+        return part(m, n_blocks, 2), part(0, len(tiles), 4), (rows, part(n, len(runs) // 2, 2), dev[n + len(runs):]) if rest else None
 
     def _units(self, ctx, per):
         key = ("latent units", per)
         if key not in ctx.memo:
-            runs = []
-            for a, b in zip(ctx.h_seg_start[:-1].tolist(), ctx.h_seg_start[1:].tolist()):
-                runs += [(t, min(per, b - t)) for t in range(a, b, per)]
-            ctx.memo[key] = torch.tensor(runs, dtype=torch.int32).pin_memory().to(ctx.rt.device, non_blocking=True)
+            starts = ctx.h_seg_start.tolist()
+            runs = _runs(zip(starts, starts[1:]), per)
+            staging = torch.empty(len(runs), dtype=torch.int32, pin_memory=True)
+            staging.numpy()[:] = runs
+            ctx.memo[key] = staging.to(ctx.rt.device, non_blocking=True).view(-1, 2)
         return ctx.memo[key]
 
     def _tensor_cores(self, rt) -> bool:
