@@ -51,7 +51,6 @@ class Runtime:
         self.act_dtype = MODES[self.mode]
         self.gemm = self.options.gemm  # "auto" | "simt" | "tcgen05"
         self._side: Optional[torch.cuda.Stream] = None
-        self.held: Optional[list] = None   # while a layer's calls are noted (parts/repeat.py): the buffers it asks for
         self.status = torch.zeros(1, dtype=torch.int32, device=self.device)
         self.activate()
 
@@ -83,8 +82,9 @@ class Runtime:
     # ---------------------------------------------------------------- memory
     def empty(self, shape, dtype=None) -> torch.Tensor:
         t = torch.empty(shape, dtype=dtype or self.act_dtype, device=self.device)
-        if self.held is not None:
-            self.held.append(t)
+        held = L.notes.held
+        if held is not None:
+            held.append(t)
         return t
 
     def upload(self, t: torch.Tensor, dtype=None) -> torch.Tensor:

@@ -135,6 +135,7 @@ KERNELS_PER_CALL = {"ib_sample_rows": 3, "ib_attention_decode": 2, "ib_attention
 
 class _Notes(threading.local):
     calls = None   # a list that every `call` of this thread is added to as (name, arguments), while somebody notes them
+    held = None    # and one of the buffers that this thread asks a runtime for meanwhile (parts/repeat.py)
 
 
 notes = _Notes()

@@ -106,12 +106,11 @@ class Decoder:
         """Run a layer and note its calls: (what it leaves for the next norm, the note or None where it cannot be repeated)."""
         block.mixer.position.tables(ctx)   # (made once a step: not among the calls)
         rep = Repeat(key, block, cache, pending)
-        rep.calls, ctx.rt.held = [], rep.held
-        L.notes.calls = rep.calls
+        L.notes.calls, L.notes.held = rep.calls, rep.held
         try:
             pending = block.forward(ctx, x, pending, cache)
         finally:
-            L.notes.calls, ctx.rt.held = None, None
+            L.notes.calls = L.notes.held = None
         return pending, rep if rep.close(pending) else None
 
     def forward(self, ctx) -> Optional[torch.Tensor]:

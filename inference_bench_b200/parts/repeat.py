@@ -22,10 +22,10 @@ class Repeat:
     """The noted layer of a step. `run` repeats it for a layer with an equal key."""
 
     def __init__(self, key, block, cache, pending):
-        self.key, self.weights, self.view, self.row0 = key, block.repeat_weights(), cache.c_view(), cache.tma()[1]
+        self.key, self.weights, self.view = key, block.repeat_weights(), cache.c_view()
         self.pending_in, self.pending = pending, None
         self.held: list = []        # the layer's buffers
-        self.calls: Optional[list] = None
+        self.calls: list = []       # (name, arguments)
         self.plan: Optional[list] = None
 
     def close(self, pending) -> bool:

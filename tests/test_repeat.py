@@ -21,3 +21,45 @@ def test_a_layer_is_repeated_behind_one_that_left_the_same_kind(before, after, a
     block = SimpleNamespace(repeat_weights=lambda: [1, 2])
     cache = SimpleNamespace(c_view=lambda: None, tma=lambda: (None, 0))
     assert Repeat("key", block, cache, before).close(after) is alike
+
+
+def test_two_threads_note_their_own_layers(monkeypatch):
+    """On one runtime, one thread's layer ends while another's is being noted: each keeps its own calls and buffers until its layers are repeated."""
+    import threading
+
+    from inference_bench_b200.engine.runtime import Runtime
+    from inference_bench_b200.kernels import lib
+    from inference_bench_b200.parts.decoder import Decoder
+    rt = SimpleNamespace(act_dtype=torch.float32, device="cpu")
+    rt.empty = lambda shape: Runtime.empty(rt, shape)
+    monkeypatch.setitem(lib._entry, "first", (lambda n: 0, 0))
+    monkeypatch.setitem(lib._entry, "second", (lambda n: 0, 0))
+    inside, other_done, reps = threading.Event(), threading.Event(), {}
+
+    def layer(name, between):
+        def forward(ctx, x, pending, cache):
+            first = rt.empty((n,))
+            lib.call(name, n)
+            between()
+            made[name] = [first, rt.empty((n,))]
+            lib.call(name, n + 1)
+            return T
+        n = len(name)
+        block = SimpleNamespace(repeat_weights=lambda: [1, 2], forward=forward, mixer=SimpleNamespace(position=SimpleNamespace(tables=lambda ctx: None)))
+        cache = SimpleNamespace(c_view=lambda: None, tma=lambda: (None, 0))
+        reps[name] = Decoder._noted(SimpleNamespace(rt=rt), block, None, T, cache, "key")[1]
+
+    made = {}
+
+    def other():
+        inside.wait(10)
+        layer("second", lambda: None)
+        other_done.set()
+
+    t = threading.Thread(target=other)
+    t.start()
+    layer("first", lambda: (inside.set(), other_done.wait(10)))
+    t.join()
+    for name in ("first", "second"):
+        assert reps[name].calls == [(name, (len(name),)), (name, (len(name) + 1,))]
+        assert [id(b) for b in reps[name].held] == [id(b) for b in made[name]]
