@@ -419,16 +419,16 @@ DESIGN_SIZES = {
     "lite": dict(width=2048, heads=16, dim=128, rot=64, vdim=128, rank=512, dense_ff=10944, experts=64, top=6, expert_ff=1408, shared_ff=2816, groups=(8, 4), vocab=32768),
 }
 DESIGN_KINDS = {   # kinds of kernel by the library entry points that launch them
-    "zabonex": {"attention": ["ib_latent_attention", "ib_latent_attention_mma"], "experts": ["ib_gemm_grouped", "ib_gemm_grouped_mma", "ib_gemm_grouped_tcgen05", "ib_gemm_grouped_swiglu_tcgen05", "ib_gemm_grouped_2cta", "ib_gemm_grouped_swiglu_2cta", "ib_gather_rows"],
+    "zabonex": {"attention": ["ib_latent_attention", "ib_latent_attention_mma", "ib_latent_gather", "ib_gemm_bf16_2cta", "ib_latent_prefill"], "experts": ["ib_gemm_grouped", "ib_gemm_grouped_mma", "ib_gemm_grouped_tcgen05", "ib_gemm_grouped_swiglu_tcgen05", "ib_gemm_grouped_2cta", "ib_gemm_grouped_swiglu_2cta", "ib_gather_rows"],
                 "heads": ["ib_gemm_heads", "ib_gemm_heads_mma"], "route": ["ib_moe_route", "ib_moe_sort", "ib_moe_route_sort", "ib_moe_combine"],
                 "norm": ["ib_norm_residual", "ib_latent_prepare", "ib_cast_rows"], "gemm": LEAVE_OUT["gemm"]},
     "qwen3": {"attention": LEAVE_OUT["attention"], "norm": LEAVE_OUT["norm"] + LEAVE_OUT["qk"], "gemm": LEAVE_OUT["gemm"] + LEAVE_OUT["qkv"]},
-    "busadra": {"attention": ["ib_attention_generic", "ib_attention_decode_capped", "ib_attention_decode_stream_capped", "ib_attention_prefill_ws_capped"],
+    "busadra": {"attention": ["ib_attention_generic", "ib_attention_prompt_f32", "ib_attention_decode_capped", "ib_attention_decode_stream_capped", "ib_attention_prefill_ws_capped"],
                 "recurrence": ["ib_gated_recurrence", "ib_recurrence_chunks_finish", "ib_head_rmsnorm"],
                 "experts": ["ib_gemm_grouped", "ib_gemm_grouped_mma", "ib_gemm_grouped_tcgen05", "ib_gemm_grouped_swiglu_tcgen05", "ib_gemm_grouped_2cta", "ib_gemm_grouped_swiglu_2cta", "ib_scatter_scaled_rows"],
                 "route": ["ib_moe_route", "ib_moe_sort", "ib_moe_route_sort", "ib_moe_combine"],
                 "norm": ["ib_add_layernorm", "ib_causal_conv_rows", "ib_add_layernorm_conv_single", "ib_depth_average", "ib_qk_norm_rope_kv"], "gemm": LEAVE_OUT["gemm"]},
-    "lulenex": {"attention": ["ib_attention_generic", "ib_attention_decode_capped", "ib_attention_decode_stream_capped", "ib_attention_prefill_ws_capped"],
+    "lulenex": {"attention": ["ib_attention_generic", "ib_attention_prompt_f32", "ib_attention_decode_capped", "ib_attention_decode_stream_capped", "ib_attention_prefill_ws_capped"],
                 "recurrence": ["ib_gated_recurrence", "ib_recurrence_chunks_finish", "ib_gated_rmsnorm"],
                 "scan": ["ib_conv_silu", "ib_selective_scan"],
                 "norm": ["ib_add_rmsnorm", "ib_add_rmsnorm_ext", "ib_token_shift_rows", "ib_qk_norm_rope_kv", "ib_loop_pack", "ib_xielu_rows", "ib_add_bias_rows"],
@@ -441,7 +441,7 @@ DITALORN_SIZES = {
     "lite": dict(DESIGN_SIZES["lite"], q_rank=768, window=1024, att_heads=16, att_kv_heads=4, att_dim=128, att_vdim=128, conv=4),
 }
 DESIGN_KINDS["ditalorn"] = {
-    "attention": ["ib_latent_attention", "ib_latent_attention_mma"], "sigmoid": ["ib_sigmoid_attention", "ib_sigmoid_attention_mma"],
+    "attention": ["ib_latent_attention", "ib_latent_attention_mma", "ib_latent_gather", "ib_gemm_bf16_2cta", "ib_latent_prefill"], "sigmoid": ["ib_sigmoid_attention", "ib_sigmoid_attention_mma"],
     "experts": ["ib_gemm_grouped", "ib_gemm_grouped_mma", "ib_gemm_grouped_tcgen05", "ib_gemm_grouped_swiglu_tcgen05", "ib_gemm_grouped_2cta", "ib_gemm_grouped_swiglu_2cta", "ib_gather_rows"],
     "heads": ["ib_gemm_heads", "ib_gemm_heads_mma"], "route": ["ib_moe_route", "ib_moe_sort", "ib_moe_route_sort", "ib_moe_combine"],
     "norm": ["ib_add_rmsnorm", "ib_post_norm", "ib_latent_down", "ib_latent_prepare", "ib_qkv_conv", "ib_embed_pos"], "gemm": LEAVE_OUT["gemm"]}
@@ -471,9 +471,8 @@ def ditalorn_work(z: dict, layers: int, T: int, ctx: int, batch: int) -> tuple:
     norm_row = layers * W * (4.0 * 4 + 2 + 4 + 4 + 2) + n_lat * (4.0 * (z["q_rank"] + r) + 2 * (z["q_rank"] + r) + 6.0 * H * z["dim"]) + n_att * R * (4.0 * z["conv"] + 2)
     lin = n_lat * ((z["q_rank"] + r + H) * W + H * z["dim"] * z["q_rank"] + H * z["vdim"] * W) + n_att * (R * W + AH * AV * W) + layers * z["experts"] * W + z["vocab"] * W
     work = {
-        "prefill": {"attention": {"flops": n_lat * 4.0 * H * pairs_w * r}, "sigmoid": {"flops": n_att * 2.0 * AH * pairs * (AD + AV)},
-                    "experts": {"flops": layers * 2.0 * T * z["top"] * 3 * z["expert_ff"] * W},
-                    "heads": {"flops": n_lat * 2.0 * T * H * r * (z["dim"] + z["vdim"])}, "norm": {"flops": 0.0, "bytes": T * norm_row}},
+        "prefill": {"attention": {"flops": n_lat * 2.0 * H * (T * r + pairs_w) * (z["dim"] + z["vdim"])}, "sigmoid": {"flops": n_att * 2.0 * AH * pairs * (AD + AV)},
+                    "experts": {"flops": layers * 2.0 * T * z["top"] * 3 * z["expert_ff"] * W}, "norm": {"flops": 0.0, "bytes": T * norm_row}},
         "decode": {"attention": {"flops": n_lat * 4.0 * H * batch * seen * r, "bytes": n_lat * 2.0 * batch * seen * r},
                    "sigmoid": {"flops": n_att * 2.0 * AH * batch * ctx * (AD + AV), "bytes": n_att * 2.0 * batch * ctx * AG * (AD + AV)},
                    "experts": {"flops": layers * 2.0 * batch * z["top"] * 3 * z["expert_ff"] * W, "bytes": layers * 2.0 * min(batch * z["top"], z["experts"]) * 3 * z["expert_ff"] * W},
@@ -613,7 +612,7 @@ FEDIPEL_SIZES = {
     "mid": dict(BUSADRA_SIZES["mid"], att_heads=16, att_kv_heads=4, map_dim=64, att_vdim=128, keep=4, wkv_heads=32, wkv_dim=64, decay_rank=64, shared_ff=2816),
 }
 DESIGN_KINDS["fedipel"] = {
-    "attention": ["ib_attention_generic", "ib_attention_decode_capped", "ib_attention_decode_stream_capped", "ib_attention_prefill_ws_capped"],
+    "attention": ["ib_attention_generic", "ib_attention_prompt_f32", "ib_attention_decode_capped", "ib_attention_decode_stream_capped", "ib_attention_prefill_ws_capped"],
     "recurrence": ["ib_recurrence_parts", "ib_recurrence_chunks_finish", "ib_head_norm_gate"],
     "experts": ["ib_gemm_grouped", "ib_gemm_grouped_mma", "ib_gemm_grouped_tcgen05", "ib_gemm_grouped_relu2_tcgen05", "ib_gemm_grouped_2cta", "ib_gather_rows"],
     "route": ["ib_moe_route", "ib_moe_sort", "ib_moe_route_sort", "ib_moe_combine"],
@@ -670,8 +669,8 @@ GOKOSUN_SIZES = {name: dict(FEDIPEL_SIZES[name], att_dim=128, lat_heads=d["heads
                             dense_ff=FEDIPEL_SIZES[name]["top"] * FEDIPEL_SIZES[name]["expert_ff"] + FEDIPEL_SIZES[name]["shared_ff"], ditalorn=d)
                  for name, d in (("small", DITALORN_SIZES["small"]), ("mid", DITALORN_SIZES["lite"]))}
 DESIGN_KINDS["gokosun"] = {
-    "attention": ["ib_attention_generic", "ib_attention_decode", "ib_attention_decode_stream", "ib_attention_prefill_ws", "ib_attention_prefill_tc"],
-    "latent": ["ib_latent_attention", "ib_latent_attention_mma"], "heads": ["ib_gemm_heads", "ib_gemm_heads_mma"],
+    "attention": ["ib_attention_generic", "ib_attention_prompt_f32", "ib_attention_decode", "ib_attention_decode_stream", "ib_attention_prefill_ws", "ib_attention_prefill_tc"],
+    "latent": ["ib_latent_attention", "ib_latent_attention_mma", "ib_latent_gather", "ib_gemm_bf16_2cta", "ib_latent_prefill"], "heads": ["ib_gemm_heads", "ib_gemm_heads_mma"],
     "recurrence": ["ib_memory_gates", "ib_memory_walk", "ib_recurrence_chunks_finish", "ib_memory_out"],
     "experts": ["ib_gemm_grouped", "ib_gemm_grouped_mma", "ib_gemm_grouped_tcgen05", "ib_gemm_grouped_swiglu_tcgen05", "ib_gemm_grouped_2cta", "ib_gemm_grouped_swiglu_2cta", "ib_gather_rows"],
     "route": ["ib_moe_route", "ib_moe_sort", "ib_moe_route_sort", "ib_moe_combine"],
@@ -707,8 +706,8 @@ def gokosun_work(z: dict, layers: int, T: int, ctx: int, batch: int) -> tuple:
         n_lat * ((Q + K + LR) * W + LH * (LD + LR) * Q + LH * LV * W) + n_moe * (E + 3 * S) * W + n_dense * 3 * z["dense_ff"] * W + z["vocab"] * W
     used = min(batch * top, E)
     work = {
-        "prefill": {"attention": {"flops": n_att * 2.0 * H * (D + V) * pairs}, "latent": {"flops": n_lat * 2.0 * LH * pairs * (2 * K + LR)},
-                    "heads": {"flops": n_lat * 2.0 * T * LH * K * (LD + LV)}, "recurrence": {"flops": 0.0, "bytes": n_mem * T * mem_row},
+        "prefill": {"attention": {"flops": n_att * 2.0 * H * (D + V) * pairs}, "latent": {"flops": n_lat * 2.0 * LH * (T * K * (LD + LV) + pairs * (LD + LR + LV))},
+                    "recurrence": {"flops": 0.0, "bytes": n_mem * T * mem_row},
                     "experts": {"flops": n_moe * 2.0 * T * top * 3 * F * W}, "norm": {"flops": 0.0, "bytes": T * norm_row}},
         # (up to 64 tokens the shared expert's products run among the experts')
         "decode": {"attention": {"flops": n_att * 2.0 * H * (D + V) * batch * ctx, "bytes": n_att * 2.0 * batch * ctx * G * (D + V)},
@@ -776,9 +775,9 @@ def design_work(z: dict, layers: int, T: int, ctx: int, batch: int) -> dict:
     moe_layers = layers - 1
     pairs = T * (T + 1) / 2
     return {
-        "prefill": {"attention": {"flops": layers * 2.0 * H * pairs * (D + r)},
-                    "experts": {"flops": moe_layers * 2.0 * T * z["top"] * 3 * z["expert_ff"] * z["width"]},
-                    "heads": {"flops": layers * 2.0 * T * H * r * (z["dim"] + z["vdim"])}},
+        # (a portion's attention makes every head's keys and values first; a decoded token's queries go to the latents through the heads' maps)
+        "prefill": {"attention": {"flops": layers * 2.0 * H * (T * r * (z["dim"] + z["vdim"]) + pairs * (z["dim"] + z["rot"] + z["vdim"]))},
+                    "experts": {"flops": moe_layers * 2.0 * T * z["top"] * 3 * z["expert_ff"] * z["width"]}},
         "decode": {"attention": {"flops": layers * 2.0 * H * batch * ctx * (D + r), "bytes": layers * 2.0 * batch * ctx * D},
                    "experts": {"flops": moe_layers * 2.0 * batch * z["top"] * 3 * z["expert_ff"] * z["width"],
                                "bytes": moe_layers * 2.0 * min(batch * z["top"], z["experts"]) * 3 * z["expert_ff"] * z["width"]},
