@@ -11,9 +11,9 @@
 //   latent_prefill_kernel   a CTA per 128 query rows of one head: the roles of attention_prefill_ws.cu (four softmax warps, a warp that issues
 //                           the MMAs one score tile ahead, a warp each for the key and value tiles), with a query of dim + rot values
 // Bound by the softmax warps' chain from a score tile to the next (two CTAs an SM fill each other's gaps), then by the scores' operand reads.
-// Which segments of a step come here is decided in parts/latent.py. Measured, 16 heads of 128 + 64 on a latent of 512: 2,048 tokens 8 + 19 + 47 us (gather, product, attention) where the maps to the latents'
-// space and attention there took 70 + 666; 333 tokens of three requests behind 116 to 583 cached positions 8 + 19 + 25 against 31 + 80; 64
-// tokens behind 900 8 + 15 + 25 against 21 + 92; 32 tokens alone 9 + 13 + 11 against 19 + 17.
+// Which segments of a step come here is decided in parts/latent.py. Measured, 16 heads of 128 + 64 on a latent of 512: 2,048 tokens 8 + 19 + 47 us
+// (gather, product, attention) where the maps to the latents' space and attention there took 70 + 666; 333 tokens of three requests behind 116 to
+// 583 cached positions 8 + 19 + 25 against 31 + 80; 64 tokens behind 900 8 + 15 + 25 against 21 + 92; 32 tokens alone 9 + 13 + 11 against 19 + 17.
 #include <cuda.h>
 
 #include <type_traits>
