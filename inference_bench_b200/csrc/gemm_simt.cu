@@ -11,7 +11,8 @@
 // for FMAs on two registers, 49 on three), and too few threads where it is not: one chain an output left a product of 777 x 1,024 x 2,048 with
 // three warps an SM. Hence four groups of 64 threads a tile, each with its own chain; their sums meet in shared memory at the end. A thread
 // holds TM x TN outputs and reads four k's of a row in one 16-byte access (rows are 68 values apart, so eight neighbouring rows meet every
-// bank once); three stages of 64 k's arrive by cp.async.
+// bank once); three stages of 64 k's arrive by cp.async. 16 x 64 and smaller tiles are bound by the shared-memory reads (16 bytes a lane, 4 cycles
+// of the SM's port a warp), larger ones by how the FMAs' operands leave the registers.
 #include "common.cuh"
 
 namespace {
@@ -160,21 +161,54 @@ int run(const X* x, const W* w, float* out, int T, int N, int K, cudaStream_t st
   return 0;
 }
 
-// The larger the tile, the fewer shared-memory reads an FMA costs, and the fewer CTAs share the work. Measured (us, tiles of 64 x 64 | 32 x 64 |
-// 32 x 32; the form before, one chain an output on 64 x 64 tiles of 4 x 4, took 3,058, 498, 414, 208 and 155): 2,048 x 4,096 x 4,096 rows, columns
-// and k's 1,679 | 1,816 | 2,030 (41 TFLOP/s); 777 x 6,144 x 1,024 280 | 293 | 316; 777 x 1,024 x 2,048 123 | 108 | 113; 300 x 1,024 x 2,048
-// 63 | 69 | 61; 96 x 4,096 x 1,024 34 | 37 | 32. Hence 64 x 64 from four CTAs an SM on, 32 x 64 from two, 32 x 32 from one, 16 x 16 below. Up to
-// 16 rows a tile has 16, and as many columns as leave every SM a CTA (2 x 32,768 x 1,024: 50 us against 230; 8 x 1,024 x 3,072: 26 against 236).
+// The larger the tile, the fewer shared-memory reads an FMA costs, and the worse its CTAs fill the SMs: a tile's last round of CTAs takes as long as
+// a full one. So the form is the one with the least of rounds x (a tile's FMAs / the rate of a full SM) over the sizes; the rates, in FMAs an
+// SM and us, are those of 2,048 x 4,096 x 4,096 rows, columns and k's (64 x 128: 1,565 us, 44 TFLOP/s; 64 x 64: 1,683; 32 x 64: 1,819; 32 x 32:
+// 2,034), with which a product of 40 to 777 rows takes 7 to 12 us more than said here, whatever the tile. Measured (us, the tile by a count of
+// CTAs alone before | now): 777 x 1,024 x 2,048 113 | 94 (143 tiles of 64 x 96 where 64 x 64 makes 208); 777 x 1,024 x 3,072 166 | 137;
+// 777 x 6,144 x 1,024 288 | 257; 777 x 4,096 x 1,024 195 | 180; 300 x 1,024 x 2,048 68 | 57; 100 x 6,144 x 1,024 61 | 47. (Two-wide FMAs, tiles stored
+// k by k, operands read a step ahead and two tiles an SM were all slower: 29 to 43 TFLOP/s at the large size; registers alone reach 66.)
+// Up to 16 rows a tile has 16, and as many columns as leave every SM a CTA (2 x 32,768 x 1,024: 50 us against 230; 8 x 1,024 x 3,072: 26 against 236).
+constexpr int SMS = 148;
+struct Form {
+  int bm, bn, per_sm;   // rows and columns of a tile, CTAs that share an SM
+  float rate;
+};
+constexpr Form FORMS[] = {{16, 16, 2, 45e3f},   {16, 64, 2, 93e3f},  {32, 32, 2, 115e3f}, {32, 64, 2, 129e3f},  {48, 64, 1, 125e3f},
+                          {64, 64, 1, 140e3f}, {40, 128, 1, 140e3f}, {48, 128, 1, 146e3f}, {56, 128, 1, 150e3f}, {64, 96, 1, 150e3f}, {64, 128, 1, 150e3f}};
+
+inline int best_form(int T, int N) {
+  int best = 0;
+  float least = 0.f;
+  for (int i = 0; i < (int)(sizeof(FORMS) / sizeof(FORMS[0])); i++) {
+    const Form& f = FORMS[i];
+    const long long tiles = (long long)((N + f.bn - 1) / f.bn) * ((T + f.bm - 1) / f.bm);
+    const float rate = f.per_sm > 1 && tiles <= SMS ? 0.75f * f.rate : f.rate;   // (an SM with one of its two)
+    const float cost = (float)((tiles + SMS - 1) / SMS) * (float)(f.bm * f.bn) / rate;
+    if (i == 0 || cost < least) best = i, least = cost;
+  }
+  return best;
+}
+
 template <typename X, typename W>
 int go(const X* x, const W* w, float* out, int T, int N, int K, cudaStream_t stream) {
-  auto tiles = [&](int bm, int bn) { return (long long)((N + bn - 1) / bn) * ((T + bm - 1) / bm); };
-  constexpr int SMS = 148;
-  if (T <= 16 && tiles(16, 64) >= SMS) return run<X, W, 16, 64, 2, 8>(x, w, out, T, N, K, stream);
-  if (T <= 16) return run<X, W, 16, 16, 2, 2>(x, w, out, T, N, K, stream);
-  if (tiles(64, 64) >= 4 * SMS) return run<X, W, 64, 64, 8, 8, 1>(x, w, out, T, N, K, stream);   // (one CTA an SM: 64 sums and 32 operands a thread do not fit 128 registers)
-  if (tiles(32, 64) >= 2 * SMS) return run<X, W, 32, 64, 4, 8>(x, w, out, T, N, K, stream);
-  if (tiles(32, 32) >= SMS) return run<X, W, 32, 32, 4, 4>(x, w, out, T, N, K, stream);
-  return run<X, W, 16, 16, 2, 2>(x, w, out, T, N, K, stream);
+  if (T <= 16) {
+    if ((N + 63) / 64 >= SMS) return run<X, W, 16, 64, 2, 8>(x, w, out, T, N, K, stream);
+    return run<X, W, 16, 16, 2, 2>(x, w, out, T, N, K, stream);
+  }
+  switch (best_form(T, N)) {   // (one CTA an SM: 48 and more sums and the operands of a thread do not fit 128 registers)
+    case 0: return run<X, W, 16, 16, 2, 2>(x, w, out, T, N, K, stream);
+    case 1: return run<X, W, 16, 64, 2, 8>(x, w, out, T, N, K, stream);
+    case 2: return run<X, W, 32, 32, 4, 4>(x, w, out, T, N, K, stream);
+    case 3: return run<X, W, 32, 64, 4, 8>(x, w, out, T, N, K, stream);
+    case 4: return run<X, W, 48, 64, 6, 8, 1>(x, w, out, T, N, K, stream);
+    case 5: return run<X, W, 64, 64, 8, 8, 1>(x, w, out, T, N, K, stream);
+    case 6: return run<X, W, 40, 128, 5, 16, 1>(x, w, out, T, N, K, stream);
+    case 7: return run<X, W, 48, 128, 6, 16, 1>(x, w, out, T, N, K, stream);
+    case 8: return run<X, W, 56, 128, 7, 16, 1>(x, w, out, T, N, K, stream);
+    case 9: return run<X, W, 64, 96, 8, 12, 1>(x, w, out, T, N, K, stream);
+    default: return run<X, W, 64, 128, 8, 16, 1>(x, w, out, T, N, K, stream);
+  }
 }
 
 }  // namespace

@@ -30,6 +30,14 @@ def test_product_at_tile_edges(T, N, K, x_dtype, w_dtype):
     assert torch.equal(alone[0], out[-1])
 
 
+# the tiles that only some sizes are given (csrc/gemm_simt.cu, FORMS): 16 x 64 above 16 rows, 48 x 64, 64 x 64, 40 x 128, 48 x 128, 56 x 128, 64 x 96 and
+# 64 x 128, with remainders in rows and columns and inner sizes with and without vector loads
+@pytest.mark.parametrize("T,N,K", [(33, 2563, 33), (129, 2050, 72), (193, 2050, 65), (33, 9473, 36), (513, 1540, 68), (193, 4099, 41), (41, 9473, 130), (289, 3077, 64)])
+@pytest.mark.parametrize("x_dtype,w_dtype", [(torch.float32, torch.float32), (torch.bfloat16, torch.bfloat16)])
+def test_product_at_the_edges_of_wide_tiles(T, N, K, x_dtype, w_dtype):
+    test_product_at_tile_edges(T, N, K, x_dtype, w_dtype)
+
+
 @pytest.mark.parametrize("hd,heads,kvh,page", [(128, 4, 2, 16), (64, 6, 1, 8), (128, 3, 3, 64)])
 @pytest.mark.parametrize("variant", ["plain", "window", "window_keep", "chunk", "cap_sink", "tail"])
 def test_prompt_attention_matches_the_row_kernel(status, hd, heads, kvh, page, variant):  # noqa: F811
