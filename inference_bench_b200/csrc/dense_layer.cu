@@ -1,0 +1,123 @@
+// The kernels of one dense layer (norm, q/k/v, attention, output, norm, gate/up, down) of a bfloat16 step outside a graph, launched by one call.
+//
+// Nothing here runs on the device: the call is the list of launches that the parts make one by one from Python, in the same order with the same
+// arguments. What bounds a step of a short prompt portion is the host: a part's wrapper checks its tensors, asks for an output and works out a tile in
+// about 15 us, a launch takes 3, and the kernel itself 3 to 10. The forms of the products and the buffers are worked out once a step
+// (kernels/dense.py); a layer then costs its launches. 100 tokens in two layers of the 0.6B sizes: 514 to 277 us of host a step (with the step's arrays
+// in one transfer), 61 tokens behind 900 in eight layers 883 to 445, as long as its kernels.
+#include "kv_view.cuh"
+
+extern "C" {
+int ib_add_rmsnorm(float* x, const float* delta, int P, long long delta_stride, const float* w, void* out, int out_dtype, const int* rows, int n_rows, int H, float eps, int write_x,
+                   cudaStream_t stream);
+int ib_silu_mul(const float* gu, int P, long long stride, void* act, int act_dtype, int T, int I, const float* limit, float slope, cudaStream_t stream);
+int ib_qk_norm_rope_kv(const float* qkv, int P, long long stride_p, const float* q_norm_w, const float* k_norm_w, float eps, const float* cos_t, const float* sin_t, int rot_half,
+                       const int* positions, const int* seg_of_token, void* q_out, int act_dtype, const IbKvView* kv, int write_kv, int T, int heads, unsigned* status,
+                       const float* bias, int qk_dim, int v_dim, int row, int q_col, int k_col, int v_col, int unit_norm_after, cudaStream_t stream);
+int ib_attention_prefill_ws(const void* q, const IbKvView* kv, const int* tile_seg, const int* tile_row0, int n_tiles, const int* seg_start, const int* seg_pos0, int window, float scale,
+                            void* out, int heads, const void* kv_map, long long view_row0, unsigned* status, cudaStream_t stream);
+int ib_attention_decode_stream(const void* q, const IbKvView* kv, const int* dec_tokens, int n_dec, const int* positions, const int* seg_of_token, int window, float scale, float* part_o,
+                               float* part_ml, void* out, int heads, int max_slices, int tiles_per_slice, const void* kv_map, long long view_row0, unsigned* status, cudaStream_t stream);
+int ib_gemm_tcgen05(const void* x, const void* w, float* out, int T, int N, int K, int bn, int splits, int wide, unsigned* status, cudaStream_t stream);
+int ib_gemm_swiglu_tcgen05(const void* x, const void* w, void* act, int T, int I, int K, int bn, int half, const float* limit, float slope, unsigned* status, cudaStream_t stream);
+int ib_gemm_tcgen05_2cta(const void* x, const void* w, float* out, int T, int N, int K, unsigned* status, cudaStream_t stream);
+int ib_gemm_tcgen05_2cta_add(const void* x, const void* w, float* out, int T, int N, int K, unsigned* status, cudaStream_t stream);
+int ib_gemm_swiglu_tcgen05_2cta(const void* x, const void* w, void* act, int T, int I, int K, const float* limit, float slope, unsigned* status, cudaStream_t stream);
+int ib_gemm_qkv_tcgen05_2cta(const void* x, const void* w, int T, int K, const float* q_norm_w, const float* k_norm_w, float eps, const float* cos_t, const float* sin_t,
+                             const int* positions, const int* seg_of_token, void* q_out, const IbKvView* kv, int write_kv, int heads, unsigned* status, cudaStream_t stream);
+}
+
+// How a product runs. kind 0: the single-CTA kernel, `splits` partial sums of tiles of bn tokens; 1: CTA pairs, one sum; 2: CTA pairs, added to the
+// residual stream; 3: with the epilogue that finishes it (q/k/v: norm, rotation and cache write on CTA pairs; gate/up: the activation, on CTA pairs where
+// bn is 0, else tiles of bn tokens, `wide` telling whether gate and up share an accumulator).
+struct IbDenseProduct {
+  int kind, bn, splits, wide;
+};
+
+struct IbDenseStep {   // what the layers of a step have in common
+  float* x;            // the residual stream [T, hidden]
+  void* h;             // [T, hidden]
+  float* partial;      // partial sums of any one product
+  void* q;             // [T, heads * head_dim]
+  void* o;             // the same
+  void* act;           // [T, inter]
+  float* part_o;       // decoded tokens: [n_dec, heads, max_slices, head_dim] and two numbers each
+  float* part_ml;
+  const float* cos_t;
+  const float* sin_t;
+  const int* positions;
+  const int* seg_of_token;
+  const int* seg_start;
+  const int* seg_pos0;
+  const int* dec_tokens;
+  const int* tile_seg;
+  const int* tile_row0;
+  const void* kv_map;
+  unsigned* status;
+  cudaStream_t stream;
+  IbDenseProduct qkv, out, gate_up, down;
+  int T, hidden, inter, heads, kv_heads, head_dim, rot_half, window, n_dec, n_tiles, max_slices, tiles_per_slice;
+  float norm_eps, ff_norm_eps, qk_eps, scale;
+};
+
+struct IbDenseLayer {
+  const float* norm;
+  const void* w_qkv;
+  const void* w_out;
+  const float* ff_norm;
+  const void* w_gate_up;
+  const void* w_down;
+  const float* q_norm;
+  const float* k_norm;
+  const IbKvView* kv;
+  long long kv_row0;    // the view's first row in the pool's tensor map
+  const float* delta;   // what the layer before left to add: delta_parts sums of [T, hidden], or null
+  int delta_parts;
+};
+
+// Returns the number of kernels launched, or -1 with the error's text set.
+extern "C" int ib_dense_layer(const IbDenseStep* s, const IbDenseLayer* l) {
+  const int T = s->T, H = s->hidden, Q = s->heads * s->head_dim, R = Q + 2 * s->kv_heads * s->head_dim;
+  if (T <= 0 || (s->n_dec > 0 && !s->part_o) || s->n_dec + s->n_tiles <= 0) {
+    ib_set_error("dense_layer: bad sizes T=%d n_dec=%d n_tiles=%d", T, s->n_dec, s->n_tiles);
+    return -1;
+  }
+  int n = 0;
+  bool bad = false;
+  auto run = [&](int code, int kernels = 1) { bad = bad || code != 0, n += kernels; };
+  auto product = [&](const IbDenseProduct& p, const void* in, const void* w, int N, int K) {
+    if (p.kind == 2) run(ib_gemm_tcgen05_2cta_add(in, w, s->x, T, N, K, s->status, s->stream));
+    else if (p.kind == 1) run(ib_gemm_tcgen05_2cta(in, w, s->partial, T, N, K, s->status, s->stream));
+    else run(ib_gemm_tcgen05(in, w, s->partial, T, N, K, p.bn, p.splits, p.wide, s->status, s->stream));
+  };
+  auto norm = [&](const float* delta, int parts, const float* w, float eps) {
+    run(ib_add_rmsnorm(s->x, delta, delta ? parts : 0, delta ? (long long)T * H : 0, w, s->h, IB_BF16, nullptr, T, H, eps, 1, s->stream));
+  };
+  norm(l->delta, l->delta_parts, l->norm, s->norm_eps);
+  if (s->qkv.kind == 3) {
+    run(ib_gemm_qkv_tcgen05_2cta(s->h, l->w_qkv, T, H, l->q_norm, l->k_norm, s->qk_eps, s->cos_t, s->sin_t, s->positions, s->seg_of_token, s->q, l->kv, 1, s->heads, s->status, s->stream));
+  } else {
+    product(s->qkv, s->h, l->w_qkv, R, H);
+    run(ib_qk_norm_rope_kv(s->partial, s->qkv.kind == 1 ? 1 : s->qkv.splits, (long long)T * R, l->q_norm, l->k_norm, s->qk_eps, s->cos_t, s->sin_t, s->rot_half, s->positions,
+                           s->seg_of_token, s->q, IB_BF16, l->kv, 1, T, s->heads, s->status, nullptr, s->head_dim, s->head_dim, 0, 0, 0, 0, 0, s->stream));
+  }
+  if (s->n_dec)
+    run(ib_attention_decode_stream(s->q, l->kv, s->dec_tokens, s->n_dec, s->positions, s->seg_of_token, s->window, s->scale, s->part_o, s->part_ml, s->o, s->heads, s->max_slices,
+                                   s->tiles_per_slice, s->kv_map, l->kv_row0, s->status, s->stream), 2);
+  if (s->n_tiles)
+    run(ib_attention_prefill_ws(s->q, l->kv, s->tile_seg, s->tile_row0, s->n_tiles, s->seg_start, s->seg_pos0, s->window, s->scale, s->o, s->heads, s->kv_map, l->kv_row0, s->status,
+                                s->stream));
+  product(s->out, s->o, l->w_out, H, Q);
+  norm(s->out.kind == 2 ? nullptr : s->partial, s->out.kind == 1 ? 1 : s->out.splits, l->ff_norm, s->ff_norm_eps);
+  const IbDenseProduct& g = s->gate_up;
+  if (g.kind == 3 && g.bn == 0) {
+    run(ib_gemm_swiglu_tcgen05_2cta(s->h, l->w_gate_up, s->act, T, s->inter, H, nullptr, 0.f, s->status, s->stream));
+  } else if (g.kind == 3) {
+    run(ib_gemm_swiglu_tcgen05(s->h, l->w_gate_up, s->act, T, s->inter, H, g.bn, g.wide, nullptr, 0.f, s->status, s->stream));
+  } else {
+    product(g, s->h, l->w_gate_up, 2 * s->inter, H);
+    run(ib_silu_mul(s->partial, g.kind == 1 ? 1 : g.splits, (long long)T * 2 * s->inter, s->act, IB_BF16, T, s->inter, nullptr, 0.f, s->stream));
+  }
+  product(s->down, s->act, l->w_down, H, s->inter);
+  return bad ? -1 : n;
+}

@@ -15,6 +15,7 @@ from typing import Any, Optional, Sequence
 import numpy as np
 import torch
 
+from ..kernels import attention
 from .runtime import Runtime
 
 
@@ -52,6 +53,8 @@ class StepContext:
     caches: list = field(default_factory=list)
     # parts may keep per-step results here (e.g. rotation tables shared by all layers)
     memo: dict = field(default_factory=dict)
+    # the step's block tables on the device, where `build_context` was given them
+    tables: list = field(default_factory=list)
     # True when the step is being captured into (or replayed from) a CUDA graph: launch shapes must
     # then depend on the batch's sizes only, never on the host copies of positions or tables
     fixed_shape: bool = False
@@ -68,44 +71,54 @@ class StepContext:
         return int((self.h_seg_start[1:] - self.h_seg_start[:-1]).max()) if self.segments else 0
 
 
-def build_context(rt: Runtime, segments: list[Segment], caches: Optional[list] = None) -> StepContext:
-    """Flatten segments into the arrays of a step and copy them to the device in one transfer."""
+def build_context(rt: Runtime, segments: list[Segment], caches: Optional[list] = None, tables: Optional[list] = None) -> StepContext:
+    """Flatten segments into the arrays of a step and copy them to the device in one transfer. tables: the step's block tables (int32 [segments, width]
+    each), for a caller that makes the caches' views from them (`StepContext.tables`): they and the attention kernels' work lists travel along."""
     S = len(segments)
     lens = [len(s.tokens) for s in segments]
-    T = int(sum(lens))
-    seg_start = np.zeros(S + 1, dtype=np.int32)
-    np.cumsum(lens, out=seg_start[1:])
-    token_ids = np.empty(T, dtype=np.int32)
-    positions = np.empty(T, dtype=np.int32)
-    seg_of_token = np.empty(T, dtype=np.int32)
-    rows: list[int] = []
-    for i, s in enumerate(segments):
-        a, b = int(seg_start[i]), int(seg_start[i + 1])
-        token_ids[a:b] = np.asarray(s.tokens, dtype=np.int64)
-        positions[a:b] = np.arange(s.pos0, s.pos0 + (b - a), dtype=np.int32)
-        seg_of_token[a:b] = i
+    starts, T, rows = [0], 0, []
+    for s, n in zip(segments, lens):
         for w in s.want:
-            if not 0 <= w < b - a:
-                raise ValueError(f"request {s.request!r}: wanted place {w} is outside its {b - a} tokens of this step")
-            rows.append(a + int(w))
-    seg_pos0 = np.asarray([s.pos0 for s in segments], dtype=np.int32)
-    seg_slot = np.asarray([s.slot for s in segments], dtype=np.int32)
-    logit_rows = np.asarray(rows, dtype=np.int32)
-    # one pinned staging buffer, one copy
-    parts = [token_ids, positions, seg_of_token, seg_start, seg_pos0, seg_slot, logit_rows]
-    sizes = [p.size for p in parts]
-    total = int(sum(sizes))
-    staging = torch.empty(max(total, 1), dtype=torch.int32).pin_memory()
+            if not 0 <= w < n:
+                raise ValueError(f"request {s.request!r}: wanted place {w} is outside its {n} tokens of this step")
+            rows.append(T + int(w))
+        T += n
+        starts.append(T)
+    dec, longest, tile_seg, tile_row0 = attention.work_lists(lens, starts, [s.pos0 for s in segments]) if tables else ([], None, [], [])
+    # one pinned staging buffer, one copy; the host's arrays are the buffer's parts
+    sizes = [T, T, T, S + 1, S, S, len(rows), len(dec), len(tile_seg), len(tile_seg)]
+    total = sum(sizes)
+    sizes.append(-total % 4)   # (tables start on 16 bytes)
+    for t in tables or ():
+        sizes += [t.size, -t.size % 4]
+    staging = torch.empty(max(sum(sizes), 1), dtype=torch.int32, pin_memory=True)
     flat = staging.numpy()
-    o = 0
-    for p, n in zip(parts, sizes):
-        flat[o:o + n] = p
-        o += n
+    token_ids, positions, seg_of_token = flat[:T], flat[T:2 * T], flat[2 * T:3 * T]
+    o = 3 * T
+    seg_start, seg_pos0, seg_slot = flat[o:o + S + 1], flat[o + S + 1:o + 2 * S + 1], flat[o + 2 * S + 1:o + 3 * S + 1]
+    o += 3 * S + 1
+    logit_rows = flat[o:o + len(rows)]
+    flat[o:total] = rows + dec + tile_seg + tile_row0
+    seg_start[:], seg_pos0[:], seg_slot[:] = starts, [s.pos0 for s in segments], [s.slot for s in segments]
+    for s, a, n in zip(segments, starts, lens):
+        if n == 1:
+            token_ids[a] = s.tokens[0]
+        elif n:
+            token_ids[a:a + n] = s.tokens
+    if S == 1:
+        seg_of_token[:] = 0
+        positions[:] = np.arange(segments[0].pos0, segments[0].pos0 + T, dtype=np.int32)
+    elif T:
+        seg_of_token[:] = np.repeat(np.arange(S, dtype=np.int32), lens)
+        np.add(np.repeat(seg_pos0 - seg_start[:-1], lens), np.arange(T, dtype=np.int32), out=positions)
+    o = total + sizes[10]
+    for t in tables or ():
+        flat[o:o + t.size] = t.reshape(-1)
+        o += t.size + -t.size % 4
     dev = staging.to(rt.device, non_blocking=True)
-    views = []
-    o = 0
-    for n in sizes:
-        views.append(dev[o:o + n])
-        o += n
-    return StepContext(rt, segments, T, token_ids, positions, seg_of_token, seg_start, seg_pos0, seg_slot, logit_rows,
-                       *views, caches=caches or [])
+    views = dev[:sum(sizes)].split(sizes)
+    ctx = StepContext(rt, segments, T, token_ids, positions, seg_of_token, seg_start, seg_pos0, seg_slot, logit_rows, *views[:7], caches=caches or [])
+    if tables:
+        ctx.tables = [views[11 + 2 * i].view(t.shape) for i, t in enumerate(tables)]
+        ctx.memo[attention.WORK_KEY] = attention.device_work(views[7], views[8], views[9], longest)
+    return ctx

@@ -113,7 +113,7 @@ class _DecodeGraph:
             self.graph.replay()
         self.h_history.copy_(self.history, non_blocking=True)
         self.h_out.copy_(self.result, non_blocking=True)
-        torch.cuda.current_stream().synchronize()
+        torch.cuda.current_stream(self.runner.rt.device).synchronize()
         self.runner.rt.raise_for(int(self.h_out[self.rows]))
         return self.h_history[:steps, :len(entries)].tolist()
 
@@ -124,7 +124,7 @@ class _DecodeGraph:
         self.dev.copy_(self.host, non_blocking=True)
         self.graph.replay()
         self.h_out.copy_(self.result, non_blocking=True)
-        torch.cuda.current_stream().synchronize()
+        torch.cuda.current_stream(self.runner.rt.device).synchronize()
         self.runner.rt.raise_for(int(self.h_out[self.rows]))
         return self.h_out[:n].tolist()
 

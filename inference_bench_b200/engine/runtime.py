@@ -14,8 +14,8 @@ from typing import Optional
 import torch
 
 from ..config.runtime_options import RuntimeOptions
+from ..kernels import gemm_tcgen05, ops
 from ..kernels import lib as L
-from ..kernels import ops
 
 MODES = {"float32": torch.float32, "fp32": torch.float32, "bfloat16": torch.bfloat16, "bf16": torch.bfloat16}
 
@@ -116,7 +116,6 @@ class Runtime:
             raise L.KernelError(f"linear: x has {x.shape[1]} columns, the matrix has {lw.k}")
         use_tc = self.mode == "bfloat16" and self.gemm != "simt"
         if use_tc:
-            from ..kernels import gemm_tcgen05
             if gemm_tcgen05.supports(lw.k):
                 return gemm_tcgen05.linear(self, x, lw, allow_split, add_to)
             if self.gemm == "tcgen05":
@@ -131,7 +130,6 @@ class Runtime:
         whose epilogue applies the activation; otherwise the product and the SiLU-mul kernel."""
         T, inter = x.shape[0], lw.n // 2
         if self.mode == "bfloat16" and self.gemm != "simt":
-            from ..kernels import gemm_tcgen05
             if self.options.swiglu_epilogue and gemm_tcgen05.swiglu_supported(T, lw.k, inter):
                 act = self.empty((T, inter))
                 gemm_tcgen05.gemm_swiglu(x, lw.weight, act, self.status, pair_min_tokens=self.options.pair_min_tokens, clamp=clamp)
@@ -148,7 +146,6 @@ class Runtime:
         otherwise the product and the row-wise kernel that adds the partial sums."""
         T = x.shape[0]
         if self.mode == "bfloat16" and self.gemm != "simt" and self.options.swiglu_epilogue:
-            from ..kernels import gemm_tcgen05
             if gemm_tcgen05.act_in_epilogue(T, lw.n, lw.k, self.sm_count):
                 act = self.empty((T, lw.n))
                 gemm_tcgen05.gemm_act(self, x, lw, kind, act, pq)

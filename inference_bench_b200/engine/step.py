@@ -44,33 +44,38 @@ class ModelRunner:
         if not entries:
             return None
         self.rt.activate()
-        seen = set()
+        reqs, tokens, vocab = [e.request for e in entries], [], self.vocab
+        if len(set(reqs)) != len(reqs):
+            twice = next(r for i, r in enumerate(reqs) if r in reqs[:i])
+            raise ValueError(f"request {twice!r} appears twice in one step")
         for e in entries:
-            if e.request in seen:
-                raise ValueError(f"request {e.request!r} appears twice in one step")
-            seen.add(e.request)
-            toks = np.asarray(e.tokens)
-            if toks.min() < 0 or toks.max() >= self.vocab:
-                bad = int(toks[(toks < 0) | (toks >= self.vocab)][0])
-                raise ValueError(f"request {e.request!r}: token id {bad} is outside the vocabulary of {self.vocab}")
+            if len(e.tokens) == 1:
+                toks = e.tokens
+                lo = hi = toks[0]
+            else:
+                toks = np.asarray(e.tokens)
+                lo, hi = toks.min(), toks.max()
+            if lo < 0 or hi >= vocab:
+                toks = np.asarray(toks)
+                raise ValueError(f"request {e.request!r}: token id {int(toks[(toks < 0) | (toks >= vocab)][0])} is outside the vocabulary of {vocab}")
+            tokens.append(toks)
         # pages first, all or nothing across the batch
-        done = []
+        cache, lengths, done = self.cache, [self.cache.length(r) for r in reqs], []
         try:
-            for e in entries:
-                self.cache.extend(e.request, self.cache.length(e.request) + len(e.tokens))
-                done.append(e)
+            for r, toks, at in zip(reqs, tokens, lengths):
+                cache.extend(r, at + len(toks))
+                done.append(r)
         except Exception:
-            for e in done:  # give back what this step took: shrink to the committed length
-                self.cache.shrink_to_committed(e.request)
+            for r in done:  # give back what this step took: shrink to the committed length
+                cache.shrink_to_committed(r)
             raise
-        segments = [Segment(e.request, self.cache.slot(e.request), self.cache.length(e.request), e.tokens, e.want) for e in entries]
-        tables = self.cache.step_tables([e.request for e in entries])
-        dev_tables = [torch.from_numpy(t).pin_memory().to(self.rt.device, non_blocking=True) for t in tables]
-        ctx = build_context(self.rt, segments, self.cache.views(dev_tables))
+        segments = [Segment(e.request, cache.slot(e.request), at, toks, e.want) for e, toks, at in zip(entries, tokens, lengths)]
+        ctx = build_context(self.rt, segments, tables=cache.step_tables(reqs))
+        ctx.caches = cache.views(ctx.tables)
         ctx.trace = trace
         logits = self.decoder.forward(ctx)
-        for e in entries:
-            self.cache.commit(e.request, self.cache.length(e.request) + len(e.tokens))
+        for r, toks, at in zip(reqs, tokens, lengths):
+            cache.commit(r, at + len(toks))
         if check:
             self.rt.check_status()
         return logits

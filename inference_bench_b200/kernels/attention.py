@@ -6,12 +6,13 @@ the generic kernel. All of them read keys and values through the block table and
 from __future__ import annotations
 
 import ctypes as C
+import operator
 from typing import Optional
 
-import numpy as np
 import torch
 
 from . import lib as L
+from . import gemm_tcgen05 as G
 from . import ops
 
 def decode_tile() -> int:
@@ -72,30 +73,42 @@ def has_tensor_core_kernel(dtype: torch.dtype, head_dim: int, heads: int, kv_hea
     return dtype == torch.bfloat16 and head_dim in (64, 128) and heads // kv_heads <= 16
 
 
+WORK_KEY = ("attention_work", QTILE)
+
+
+def work_lists(lens: list, starts: list, pos0: list) -> tuple:
+    """Of a step's segments (their tokens, first rows and first positions): the flat rows of decoded tokens and their last position or None, then segments
+    and first rows of the portions' query tiles, those with the most keys first."""
+    dec = [i for i, n in enumerate(lens) if n == 1]
+    tiles = [(-(p + min(r + QTILE, n)), i, r) for i, (n, p) in enumerate(zip(lens, pos0)) if n > 1 for r in range(0, n, QTILE)]
+    tiles.sort(key=_first)
+    return [starts[i] for i in dec], max((pos0[i] for i in dec), default=None), [t[1] for t in tiles], [t[2] for t in tiles]
+
+
+_first = operator.itemgetter(0)
+
+
+def device_work(dec: Optional[torch.Tensor], tile_seg: Optional[torch.Tensor], tile_row0: Optional[torch.Tensor], max_pos: Optional[int]) -> dict:
+    nd, nt = dec.shape[0], tile_seg.shape[0]
+    return dict(dec_tokens=dec if nd else None, n_dec=nd, tile_seg=tile_seg if nt else None, tile_row0=tile_row0 if nt else None, n_tiles=nt, max_pos=max_pos)
+
+
 def _work_lists(ctx):
-    """Per step, shared by all layers: flat rows of decoded tokens, and 64-row query tiles of portions."""
-    qtile = QTILE
-    key = ("attention_work", qtile)
-    if key in ctx.memo:
-        return ctx.memo[key]
+    """Per step, shared by all layers: flat rows of decoded tokens, and 128-row query tiles of portions."""
+    work = ctx.memo.get(WORK_KEY)
+    if work is not None:
+        return work
     if ctx.fixed_shape:
         work = dict(dec_tokens=ctx.seg_start[:ctx.n_tokens], n_dec=ctx.n_tokens, tile_seg=None, tile_row0=None, n_tiles=0, max_pos=None)
     else:
-        lens = np.diff(ctx.h_seg_start)
-        dec = ctx.h_seg_start[:-1][lens == 1].astype(np.int32)
-        tiles = []   # (last position the tile sees, segment, first row): the tiles with the most keys go first
-        for s in np.nonzero(lens > 1)[0]:
-            for r in range(0, int(lens[s]), qtile):
-                tiles.append((int(ctx.h_seg_pos0[s]) + min(r + qtile, int(lens[s])), int(s), r))
-        tiles.sort(key=lambda t: -t[0])
-        tile_seg, tile_row0 = [t[1] for t in tiles], [t[2] for t in tiles]
-        flat = np.concatenate([dec, np.asarray(tile_seg, np.int32), np.asarray(tile_row0, np.int32)]).astype(np.int32)
-        dev = torch.from_numpy(flat).pin_memory().to(ctx.rt.device, non_blocking=True) if flat.size else None
-        nd, nt = dec.size, len(tile_seg)
-        work = dict(dec_tokens=dev[:nd] if nd else None, n_dec=nd, tile_seg=dev[nd:nd + nt] if nt else None,
-                    tile_row0=dev[nd + nt:] if nt else None, n_tiles=nt,
-                    max_pos=int(ctx.h_positions[dec].max()) if nd else None)
-    ctx.memo[key] = work
+        starts = ctx.h_seg_start.tolist()
+        dec, longest, tile_seg, tile_row0 = work_lists([b - a for a, b in zip(starts, starts[1:])], starts, ctx.h_seg_pos0.tolist())
+        nd, nt = len(dec), len(tile_seg)
+        staging = torch.empty(max(nd + 2 * nt, 1), dtype=torch.int32, pin_memory=True)
+        staging.numpy()[:nd + 2 * nt] = dec + tile_seg + tile_row0
+        dev = staging.to(ctx.rt.device, non_blocking=True)
+        work = device_work(dev[:nd], dev[nd:nd + nt], dev[nd + nt:nd + 2 * nt], longest)
+    ctx.memo[WORK_KEY] = work
     return work
 
 
@@ -107,7 +120,6 @@ def project_qkv(ctx, h: torch.Tensor, lw, q_norm_w, k_norm_w, eps: float, cos, s
     rt = ctx.rt
     if rt.mode != "bfloat16" or rt.gemm == "simt" or h.dtype != torch.bfloat16:
         return None
-    from . import gemm_tcgen05 as G
     view = cache.c_view()
     if view.head_dim != 128 or view.dtype != L.BF16 or not G.supports(lw.k) or lw.n != (heads + 2 * view.kv_heads) * 128:
         return None

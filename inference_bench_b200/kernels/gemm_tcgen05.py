@@ -191,22 +191,24 @@ def gemm_qkv_pair(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, kv: "op
            positions.data_ptr(), seg_of_token.data_ptr(), q_out.data_ptr(), C.byref(view), 1 if write_kv else 0, heads, status.data_ptr(), ops._stream())
 
 
+def product_form(rt, T: int, n: int, k: int, allow_split: bool = True, add: bool = False) -> tuple:
+    """How a product of T tokens with an [n, k] matrix runs: ("single", tokens per CTA, k-splits, wide), ("pair",), or with `add` (the caller has a stream
+    it may be added to) ("add",) in the place of the latter."""
+    how = ("pair",) if T >= rt.options.pair_always_tokens else (plan(T, n, k, rt.sm_count, allow_split) if T > 128 else ("single", *choose(T, n, k, allow_split, rt.sm_count)))
+    return ("add",) if add and how[0] == "pair" else how
+
+
 def linear(rt, x: torch.Tensor, lw, allow_split: bool = True, add_to: Optional[torch.Tensor] = None) -> Optional[torch.Tensor]:
     T = x.shape[0]
-    how = ("pair",) if T >= rt.options.pair_always_tokens else (plan(T, lw.n, lw.k, rt.sm_count, allow_split) if T > 128 else None)
-    if how is not None and how[0] == "single":
-        _, bn, splits, wide = how
-        out = rt.empty((splits, T, lw.n), torch.float32)
-        gemm(x, lw.weight, out, bn, splits, rt.status, wide)
-        return out
-    if how is not None:
-        if add_to is not None:
-            gemm_pair(x, lw.weight, add_to, rt.status, add=True)
-            return None
+    how = product_form(rt, T, lw.n, lw.k, allow_split, add_to is not None)
+    if how[0] == "add":
+        gemm_pair(x, lw.weight, add_to, rt.status, add=True)
+        return None
+    if how[0] == "pair":
         out = rt.empty((1, T, lw.n), torch.float32)
         gemm_pair(x, lw.weight, out[0], rt.status)
         return out
-    bn, splits, wide = choose(T, lw.n, lw.k, allow_split, rt.sm_count)
+    _, bn, splits, wide = how
     out = rt.empty((splits, T, lw.n), torch.float32)
     gemm(x, lw.weight, out, bn, splits, rt.status, wide)
     return out
@@ -238,6 +240,16 @@ def half_swiglu(T: int, inter: int) -> bool:
     return T <= HALF_SWIGLU_MAX_TOKENS and inter % 64 == 0 and inter // 64 >= HALF_SWIGLU_MIN_CTAS
 
 
+def swiglu_form(T: int, inter: int, pair_min_tokens: int = 129) -> tuple[int, bool]:
+    """How the fused gate/up product of T tokens runs: (tokens per CTA, gate and up rows in one accumulator), or (0, False) for CTA pairs."""
+    if half_swiglu(T, inter) or (T <= 32 and inter % 64 == 0):
+        return (16 if T <= 16 else 32 if T <= 32 else 64), True
+    if T >= pair_min_tokens or (T > 32 and -(-inter // 256) >= PAIR_SWIGLU_MIN_TILES):
+        return 0, False
+    bn = 64 if T <= 64 else (128 if T <= 128 else 256)
+    return bn, bn in (16, 32)
+
+
 def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor, status: torch.Tensor, bn: int | None = None, pair_min_tokens: int = 129,
                 half: bool | None = None, clamp: Optional["ops.Clamp"] = None) -> None:
     """act [T, I] bfloat16 = silu(x gate^T) * (x up^T) (or the clamped pair) with w_gate_up [2I, K] = gate rows then up rows."""
@@ -246,15 +258,14 @@ def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor, sta
     ops._check("x", x, torch.bfloat16)
     ops._check("w_gate_up", w_gate_up, torch.bfloat16, (2 * I, K))
     ops._check("act", act, torch.bfloat16, (T, I))
-    if bn is None and (half_swiglu(T, I) or (T <= 32 and I % 64 == 0)):
-        bn, half = (16 if T <= 16 else 32 if T <= 32 else 64), True
+    if bn is None:
+        bn, own = swiglu_form(T, I, pair_min_tokens)
+        if bn == 0:
+            L.call("ib_gemm_swiglu_tcgen05_2cta", x.data_ptr(), w_gate_up.data_ptr(), act.data_ptr(), T, I, K, *ops._clamp_args(clamp), status.data_ptr(), ops._stream())
+            return
+        half = True if own else half
     if half is None:
         half = bn in (16, 32)
-    if bn is None and (T >= pair_min_tokens or (T > 32 and -(-I // 256) >= PAIR_SWIGLU_MIN_TILES)):
-        L.call("ib_gemm_swiglu_tcgen05_2cta", x.data_ptr(), w_gate_up.data_ptr(), act.data_ptr(), T, I, K, *ops._clamp_args(clamp), status.data_ptr(), ops._stream())
-        return
-    if bn is None:
-        bn = 64 if T <= 64 else (128 if T <= 128 else 256)
     L.call("ib_gemm_swiglu_tcgen05", x.data_ptr(), w_gate_up.data_ptr(), act.data_ptr(), T, I, K, bn, 1 if half else 0, *ops._clamp_args(clamp), status.data_ptr(), ops._stream())
 
 

@@ -155,3 +155,23 @@ def call(name: str, *args) -> None:
         noted.append((name, args))
     if e[0](*args) != 0:
         raise KernelError(load().ib_last_error().decode(errors="replace"))
+
+
+def call_counted(name: str, *args) -> None:
+    """An entry that launches several kernels and returns their number, or a negative one with its error's text set."""
+    global launches
+    e = _entry.get(name)
+    if e is None:
+        e = _entry[name] = (getattr(load(), name), 0)
+    n = e[0](*args)
+    if n < 0:
+        raise KernelError(load().ib_last_error().decode(errors="replace"))
+    launches += n
+
+
+_own_call = call
+
+
+def watched() -> bool:
+    """Whether somebody looks at this thread's calls one by one: notes them, or has put a function of its own in the place of `call`."""
+    return call is not _own_call or notes.calls is not None

@@ -27,6 +27,8 @@ def _ptr(t: Optional[torch.Tensor]) -> Optional[int]:
 
 
 def _check(name: str, t: torch.Tensor, dtype=None, shape=None) -> None:
+    if (shape is None or t.shape == shape) and (dtype is None or t.dtype is dtype) and t.is_contiguous() and t.is_cuda:   # (a wrapper checks five to ten tensors)
+        return
     if not t.is_cuda:
         raise L.KernelError(f"{name} must be a CUDA tensor: the kernels have no CPU path")
     if not t.is_contiguous():
@@ -86,9 +88,12 @@ class KvLayerView:
 
     def tma(self) -> tuple[Optional[int], int]:
         """(address of the pool's tensor map or None, pool row where this view's keys of page 0, head 0 start)."""
-        m = kv_tensor_map(self.pool)
-        _, pages, _, kv_heads, page_size, _ = self.pool.shape
-        return (m[1] if m else None), PoolRow(self.entry * pages * 2 * kv_heads * page_size)
+        made = self.__dict__.get("_tma")
+        if made is None:
+            m = kv_tensor_map(self.pool)
+            _, pages, _, kv_heads, page_size, _ = self.pool.shape
+            made = self.__dict__["_tma"] = (m[1] if m else None), PoolRow(self.entry * pages * 2 * kv_heads * page_size)
+        return made
 
     def c_view(self) -> L.KvView:
         cv = self.__dict__.get("_cv")   # made once per view: a layer asks for it several times a step
@@ -104,18 +109,8 @@ class KvLayerView:
         _check("block_table", self.block_table, torch.int32)
         per_kv = kv_heads * page_size * head_dim
         esz = self.pool.element_size()
-        return L.KvView(
-            base=self.pool.data_ptr() + self.entry * pages * planes * per_kv * esz,
-            page_stride=planes * per_kv,
-            v_offset=per_kv if planes == 2 else 0,
-            block_table=self.block_table.data_ptr(),
-            table_stride=self.block_table.shape[1],
-            page_size=page_size,
-            num_pages=pages,
-            kv_heads=kv_heads,
-            head_dim=head_dim,
-            dtype=dtype_code(self.pool.dtype),
-        )
+        return L.KvView(self.pool.data_ptr() + self.entry * pages * planes * per_kv * esz, planes * per_kv, per_kv if planes == 2 else 0, self.block_table.data_ptr(),
+                        self.block_table.shape[1], page_size, pages, kv_heads, head_dim, dtype_code(self.pool.dtype))
 
 
 def embed(table: torch.Tensor, tokens: torch.Tensor, x: torch.Tensor, status: torch.Tensor) -> None:

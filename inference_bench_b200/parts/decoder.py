@@ -10,6 +10,8 @@ from typing import Optional
 import torch
 
 from ..kernels import lib as L
+from ..kernels.dense import NO_LAYERS, DenseLayers
+from ..kernels.dense import takes as takes_dense
 from . import base
 from .plan import ModelPlan, PartSpec
 from .repeat import Repeat
@@ -130,15 +132,32 @@ class Decoder:
         if trace is not None:
             trace.append(self._residual_rows(ctx, x, None))
         # layers that repeat the calls of the one before (a captured step costs the host nothing, and a traced one looks between layers)
-        repeats = ctx.n_tokens <= REPEAT_MAX_TOKENS and not ctx.fixed_shape and trace is None and not nvtx and len(self.plan.schedule) > 2
+        alone = not ctx.fixed_shape and trace is None and not nvtx
+        repeats = alone and ctx.n_tokens <= REPEAT_MAX_TOKENS and len(self.plan.schedule) > 2
         rep: Optional[Repeat] = None
+        dense, left = {}, None   # layers launched by one call each (kernels/dense.py), by key; those whose contribution is still to be added
         for i, e in enumerate(self.plan.schedule):
             if nvtx:
                 nvtx.range_push(f"entry {i} layer {e.layer}")
+            block, cache = self.blocks[e.layer], ctx.caches[i] if ctx.caches else None
+            key = block.repeat_key(cache) if alone and e.enter is None else None
+            if key is not None and (pending is None or type(pending) is torch.Tensor):
+                layers = dense.get(key)
+                if layers is None:
+                    layers = dense[key] = DenseLayers(ctx, block, cache, x) if takes_dense(ctx, cache) else NO_LAYERS
+                if layers.fits:
+                    if left is not None:
+                        layers.run(block, cache, left.partial, left.left)
+                    else:
+                        layers.run(block, cache, None if pending is None else pending.data_ptr(), 0 if pending is None else pending.shape[0])
+                    rep, pending, left = None, None, layers if layers.left else None
+                    continue
+            if left is not None:
+                pending, left = left.pending(), None
             if e.enter is not None:
                 pending = self.stream_parts[e.enter[0]].forward(ctx, x, pending, x0, e.enter[1])
-            block, cache = self.blocks[e.layer], ctx.caches[i] if ctx.caches else None
-            key = block.repeat_key(cache) if repeats and e.enter is None else None
+            if not repeats:
+                key = None
             if rep is not None and key is not None and key == rep.key:
                 pending = rep.run(block, cache)
                 continue
@@ -151,6 +170,8 @@ class Decoder:
                 nvtx.range_pop()
             if trace is not None:
                 trace.append(self._residual_rows(ctx, x, pending))
+        if left is not None:
+            pending = left.pending()
         logits = None
         if ctx.logit_rows.shape[0] != 0:
             if nvtx:

@@ -18,8 +18,6 @@ from __future__ import annotations
 
 import torch
 
-import numpy as np
-
 from ..kernels import ops
 from . import base
 from .base import FixedState, WeightSpec
@@ -70,20 +68,22 @@ class GatedLinearRecurrence(base.Mixer):
         if ctx.fixed_shape:
             return None, None, None
         if "recurrence cut" not in ctx.memo:
-            C = ops.RECURRENCE_CHUNK
-            starts = ctx.h_seg_start
-            lens = np.diff(starts)
-            if not (lens > C).any():
+            C, starts = ops.RECURRENCE_CHUNK, ctx.h_seg_start.tolist()
+            short, long_segs, chunks = [], [], []
+            for s, (a, b) in enumerate(zip(starts, starts[1:])):
+                if b - a <= C:
+                    short.append(s)
+                    continue
+                first = len(chunks) // 2
+                for t in range(a, b, C):
+                    chunks += (t, min(C, b - t))
+                long_segs += (s, first, len(chunks) // 2 - first)
+            if not long_segs:
                 ctx.memo["recurrence cut"] = (None, None, None)
             else:
-                short = np.nonzero(lens <= C)[0].astype(np.int32)
-                long_segs, chunks = [], []
-                for s in np.nonzero(lens > C)[0].tolist():
-                    first = len(chunks)
-                    chunks += [(t, min(C, int(starts[s + 1]) - t)) for t in range(int(starts[s]), int(starts[s + 1]), C)]
-                    long_segs.append((s, first, len(chunks) - first))
-                flat = np.concatenate([short, np.asarray(long_segs, np.int32).ravel(), np.asarray(chunks, np.int32).ravel()]).astype(np.int32)
-                dev = torch.from_numpy(flat).pin_memory().to(ctx.rt.device, non_blocking=True)
-                a, b = short.size, short.size + 3 * len(long_segs)
+                a, b, n = len(short), len(short) + len(long_segs), len(short) + len(long_segs) + len(chunks)
+                staging = torch.empty(n, dtype=torch.int32, pin_memory=True)
+                staging.numpy()[:] = short + long_segs + chunks
+                dev = staging.to(ctx.rt.device, non_blocking=True)
                 ctx.memo["recurrence cut"] = (dev[:a], dev[a:b].view(-1, 3), dev[b:].view(-1, 2))
         return ctx.memo["recurrence cut"]

@@ -5,7 +5,9 @@ wrapper checks its tensors, asks for an output buffer and works out a tile (abou
 kernels take less than that, so the step waits for the host. Here the calls of one layer are noted as it runs, and the layers after it repeat them
 with their own weights and cache entry in the noted layer's buffers: everything is ordered by the stream, as it is when the allocator hands a freed
 buffer to the next layer. A layer is repeated only after one whose input and output are alike (the first of a run may have nothing to add to the
-stream yet), inside one step. Measured: 61 tokens behind 900 in eight layers of the 0.6B sizes 1,237 to 870 us a step (443 us of it on the device), a call 5 us.
+stream yet), inside one step. Measured when bfloat16 layers went this way: 61 tokens behind 900 in eight layers of the 0.6B sizes 1,237 to 870 us a step (443 us
+of it on the device), a call 5 us. Those are launched by one call a layer now (kernels/dense.py: 445 us); this form has the float32 layers and page
+or head sizes that the tensor-core attention kernels do not take.
 """
 from __future__ import annotations
 

@@ -10,7 +10,7 @@ from typing import Optional
 
 import torch
 
-from ..kernels import ops
+from ..kernels import attention, ops
 from . import base
 from .base import FixedState, PagedKV, WeightSpec
 
@@ -294,7 +294,6 @@ class Attention(base.Mixer):
         """Any of the variants: the projection's partial sums go through the q/k kernel that adds biases and takes two head sizes, then
         the attention kernels that cap scores and count the sink."""
         rt = ctx.rt
-        from ..kernels import attention
         cos, sin = self.position.tables(ctx)
         qkv = rt.linear(h, self.wqkv)
         q = rt.empty((ctx.n_tokens, self.heads * self.head_dim))
@@ -309,7 +308,6 @@ class Attention(base.Mixer):
         if not self.plain:
             return self._forward_variant(ctx, h, cache)
         cos, sin = self.position.tables(ctx)
-        from ..kernels import attention
         q = attention.project_qkv(ctx, h, self.wqkv, self.q_norm, self.k_norm, self.norm_eps, cos, sin, cache, self.heads, self.own_kv)
         if q is not None:   # many tokens: norm, rotation and cache write happened in the projection's epilogue
             out = attention.paged_attention(ctx, q, cache, self.heads, self.window, self.scale)

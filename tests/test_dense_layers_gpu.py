@@ -1,0 +1,74 @@
+"""Layers launched by one call each (csrc/dense_layer.cu) against the same layers run by their parts: the same bits, over the forms their products take."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+def _runner(hidden, inter, heads, kv_heads, head_dim, window, page, options=None):
+    from inference_bench_b200.cache.manager import CacheManager
+    from inference_bench_b200.config.runtime_options import RuntimeOptions
+    from inference_bench_b200.engine.model import plan_from_config
+    from inference_bench_b200.engine.runtime import Runtime
+    from inference_bench_b200.engine.step import ModelRunner
+    from inference_bench_b200.parts.decoder import Decoder
+    from inference_bench_b200.weights.random_init import random_weights
+    cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", vocab_size=333, hidden_size=hidden, intermediate_size=inter, num_hidden_layers=3, num_attention_heads=heads,
+               num_key_value_heads=kv_heads, head_dim=head_dim, rms_norm_eps=1e-6, rope_theta=1e6, tie_word_embeddings=True, max_position_embeddings=8192, hidden_act="silu",
+               attention_bias=False, torch_dtype="bfloat16")
+    if window:
+        cfg.update(use_sliding_window=True, sliding_window=window, max_window_layers=0, layer_types=["full_attention", "sliding_attention", "full_attention"])
+    rt = Runtime(DEV, "bfloat16", options=options or RuntimeOptions())
+    decoder = Decoder(plan_from_config(cfg)[1])
+    decoder.bind({k: v.to(DEV) for k, v in random_weights(decoder.weight_specs(), 5, std=0.05).items()}, rt)
+    cache = CacheManager(decoder.cache_needs(), page, 12000 // page, 8, 6000, device=rt.device, dtype=rt.act_dtype, sources=decoder.cache_sources())
+    return ModelRunner(decoder, cache, rt)
+
+
+# tokens of up to three requests a step: around the token tiles of the products (16, 32, 64, 128), where the q/k/v product takes its epilogue and the
+# cost model changes forms, the largest step that goes this way and one beyond it; single tokens beside portions in most of them
+STEPS = [[2], [15, 1, 1], [17, 16], [31, 1, 33], [63, 1, 1], [65], [127, 1, 1], [129], [300, 1, 7], [1000, 1, 1], [1, 1, 1], [2558, 1, 1], [1, 2560]]
+
+
+@pytest.mark.parametrize("sizes", [(256, 640, 4, 2, 64, 0, 16), (256, 640, 2, 2, 128, 70, 8), (1024, 3072, 16, 8, 128, 0, 64), (320, 9728, 4, 1, 128, 0, 128)])
+def test_the_same_bits_as_the_parts(sizes, monkeypatch):
+    from inference_bench_b200.engine.step import StepEntry
+    from inference_bench_b200.kernels import lib
+    outs, counts, native = [], [], []
+    for watch in (False, True):
+        names = []
+        if watch:   # somebody looks at every call: the parts run
+            real = lib.call
+            monkeypatch.setattr(lib, "call", lambda name, *a: (names.append(name), real(name, *a))[1])
+        else:
+            counted = lib.call_counted
+            monkeypatch.setattr(lib, "call_counted", lambda name, *a: (native.append(name), counted(name, *a))[1])
+        r, g = _runner(*sizes), torch.Generator().manual_seed(3)
+        for i in range(3):
+            r.cache.admit(i)
+        got = []
+        for lens in STEPS:
+            entries = [StepEntry(i, torch.randint(0, 333, (n,), generator=g).tolist(), [0, n - 1]) for i, n in enumerate(lens)]
+            before = lib.launches
+            got.append(r.step(entries).clone())
+            counts.append(lib.launches - before)
+        outs.append(got + [gr.tensor.clone() for gr in r.cache.groups])
+        assert not watch or "ib_attention_prefill_ws" in names
+    assert native.count("ib_dense_layer") == 3 * 11   # every step but the one of single tokens and the one of 2,561
+    assert counts[:len(STEPS)] == counts[len(STEPS):]
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
+@pytest.mark.parametrize("options", [dict(prefill_attention="tcgen05"), dict(decode_attention="split"), dict(gemm="simt")])
+def test_other_kernels_asked_for_run(options, monkeypatch):
+    """A runtime that asks for kernels this way does not have keeps its parts."""
+    from inference_bench_b200.config.runtime_options import RuntimeOptions
+    from inference_bench_b200.engine.step import StepEntry
+    from inference_bench_b200.kernels import lib
+    monkeypatch.setattr(lib, "call_counted", lambda *a: pytest.fail("a layer went past its parts"))
+    r = _runner(256, 640, 4, 2, 64, 0, 16, RuntimeOptions(**options))
+    r.cache.admit(0)
+    assert torch.isfinite(r.step([StepEntry(0, list(range(40)), [39])])).all()
