@@ -30,6 +30,8 @@ constexpr int EPI_STORE = 0, EPI_SWIGLU = 1, EPI_ADD = 2;   // float32 out; bflo
 constexpr int EPI_QKV = 3;   // the q/k/v projection finished in the epilogue: per-head norm, rotation, queries out, keys and values into the cache
 constexpr int EPI_CLAMPED = 6;   // EPI_SWIGLU with clamped halves (ib::clamped_glu): the limit in QkvEpi::act_pq[0], the slope in QkvEpi::act_slope
 constexpr bool epi_gated(int epi) { return epi == EPI_SWIGLU || epi == EPI_CLAMPED; }
+constexpr int EPI_GLU16 = 8, EPI_CLAMPED16 = 9;   // EPI_SWIGLU and EPI_CLAMPED with gate and up rows in one accumulator, sixteen of each in turn
+constexpr bool epi_16(int epi) { return epi == EPI_GLU16 || epi == EPI_CLAMPED16; }
 constexpr int EPI_RELU2 = 5;   // bfloat16 max(product, 0)^2
 constexpr int EPI_BF16 = 7;    // the product rounded to bfloat16, tokens and matrix rows exchanged as for EPI_QKV (a thread writes a token's row piece by piece)
 constexpr int EPI_XIELU = 4;   // bfloat16 xielu(product) with the activation's two numbers (QkvEpi::act_pq)
@@ -77,6 +79,13 @@ __device__ __forceinline__ void tma_load_2d_pair(void* smem_dst, const CUtensorM
       "l"(m), "r"(x), "r"(y), "r"(sm100::smem_u32(bar) & kPeerBitMask)
       : "memory");
 }
+__device__ __forceinline__ void tma_load_4d_pair(void* smem_dst, const CUtensorMap* m, int x, int y, int z, int w, uint64_t* bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];" ::"r"(
+          sm100::smem_u32(smem_dst)),
+      "l"(m), "r"(x), "r"(y), "r"(z), "r"(w), "r"(sm100::smem_u32(bar) & kPeerBitMask)
+      : "memory");
+}
 __device__ __forceinline__ void mma_bf16_ss_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
@@ -99,9 +108,10 @@ __device__ __forceinline__ void arrive_on_leader(uint64_t* bar) {
 
 // Regrouped rows (routed experts): rows offsets[e] .. offsets[e + 1] of x go through matrix e, rows e * w_rows .. of w. tiles[e] is the first token tile of
 // group e and tiles[n] their number; a tile never crosses a group's end (rows past it are multiplied and not stored). n = 0: one matrix for all.
-// The table is read into shared memory once, after the wait for the kernels before; a tile's group is a search in it. Bound by the tensor cores' operand
-// traffic at many rows a group and by the matrices' bytes at few: 12,288 rows of 64 groups, 2,816 x 2,048 each, 240 us on single CTAs, 202 here, the
-// 2,048 x 1,408 product behind it 169 and 109; 49,152 rows 696 and 501, 541 and 277 (1.1 PFLOP/s).
+// The table is read into shared memory once, after the wait for the kernels before; a tile's group is a search in it. Bound by memory at up to a few
+// hundred rows a group, so the tiles go group by group: with all groups' token tiles under one block of rows after the other, 12,288 rows of 64 groups, 2,816 x
+// 2,048 each, read 1.17 GB (the rows of x again and again) where 0.79 are there, 203 us; in this order 156 (5.1 TB/s; single CTAs 238), the 2,048 x
+// 1,408 product behind it 115 and 92 (166). 49,152 rows: 538 and 420 (711), 302 and 240 (557; 1.2 PFLOP/s).
 struct PairGroups {
   const int* offsets;
   const int* tiles;
@@ -137,7 +147,7 @@ struct QkvEpi {
 // memory holds two of them, so the next tile's MMAs also run during that store.
 template <int MT, int EPI, int BN>
 __global__ void __launch_bounds__(kThreads, 1)
-    gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, void* __restrict__ out_, int T, int N,
+    gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x, const __grid_constant__ CUtensorMap tmap_x16, void* __restrict__ out_, int T, int N,
                      int K, int token_tiles, int total_tiles, int second_off, unsigned long long wait_ns, unsigned* __restrict__ status, const QkvEpi qe, const PairGroups grp) {
   using TL = Tile<MT, BN>;
   constexpr int STAGES = TL::kStages;
@@ -157,7 +167,7 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t rank = cluster_rank();          // 0 = leader
   const int pair = blockIdx.x >> 1, n_pairs = gridDim.x >> 1;
   const int nkt = (K + BK - 1) / BK;
-  constexpr int kColsPerPair = epi_gated(EPI) ? 2 * BM : 2 * BM * MT;
+  constexpr int kColsPerPair = epi_16(EPI) ? BM : epi_gated(EPI) ? 2 * BM : 2 * BM * MT;
 
   int* g_off = (int*)(tiles + STAGES * TL::kStageBytes + 256 + 1024);   // [kMaxGroups + 1]
   int* g_tile = g_off + kMaxGroups + 1;
@@ -193,28 +203,28 @@ __global__ void __launch_bounds__(kThreads, 1)
   sm100::tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  if (grp.n) {
-    token_tiles = g_tile[grp.n];
-    total_tiles = token_tiles * ((N + kColsPerPair - 1) / kColsPerPair);
-  }
+  const int row_blocks = (N + kColsPerPair - 1) / kColsPerPair;
+  if (grp.n) total_tiles = g_tile[grp.n] * row_blocks;
   // a tile: its block of rows of W, its first token, one past its last, its group and where the group's matrix begins
   struct Place {
     int rb, t0, t_end, group, w0;
   };
   auto place = [&](int tile) {
-    const int b = tile % token_tiles;
-    Place p{tile / token_tiles, b * BN, T, 0, 0};
-    if (grp.n) {
-      int lo = 0, hi = grp.n;   // the last group whose first tile is at or before b
-      while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (g_tile[mid] <= b) lo = mid;
-        else hi = mid;
-      }
-      p.t0 = g_off[lo] + (b - g_tile[lo]) * BN, p.t_end = g_off[lo + 1], p.group = lo, p.w0 = lo * grp.w_rows;
+    if (!grp.n) return Place{tile / token_tiles, tile % token_tiles * BN, T, 0, 0};
+    // group by group, so that its rows of x and its matrix come from memory once: every block of the matrix with all of the group's token tiles in turn
+    int lo = 0, hi = grp.n;   // the last group whose first tile is at or before this one
+    while (hi - lo > 1) {
+      const int mid = (lo + hi) >> 1;
+      if (g_tile[mid] * row_blocks <= tile) lo = mid;
+      else hi = mid;
     }
-    return p;
+    const int in = tile - g_tile[lo] * row_blocks, own = g_tile[lo + 1] - g_tile[lo], rb = in / own;
+    return Place{rb, g_off[lo] + (in - rb * own) * BN, g_off[lo + 1], lo, lo * grp.w_rows};
   };
+  // Regrouped rows in tiles of 256: a tile is loaded and multiplied only as far as its rows go, in steps of 32 (each CTA has half of them; tmap_x brings
+  // 64 rows, tmap_x16 sixteen). Otherwise the tile's full width, in one load.
+  constexpr bool kTrims = MT == 1 && BN == 256;
+  auto width = [&](const Place& p) { return kTrims && grp.n ? min(BN, (p.t_end - p.t0 + 31) & ~31) : BN; };
   // W rows of accumulator m of this CTA for the pair's row block rb: plain tiles stack 256-row pairs;
   // SwiGLU takes gate rows and, second_off on, up rows
   auto w_row = [&](int rb, int m) {
@@ -230,6 +240,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       int it = 0;   // k-tiles sent so far, over all tiles: stage = it % STAGES
       for (int tile = pair; tile < total_tiles && ok; tile += n_pairs) {
         const Place at = place(tile);
+        const int wide = width(at);
         for (int i = 0; i < nkt; i++, it++) {
           const int s = it % STAGES;
           if (!sm100::mbar_wait(&empty[s], ((it / STAGES) & 1) ^ 1, wait_ns)) {
@@ -238,24 +249,37 @@ __global__ void __launch_bounds__(kThreads, 1)
             break;
           }
           uint8_t* a = tiles + s * TL::kStageBytes;
-          if (rank == 0) sm100::mbar_arrive_expect_tx(&full[s], 2 * TL::kStageBytes);   // the leader counts both CTAs' bytes
+          if (rank == 0) sm100::mbar_arrive_expect_tx(&full[s], 2 * MT * TL::kABytes + wide * BK * 2);   // the leader counts both CTAs' bytes
           if ((EPI == EPI_QKV || EPI == EPI_BF16) && !waited) {   // there the rows are the tokens, which the kernel before wrote
             ib::pdl_wait();
             waited = true;
           }
+          if constexpr (epi_16(EPI)) {   // sixteen gate rows, the sixteen up rows that go with them, four times
+            const int first = (at.w0 + at.rb * kColsPerPair + (int)rank * (BM / 2)) / 16;
 #pragma unroll
-          for (int m = 0; m < MT; m++) tma_load_2d_pair(a + m * TL::kABytes, &tmap_w, i * BK, at.w0 + w_row(at.rb, m), &full[s]);
+            for (int e = 0; e < 4; e++) tma_load_4d_pair(a + e * 32 * BK * 2, &tmap_w, i * BK, 0, first + e, 0, &full[s]);
+          } else {
+#pragma unroll
+            for (int m = 0; m < MT; m++) tma_load_2d_pair(a + m * TL::kABytes, &tmap_w, i * BK, at.w0 + w_row(at.rb, m), &full[s]);
+          }
           if (!waited) {   // the weights above do not depend on earlier kernels; x does
             ib::pdl_wait();
             waited = true;
           }
-          tma_load_2d_pair(a + MT * TL::kABytes, &tmap_x, i * BK, at.t0 + (int)rank * BNH, &full[s]);
+          if (kTrims && grp.n) {
+            const int half = wide / 2, first = at.t0 + (int)rank * half;
+            uint8_t* xs = a + MT * TL::kABytes;
+            int r = 0;
+            for (; r + 64 <= half; r += 64) tma_load_2d_pair(xs + r * BK * 2, &tmap_x, i * BK, first + r, &full[s]);
+            for (; r < half; r += 16) tma_load_2d_pair(xs + r * BK * 2, &tmap_x16, i * BK, first + r, &full[s]);
+          } else {
+            tma_load_2d_pair(a + MT * TL::kABytes, &tmap_x, i * BK, at.t0 + (int)rank * BNH, &full[s]);
+          }
         }
       }
     }
   } else if (warp == 1) {
     if (rank == 0 && sm100::elect_one()) {
-      constexpr uint32_t idesc = sm100::idesc_bf16_f32(2 * BM, BN);
       bool ok = true;
       int it = 0, tl = 0;
       for (int tile = pair; tile < total_tiles && ok; tile += n_pairs, tl++) {
@@ -266,6 +290,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           break;
         }
         sm100::tc_fence_after();
+        const uint32_t idesc = sm100::idesc_bf16_f32(2 * BM, kTrims && grp.n ? width(place(tile)) : BN);
         for (int i = 0; i < nkt; i++, it++) {
           const int s = it % STAGES;
           if (!sm100::mbar_wait(&full[s], (it / STAGES) & 1, wait_ns)) {
@@ -415,7 +440,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         for (int m = 0; m < MT; m++) {
           const int n = n_pair + m * 2 * BM + (int)rank * BM + q * 32 + lane;
 #pragma unroll 1
-          for (int c0 = 0; c0 < BN; c0 += 32) {
+          for (int c0 = 0; c0 < width(at); c0 += 32) {
             uint32_t r[32];
             sm100::tmem_ld_32x32b_x32(lane_addr + b * MT * BN + m * BN + c0, r);
             sm100::tmem_ld_wait();
@@ -440,6 +465,32 @@ __global__ void __launch_bounds__(kThreads, 1)
                 }
               }
             }
+          }
+        }
+      } else if constexpr (epi_16(EPI)) {
+        // Lane l holds gate row l or, from 16 on, up row l - 16 of the warp's sixteen: one exchange gives each half of the lanes both numbers of every
+        // second token. No branch between the numbers (as in the form below, where 128 columns take 8 us): a thread's sixteen run side by side.
+        const float limit = EPI == EPI_CLAMPED16 ? qe.act_pq[at.group] : 0.f;
+        const int n = n_pair + (int)rank * (BM / 2) + q * 16 + (lane & 15), wide = width(at), up = lane >> 4;
+        __nv_bfloat16* dst = (__nv_bfloat16*)out_ + (size_t)(t0 + up) * N + n;
+#pragma unroll 1
+        for (int c0 = 0; c0 < wide; c0 += 32) {
+          uint32_t r[32];
+          sm100::tmem_ld_32x32b_x32(lane_addr + b * BN + c0, r);
+          sm100::tmem_ld_wait();
+          __nv_bfloat16 v[16];
+#pragma unroll
+          for (int c = 0; c < 16; c++) {
+            const uint32_t got = __shfl_xor_sync(0xffffffffu, up ? r[2 * c] : r[2 * c + 1], 16);
+            const float gv = __uint_as_float(up ? got : r[2 * c]), uv = __uint_as_float(up ? r[2 * c + 1] : got);
+            if constexpr (EPI == EPI_CLAMPED16) v[c] = __float2bfloat16_rn(ib::clamped_glu<true>(gv, uv, limit, qe.act_slope));
+            else v[c] = __float2bfloat16_rn(__fdividef(gv, 1.f + __expf(-gv)) * uv);
+          }
+          if (n < N) {
+            const int left = t_end - t0 - c0 - up;   // tokens of this chunk that are stored: every second one below this
+#pragma unroll
+            for (int c = 0; c < 16; c++)
+              if (2 * c < left) dst[(size_t)(c0 + 2 * c) * N] = v[c];
           }
         }
       } else {
@@ -492,6 +543,23 @@ int make_tmap(CUtensorMap* m, const void* ptr, int rows, int K, int box_rows) {
   return 0;
 }
 
+// The [E][2 I][K] gate and up rows as (k, sixteen rows, sixteens, gate or up): a box brings sixteen gate rows and the up rows that go with them. The last
+// sixteens, whose up rows would lie behind the buffer, are outside.
+int make_tmap_glu16(CUtensorMap* m, const void* ptr, int rows, int I, int K) {
+  tma_host::EncodeTiledFn fn = tma_host::encode_fn();
+  IB_CHECK_ARG(fn, "gemm_tcgen05_2cta: the driver has no cuTensorMapEncodeTiled");
+  IB_CHECK_ARG(I % 16 == 0 && rows % (2 * I) == 0, "gemm_tcgen05_2cta: %d gate rows are no whole sixteens", I);
+  const cuuint64_t row = (cuuint64_t)K * 2;
+  cuuint64_t dims[4] = {(cuuint64_t)K, 16, (cuuint64_t)(rows - I) / 16, 2};
+  cuuint64_t strides[3] = {row, row * 16, row * I};
+  cuuint32_t box[4] = {(cuuint32_t)BK, 16, 1, 2};
+  cuuint32_t estr[4] = {1, 1, 1, 1};
+  CUresult r = fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                  CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  IB_CHECK_ARG(r == CUDA_SUCCESS, "gemm_tcgen05_2cta: cuTensorMapEncodeTiled failed with code %d", (int)r);
+  return 0;
+}
+
 template <int MT, int EPI, int BN>
 int launch(const void* x, const void* w, void* out, int T, int N, int K, int w_rows, int second_off, unsigned* status, cudaStream_t stream,
            const QkvEpi& qe = QkvEpi{}, const PairGroups& grp = PairGroups{}) {
@@ -504,10 +572,13 @@ int launch(const void* x, const void* w, void* out, int T, int N, int K, int w_r
     IB_CHECK_ARG(e == cudaSuccess, "gemm_tcgen05_2cta: cannot reserve %d bytes of shared memory: %s", TL::kSmemBytes, cudaGetErrorString(e));
     configured = true;
   }
-  CUtensorMap tw, tx;
-  if (make_tmap(&tw, w, w_rows, K, BM)) return 1;
-  if (make_tmap(&tx, x, T, K, BN / 2)) return 1;
-  const int cols_per_pair = epi_gated(EPI) ? 2 * BM : 2 * BM * MT;
+  CUtensorMap tw, tx, tx16;
+  const bool trims = MT == 1 && BN == 256 && grp.n;
+  if (epi_16(EPI) ? make_tmap_glu16(&tw, w, w_rows, N, K) : make_tmap(&tw, w, w_rows, K, BM)) return 1;
+  if (make_tmap(&tx, x, T, K, trims ? 64 : BN / 2)) return 1;
+  if (!trims) tx16 = tx;
+  else if (make_tmap(&tx16, x, T, K, 16)) return 1;
+  const int cols_per_pair = epi_16(EPI) ? BM : epi_gated(EPI) ? 2 * BM : 2 * BM * MT;
   const int token_tiles = grp.n ? T / BN + grp.n : (T + BN - 1) / BN, row_blocks = (N + cols_per_pair - 1) / cols_per_pair;
   const int total_tiles = token_tiles * row_blocks;
   static int sm_count = 0;
@@ -531,7 +602,7 @@ int launch(const void* x, const void* w, void* out, int T, int N, int K, int w_r
   attr[1].val.programmaticStreamSerializationAllowed = ib_pdl_enabled();
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_2cta_kernel<MT, EPI, BN>, tw, tx, out, T, N, K, token_tiles, total_tiles, second_off, ib_wait_limit_ns(), status, qe, grp);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, gemm_2cta_kernel<MT, EPI, BN>, tw, tx, tx16, out, T, N, K, token_tiles, total_tiles, second_off, ib_wait_limit_ns(), status, qe, grp);
   IB_CHECK_ARG(e == cudaSuccess, "gemm_tcgen05_2cta: launch failed: %s", cudaGetErrorString(e));
   return 0;
 }
@@ -586,27 +657,33 @@ extern "C" int ib_gemm_swiglu_tcgen05_2cta(const void* x, const void* w, void* a
   return launch<2, EPI_SWIGLU, 128>(x, w, act, T, I, K, 2 * I, I, status, stream);
 }
 
-// The products of regrouped rows on CTA pairs, tiles of 128 rows (the table: ib_moe_sort with tile_rows = 128): x [R, K] bfloat16 and w [E, N or 2 I, K];
+// The products of regrouped rows on CTA pairs, tiles of `tile` rows, 128 or 256 (the table: ib_moe_sort with tile_rows = tile): x [R, K] bfloat16 and w [E, N or 2 I, K];
 // offsets, tiles [E + 1] (see PairGroups). Store: out [R, N] float32; act 2: [R, N] bfloat16 max(product, 0)^2.
-extern "C" int ib_gemm_grouped_2cta(const void* x, const void* w, void* out, int R, int N, int K, const int* offsets, const int* tiles, int E, int act, unsigned* status,
+extern "C" int ib_gemm_grouped_2cta(const void* x, const void* w, void* out, int R, int N, int K, const int* offsets, const int* tiles, int E, int tile, int act, unsigned* status,
                                     cudaStream_t stream) {
   if (R == 0 || N == 0) return 0;
   IB_CHECK_ARG(E > 0 && E <= kMaxGroups && offsets && tiles && (act == 0 || act == 2), "gemm_grouped_2cta: %d groups (up to %d) or activation %d", E, kMaxGroups, act);
+  IB_CHECK_ARG(tile == 128 || tile == 256, "gemm_grouped_2cta: tiles of %d rows (128 and 256 are built)", tile);
   IB_CHECK_ARG((long long)E * N < (1ll << 31), "gemm_grouped_2cta: %d matrices of %d rows", E, N);
   const PairGroups grp{offsets, tiles, E, N};
+  if (tile == 256 && act == 2) return launch<1, EPI_RELU2, 256>(x, w, out, R, N, K, E * N, 0, status, stream, QkvEpi{}, grp);
+  if (tile == 256) return launch<1, EPI_STORE, 256>(x, w, out, R, N, K, E * N, 0, status, stream, QkvEpi{}, grp);
   if (act == 2) return launch<2, EPI_RELU2, 128>(x, w, out, R, N, K, E * N, BM * 2, status, stream, QkvEpi{}, grp);
   return launch<2, EPI_STORE, 128>(x, w, out, R, N, K, E * N, BM * 2, status, stream, QkvEpi{}, grp);
 }
 
 // act [R, I] bfloat16 = silu(gate) * up per group, w [E, 2 I, K] = every group's gate rows then its up rows; limits: null, or float32 [E]: clamped halves.
-extern "C" int ib_gemm_grouped_swiglu_2cta(const void* x, const void* w, void* act, int R, int I, int K, const int* offsets, const int* tiles, int E, const float* limits,
+extern "C" int ib_gemm_grouped_swiglu_2cta(const void* x, const void* w, void* act, int R, int I, int K, const int* offsets, const int* tiles, int E, int tile, const float* limits,
                                            float slope, unsigned* status, cudaStream_t stream) {
   if (R == 0 || I == 0) return 0;
   IB_CHECK_ARG(E > 0 && E <= kMaxGroups && offsets && tiles, "gemm_grouped_swiglu_2cta: %d groups (up to %d)", E, kMaxGroups);
+  IB_CHECK_ARG(tile == 128 || (tile == 256 && I % 16 == 0), "gemm_grouped_swiglu_2cta: tiles of %d rows with %d gate rows (128, or 256 with a multiple of 16)", tile, I);
   IB_CHECK_ARG((long long)E * 2 * I < (1ll << 31), "gemm_grouped_swiglu_2cta: %d matrices of %d rows", E, 2 * I);
   const PairGroups grp{offsets, tiles, E, 2 * I};
   QkvEpi qe{};
   qe.act_pq = limits, qe.act_slope = slope;
+  if (tile == 256 && limits) return launch<1, EPI_CLAMPED16, 256>(x, w, act, R, I, K, E * 2 * I, I, status, stream, qe, grp);
+  if (tile == 256) return launch<1, EPI_GLU16, 256>(x, w, act, R, I, K, E * 2 * I, I, status, stream, qe, grp);
   if (limits) return launch<2, EPI_CLAMPED, 128>(x, w, act, R, I, K, E * 2 * I, I, status, stream, qe, grp);
   return launch<2, EPI_SWIGLU, 128>(x, w, act, R, I, K, E * 2 * I, I, status, stream, qe, grp);
 }

@@ -32,8 +32,8 @@ L.register("ib_gemm_qkv_tcgen05_2cta", [L._p, L._p, L._i, L._i, L._p, L._p, L._f
 
 L.register("ib_gemm_grouped_tcgen05", [L._p, L._p, L._p, L._i, L._i, L._i, L._i, L._p, L._p, L._i, L._p, L._p])
 L.register("ib_gemm_parts_tcgen05", [L._p, L._p, L._p, L._i, L._i, L._i, L._i, L._i, L._i, L._p, L._p])
-L.register("ib_gemm_grouped_2cta", [L._p, L._p, L._p, L._i, L._i, L._i, L._p, L._p, L._i, L._i, L._p, L._p])
-L.register("ib_gemm_grouped_swiglu_2cta", [L._p, L._p, L._p, L._i, L._i, L._i, L._p, L._p, L._i, L._p, L._f, L._p, L._p])
+L.register("ib_gemm_grouped_2cta", [L._p, L._p, L._p, L._i, L._i, L._i, L._p, L._p, L._i, L._i, L._i, L._p, L._p])
+L.register("ib_gemm_grouped_swiglu_2cta", [L._p, L._p, L._p, L._i, L._i, L._i, L._p, L._p, L._i, L._i, L._p, L._f, L._p, L._p])
 L.register("ib_gemm_grouped_relu2_tcgen05", [L._p, L._p, L._p, L._i, L._i, L._i, L._i, L._p, L._p, L._i, L._p, L._p])
 L.register("ib_gemm_grouped_swiglu_tcgen05", [L._p, L._p, L._p, L._i, L._i, L._i, L._i, L._p, L._p, L._i, L._p, L._f, L._p, L._p])
 
@@ -305,7 +305,7 @@ def gemm_act(rt, x: torch.Tensor, lw, kind: str, act: torch.Tensor, pq: Optional
 # ---------------------------------------------------------------- products on regrouped rows (routed experts)
 def grouped_token_tile(rows: int, groups: int, inter: int = 0, sm_count: int = FITTED_SM_COUNT) -> int:
     """Tokens per CTA for a product on `rows` regrouped rows of `groups` experts: the smallest tile that holds an expert's average share,
-    up to 128 (from there on `grouped_pairs` takes up to 256 experts); 256 where the experts' shares are larger and tiles of 256 still give every SM two CTAs (measured alone, 2,048 tokens: 64
+    up to 128 (most sizes from 32 rows an expert on go to `grouped_pairs`, which takes up to 256 experts); 256 where the experts' shares are larger and tiles of 256 still give every SM two CTAs (measured alone, 2,048 tokens: 64
     experts of 1,408 x 2,048 with 6 a token 421 against 468 us; 16 experts of 1,024 x 1,024 with 2 a token 87 against 83 us). A function of
     the sizes only."""
     avg = -(-rows // groups)
@@ -321,38 +321,49 @@ def grouped_supported(k: int, inter: int, bn: int, gated: bool = True) -> bool:
     return k % 8 == 0 and inter % 8 == 0 and (not gated or bn >= 64 or inter % 64 == 0)
 
 
-PAIR_TILE = 128   # rows of a token tile of the CTA-pair form of these products
+PAIR_TILE, PAIR_WIDE_TILE = 128, 256   # rows of a token tile of the CTA-pair forms of these products
 PAIR_MAX_GROUPS = 256
 
 
 def grouped_pairs(rows: int, groups: int, inter: int, sm_count: int = FITTED_SM_COUNT) -> bool:
-    """Whether the experts' products run on CTA pairs (256 or 512 matrix rows by 128 regrouped rows a tile, stored while the next tile is multiplied):
-    from 128 rows an expert on, and from 64 on where the experts' matrices alone give every pair a tile; below that the tiles are mostly
-    padding. A function of the sizes only. Both products alone, L2 flushed, single CTAs against pairs in us: 64 experts of 1,408 x 2,048, 48
-    rows an expert 243 / 244, 65 280 / 249, 96 299 / 262, 192 409 / 310, 768 1,237 / 777; 128 experts of 768 x 2,048, 64 rows 318 / 262, 256
-    673 / 385; 32 experts of 2,880 x 2,880, 64 rows 346 / 326, 256 633 / 486; 16 experts of 1,024 x 1,024 (64 tiles a product and few rows), 65
-    rows 50.1 / 51.2, 97 51.3 / 52.2, 128 68.7 / 59.4."""
+    """Whether the experts' products run on CTA pairs (their tiles stored while the next is multiplied): from 128 rows an expert on, and from 32 on where the
+    experts' matrices alone give every pair a tile; below that the matrices' bytes are all that counts and single CTAs stream them a little faster.
+    A function of the sizes only. Both products alone, L2 flushed, single CTAs against pairs in us: 64 experts of 1,408 x 2,048, 24 rows an expert 213 /
+    215, 48 242 / 219, 96 295 / 227, 192 404 / 248, 768 1,268 / 659; 128 experts of 768 x 2,048, 32 rows 263 / 239, 256 668 / 356; 32 experts of
+    2,880 x 2,880, 64 rows 352 / 305, 256 635 / 399; 16 experts of 1,024 x 1,024, 37 rows 47.1 / 45.1, 128 69.7 / 49.2."""
     avg = -(-rows // groups)
-    return groups <= PAIR_MAX_GROUPS and (avg >= 128 or avg >= 64 and groups * -(-inter // 256) >= sm_count // 2)
+    return groups <= PAIR_MAX_GROUPS and (avg >= 128 or avg >= 32 and groups * -(-inter // 128) >= sm_count // 2)
+
+
+def pair_tile(rows: int, groups: int, inter: int, gated: bool = True, sm_count: int = FITTED_SM_COUNT) -> int:
+    """Rows of a token tile of that form. 256: an expert's share is mostly one tile, loaded and multiplied as far as it goes, so that its matrix passes through
+    the SMs once (gate and up of 64 experts, 192 rows each: 156 us against 174). 128 where gate and up rows cannot be taken sixteen at a time, and
+    where large shares make fewer than four rounds of the wide tiles, whose last is then nearly empty (16 experts of 1,024 x 1,024, 512 rows each:
+    82 us against 90)."""
+    avg = -(-rows // groups)
+    if gated and inter % 16:
+        return PAIR_TILE
+    rounds = groups * -(-avg // PAIR_WIDE_TILE) * -(-inter // 128) / (sm_count // 2)
+    return PAIR_TILE if avg > PAIR_WIDE_TILE and rounds < 4 else PAIR_WIDE_TILE
 
 
 def gemm_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bn: int, offsets: torch.Tensor, tiles: torch.Tensor, status: torch.Tensor, pair: bool = False) -> None:
     """out [R, N] float32 = per expert w[e] x[r] for the regrouped rows x [R, K] (expert e's rows: offsets[e] .. offsets[e + 1]); w [E, N, K];
-    tiles: first token tile of `bn` rows of every expert, then their number (`ops.moe_sort` with tile_rows=bn). pair: on CTA pairs (bn = 128)."""
+    tiles: first token tile of `bn` rows of every expert, then their number (`ops.moe_sort` with tile_rows=bn). pair: on CTA pairs (bn = 128 or 256)."""
     R, K = x.shape
     E, N, _ = w.shape
     ops._check("x", x, torch.bfloat16)
     ops._check("w", w, torch.bfloat16, (E, N, K))
     ops._check("out", out, torch.float32, (R, N))
     if _pair_tile(pair, bn):
-        L.call("ib_gemm_grouped_2cta", x.data_ptr(), w.data_ptr(), out.data_ptr(), R, N, K, offsets.data_ptr(), tiles.data_ptr(), E, 0, status.data_ptr(), ops._stream())
+        L.call("ib_gemm_grouped_2cta", x.data_ptr(), w.data_ptr(), out.data_ptr(), R, N, K, offsets.data_ptr(), tiles.data_ptr(), E, bn, 0, status.data_ptr(), ops._stream())
         return
     L.call("ib_gemm_grouped_tcgen05", x.data_ptr(), w.data_ptr(), out.data_ptr(), R, N, K, bn, offsets.data_ptr(), tiles.data_ptr(), E, status.data_ptr(), ops._stream())
 
 
 def _pair_tile(pair: bool, bn: int) -> bool:
-    if pair and bn != PAIR_TILE:
-        raise L.KernelError(f"products of regrouped rows on CTA pairs take tiles of {PAIR_TILE} rows, not {bn}")
+    if pair and bn not in (PAIR_TILE, PAIR_WIDE_TILE):
+        raise L.KernelError(f"products of regrouped rows on CTA pairs take tiles of {PAIR_TILE} or {PAIR_WIDE_TILE} rows, not {bn}")
     return pair
 
 
@@ -380,7 +391,7 @@ def gemm_grouped_relu2(x: torch.Tensor, w: torch.Tensor, act: torch.Tensor, bn: 
     ops._check("w", w, torch.bfloat16, (E, N, K))
     ops._check("act", act, torch.bfloat16, (R, N))
     if _pair_tile(pair, bn):
-        L.call("ib_gemm_grouped_2cta", x.data_ptr(), w.data_ptr(), act.data_ptr(), R, N, K, offsets.data_ptr(), tiles.data_ptr(), E, 2, status.data_ptr(), ops._stream())
+        L.call("ib_gemm_grouped_2cta", x.data_ptr(), w.data_ptr(), act.data_ptr(), R, N, K, offsets.data_ptr(), tiles.data_ptr(), E, bn, 2, status.data_ptr(), ops._stream())
         return
     L.call("ib_gemm_grouped_relu2_tcgen05", x.data_ptr(), w.data_ptr(), act.data_ptr(), R, N, K, bn, offsets.data_ptr(), tiles.data_ptr(), E, status.data_ptr(), ops._stream())
 
@@ -394,7 +405,7 @@ def gemm_grouped_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Ten
     ops._check("w_gate_up", w_gate_up, torch.bfloat16, (E, I2, K))
     ops._check("act", act, torch.bfloat16, (R, I2 // 2))
     if _pair_tile(pair, bn):
-        L.call("ib_gemm_grouped_swiglu_2cta", x.data_ptr(), w_gate_up.data_ptr(), act.data_ptr(), R, I2 // 2, K, offsets.data_ptr(), tiles.data_ptr(), E,
+        L.call("ib_gemm_grouped_swiglu_2cta", x.data_ptr(), w_gate_up.data_ptr(), act.data_ptr(), R, I2 // 2, K, offsets.data_ptr(), tiles.data_ptr(), E, bn,
                *ops._clamp_args(clamp, E), status.data_ptr(), ops._stream())
         return
     L.call("ib_gemm_grouped_swiglu_tcgen05", x.data_ptr(), w_gate_up.data_ptr(), act.data_ptr(), R, I2 // 2, K, bn, offsets.data_ptr(), tiles.data_ptr(), E,

@@ -139,7 +139,7 @@ class RoutedExperts(base.FeedForward):
             raise ValueError(f"expert_gemm = \"tcgen05\" needs bfloat16 and inner sizes that are multiples of 8 (of 64 for few tokens), got {self.hidden} and {self.expert_ff}")
         pair = tcgen05 and G.grouped_pairs(R, n, self.expert_ff, rt.sm_count)
         if pair:
-            bn = G.PAIR_TILE
+            bn = G.pair_tile(R, n, self.expert_ff, self.gated, rt.sm_count)
         tile_rows = bn if tcgen05 else ops.moe_tile_rows()
         one = T <= ROUTE_SORT_TOKENS and ops.moe_route_sort_fits(T, E, self.groups, always)     # the choice and the regrouping in one kernel
         ops.moe_route(logits, self.groups, self.groups_keep, top, self.route_scale, self.renorm, idx, wt, self.score, correction=self.w_correction, group_top=self.group_top,
