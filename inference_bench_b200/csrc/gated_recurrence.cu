@@ -12,7 +12,8 @@
 //    With `chunks` the same kernel walks chunks of a long segment instead, each from a zero state: it leaves the chunk's own
 //    outputs, its closing state and decay, and q_t times the decay from the chunk's start to t; `chunk_carry` then walks a segment's
 //    chunks in order (S_in of the next = decay * S_in + the chunk's closing state, elementwise, ending in the request's state) and
-//    `chunk_apply` adds (q_t * decay)^T S_in to every output. The three give what the walk over the whole segment gives, up to
+//    `chunk_apply` adds (q_t * decay)^T S_in to every output. (The gated form's chunks with heads of more than 64 are products instead of a walk:
+//    gated_chunk_kernel.) The three give what the walk over the whole segment gives, up to
 //    rounding, with as many CTAs as the segment has chunks; which path a segment takes depends on its own length only.
 //  * Other forms of the same walk: a fixed decay per head with a key (form 1: q, k, v behind a SiLU; form 2: q and k turned by the token's
 //    angles, the key scaled, v as it is), and a decay per channel and token with a bonus for the current token (form 3:
@@ -404,6 +405,229 @@ __global__ void __launch_bounds__(MAXT, MAXT == 256 && RPT == 8 ? (NC == 2 ? 3 :
   }
 }
 
+// The gated form's chunks (form 0) as products instead of a walk. With A(s, t) the product of the f's after token s up to token t, channel by channel:
+//     o_t = sum over s <= t of p_ts v_s,  p_ts = sum_d q_td k_sd A_d(s, t),     closing state = sum_s k_s A(s, end) v_s^T,     k = 1 - f.
+// A CTA of 512 threads takes a chunk of up to 64 tokens of one head with 128 value columns, everything in shared memory: a multiply-add an entry of the
+// state and token where the walk needs three. A(s, t) is never a quotient of running products, which would overflow: tokens go in four blocks of
+// sixteen, and across blocks A is (f's after s in its block) x (whole blocks between) x (f's of t's block up to t), each a product of numbers below
+// one. Inside a block the p's are made channel by channel, s fixed and t rising.
+// What bounds it is issue (58 % of the slots) and shared-memory reads (the state's 8 x 8 outputs a thread cost 4 of 16 bytes for 64 FMAs) with one CTA an
+// SM, whose phases nothing overlaps: 2,048 tokens of 16 heads of 128 x 128 take 104 us, four rounds, where the walk took 187 (8 heads: two rounds).
+// Smaller heads keep the walk: half of the threads here would have nothing to do.
+constexpr int kMatTokens = 64, kMatBlock = 16, kMatCols = 128, kMatThreads = 512, kMatRow = kMatCols + 4, kMatPRow = kMatTokens + 4;
+constexpr size_t kMatSmem = sizeof(float) * (4 * kMatTokens * kMatRow + kMatTokens * kMatPRow + (kMatTokens / kMatBlock) * kMatCols);
+
+__global__ void __launch_bounds__(kMatThreads, 1)
+    gated_chunk_kernel(const float* __restrict__ q_src, const float* __restrict__ f_src, const float* __restrict__ v_src, int P, size_t stride_p, int R,
+                       const float* __restrict__ f_bias, const float* __restrict__ lower, float* __restrict__ o_out, int heads, int D, int V, const int* __restrict__ chunks,
+                       float* __restrict__ chunk_state, float* __restrict__ chunk_decay, float* __restrict__ qa_out) {
+  extern __shared__ __align__(16) float sm[];
+  float *sq = sm, *sf = sq + kMatTokens * kMatRow, *sk = sf + kMatTokens * kMatRow, *sv = sk + kMatTokens * kMatRow, *sp = sv + kMatTokens * kMatRow,   // sp[s][t]
+        *sg = sp + kMatTokens * kMatPRow;   // a block's whole decay [4][128]
+  ib::pdl_launch_dependents();
+  ib::pdl_wait();
+  const int t0 = chunks[2 * blockIdx.x], n = chunks[2 * blockIdx.x + 1], a = blockIdx.y, j0 = blockIdx.z * kMatCols;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  // ---- q, f, k and v of the chunk: a thread keeps its channel (and value column) and takes every fourth token; tokens and channels that are not there
+  // have q = k = v = 0 and f = 1
+  {
+    const int d = tid & 127, j = j0 + d;
+    const bool in_d = d < D, in_j = j < V;
+    const float bias = in_d ? f_bias[a * D + d] : 0.f, lo = in_d ? lower[a * D + d] : 0.f;
+    float zq[16], zf[16], zv[16];   // (everything is requested before the first value is used: one trip to memory)
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      const int t = (tid >> 7) + 4 * e;
+      const size_t row = (size_t)(t0 + t) * R;
+      zq[e] = in_d && t < n ? q_src[row + a * D + d] : 0.f, zf[e] = in_d && t < n ? f_src[row + a * D + d] : 0.f, zv[e] = in_j && t < n ? v_src[row + a * V + j] : 0.f;
+    }
+    for (int p = 1; p < P; p++) {
+#pragma unroll
+      for (int e = 0; e < 16; e++) {
+        const int t = (tid >> 7) + 4 * e;
+        const size_t row = p * stride_p + (size_t)(t0 + t) * R;
+        if (in_d && t < n) zq[e] += q_src[row + a * D + d], zf[e] += f_src[row + a * D + d];
+        if (in_j && t < n) zv[e] += v_src[row + a * V + j];
+      }
+    }
+#pragma unroll
+    for (int e = 0; e < 16; e++) {
+      const int t = (tid >> 7) + 4 * e, at = t * kMatRow + d;
+      const bool live = in_d && t < n;
+      const float sig = 1.f / (1.f + expf(-(zf[e] + bias))), f = live ? __fmaf_rn(1.f - lo, sig, lo) : 1.f;
+      sq[at] = live ? zq[e] / (1.f + expf(-zq[e])) : 0.f;
+      sf[at] = f, sk[at] = 1.f - f, sv[at] = zv[e];
+    }
+    for (int i = tid; i < kMatTokens * kMatPRow; i += kMatThreads) sp[i] = 0.f;
+  }
+  __syncthreads();
+  // ---- p inside the blocks: a warp has four s, eight lanes each with sixteen channels (every eighth group of four)
+  {
+    const int s = 4 * warp + (lane >> 3), ds = lane & 7, end = (warp / 4 + 1) * kMatBlock;
+    float4 w[4];
+#pragma unroll
+    for (int c = 0; c < 4; c++) w[c] = *(const float4*)&sk[s * kMatRow + 4 * (ds + 8 * c)];
+    for (int t = 4 * warp; t < end; t++) {
+      float acc = 0.f;
+#pragma unroll
+      for (int c = 0; c < 4; c++) {
+        const float4 f = *(const float4*)&sf[t * kMatRow + 4 * (ds + 8 * c)], q = *(const float4*)&sq[t * kMatRow + 4 * (ds + 8 * c)];
+        if (t > s) w[c] = make_float4(w[c].x * f.x, w[c].y * f.y, w[c].z * f.z, w[c].w * f.w);
+        acc = fmaf(w[c].x, q.x, fmaf(w[c].y, q.y, fmaf(w[c].z, q.z, fmaf(w[c].w, q.w, acc))));
+      }
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
+      if (ds == 0 && t >= s) sp[s * kMatPRow + t] = acc;
+    }
+  }
+  __syncthreads();
+  // ---- q times the f's of its block up to its token, k times those after it, and the block's product
+  {
+    const int d = tid & 127, b = tid >> 7;
+    float run = 1.f;
+#pragma unroll 4
+    for (int t = b * kMatBlock; t < (b + 1) * kMatBlock; t++) {
+      run *= sf[t * kMatRow + d];
+      sq[t * kMatRow + d] *= run;
+    }
+    float after = 1.f;
+#pragma unroll 4
+    for (int t = (b + 1) * kMatBlock - 1; t >= b * kMatBlock; t--) {
+      sk[t * kMatRow + d] *= after;
+      after *= sf[t * kMatRow + d];
+    }
+    sg[b * kMatCols + d] = run;
+  }
+  __syncthreads();
+  // ---- p across blocks: six pairs of blocks, two warps each; a thread has 4 x 4 of the 16 x 16 over every fourth group of four channels
+  if (warp < 12) {
+    const int pair = warp >> 1, bt = pair < 1 ? 1 : pair < 3 ? 2 : 3, bs = pair - (bt * (bt - 1)) / 2;   // (1,0) (2,0) (2,1) (3,0) (3,1) (3,2)
+    const int ds = lane & 3, th = (warp & 1) * 8 + (lane >> 2), ti = bt * kMatBlock + 4 * (th >> 2), si = bs * kMatBlock + 4 * (th & 3);
+    float acc[4][4];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[i][j] = 0.f;
+#pragma unroll 2
+    for (int c = 4 * ds; c < kMatCols; c += 16) {
+      float4 between = make_float4(1.f, 1.f, 1.f, 1.f);
+      for (int b = bs + 1; b < bt; b++) {
+        const float4 g = *(const float4*)&sg[b * kMatCols + c];
+        between = make_float4(between.x * g.x, between.y * g.y, between.z * g.z, between.w * g.w);
+      }
+      float4 q[4], k[4];
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        q[i] = *(const float4*)&sq[(ti + i) * kMatRow + c], k[i] = *(const float4*)&sk[(si + i) * kMatRow + c];
+        q[i] = make_float4(q[i].x * between.x, q[i].y * between.y, q[i].z * between.z, q[i].w * between.w);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[i][j] = fmaf(q[i].x, k[j].x, fmaf(q[i].y, k[j].y, fmaf(q[i].z, k[j].z, fmaf(q[i].w, k[j].w, acc[i][j]))));
+    }
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 4; j++) {
+        float v = acc[i][j];
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        if (ds == i) sp[(si + j) * kMatPRow + ti + i] = v;
+      }
+  } else if (blockIdx.z == 0) {   // the queries with the decay since the chunk's start, for the incoming state's share, and the chunk's whole decay
+    const int d = tid & 127;
+    if (d < D) {
+      float before = 1.f;
+      for (int b = 0; b < kMatTokens / kMatBlock; b++) {
+#pragma unroll 4
+        for (int t = b * kMatBlock; t < (b + 1) * kMatBlock; t++)
+          if (t < n) qa_out[((size_t)(t0 + t) * heads + a) * D + d] = sq[t * kMatRow + d] * before;
+        before *= sg[b * kMatCols + d];
+      }
+      chunk_decay[((size_t)blockIdx.x * heads + a) * D + d] = before;
+    }
+  }
+  __syncthreads();
+  // ---- k times the f's up to the chunk's end
+  {
+    const int d = tid & 127, b = tid >> 7;
+    float after = 1.f;
+    for (int c = b + 1; c < kMatTokens / kMatBlock; c++) after *= sg[c * kMatCols + d];
+    if (b + 1 < kMatTokens / kMatBlock) {
+#pragma unroll 4
+      for (int t = b * kMatBlock; t < (b + 1) * kMatBlock; t++) sk[t * kMatRow + d] *= after;
+    }
+  }
+  __syncthreads();
+  const int tx = tid & 15, ty = (tid >> 4) & 15;
+  const bool wide = V % 4 == 0 && ((uintptr_t)o_out | (uintptr_t)chunk_state) % 16 == 0;
+  auto store = [&](float* row, const float* v, int j) {   // four values from column j0 + j on
+    if (wide && j0 + j + 3 < V) {
+      *(float4*)(row + j) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; e++)
+        if (j0 + j + e < V) row[j + e] = v[e];
+    }
+  };
+  if (warp < 8) {   // ---- the closing state: rows 4 ty .. and 64 + 4 ty .., columns 4 tx .. and 64 + 4 tx ..
+    float acc[8][8];
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+#pragma unroll
+      for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < kMatTokens; s++) {
+      const float4 k0 = *(const float4*)&sk[s * kMatRow + 4 * ty], k1 = *(const float4*)&sk[s * kMatRow + 64 + 4 * ty];
+      const float4 v0 = *(const float4*)&sv[s * kMatRow + 4 * tx], v1 = *(const float4*)&sv[s * kMatRow + 64 + 4 * tx];
+      const float k[8] = {k0.x, k0.y, k0.z, k0.w, k1.x, k1.y, k1.z, k1.w}, v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+      for (int j = 0; j < 8; j++)
+#pragma unroll
+        for (int i = 0; i < 8; i++) acc[i][j] = fmaf(k[i], v[j], acc[i][j]);
+    }
+    float* S = chunk_state + ((size_t)blockIdx.x * heads + a) * D * V + j0;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      const int d = (i >> 2) * 64 + 4 * ty + (i & 3);
+      if (d >= D) continue;
+      store(S + (size_t)d * V, acc[i], 4 * tx);
+      store(S + (size_t)d * V, acc[i] + 4, 64 + 4 * tx);
+    }
+  } else {   // ---- the outputs: tokens 4 ty .., the same columns
+    float acc[4][8];
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+#pragma unroll
+      for (int j = 0; j < 8; j++) acc[i][j] = 0.f;
+    auto add = [&](int s, auto guard) {
+      const float4 p4 = *(const float4*)&sp[s * kMatPRow + 4 * ty];
+      const float4 v0 = *(const float4*)&sv[s * kMatRow + 4 * tx], v1 = *(const float4*)&sv[s * kMatRow + 64 + 4 * tx];
+      const float p[4] = {p4.x, p4.y, p4.z, p4.w}, v[8] = {v0.x, v0.y, v0.z, v0.w, v1.x, v1.y, v1.z, v1.w};
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        if (decltype(guard)::value && s > 4 * ty + i) continue;   // (a later token adds nothing, whatever its value holds)
+#pragma unroll
+        for (int j = 0; j < 8; j++) acc[i][j] = fmaf(p[i], v[j], acc[i][j]);
+      }
+    };
+    const int first = 8 * (warp - 8);   // a warp's tokens are eight in a row
+#pragma unroll 4
+    for (int s = 0; s < first; s++) add(s, std::false_type());
+#pragma unroll 2
+    for (int s = first; s < first + 8; s++) add(s, std::true_type());
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+      const int t = 4 * ty + i;
+      if (t >= n) continue;
+      float* row = o_out + ((size_t)(t0 + t) * heads + a) * V + j0;
+      store(row, acc[i], 4 * tx);
+      store(row, acc[i] + 4, 64 + 4 * tx);
+    }
+  }
+}
+
 // One thread per element (d, j) of a head's state walks a long segment's chunks in order: the chunk's place in chunk_state receives
 // the state the chunk starts from, and the request's state slot the state after the last chunk.
 __global__ void chunk_carry_kernel(const int* __restrict__ long_segs, const int* __restrict__ seg_slot, float* __restrict__ state, size_t slot_stride,
@@ -678,6 +902,15 @@ int launch_recurrence(const float* q_src, const float* f_src, const float* v_src
   IB_CHECK_ARG(n_segments > 0 && P >= 1 && heads > 0 && D > 0 && V > 0, "recurrence: bad sizes segments=%d P=%d heads=%d D=%d V=%d", n_segments, P, heads, D, V);
   IB_CHECK_ARG(D <= 512, "recurrence: a head's key size %d is above 512", D);
   IB_CHECK_ARG(R >= heads * D && R >= heads * V, "recurrence: rows of %d entries do not hold %d heads of %d and %d", R, heads, D, V);
+  if (chunks && form == 0 && D > 64 && D <= kMatCols && V > 64) {   // see gated_chunk_kernel
+    IB_CHECK_ARG(heads <= 65535 && (V + kMatCols - 1) / kMatCols <= 65535, "recurrence: the grid is too large");
+    cudaError_t e = cudaFuncSetAttribute(gated_chunk_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMatSmem);
+    IB_CHECK_ARG(e == cudaSuccess, "recurrence: cannot reserve %d bytes of shared memory: %s", (int)kMatSmem, cudaGetErrorString(e));
+    ib::launch(gated_chunk_kernel, dim3((unsigned)n_segments, (unsigned)heads, (unsigned)((V + kMatCols - 1) / kMatCols)), kMatThreads, kMatSmem, stream, q_src, f_src, v_src, P,
+               (size_t)stride_p, R, f_bias, lower, o_out, heads, D, V, chunks, chunk_state, chunk_decay, qa);
+    IB_CHECK_LAUNCH("recurrence");
+    return 0;
+  }
   // Four columns a thread halve the work of preparing tokens, which every CTA of a head repeats, and the shared-memory reads a state entry costs;
   // two leave twice the CTAs. Chunk walks of 16 heads of 128 x 128 (us, the form before: one row and column an instruction, items by division):
   // 2,048 tokens 318 to 187 with four; 8 heads 172 to 105; 130 tokens 80 to 51 and 300 of 8 heads 70 to 46 with two. Which one runs changes no
