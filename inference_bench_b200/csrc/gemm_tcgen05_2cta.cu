@@ -469,10 +469,10 @@ __global__ void __launch_bounds__(kThreads, 1)
         }
       } else if constexpr (epi_16(EPI)) {
         // Lane l holds gate row l or, from 16 on, up row l - 16 of the warp's sixteen: one exchange gives each half of the lanes both numbers of every
-        // second token. No branch between the numbers (as in the form below, where 128 columns take 8 us): a thread's sixteen run side by side.
+        // second token. No branch stands between the numbers: a thread's sixteen run side by side.
         const float limit = EPI == EPI_CLAMPED16 ? qe.act_pq[at.group] : 0.f;
         const int n = n_pair + (int)rank * (BM / 2) + q * 16 + (lane & 15), wide = width(at), up = lane >> 4;
-        __nv_bfloat16* dst = (__nv_bfloat16*)out_ + (size_t)(t0 + up) * N + n;
+        __nv_bfloat16* dst = (__nv_bfloat16*)out_;
 #pragma unroll 1
         for (int c0 = 0; c0 < wide; c0 += 32) {
           uint32_t r[32];
@@ -487,10 +487,11 @@ __global__ void __launch_bounds__(kThreads, 1)
             else v[c] = __float2bfloat16_rn(__fdividef(gv, 1.f + __expf(-gv)) * uv);
           }
           if (n < N) {
-            const int left = t_end - t0 - c0 - up;   // tokens of this chunk that are stored: every second one below this
 #pragma unroll
-            for (int c = 0; c < 16; c++)
-              if (2 * c < left) dst[(size_t)(c0 + 2 * c) * N] = v[c];
+            for (int c = 0; c < 16; c++) {
+              const int t = t0 + c0 + 2 * c + up;
+              if (t < t_end) dst[(size_t)t * N + n] = v[c];
+            }
           }
         }
       } else {
@@ -503,14 +504,19 @@ __global__ void __launch_bounds__(kThreads, 1)
           sm100::tmem_ld_32x32b_x32(lane_addr + b * MT * BN + c0, g);
           sm100::tmem_ld_32x32b_x32(lane_addr + b * MT * BN + BN + c0, u);
           sm100::tmem_ld_wait();
+          // All 32 are made before the first is stored: a branch a token kept them from running side by side (2,048 tokens of 12,288 x 4,096
+          // 259 -> 253 us, of 3,072 x 1,024 40 -> 32; 1,003 tokens 148.5 -> 144.4 and 30 -> 26).
+#pragma unroll
+          for (int c = 0; c < 32; c++) {
+            const float gv = __uint_as_float(g[c]), uv = __uint_as_float(u[c]);
+            if constexpr (EPI == EPI_CLAMPED) g[c] = __float_as_uint(ib::clamped_glu<true>(gv, uv, limit, qe.act_slope));
+            else g[c] = __float_as_uint(__fdividef(gv, 1.f + __expf(-gv)) * uv);
+          }
           if (n < N) {
 #pragma unroll
             for (int c = 0; c < 32; c++) {
               const int t = t0 + c0 + c;
-              const float gv = __uint_as_float(g[c]), uv = __uint_as_float(u[c]);
-              if (t >= t_end) continue;
-              if constexpr (EPI == EPI_CLAMPED) dst[(size_t)t * N + n] = __float2bfloat16_rn(ib::clamped_glu<true>(gv, uv, limit, qe.act_slope));
-              else dst[(size_t)t * N + n] = __float2bfloat16_rn(__fdividef(gv, 1.f + __expf(-gv)) * uv);
+              if (t < t_end) dst[(size_t)t * N + n] = __float2bfloat16_rn(__uint_as_float(g[c]));
             }
           }
         }
