@@ -3,7 +3,7 @@
 Steps that hold only decoded tokens are the launch-bound inner loop of generation, so they are
 replayed as CUDA graphs, one per padded batch size (1, 2, 4, ... rows), like the reference's
 `Stepper` (crates/specrt/src/runtime/step.rs:8-20, 197-228): all inputs of such a step live in one
-static device buffer that a single copy fills, padded rows write to a scratch page and a scratch
+static device buffer that a single copy (or the step itself) fills, padded rows write to a scratch page and a scratch
 slot, and the graph holds the whole model, the sampling kernel included.
 """
 from __future__ import annotations
@@ -13,6 +13,7 @@ from typing import Optional
 import numpy as np
 import torch
 
+from ..kernels import ops
 from ..sampling.params import SamplingParams
 from ..sampling.sampler import Sampler
 from .context import Segment, StepContext
@@ -23,15 +24,16 @@ RUN_AHEAD_MAX = 64
 
 
 class _DecodeGraph:
-    """The captured decode step for `rows` rows and the static buffers it reads and writes."""
+    """The captured decode step for `rows` rows and the static buffers it reads and writes. alone: a step that the host waits for (`run`); it fetches its
+    inputs from the pinned block and leaves its tokens there itself. Otherwise the inputs are copied in front of it (`launch`, `run_ahead`)."""
 
-    def __init__(self, runner: ModelRunner, rows: int):
-        self.runner, self.rows = runner, rows
+    def __init__(self, runner: ModelRunner, rows: int, alone: bool):
+        self.runner, self.rows, self.alone = runner, rows, alone
         cache, rt = runner.cache, runner.rt
         B, W = rows, cache.table_width
         n_groups = len(cache.groups)
         # layout of the int32 input block: tokens | positions | seg_pos0 | seg_slot | params[B,6] | tables[g][B,W] | count
-        self.n_ints = 4 * B + 6 * B + n_groups * B * W + 1
+        self.n_ints = (4 * B + 6 * B + n_groups * B * W + 1 + 3) // 4 * 4
         self.host = torch.zeros(self.n_ints, dtype=torch.int32).pin_memory()
         self.dev = torch.zeros(self.n_ints, dtype=torch.int32, device=rt.device)
         h = self.host.numpy()
@@ -55,6 +57,7 @@ class _DecodeGraph:
         self.result = torch.zeros(B + 1, dtype=torch.int32, device=rt.device)   # the step's tokens, then the status word after the step
         self.tokens = self.result[:B]
         self.h_out = torch.zeros(B + 1, dtype=torch.int32).pin_memory()
+        self.np_out = self.h_out.numpy()
         # for steps launched without waiting (two may be in flight): a staging copy of the inputs, a place for the tokens and an event each
         self.stages = [torch.zeros(self.n_ints, dtype=torch.int32).pin_memory() for _ in range(2)]
         self.h_outs = [torch.zeros(B + 1, dtype=torch.int32).pin_memory() for _ in range(2)]
@@ -76,16 +79,15 @@ class _DecodeGraph:
             t[:] = cache.scratch_page(g)
 
     def _forward(self) -> None:
-        from ..kernels import ops
         self.ctx.memo = {}
         self.logits = self.runner.decoder.forward(self.ctx)
         ops.sample_rows(self.logits, self.d_params, self.result, self.runner.rt.status)
         c = self.ctx
-        ops.advance_rows(self.tokens, c.token_ids, c.positions, c.seg_pos0, self.d_params, self.history, self.d_count)
+        ops.advance_rows(self.tokens, c.token_ids, c.positions, c.seg_pos0, self.d_params, self.history, self.d_count, self.h_out if self.alone else None)
 
     def capture(self) -> None:
         self.runner.rt.activate()
-        self.dev.copy_(self.host, non_blocking=True)
+        ops.fetch_ints(self.host, self.dev)
         stream = torch.cuda.Stream(device=self.runner.rt.device)
         stream.wait_stream(torch.cuda.current_stream())
         with torch.cuda.stream(stream):
@@ -97,6 +99,8 @@ class _DecodeGraph:
         before = lib.launches
         self.graph = torch.cuda.CUDAGraph()
         with torch.cuda.graph(self.graph):
+            if self.alone:
+                ops.fetch_ints(self.host, self.dev)
             self._forward()
         self.launches = lib.launches - before    # kernels in one replay
 
@@ -119,14 +123,12 @@ class _DecodeGraph:
 
     def run(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], reqs: list, rows) -> list[int]:
         """reqs, rows: the entries' requests and their slots (`CacheManager.rows`)."""
-        n = len(entries)
         self._fill(entries, sampling, reqs, rows)
-        self.dev.copy_(self.host, non_blocking=True)
         self.graph.replay()
-        self.h_out.copy_(self.result, non_blocking=True)
         torch.cuda.current_stream(self.runner.rt.device).synchronize()
-        self.runner.rt.raise_for(int(self.h_out[self.rows]))
-        return self.h_out[:n].tolist()
+        out = self.np_out.tolist()
+        self.runner.rt.raise_for(out[self.rows])
+        return out[:len(entries)]
 
     def launch(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], feed: bool, reqs: list, rows) -> tuple[int, int]:
         """Enqueue one step and return at once. With `feed` the input tokens stay what the step before
@@ -178,26 +180,27 @@ class GpuExecutor:
         self.runner = runner
         self.sampler = Sampler(runner.rt.device)
         self.use_graphs, self.max_graph_rows = use_graphs, max_graph_rows
-        self._graphs: dict[int, _DecodeGraph] = {}
+        self._graphs: dict[tuple[int, bool], _DecodeGraph] = {}
         self.last_logits: Optional[torch.Tensor] = None
         self.steps = 0
         self.h2d_bytes = 0
         self.d2h_bytes = 0
 
-    def graph_for(self, n_rows: int) -> _DecodeGraph:
+    def graph_for(self, n_rows: int, alone: bool = True) -> _DecodeGraph:
+        """The captured step for this many rows, in the form of `execute` or that of `launch_decode` and `decode_ahead`."""
         rows = 1
         while rows < n_rows:
             rows *= 2
-        g = self._graphs.get(rows)
+        g = self._graphs.get((rows, alone))
         if g is None:
-            g = self._graphs[rows] = _DecodeGraph(self.runner, rows)
+            g = self._graphs[rows, alone] = _DecodeGraph(self.runner, rows, alone)
             g.capture()
         return g
 
     def decode_ahead(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], steps: int) -> list[list[int]]:
         """Several decode steps of the same requests in a row, tokens fed back on the device."""
         cache = self.runner.cache
-        g = self.graph_for(len(entries))
+        g = self.graph_for(len(entries), alone=False)
         reqs = [e.request for e in entries]
         rows = cache.rows(reqs)
         cache.extend_rows(reqs, rows, steps)
@@ -219,7 +222,7 @@ class GpuExecutor:
             for e in entries:
                 if not 0 <= e.tokens[0] < self.runner.vocab:
                     raise ValueError(f"request {e.request!r}: token id {e.tokens[0]} is outside the vocabulary of {self.runner.vocab}")
-        g = self.graph_for(len(entries))
+        g = self.graph_for(len(entries), alone=False)
         reqs = [e.request for e in entries]
         rows = cache.rows(reqs)
         try:

@@ -85,7 +85,8 @@ _SIGNATURES = {
     "ib_attention_generic": [_p, _i, C.POINTER(KvView), _p, _p, _i, _f, _p, _i, _i, _p, _i, _i, _f, _i, _i, _p, _p, _i, _ll, _i, _f, _i, _i, _p, _p],
     "ib_gemm_simt": [_p, _i, _p, _i, _p, _i, _i, _i, _p],
     "ib_sample_rows": [_p, _i, _i, _p, _p, _p, _p, _p],
-    "ib_advance_rows": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _p],
+    "ib_advance_rows": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _p, _p],
+    "ib_fetch_ints": [_p, _p, _i, _p],
 }
 
 _lib: Optional[C.CDLL] = None

@@ -326,16 +326,27 @@ def sample_rows(logits: torch.Tensor, params: torch.Tensor, tokens: torch.Tensor
 
 
 def advance_rows(sampled: torch.Tensor, token_in: torch.Tensor, positions: torch.Tensor, pos0: torch.Tensor, params: torch.Tensor,
-                 history: torch.Tensor, count: torch.Tensor) -> None:
-    """Feed sampled tokens back as the next inputs of a decode batch and log them: history[count, :] = sampled."""
+                 history: torch.Tensor, count: torch.Tensor, host: Optional[torch.Tensor] = None) -> None:
+    """Feed sampled tokens back as the next inputs of a decode batch and log them: history[count, :] = sampled. host: pinned int32 [rows + 1] that receives
+    them as well, and the word behind them (`sample_rows` with a status word leaves one there)."""
     rows = sampled.shape[0]
+    if host is not None and not (host.is_pinned() and host.is_contiguous() and host.dtype == torch.int32 and host.shape == (rows + 1,)):
+        raise L.KernelError(f"advance_rows: the host's copy must be pinned int32 [{rows + 1}]")
     for name, t in (("sampled", sampled), ("token_in", token_in), ("positions", positions), ("pos0", pos0)):
         _check(name, t, torch.int32, (rows,))
     _check("params", params, torch.int32, (rows, 6))
     _check("history", history, torch.int32)
     _check("count", count, torch.int32, (1,))
     L.call("ib_advance_rows", sampled.data_ptr(), token_in.data_ptr(), positions.data_ptr(), pos0.data_ptr(), params.data_ptr(), history.data_ptr(),
-           count.data_ptr(), rows, history.shape[0], _stream())
+           count.data_ptr(), rows, history.shape[0], _ptr(host), _stream())
+
+
+def fetch_ints(host: torch.Tensor, dev: torch.Tensor) -> None:
+    """dev = host (pinned memory), both int32 of one length, a multiple of four."""
+    _check("dev", dev, torch.int32, (host.shape[0],))
+    if not (host.is_pinned() and host.is_contiguous() and host.dtype == torch.int32):
+        raise L.KernelError("fetch_ints: the source must be pinned int32")
+    L.call("ib_fetch_ints", host.data_ptr(), dev.data_ptr(), host.shape[0], _stream())
 
 
 # ---------------------------------------------------------------- norm on a sublayer's output
