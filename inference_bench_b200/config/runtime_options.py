@@ -32,7 +32,7 @@ class RuntimeOptions:
     dtype: str = "bfloat16"            # "bfloat16": what serving uses; "float32": every tensor and product in IEEE float32
     gemm: str = "auto"                 # "auto": tcgen05 in bfloat16 where the sizes allow; "simt": the FMA kernel; "tcgen05": refuse sizes it cannot take
     pair_min_tokens: int = 129         # the fused gate/up product runs on the CTA-pair kernel from this many tokens on
-    pair_always_tokens: int = 2048     # every product does from here on; between the two a cost model decides
+    pair_always_tokens: int = 2048     # every product that gives each CTA pair a tile, or adds to the stream, does from here on; otherwise a cost model decides
     # ---- launches
     graphs: bool = True                # replay steps of decoded tokens as CUDA graphs
     pdl: bool = True                   # programmatic dependent launch: a kernel's set-up overlaps the tail of the one before

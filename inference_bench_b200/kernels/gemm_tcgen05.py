@@ -39,7 +39,7 @@ L.register("ib_gemm_grouped_swiglu_tcgen05", [L._p, L._p, L._p, L._i, L._i, L._i
 
 # Runtime options that steer the choice (config/runtime_options.py): `pair_min_tokens` (129: the fused gate/up product runs on the
 # persistent CTA-pair kernel, csrc/gemm_tcgen05_2cta.cu, from here on whatever its size), `pair_always_tokens` (2,048: every
-# product from here on; between the two, `plan` decides by its cost model) and `fuse_qkv_epilogue`.
+# product that gives each pair a tile or adds to the stream from here on; otherwise `plan` decides by its cost model) and `fuse_qkv_epilogue`.
 
 
 def supports(k: int) -> bool:
@@ -191,10 +191,19 @@ def gemm_qkv_pair(x: torch.Tensor, w: torch.Tensor, q_out: torch.Tensor, kv: "op
            positions.data_ptr(), seg_of_token.data_ptr(), q_out.data_ptr(), C.byref(view), 1 if write_kv else 0, heads, status.data_ptr(), ops._stream())
 
 
+def _fills_pairs(T: int, n: int, sm_count: int) -> bool:
+    """Whether a product's 256 x 256 tiles give every CTA pair one. Below that the cost model decides at any number of tokens, for a product that nothing is
+    added to: 2,048 tokens of 64 x 2,048 20.5 us on pairs, 14.3 with the k-range cut; of 2,048 x 2,816 27.6 and 32.8 (it stays)."""
+    return -(-n // 256) * -(-T // 256) >= sm_count // 2
+
+
 def product_form(rt, T: int, n: int, k: int, allow_split: bool = True, add: bool = False) -> tuple:
     """How a product of T tokens with an [n, k] matrix runs: ("single", tokens per CTA, k-splits, wide), ("pair",), or with `add` (the caller has a stream
     it may be added to) ("add",) in the place of the latter."""
-    how = ("pair",) if T >= rt.options.pair_always_tokens else (plan(T, n, k, rt.sm_count, allow_split) if T > 128 else ("single", *choose(T, n, k, allow_split, rt.sm_count)))
+    if T >= rt.options.pair_always_tokens and (add or T <= 128 or _fills_pairs(T, n, rt.sm_count)):
+        how = ("pair",)
+    else:
+        how = plan(T, n, k, rt.sm_count, allow_split) if T > 128 else ("single", *choose(T, n, k, allow_split, rt.sm_count))
     return ("add",) if add and how[0] == "pair" else how
 
 
