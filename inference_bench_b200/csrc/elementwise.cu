@@ -55,24 +55,27 @@ __global__ void embed_kernel(const W* __restrict__ table, const int* __restrict_
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < H; i += gridDim.x * blockDim.x) dst[i] = ib::to_f32<W>(src[i]);
 }
 
-// The same with 16-byte accesses (rows of a multiple of 16 bytes): a CTA per token, four chunks requested a thread before the first is used. With one
-// value a thread and 256 a CTA the launch of the CTAs was the bound: 2,048 tokens of 4,096 48 us, now 26; 4,152 tokens 86 us, now 39; 64 tokens 17 us, now 12.
+// The same with four values an access (rows of a multiple of 16 bytes): a CTA per token, eight accesses requested a thread before the first is used, and
+// neighbouring threads' stores side by side (with eight bfloat16 values a thread, every store filled half of each 32 bytes it touched). Bound by the
+// bytes and three trips to memory. 2,048 tokens of 4,096 bfloat16 values: 48 us with one value a thread, 18.5 with a CTA a token and eight
+// values an access, 14.3 now (timed with the caches cold, 2 us of it the launch); 4,152 tokens 26.6 and 22.6.
 template <typename W>
 __global__ void __launch_bounds__(128) embed_vec_kernel(const W* __restrict__ table, const int* __restrict__ tokens, float* __restrict__ x, int H, int V,
                                                         unsigned* __restrict__ status) {
-  constexpr int PER = 16 / sizeof(W), U = 4;
+  constexpr int U = 8;
+  using V4 = std::conditional_t<sizeof(W) == 4, uint4, uint2>;   // four values
   ib::pdl_launch_dependents();
   ib::pdl_wait();
-  const int t = blockIdx.x, chunks = H / PER;
+  const int t = blockIdx.x, chunks = H / 4;
   int tok = tokens[t];
   if (tok < 0 || tok >= V) {
     if (threadIdx.x == 0) atomicOr(status, IB_ERR_BAD_TOKEN);
     tok = 0;
   }
-  const uint4* src = (const uint4*)(table + (size_t)tok * H);
+  const V4* src = (const V4*)(table + (size_t)tok * H);
   float4* dst = (float4*)(x + (size_t)t * H);
   for (int c0 = threadIdx.x; c0 < chunks; c0 += U * 128) {
-    uint4 v[U];
+    V4 v[U];
 #pragma unroll
     for (int u = 0; u < U; u++)
       if (c0 + u * 128 < chunks) v[u] = src[c0 + u * 128];
@@ -85,8 +88,7 @@ __global__ void __launch_bounds__(128) embed_vec_kernel(const W* __restrict__ ta
       } else {
         auto lo = [](uint32_t w) { return __uint_as_float(w << 16); };
         auto hi = [](uint32_t w) { return __uint_as_float(w & 0xffff0000u); };
-        dst[2 * c] = make_float4(lo(v[u].x), hi(v[u].x), lo(v[u].y), hi(v[u].y));
-        dst[2 * c + 1] = make_float4(lo(v[u].z), hi(v[u].z), lo(v[u].w), hi(v[u].w));
+        dst[c] = make_float4(lo(v[u].x), hi(v[u].x), lo(v[u].y), hi(v[u].y));
       }
     }
   }
@@ -310,6 +312,37 @@ __global__ void rope_table_kernel(const int* __restrict__ positions, const float
 // gu[p][t][0:I] = gate, gu[p][t][I:2I] = up (partials summed first); act = g / (1 + exp(-g)) * u, or with a limit the
 // pair with clamped halves (ib::clamped_glu).
 template <typename O>
+__device__ __forceinline__ O silu_mul_one(float g, float u, const float* limit, float slope) {
+  return ib::from_f32<O>(limit ? ib::clamped_glu<false>(g, u, limit[0], slope) : (g / (1.f + expf(-g))) * u);
+}
+
+// Four values a thread (I a multiple of four, rows on 16 bytes), the partial sums of both halves requested four at a time and added in order: a trip to
+// memory where there were as many as partial sums. 777 tokens of 3,072 float32 values: 18.4 us with one value a thread, 12.3 now; 300 of 12,288: 24.5 and
+// 16.4; 64 tokens of 3,072 in four partial sums 10.2 and 8.2 (timed with the caches cold).
+template <typename O>
+__global__ void __launch_bounds__(128) silu_mul_vec_kernel(const float* __restrict__ gu, int P, size_t stride, O* __restrict__ act, int I, const float* __restrict__ limit, float slope) {
+  ib::pdl_launch_dependents();
+  ib::pdl_wait();
+  const int t = blockIdx.y, i = (blockIdx.x * 128 + threadIdx.x) * 4;
+  if (i >= I) return;
+  const float* row = gu + (size_t)t * 2 * I + i;
+  float4 g = *(const float4*)row, u = *(const float4*)(row + I);
+  for (int p0 = 1; p0 < P; p0 += 4) {
+    float4 a[4], b[4];
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+      if (p0 + p < P) a[p] = *(const float4*)(row + (p0 + p) * stride), b[p] = *(const float4*)(row + (p0 + p) * stride + I);
+#pragma unroll
+    for (int p = 0; p < 4; p++)
+      if (p0 + p < P) g.x += a[p].x, g.y += a[p].y, g.z += a[p].z, g.w += a[p].w, u.x += b[p].x, u.y += b[p].y, u.z += b[p].z, u.w += b[p].w;
+  }
+  alignas(16) O v[4] = {silu_mul_one<O>(g.x, u.x, limit, slope), silu_mul_one<O>(g.y, u.y, limit, slope), silu_mul_one<O>(g.z, u.z, limit, slope), silu_mul_one<O>(g.w, u.w, limit, slope)};
+  O* to = act + (size_t)t * I + i;
+  if constexpr (sizeof(O) == 4) *(float4*)to = make_float4(v[0], v[1], v[2], v[3]);
+  else *(uint2*)to = *(uint2*)v;
+}
+
+template <typename O>
 __global__ void silu_mul_kernel(const float* __restrict__ gu, int P, size_t stride, O* __restrict__ act, int I, const float* __restrict__ limit, float slope) {
   ib::pdl_launch_dependents();
   ib::pdl_wait();
@@ -321,7 +354,7 @@ __global__ void silu_mul_kernel(const float* __restrict__ gu, int P, size_t stri
       g += row[p * stride + i];
       u += row[p * stride + I + i];
     }
-    act[(size_t)t * I + i] = ib::from_f32<O>(limit ? ib::clamped_glu<false>(g, u, limit[0], slope) : (g / (1.f + expf(-g))) * u);
+    act[(size_t)t * I + i] = silu_mul_one<O>(g, u, limit, slope);
   }
 }
 
@@ -514,6 +547,13 @@ extern "C" int ib_silu_mul(const float* gu, int P, long long stride, void* act, 
   if (T == 0) return 0;
   IB_CHECK_ARG(T > 0 && I > 0 && P >= 1, "silu_mul: bad sizes T=%d I=%d P=%d", T, I, P);
   IB_CHECK_ARG(T <= 65535, "silu_mul: T=%d rows exceed the grid limit 65535", T);
+  if (I % 4 == 0 && stride % 4 == 0 && (((uintptr_t)gu | (uintptr_t)act) & 15) == 0 && (act_dtype == IB_F32 || act_dtype == IB_BF16)) {
+    const dim3 vec((I / 4 + 127) / 128, T);
+    if (act_dtype == IB_F32) ib::launch(silu_mul_vec_kernel<float>, vec, 128, 0, stream, gu, P, (size_t)stride, (float*)act, I, limit, slope);
+    else ib::launch(silu_mul_vec_kernel<__nv_bfloat16>, vec, 128, 0, stream, gu, P, (size_t)stride, (__nv_bfloat16*)act, I, limit, slope);
+    IB_CHECK_LAUNCH("silu_mul");
+    return 0;
+  }
   dim3 grid((I + 255) / 256, T);
   if (grid.x > 64) grid.x = 64;
   if (act_dtype == IB_F32)
