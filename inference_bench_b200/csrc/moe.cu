@@ -26,14 +26,11 @@ namespace {
 
 constexpr int kRouteWarps = 4;
 
-// (value, index) argmax over a warp: larger value wins, then the lower index.
-__device__ __forceinline__ void warp_argmax(float& v, int& i) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    const float ov = __shfl_xor_sync(0xffffffffu, v, o);
-    const int oi = __shfl_xor_sync(0xffffffffu, i, o);
-    if (ov > v || (ov == v && oi < i)) v = ov, i = oi;
-  }
+// Index of the largest value over a warp (no NaN): the larger value wins, then the lower index. Two reductions over whole numbers (the
+// value's bits in an order that is the numbers', zeros of both signs alike) where exchanges of value and index take ten.
+__device__ __forceinline__ int warp_argmax(float v, int i) {
+  const unsigned b = __float_as_uint(v + 0.f), key = b ^ ((int)b < 0 ? 0xffffffffu : 0x80000000u);
+  return __reduce_min_sync(0xffffffffu, key == __reduce_max_sync(0xffffffffu, key) ? i : 0x7fffffff);
 }
 
 struct RouteArgs {
@@ -54,15 +51,26 @@ struct RouteArgs {
 };
 
 // One warp routes token t; `s` holds 2 E + n_groups floats of shared memory of its own. Choice scores may be negative: what cannot be
-// chosen counts as minus infinity.
+// chosen counts as minus infinity. A chain of dependent steps bounds it, one a kept group and one a choice, not bytes: each is two warp
+// reductions, the weights stay in registers until they are scaled and stored once, and partial sums are requested together. 2,048 tokens,
+// 64 experts in 8 groups of which 4 are kept, 6 choices, 6 partial sums: 18.4 us with exchanges, one load after the other and weights
+// rescaled in memory, 12.3 us so (about 4 us of both are the launch).
 __device__ __forceinline__ void route_token(const RouteArgs& a, int t, float* s, int lane) {
   const int E = a.E;
   float* c = s + E;
   float* g = c + E;
   float mx = -INFINITY;
   for (int e = lane; e < E; e += 32) {
-    float z = a.logits[(size_t)t * a.row + e];
-    for (int p = 1; p < a.P; p++) z += a.logits[p * a.stride_p + (size_t)t * a.row + e];
+    const float* src = a.logits + (size_t)t * a.row + e;
+    float z = src[0];
+    for (int p0 = 1; p0 < a.P; p0 += 8) {   // eight partial sums requested together, added in order
+      float v[8];
+#pragma unroll
+      for (int p = 0; p < 8; p++) v[p] = p0 + p < a.P ? src[(p0 + p) * a.stride_p] : 0.f;
+#pragma unroll
+      for (int p = 0; p < 8; p++)
+        if (p0 + p < a.P) z += v[p];
+    }
     if (a.logit_bias) z += a.logit_bias[e];
     s[e] = z;
     mx = fmaxf(mx, z);
@@ -107,7 +115,7 @@ __device__ __forceinline__ void route_token(const RouteArgs& a, int t, float* s,
       int bi = 0x7fffffff;
       for (int k = lane; k < a.n_groups; k += 32)
         if (g[k] == g[k] && (bi == 0x7fffffff || g[k] > bv)) bv = g[k], bi = k;
-      warp_argmax(bv, bi);
+      bi = warp_argmax(bv, bi);
       if (lane == 0 && bi < a.n_groups) g[bi] = __int_as_float(0x7fc00000);
       __syncwarp();
     }
@@ -115,13 +123,14 @@ __device__ __forceinline__ void route_token(const RouteArgs& a, int t, float* s,
       if (g[e / per] == g[e / per]) c[e] = -INFINITY;   // its group was not kept
     __syncwarp();
   }
-  float chosen_sum = 0.f, chosen_max = 0.f;
+  float chosen_sum = 0.f, chosen_max = 0.f, own_w = 0.f;   // lane r % 32 holds choice r until it is stored
+  int own = 0;
   for (int r = 0; r < a.top; r++) {
     float bv = -INFINITY;
     int bi = 0x7fffffff;
     for (int e = lane; e < E; e += 32)
       if (c[e] > bv) bv = c[e], bi = e;
-    warp_argmax(bv, bi);
+    bi = warp_argmax(bv, bi);
     float w = 0.f;
     if (bi >= E) {   // fewer experts that can be chosen than choices: weight zero
       bi = 0;
@@ -131,17 +140,23 @@ __device__ __forceinline__ void route_token(const RouteArgs& a, int t, float* s,
     } else {
       w = s[bi];
     }
-    if (lane == 0) {
-      a.idx_out[(size_t)t * a.row_out() + r] = bi;
-      a.wt_out[(size_t)t * a.row_out() + r] = w;
-      c[bi] = -INFINITY;
+    if (lane == r % 32) {   // choices 32, 64, ... of a token with more are stored as they come
+      if (r >= 32) {
+        a.idx_out[(size_t)t * a.row_out() + r - 32] = own;
+        a.wt_out[(size_t)t * a.row_out() + r - 32] = own_w;
+      }
+      own = bi, own_w = w;
     }
+    if (lane == 0) c[bi] = -INFINITY;
     chosen_sum += w;
     __syncwarp();
   }
-  if (lane == 0) {
-    const float f = a.renorm ? a.route_scale / (chosen_sum + 1e-20f) : a.route_scale;
-    for (int r = 0; r < a.top; r++) a.wt_out[(size_t)t * a.row_out() + r] *= f;
+  const float f = a.renorm ? a.route_scale / (chosen_sum + 1e-20f) : a.route_scale;
+  const int last = a.top - 1 - (a.top - 1 - lane) % 32;   // the choice that is still here
+  if (lane < a.top) {
+    a.idx_out[(size_t)t * a.row_out() + last] = own;
+    a.wt_out[(size_t)t * a.row_out() + last] = own_w * f;
+    for (int r = lane; r < last; r += 32) a.wt_out[(size_t)t * a.row_out() + r] *= f;
   }
   for (int r = lane; r < a.always; r += 32) {
     float w = 1.f;
