@@ -17,9 +17,13 @@
 // (MMAs, copies) run one instruction stream each, and the loop is as fast as the slowest of them: what
 // they do per tile is kept to the instructions themselves (descriptors are a constant apart, buffers and
 // parities are counted, a wait that is already over costs one try).
+// With few query tiles their keys are cut into slices (SLICED): a thread-block cluster has a CTA per slice, each leaves its (maximum, sum, O) in shared
+// memory, and each merges a share of the rows out of the others', in float32 and in the order of the slices.
 // Needs the tensor map of the cache pool (ib_make_kv_map): page sizes that are a multiple of 8 and
 // divide 64, or a multiple of 64. Reference design: crates/kir/src/cuda/attention/flash_mma.rs.
 #include <cuda.h>
+
+#include <algorithm>
 
 #include "kv_view.cuh"
 #include "mma_tiles.cuh"
@@ -69,6 +73,25 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
+// The same place of shared memory in CTA `rank` of the cluster, and loads from there.
+__device__ __forceinline__ uint32_t peer_addr(uint32_t addr, int rank) {
+  uint32_t d;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(d) : "r"(addr), "r"(rank));
+  return d;
+}
+__device__ __forceinline__ float2 peer_ld2(uint32_t addr) {
+  float2 v;
+  asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ float4 peer_ld4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ void cluster_sync() {   // every thread of every CTA of the cluster (one that has left counts as arrived)
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void bar_sync_softmax() { asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxWarps * 32) : "memory"); }
 
 template <int HD>
@@ -79,9 +102,16 @@ struct Smem {
   static constexpr int kBars = KS + 2 * VS + 5;
   static constexpr int kBytes = oBar + kBars * 8 + 16;
   static_assert(kBytes <= 113 * 1024, "two CTAs must fit one SM");
+  // a slice's result, once no tile is needed any more: (maximum, sum) of the rows over Q, O over the K and V tiles in rows of HD + 4 floats
+  // (threads of neighbouring rows then store 16 bytes each without bank conflicts)
+  static constexpr int kRowO = HD + 4;
+  static_assert(BM * kRowO * 4 <= oBar - oK && BM * 8 + BM * 9 * 4 <= kQ, "a slice's result must fit the tiles");
 };
 
-template <int HD>
+constexpr int kMaxSlices = 8;
+
+// SLICED: the key tiles of a query tile are cut into as many slices as the cluster has CTAs (blockIdx.z is the rank).
+template <int HD, bool SLICED>
 __global__ void __launch_bounds__(kThreads, 2)
     prefill_ws_kernel(const __nv_bfloat16* __restrict__ q, IbKvView kv, const int* __restrict__ tile_seg, const int* __restrict__ tile_row0,
                       const int* __restrict__ seg_start, const int* __restrict__ seg_pos0, int window, float scale_log2e,
@@ -141,8 +171,11 @@ __global__ void __launch_bounds__(kThreads, 2)
   const int lo_last = ib::first_visible(pos_last, window);   // a tile of keys from here on is seen by every row whose position has come
   const int kt_begin = key_lo / BN, kt_end = pos_last / BN + 1;
   const int n_pre = min((keep + BN - 1) / BN, kt_begin);   // tiles of kept keys before the window's first tile
-  const int n_kt = n_pre + kt_end - kt_begin;
-  auto key_tile = [&](int j) { return j < n_pre ? j : kt_begin + j - n_pre; };   // the j-th tile of keys that this CTA walks
+  const int n_all = n_pre + kt_end - kt_begin;
+  const int slices = SLICED ? gridDim.z : 1, slice = SLICED ? blockIdx.z : 0;
+  const int j0 = SLICED ? n_all * slice / slices : 0;   // this CTA's tiles: j0 .. j0 + n_kt - 1 of the query tile's (there may be none)
+  const int n_kt = SLICED ? n_all * (slice + 1) / slices - j0 : n_all;
+  auto key_tile = [&](int j) { return j < n_pre ? j : kt_begin + j - n_pre; };   // the j-th tile of keys that the query tile sees
   // a wait that ran out: say so once, and from then on nobody waits (the results are void, the status says so)
   auto wait = [&](uint64_t* bar, uint32_t parity) {
     if (sm100::mbar_try_wait(bar, parity) || *gave_up) return;
@@ -174,9 +207,10 @@ __global__ void __launch_bounds__(kThreads, 2)
     int st = 0;
     uint32_t par = 1;   // the parity to wait for before a buffer is filled again: of s_full (K), of v_empty (V)
     for (int j = 0; j < n_kt; j++) {
-      const int rel = j * ppt;
-      if ((rel & 31) == 0) {   // the pages of the next 32 boxes, one per lane
-        const int box = rel + lane < n_pre * ppt ? rel + lane : (kt_begin - n_pre) * ppt + rel + lane;
+      const int rel = (j0 + j) * ppt;
+      if ((rel & 31) == 0 || (SLICED && j == 0)) {   // the pages of these 32 boxes, one per lane
+        const int at = (rel & ~31) + lane;
+        const int box = at < n_pre * ppt ? at : (kt_begin - n_pre) * ppt + at;
         const int key0 = box * box_rows;
         held_row = -1;
         if (key0 <= pos_last && (key0 + box_rows > key_lo || key0 < keep)) {
@@ -214,7 +248,7 @@ __global__ void __launch_bounds__(kThreads, 2)
     }
   } else if (warp == kSoftmaxWarps) {
     // ------------------------------------------------------------ the MMA warp (one lane issues)
-    if (lane == 0) {
+    if (lane == 0 && n_kt > 0) {
       constexpr uint32_t idesc_s = sm100::idesc_bf16_f32(BM, BN);
       constexpr uint32_t idesc_o = sm100::idesc_bf16_f32_b_mn(BM, HD);
       // Only the address field of a shared-memory descriptor changes from one MMA to the next (16-byte units), so every
@@ -273,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 
     float m_ref = -INFINITY, l = 0.f;
     for (int j = 0; j < n_kt; j++) {
-      const int kt = key_tile(j);
+      const int kt = key_tile(j0 + j);
       wait(&s_full[j & 1], (j >> 1) & 1);
       sm100::tc_fence_after();
       uint32_t sr[BN];
@@ -352,10 +386,26 @@ __global__ void __launch_bounds__(kThreads, 2)
       __syncwarp();
       if (lane == 0) sm100::mbar_arrive(&p_full[j & 1]);
     }
-    // ---- O / l -> out
-    wait(&v_empty[(n_kt - 1) % VS], ((n_kt - 1) / VS) & 1);
-    sm100::tc_fence_after();
-    if (!*gave_up) {
+    if (!SLICED || n_kt > 0) {
+      wait(&v_empty[(n_kt - 1) % VS], ((n_kt - 1) / VS) & 1);
+      sm100::tc_fence_after();
+    }
+    if constexpr (SLICED) {   // ---- (maximum, sum) and O -> shared memory, for the cluster's CTAs to merge
+      const bool has = n_kt > 0 && !*gave_up;
+      ((float2*)(sm + SM::oQ))[row] = make_float2(has ? m_ref : -INFINITY, has ? l : 0.f);
+      float4* dst = (float4*)((float*)(sm + SM::oK) + row * SM::kRowO);
+      if (has) {
+#pragma unroll 1
+        for (int c0 = 0; c0 < HD; c0 += 32) {
+          uint32_t o[32];
+          sm100::tmem_ld_32x32b_x32(t_lane + 2 * BN + c0, o);
+          sm100::tmem_ld_wait();
+#pragma unroll
+          for (int c = 0; c < 32; c += 4)
+            dst[(c0 + c) / 4] = make_float4(__uint_as_float(o[c]), __uint_as_float(o[c + 1]), __uint_as_float(o[c + 2]), __uint_as_float(o[c + 3]));
+        }
+      }
+    } else if (!*gave_up) {   // ---- O / l -> out
       // the sink's weight in the units of the running sum (a row that saw no key: infinite, the output is zero)
       if (sink) l += ex2((tail.sink_values ? tail.sink_values[h] * 1.4426950408889634f : 0.f) - m_ref);
       float inv = l > 0.f ? 1.f / l : 0.f;
@@ -387,21 +437,117 @@ __global__ void __launch_bounds__(kThreads, 2)
     __syncwarp();
     sm100::tmem_dealloc(tmem, kTmemCols);
   }
+  if constexpr (SLICED) {   // each CTA merges its share of the rows: O = sum of 2^(m_i - M) O_i over the slices, in their order, and the same of the sums
+    __syncwarp();
+    cluster_sync();
+    constexpr int QPR = HD / 4, U = 2;
+    const int share = (rows + slices - 1) / slices, r0 = slice * share, n_own = max(min(rows - r0, share), 0);
+    float* const f_s = (float*)(sm + SM::oQ + BM * 8);   // [share][kMaxSlices]: the factors of a row's slices, -1 for one in which it saw no key
+    if (tid < n_own) {
+      float2 ml[kMaxSlices];
+      float M = -INFINITY, l = 0.f;
+#pragma unroll
+      for (int i = 0; i < kMaxSlices; i++) ml[i] = i < slices ? peer_ld2(peer_addr(q_s + (r0 + tid) * 8, i)) : make_float2(-INFINITY, 0.f);
+#pragma unroll
+      for (int i = 0; i < kMaxSlices; i++) M = fmaxf(M, ml[i].x);
+#pragma unroll
+      for (int i = 0; i < kMaxSlices; i++)
+        if (ml[i].x != -INFINITY) l = fmaf(ml[i].y, ex2(ml[i].x - M), l);
+      if (sink) l += ex2((tail.sink_values ? tail.sink_values[h] * 1.4426950408889634f : 0.f) - M);
+      const float inv = (l > 0.f ? 1.f / l : 0.f) * ib::tail_factor(tail, t0 + r0 + tid, h);
+      f_s[tid * (kMaxSlices + 1) + kMaxSlices] = inv;
+#pragma unroll
+      for (int i = 0; i < kMaxSlices; i++) f_s[tid * (kMaxSlices + 1) + i] = ml[i].x == -INFINITY ? -1.f : ex2(ml[i].x - M);
+    }
+    __syncthreads();
+    for (int idx0 = tid; idx0 < n_own * QPR; idx0 += U * kThreads) {
+      float4 o[U][kMaxSlices];   // every slice's part of U places is requested before the first is used
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int idx = min(idx0 + u * kThreads, n_own * QPR - 1);
+#pragma unroll
+        for (int i = 0; i < kMaxSlices; i++)
+          if (i < slices) o[u][i] = peer_ld4(peer_addr(k_s + ((r0 + idx / QPR) * SM::kRowO + idx % QPR * 4) * 4, i));
+      }
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int idx = idx0 + u * kThreads, r = idx / QPR, c = idx % QPR * 4;
+        if (idx >= n_own * QPR) continue;
+        const float* fr = f_s + r * (kMaxSlices + 1);
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < kMaxSlices; i++) {
+          const float f = fr[i];
+          if (f >= 0.f && i < slices) a.x = fmaf(o[u][i].x, f, a.x), a.y = fmaf(o[u][i].y, f, a.y), a.z = fmaf(o[u][i].z, f, a.z), a.w = fmaf(o[u][i].w, f, a.w);
+        }
+        const float inv = fr[kMaxSlices];
+        uint2 v;
+        v.x = mt::pack_bf16(a.x * inv, a.y * inv);
+        v.y = mt::pack_bf16(a.z * inv, a.w * inv);
+        *(uint2*)(out + (size_t)(t0 + r0 + r) * (tail.out_row ? tail.out_row : heads * HD) + h * HD + c) = v;
+      }
+    }
+    __syncwarp();
+    cluster_sync();   // nobody leaves while its slice may still be read
+  }
+}
+
+// Into how many slices the keys of a query tile are cut: a short portion behind a long context has few query tiles, each a chain of key tiles
+// of 0.6 us; the merge takes 4 us more. 61 tokens behind 900 in eight layers of the 0.6B sizes: 588 -> 535 us a step, behind 3,000 785 -> 560. A row: CTAs of the cluster, the fewest key tiles (of the tile that sees the most) with one CTA an SM
+// and with two. Measured alone (us, 1 | 2 | 4 | 8 slices; query tiles x heads, most key tiles): 16 CTAs of 16 tiles 20.5 | 18.5 | 16.4 | 16.4, of 32
+// 32.8 | 25.6 | 18.4 | 17.5; 16 of 10 16.4 | 16.4 | 14.4 | 16.4, of 5 12.3 | 14.3 | 14.3 | 13.2; 32 of 47 46.0 | 32.8 | 23.6 | 22.6, of 126 107 | 64 |
+// 41 | 35; 48 of 10 16.6 | 19.4 | 18.4 | 28.7; 64 of 17 23.5 | 21.4 | 20.5 | 31.7, of 8 15.4 | 17.3 | 19.2; 128 of 16 23.5 | 21.4 | 31.7, of 24 29.6 |
+// 26.6 | 36.9, of 32 35.8 | 29.7 | 34.8.
+struct SliceRule {
+  int slices, tiles_one, tiles_two;
+};
+constexpr SliceRule kSliceRules[] = {{8, 16, 64}, {4, 10, 16}, {2, 16, 16}};
+static_assert(kSliceRules[0].slices == kMaxSlices, "the merge takes every slice");
+
+int slices_for(long long ctas, int max_keys, int window, int keep, int sm_count) {
+  const long long seen = window == 0 ? max_keys : std::min((long long)max_keys, (window > 0 ? (long long)window + keep : -(long long)window) + BM);
+  const long long tiles = (seen + BN - 1) / BN;
+  for (const SliceRule& r : kSliceRules)
+    if ((ctas * r.slices <= sm_count && tiles >= r.tiles_one) || (ctas * r.slices <= 2 * sm_count && tiles >= r.tiles_two)) return r.slices;
+  return 1;
 }
 
 template <int HD>
 int launch(const void* q, const IbKvView* kv, const int* tile_seg, const int* tile_row0, int n_tiles, const int* seg_start, const int* seg_pos0,
            int window, float scale, void* out, int heads, const CUtensorMap* kv_map, long long view_row0, unsigned* status, cudaStream_t stream,
-           float softcap, int sink, const IbAttnTail& tail, int keep) {
+           float softcap, int sink, const IbAttnTail& tail, int keep, int max_keys) {
   const float scale_log2e = (softcap > 0.f ? softcap : scale) * 1.4426950408889634f, cap_pre = softcap > 0.f ? scale / softcap : 0.f;
   static bool configured = false;
+  static int sm_count = 0;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_ws_kernel<HD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<HD>::kBytes);
+    cudaError_t e = cudaFuncSetAttribute(prefill_ws_kernel<HD, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<HD>::kBytes);
+    if (e == cudaSuccess) e = cudaFuncSetAttribute(prefill_ws_kernel<HD, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, Smem<HD>::kBytes);
     IB_CHECK_ARG(e == cudaSuccess, "attention_prefill_ws: cannot reserve %d bytes of shared memory: %s", Smem<HD>::kBytes, cudaGetErrorString(e));
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
     configured = true;
   }
-  ib::launch(prefill_ws_kernel<HD>, dim3(heads, n_tiles), kThreads, Smem<HD>::kBytes, stream, (const __nv_bfloat16*)q, *kv, tile_seg, tile_row0,
-             seg_start, seg_pos0, window, scale_log2e, (__nv_bfloat16*)out, heads, *kv_map, view_row0, ib_wait_limit_ns(), status, cap_pre, sink, tail, keep);
+  const int slices = slices_for((long long)heads * n_tiles, max_keys, window, keep, sm_count);
+  auto run = [&](auto kernel, int z) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(heads, n_tiles, z);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = Smem<HD>::kBytes;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = ib_pdl_enabled();
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = z;
+    cfg.attrs = attr;
+    cfg.numAttrs = z > 1 ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16*)q, *kv, tile_seg, tile_row0, seg_start, seg_pos0, window, scale_log2e, (__nv_bfloat16*)out, heads, *kv_map,
+                              view_row0, ib_wait_limit_ns(), status, cap_pre, sink, tail, keep);
+  };
+  const cudaError_t e = slices > 1 ? run(prefill_ws_kernel<HD, true>, slices) : run(prefill_ws_kernel<HD, false>, 1);
+  IB_CHECK_ARG(e == cudaSuccess, "attention_prefill_ws: launch failed: %s", cudaGetErrorString(e));
   IB_CHECK_LAUNCH("attention_prefill_ws");
   return 0;
 }
@@ -411,13 +557,14 @@ int launch(const void* q, const IbKvView* kv, const int* tile_seg, const int* ti
 // Attention for query tiles of 128 rows: tile i covers rows tile_row0[i].. of segment tile_seg[i]; list the
 // tiles that see the most keys first. kv_map: the tensor map of the view's pool (ib_make_kv_map), view_row0
 // the pool row where this view's keys of page 0, head 0 start.
+// max_keys: how many keys the first of the tiles sees (its last row's position plus one), from which the number of slices follows, or 0 (no slices).
 // softcap > 0: scores become softcap * tanh(score / softcap) after the scale; sink: the softmax's denominator has one added (or
 // exp(tail->sink_values[head])). window < 0: a position sees the earlier positions of its own block of -window positions. keep (with a
 // window): the first positions of the request that are seen beside the window. tail (may be
 // null): the sink's scores, a gate and a constant on the output, the output's row length (IbAttnTail).
 extern "C" int ib_attention_prefill_ws_capped(const void* q, const IbKvView* kv, const int* tile_seg, const int* tile_row0, int n_tiles,
                                               const int* seg_start, const int* seg_pos0, int window, float scale, void* out, int heads,
-                                              const void* kv_map, long long view_row0, float softcap, int sink, const IbAttnTail* tail_in, int keep,
+                                              const void* kv_map, long long view_row0, int max_keys, float softcap, int sink, const IbAttnTail* tail_in, int keep,
                                               unsigned* status, cudaStream_t stream) {
   if (n_tiles == 0) return 0;
   IB_CHECK_ARG(keep >= 0 && (keep == 0 || window > 0), "attention_prefill_ws: %d kept positions need a window", keep);
@@ -437,16 +584,16 @@ extern "C" int ib_attention_prefill_ws_capped(const void* q, const IbKvView* kv,
   IB_CHECK_ARG(kv->page_stride % kv->head_dim == 0 && kv->v_offset % kv->head_dim == 0, "attention_prefill_ws: strides are not whole rows");
   if (kv->head_dim == 128)
     return launch<128>(q, kv, tile_seg, tile_row0, n_tiles, seg_start, seg_pos0, window, scale, out, heads, (const CUtensorMap*)kv_map, view_row0,
-                       status, stream, softcap, sink, tail, keep);
+                       status, stream, softcap, sink, tail, keep, max_keys);
   if (kv->head_dim == 64)
     return launch<64>(q, kv, tile_seg, tile_row0, n_tiles, seg_start, seg_pos0, window, scale, out, heads, (const CUtensorMap*)kv_map, view_row0,
-                      status, stream, softcap, sink, tail, keep);
+                      status, stream, softcap, sink, tail, keep, max_keys);
   return ib_set_error("attention_prefill_ws: head_dim %d has no tensor-core kernel (64 and 128 have)", kv->head_dim);
 }
 
 extern "C" int ib_attention_prefill_ws(const void* q, const IbKvView* kv, const int* tile_seg, const int* tile_row0, int n_tiles,
                                        const int* seg_start, const int* seg_pos0, int window, float scale, void* out, int heads,
-                                       const void* kv_map, long long view_row0, unsigned* status, cudaStream_t stream) {
-  return ib_attention_prefill_ws_capped(q, kv, tile_seg, tile_row0, n_tiles, seg_start, seg_pos0, window, scale, out, heads, kv_map, view_row0, 0.f, 0, nullptr, 0,
+                                       const void* kv_map, long long view_row0, int max_keys, unsigned* status, cudaStream_t stream) {
+  return ib_attention_prefill_ws_capped(q, kv, tile_seg, tile_row0, n_tiles, seg_start, seg_pos0, window, scale, out, heads, kv_map, view_row0, max_keys, 0.f, 0, nullptr, 0,
                                         status, stream);
 }

@@ -15,7 +15,7 @@ int ib_qk_norm_rope_kv(const float* qkv, int P, long long stride_p, const float*
                        const int* positions, const int* seg_of_token, void* q_out, int act_dtype, const IbKvView* kv, int write_kv, int T, int heads, unsigned* status,
                        const float* bias, int qk_dim, int v_dim, int row, int q_col, int k_col, int v_col, int unit_norm_after, cudaStream_t stream);
 int ib_attention_prefill_ws(const void* q, const IbKvView* kv, const int* tile_seg, const int* tile_row0, int n_tiles, const int* seg_start, const int* seg_pos0, int window, float scale,
-                            void* out, int heads, const void* kv_map, long long view_row0, unsigned* status, cudaStream_t stream);
+                            void* out, int heads, const void* kv_map, long long view_row0, int max_keys, unsigned* status, cudaStream_t stream);
 int ib_attention_decode_stream(const void* q, const IbKvView* kv, const int* dec_tokens, int n_dec, const int* positions, const int* seg_of_token, int window, float scale, float* part_o,
                                float* part_ml, void* out, int heads, int max_slices, int tiles_per_slice, const void* kv_map, long long view_row0, unsigned* status, cudaStream_t stream);
 int ib_gemm_tcgen05(const void* x, const void* w, float* out, int T, int N, int K, int bn, int splits, int wide, unsigned* status, cudaStream_t stream);
@@ -56,7 +56,7 @@ struct IbDenseStep {   // what the layers of a step have in common
   unsigned* status;
   cudaStream_t stream;
   IbDenseProduct qkv, out, gate_up, down;
-  int T, hidden, inter, heads, kv_heads, head_dim, rot_half, window, n_dec, n_tiles, max_slices, tiles_per_slice;
+  int T, hidden, inter, heads, kv_heads, head_dim, rot_half, window, n_dec, n_tiles, max_slices, tiles_per_slice, tile_keys;
   float norm_eps, ff_norm_eps, qk_eps, scale;
 };
 
@@ -105,8 +105,8 @@ extern "C" int ib_dense_layer(const IbDenseStep* s, const IbDenseLayer* l) {
     run(ib_attention_decode_stream(s->q, l->kv, s->dec_tokens, s->n_dec, s->positions, s->seg_of_token, s->window, s->scale, s->part_o, s->part_ml, s->o, s->heads, s->max_slices,
                                    s->tiles_per_slice, s->kv_map, l->kv_row0, s->status, s->stream), 2);
   if (s->n_tiles)
-    run(ib_attention_prefill_ws(s->q, l->kv, s->tile_seg, s->tile_row0, s->n_tiles, s->seg_start, s->seg_pos0, s->window, s->scale, s->o, s->heads, s->kv_map, l->kv_row0, s->status,
-                                s->stream));
+    run(ib_attention_prefill_ws(s->q, l->kv, s->tile_seg, s->tile_row0, s->n_tiles, s->seg_start, s->seg_pos0, s->window, s->scale, s->o, s->heads, s->kv_map, l->kv_row0, s->tile_keys,
+                                s->status, s->stream));
   product(s->out, s->o, l->w_out, H, Q);
   norm(s->out.kind == 2 ? nullptr : s->partial, s->out.kind == 1 ? 1 : s->out.splits, l->ff_norm, s->ff_norm_eps);
   const IbDenseProduct& g = s->gate_up;

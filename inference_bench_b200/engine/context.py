@@ -84,7 +84,7 @@ def build_context(rt: Runtime, segments: list[Segment], caches: Optional[list] =
             rows.append(T + int(w))
         T += n
         starts.append(T)
-    dec, longest, tile_seg, tile_row0 = attention.work_lists(lens, starts, [s.pos0 for s in segments]) if tables else ([], None, [], [])
+    dec, longest, tile_seg, tile_row0, tile_keys = attention.work_lists(lens, starts, [s.pos0 for s in segments]) if tables else ([], None, [], [], 0)
     # one pinned staging buffer, one copy; the host's arrays are the buffer's parts
     sizes = [T, T, T, S + 1, S, S, len(rows), len(dec), len(tile_seg), len(tile_seg)]
     total = sum(sizes)
@@ -120,5 +120,5 @@ def build_context(rt: Runtime, segments: list[Segment], caches: Optional[list] =
     ctx = StepContext(rt, segments, T, token_ids, positions, seg_of_token, seg_start, seg_pos0, seg_slot, logit_rows, *views[:7], caches=caches or [])
     if tables:
         ctx.tables = [views[11 + 2 * i].view(t.shape) for i, t in enumerate(tables)]
-        ctx.memo[attention.WORK_KEY] = attention.device_work(views[7], views[8], views[9], longest)
+        ctx.memo[attention.WORK_KEY] = attention.device_work(views[7], views[8], views[9], longest, tile_keys)
     return ctx

@@ -55,15 +55,15 @@ L.register("ib_attention_decode_stream", [L._p, C.POINTER(L.KvView), L._p, L._i,
 L.register("ib_attention_decode_fused", [L._p, L._i, L._ll, L._p, L._p, L._f, L._p, L._p, L._i, C.POINTER(L.KvView), L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._p,
                                          L._p, L._i, L._i, L._i, L._p, L._ll, L._p, L._p])
 L.register("ib_attention_prefill_tc", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._p])
-L.register("ib_attention_prefill_ws", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._ll, L._p, L._p])
+L.register("ib_attention_prefill_ws", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._ll, L._i, L._p, L._p])
 # the same with capped scores and a sink (softcap, sink before the status word)
 # (softcap, sink, the output's tail or null, the kept first positions, then the status word)
 L.register("ib_attention_decode_capped", [L._p, C.POINTER(L.KvView), L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._p, L._p, L._i, L._i, L._i, L._f, L._i, C.POINTER(L.AttnTail),
                                           L._i, L._p, L._p])
 L.register("ib_attention_decode_stream_capped", [L._p, C.POINTER(L.KvView), L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._p, L._p, L._i, L._i, L._i, L._p, L._ll, L._f, L._i,
                                                  C.POINTER(L.AttnTail), L._i, L._p, L._p])
-L.register("ib_attention_prefill_ws_capped", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._ll, L._f, L._i, C.POINTER(L.AttnTail),
-                                              L._i, L._p, L._p])
+L.register("ib_attention_prefill_ws_capped", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._ll, L._i, L._f, L._i,
+                                              C.POINTER(L.AttnTail), L._i, L._p, L._p])
 L.register("ib_attention_prompt_f32", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._f, L._i, C.POINTER(L.AttnTail), L._i, L._p, L._p])
 L.KERNELS_PER_CALL["ib_attention_decode_capped"] = 2
 L.KERNELS_PER_CALL["ib_attention_decode_stream_capped"] = 2
@@ -78,19 +78,20 @@ WORK_KEY = ("attention_work", QTILE)
 
 def work_lists(lens: list, starts: list, pos0: list) -> tuple:
     """Of a step's segments (their tokens, first rows and first positions): the flat rows of decoded tokens and their last position or None, then segments
-    and first rows of the portions' query tiles, those with the most keys first."""
+    and first rows of the portions' query tiles, those with the most keys first, and how many keys the first of them has."""
     dec = [i for i, n in enumerate(lens) if n == 1]
     tiles = [(-(p + min(r + QTILE, n)), i, r) for i, (n, p) in enumerate(zip(lens, pos0)) if n > 1 for r in range(0, n, QTILE)]
     tiles.sort(key=_first)
-    return [starts[i] for i in dec], max((pos0[i] for i in dec), default=None), [t[1] for t in tiles], [t[2] for t in tiles]
+    return [starts[i] for i in dec], max((pos0[i] for i in dec), default=None), [t[1] for t in tiles], [t[2] for t in tiles], -tiles[0][0] if tiles else 0
 
 
 _first = operator.itemgetter(0)
 
 
-def device_work(dec: Optional[torch.Tensor], tile_seg: Optional[torch.Tensor], tile_row0: Optional[torch.Tensor], max_pos: Optional[int]) -> dict:
+def device_work(dec: Optional[torch.Tensor], tile_seg: Optional[torch.Tensor], tile_row0: Optional[torch.Tensor], max_pos: Optional[int], tile_keys: int) -> dict:
     nd, nt = dec.shape[0], tile_seg.shape[0]
-    return dict(dec_tokens=dec if nd else None, n_dec=nd, tile_seg=tile_seg if nt else None, tile_row0=tile_row0 if nt else None, n_tiles=nt, max_pos=max_pos)
+    return dict(dec_tokens=dec if nd else None, n_dec=nd, tile_seg=tile_seg if nt else None, tile_row0=tile_row0 if nt else None, n_tiles=nt, tile_keys=tile_keys,
+                max_pos=max_pos)
 
 
 def _work_lists(ctx):
@@ -99,15 +100,15 @@ def _work_lists(ctx):
     if work is not None:
         return work
     if ctx.fixed_shape:
-        work = dict(dec_tokens=ctx.seg_start[:ctx.n_tokens], n_dec=ctx.n_tokens, tile_seg=None, tile_row0=None, n_tiles=0, max_pos=None)
+        work = dict(dec_tokens=ctx.seg_start[:ctx.n_tokens], n_dec=ctx.n_tokens, tile_seg=None, tile_row0=None, n_tiles=0, tile_keys=0, max_pos=None)
     else:
         starts = ctx.h_seg_start.tolist()
-        dec, longest, tile_seg, tile_row0 = work_lists([b - a for a, b in zip(starts, starts[1:])], starts, ctx.h_seg_pos0.tolist())
+        dec, longest, tile_seg, tile_row0, tile_keys = work_lists([b - a for a, b in zip(starts, starts[1:])], starts, ctx.h_seg_pos0.tolist())
         nd, nt = len(dec), len(tile_seg)
         staging = torch.empty(max(nd + 2 * nt, 1), dtype=torch.int32, pin_memory=True)
         staging.numpy()[:nd + 2 * nt] = dec + tile_seg + tile_row0
         dev = staging.to(ctx.rt.device, non_blocking=True)
-        work = device_work(dev[:nd], dev[nd:nd + nt], dev[nd + nt:nd + 2 * nt], longest)
+        work = device_work(dev[:nd], dev[nd:nd + nt], dev[nd + nt:nd + 2 * nt], longest, tile_keys)
     ctx.memo[WORK_KEY] = work
     return work
 
@@ -296,7 +297,7 @@ def paged_attention(ctx, q: torch.Tensor, cache: ops.KvLayerView, heads: int, wi
         if rt.options.prefill_attention == "ws" and not kv_map:
             raise L.KernelError(f"prefill_attention = \"ws\" needs a page size that TMA can serve (a multiple of 8 that divides 64, or a multiple of 64), got {view.page_size}")
         if kv_map:
-            L.call("ib_attention_prefill_ws" + tail, *args, kv_map, row0, *extra, rt.status.data_ptr(), stream)
+            L.call("ib_attention_prefill_ws" + tail, *args, kv_map, row0, work["tile_keys"], *extra, rt.status.data_ptr(), stream)
         else:
             L.call("ib_attention_prefill_tc", *args, rt.status.data_ptr(), stream)
     return out

@@ -30,7 +30,7 @@ class DenseStep(C.Structure):
     """Mirror of IbDenseStep."""
     _fields_ = ([(n, _p) for n in ("x", "h", "partial", "q", "o", "act", "part_o", "part_ml", "cos_t", "sin_t", "positions", "seg_of_token", "seg_start", "seg_pos0", "dec_tokens",
                                    "tile_seg", "tile_row0", "kv_map", "status", "stream")] + [(n, Product) for n in ("qkv", "out", "gate_up", "down")] +
-                [(n, _i) for n in ("T", "hidden", "inter", "heads", "kv_heads", "head_dim", "rot_half", "window", "n_dec", "n_tiles", "max_slices", "tiles_per_slice")] +
+                [(n, _i) for n in ("T", "hidden", "inter", "heads", "kv_heads", "head_dim", "rot_half", "window", "n_dec", "n_tiles", "max_slices", "tiles_per_slice", "tile_keys")] +
                 [(n, _f) for n in ("norm_eps", "ff_norm_eps", "qk_eps", "scale")])
 
 
@@ -109,7 +109,7 @@ class DenseLayers:
         self.step = DenseStep(x.data_ptr(), h, partial, q, q + 2 * T * Q, q, part_o if work["n_dec"] else None, part_ml, ptr(cos), ptr(sin), ctx.positions.data_ptr(),
                               ctx.seg_of_token.data_ptr(), ctx.seg_start.data_ptr(), ctx.seg_pos0.data_ptr(), ptr(work["dec_tokens"]), ptr(work["tile_seg"]), ptr(work["tile_row0"]),
                               kv_map, rt.status.data_ptr(), ops._stream(), qkv, out, gate_up, down, T, H, I, m.heads, m.kv_heads, hd, rot_half, int(m.window or 0), work["n_dec"],
-                              work["n_tiles"], max_slices, tps, block.mixer_norm.eps, block.feed_forward_norm.eps, m.norm_eps, m.scale)
+                              work["n_tiles"], max_slices, tps, work["tile_keys"], block.mixer_norm.eps, block.feed_forward_norm.eps, m.norm_eps, m.scale)
         self.left = down.splits if down.kind < 2 else 0   # partial sums the layers leave to add
         self._ref = C.byref(self.step)
         self.layer = DenseLayer()

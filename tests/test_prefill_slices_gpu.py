@@ -1,0 +1,48 @@
+"""Prompt portions whose keys are cut into slices over a thread-block cluster: every number of slices, slices without keys (a segment much shorter than the
+longest, rows that see none of a slice), windows, kept positions, sinks and gates, page sizes on both sides of a tile."""
+from __future__ import annotations
+
+import math
+
+import pytest
+import torch
+from test_kernels_gpu import _attention_case
+
+pytestmark = pytest.mark.gpu
+DEV = "cuda:0"
+
+
+@pytest.mark.parametrize("hd,heads,kvh,page,shapes", [
+    (128, 4, 2, 64, [(1100, 61)]),                          # 8 slices of 18 tiles, one query tile that is half full
+    (64, 6, 3, 8, [(1025, 128), (70, 2), (3, 3)]),          # 8 slices: segments of 17, 2 and 1 key tiles; eight pages a tile
+    (128, 16, 8, 16, [(700, 100), (641, 129)]),             # 4 slices of 11 tiles, a query tile of one row
+    (128, 32, 8, 192, [(1300, 256), (130, 130)]),           # 2 slices at two CTAs an SM: 128 CTAs, tiles of causal keys only beside long ones
+    (64, 2, 1, 128, [(4500, 2), (2500, 300)]),
+])
+@pytest.mark.parametrize("window,keep", [(None, 0), (1000, 0), (1030, 70)])
+def test_sliced_portions(hd, heads, kvh, page, shapes, window, keep):
+    from inference_bench_b200.engine.context import Segment, build_context
+    from inference_bench_b200.engine.runtime import Runtime
+    from inference_bench_b200.kernels import attention, ops
+    q, view, pos, seg, ref, _ = _attention_case(torch.bfloat16, heads, kvh, hd, page, window, shapes, 31, needle=True)
+    rt = Runtime(DEV)
+    ctx = build_context(rt, [Segment(i, i, L - n, [0] * n) for i, (L, n) in enumerate(shapes)])
+    scale = 1 / math.sqrt(hd)
+    out = attention.paged_attention(ctx, q, view, heads, window, scale, keep_first=keep)
+    again = attention.paged_attention(ctx, q, view, heads, window, scale, keep_first=keep)
+    rt.check_status()
+    assert torch.equal(out, again)
+    other = torch.empty_like(out)
+    ops.attention_generic(q, view, pos, seg, window, scale, other, heads, rt.status, keep_first=keep)
+    # P is rounded to bfloat16 (2^-9 of each weight) and so is the output, on both sides
+    top = ref.abs().max()
+    assert (out.double() - other.double()).abs().max() <= 2e-2 * top
+    if not keep:
+        assert (out.cpu().double() - ref).abs().max() <= 1.5e-2 * top
+    sinks, gate = torch.randn(heads, device=DEV), torch.randn((2, q.shape[0], heads), device=DEV)
+    kw = dict(softcap=20.0, sink=True, sink_values=sinks, gate=(gate, 0), out_scale=0.5, keep_first=keep)
+    out = attention.paged_attention(ctx, q, view, heads, window, scale, **kw)
+    kw["gate"] = (gate, 0)
+    ops.attention_generic(q, view, pos, seg, window, scale, other, heads, rt.status, **kw)
+    rt.check_status()
+    assert (out.double() - other.double()).abs().max() <= 2e-2 * top
