@@ -89,9 +89,6 @@ __device__ __forceinline__ float4 peer_ld4(uint32_t addr) {
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(addr));
   return v;
 }
-__device__ __forceinline__ void cluster_sync() {   // every thread of every CTA of the cluster (one that has left counts as arrived)
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 __device__ __forceinline__ void bar_sync_softmax() { asm volatile("bar.sync 1, %0;" ::"n"(kSoftmaxWarps * 32) : "memory"); }
 
 template <int HD>
@@ -439,7 +436,7 @@ __global__ void __launch_bounds__(kThreads, 2)
   }
   if constexpr (SLICED) {   // each CTA merges its share of the rows: O = sum of 2^(m_i - M) O_i over the slices, in their order, and the same of the sums
     __syncwarp();
-    cluster_sync();
+    ib::cluster_sync();
     constexpr int QPR = HD / 4, U = 2;
     const int share = (rows + slices - 1) / slices, r0 = slice * share, n_own = max(min(rows - r0, share), 0);
     float* const f_s = (float*)(sm + SM::oQ + BM * 8);   // [share][kMaxSlices]: the factors of a row's slices, -1 for one in which it saw no key
@@ -488,7 +485,7 @@ __global__ void __launch_bounds__(kThreads, 2)
       }
     }
     __syncwarp();
-    cluster_sync();   // nobody leaves while its slice may still be read
+    ib::cluster_sync();   // nobody leaves while its slice may still be read
   }
 }
 
@@ -530,21 +527,8 @@ int launch(const void* q, const IbKvView* kv, const int* tile_seg, const int* ti
   }
   const int slices = slices_for((long long)heads * n_tiles, max_keys, window, keep, sm_count);
   auto run = [&](auto kernel, int z) {
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(heads, n_tiles, z);
-    cfg.blockDim = dim3(kThreads);
-    cfg.dynamicSmemBytes = Smem<HD>::kBytes;
-    cfg.stream = stream;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = ib_pdl_enabled();
-    attr[1].id = cudaLaunchAttributeClusterDimension;
-    attr[1].val.clusterDim.x = attr[1].val.clusterDim.y = 1;
-    attr[1].val.clusterDim.z = z;
-    cfg.attrs = attr;
-    cfg.numAttrs = z > 1 ? 2 : 1;
-    return cudaLaunchKernelEx(&cfg, kernel, (const __nv_bfloat16*)q, *kv, tile_seg, tile_row0, seg_start, seg_pos0, window, scale_log2e, (__nv_bfloat16*)out, heads, *kv_map,
-                              view_row0, ib_wait_limit_ns(), status, cap_pre, sink, tail, keep);
+    return ib::launch_cluster(kernel, dim3(heads, n_tiles, z), dim3(1, 1, z), kThreads, Smem<HD>::kBytes, stream, (const __nv_bfloat16*)q, *kv, tile_seg, tile_row0, seg_start,
+                              seg_pos0, window, scale_log2e, (__nv_bfloat16*)out, heads, *kv_map, view_row0, ib_wait_limit_ns(), status, cap_pre, sink, tail, keep);
   };
   const cudaError_t e = slices > 1 ? run(prefill_ws_kernel<HD, true>, slices) : run(prefill_ws_kernel<HD, false>, 1);
   IB_CHECK_ARG(e == cudaSuccess, "attention_prefill_ws: launch failed: %s", cudaGetErrorString(e));

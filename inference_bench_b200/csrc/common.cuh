@@ -49,6 +49,38 @@ namespace ib {
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
+// Of a thread-block cluster: the barrier of every thread of every CTA (whole warps; a CTA that has left counts as arrived), and a load from the same place of
+// shared memory in CTA `rank`.
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float peer_ld(const float* own, int rank) {
+  unsigned addr;
+  float v;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(addr) : "r"((unsigned)__cvta_generic_to_shared(own)), "r"(rank));
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+
+template <typename... Exp, typename... Act>
+inline cudaError_t launch_cluster(void (*kernel)(Exp...), dim3 grid, dim3 cluster, dim3 block, size_t smem, cudaStream_t stream, Act&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = ib_pdl_enabled();
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster.x;
+  attr[1].val.clusterDim.y = cluster.y;
+  attr[1].val.clusterDim.z = cluster.z;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster.x * cluster.y * cluster.z > 1 ? 2 : 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<Exp>(args)...);
+}
+
 template <typename... Exp, typename... Act>
 inline cudaError_t launch(void (*kernel)(Exp...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Act&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -1,16 +1,19 @@
-// Next-token choice on the device, one block per logits row.
+// Next-token choice on the device, one thread-block cluster per logits row.
 //
 // Temperature 0: argmax, the lowest index winning ties. Otherwise Gumbel-max over the candidates
 // that survive top-k, top-p and min-p, on v = logit / T: token = argmax_i (v_i + g_i),
 // g_i = -ln(-ln u_i), u_i from an integer hash of (seed, step, i). Same semantics and the same
 // hash as the reference's sample_rows (crates/kir/tests/golden/prims/prims_sm120.cu:34-39,
-// 51-163, 208-250); the threshold search here is a byte-wise radix descent for top-k and a
-// bisection with ordered block sums for top-p, so a row's result never depends on thread timing.
+// 51-163, 208-250); the thresholds here are found digit by digit of the value's bits, four at a
+// time, by count (top-k) or by mass with ordered sums (top-p), so a row's result never depends on
+// thread timing.
 #include "common.cuh"
 
 namespace {
 
-constexpr int kThreads = 1024;
+constexpr int kThreads = 512, kWarpsOfRow = kThreads / 32;
+constexpr int kMaxCtas = 8;    // CTAs of a row's cluster
+constexpr int kCtaValues = 4096;   // of the vocabulary, from which on a row takes another CTA
 
 struct RowParams {  // six 32-bit words per row, as the reference packs them (crates/specrt/src/runtime/step.rs:76-85)
   float inv_temp;   // 0 = greedy
@@ -32,111 +35,12 @@ __device__ __forceinline__ float gumbel(unsigned seed, unsigned step, unsigned i
   return -logf(-logf(u));
 }
 
-// Monotone map float -> unsigned (larger float, larger key).
+// Monotone map float -> unsigned (larger float, larger key), zeros of both signs alike.
 __device__ __forceinline__ unsigned order_key(float v) {
-  unsigned b = __float_as_uint(v);
+  unsigned b = __float_as_uint(v + 0.f);
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
 __device__ __forceinline__ float order_value(unsigned k) { return __uint_as_float((k & 0x80000000u) ? (k & 0x7fffffffu) : ~k); }
-
-__device__ float block_max(float v, float* scratch) {
-  int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  v = ib::warp_max(v);
-  __syncthreads();
-  if (lane == 0) scratch[warp] = v;
-  __syncthreads();
-  float r = lane < (blockDim.x >> 5) ? scratch[lane] : -INFINITY;
-  return ib::warp_max(r);
-}
-
-// The k-th largest value of v_i = row[i] * inv_temp, by four passes over one byte of the key each.
-__device__ float kth_largest(const float* row, int V, float inv_temp, int k) {
-  __shared__ unsigned hist[256];
-  __shared__ unsigned sh_prefix;
-  __shared__ int sh_need;
-  unsigned prefix = 0, mask = 0;
-  int need = k;
-  for (int pass = 0; pass < 4; pass++) {
-    int shift = 24 - 8 * pass;
-    for (int i = threadIdx.x; i < 256; i += blockDim.x) hist[i] = 0;
-    __syncthreads();
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      unsigned key = order_key(row[i] * inv_temp);
-      if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int c = need, b = 255;
-      for (; b > 0; b--) {
-        if ((int)hist[b] >= c) break;
-        c -= (int)hist[b];
-      }
-      sh_need = c;
-      sh_prefix = prefix | ((unsigned)b << shift);
-    }
-    __syncthreads();
-    need = sh_need;
-    prefix = sh_prefix;
-    mask |= 255u << shift;
-    __syncthreads();
-  }
-  return order_value(prefix);
-}
-
-__device__ float mass_at_least(const float* row, int V, float inv_temp, float m, float floor_v, float* scratch) {
-  float z = 0.f;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) {
-    float v = row[i] * inv_temp;
-    if (v >= floor_v) z += expf(v - m);
-  }
-  return ib::block_sum(z, scratch);
-}
-
-// Stage 1, one block per row: the candidate threshold on v = logit / T. Rows that are greedy or
-// have no filter leave at once with -inf.
-__global__ void __launch_bounds__(kThreads) sample_threshold_kernel(const float* __restrict__ logits, int V, const RowParams* __restrict__ params,
-                                                                    float* __restrict__ threshold) {
-  __shared__ float scratch[32];
-  ib::pdl_launch_dependents();
-  ib::pdl_wait();
-  const float* row = logits + (size_t)blockIdx.x * V;
-  const RowParams p = params[blockIdx.x];
-  const bool use_k = p.top_k > 0 && p.top_k < V, use_p = p.top_p < 1.f, use_m = p.min_p > 0.f;
-  if (!(p.inv_temp > 0.f) || !(use_k || use_p || use_m)) {
-    if (threadIdx.x == 0) threshold[blockIdx.x] = -INFINITY;
-    return;
-  }
-  float thr = -INFINITY;
-  float m = -INFINITY;
-  for (int i = threadIdx.x; i < V; i += blockDim.x) m = fmaxf(m, row[i] * p.inv_temp);
-  m = block_max(m, scratch);
-  if (use_k) thr = kth_largest(row, V, p.inv_temp, p.top_k);
-  if (use_p) {
-    // Largest threshold whose candidates (also above the top-k threshold) hold mass >= top_p * total.
-    float z = mass_at_least(row, V, p.inv_temp, m, thr, scratch);
-    float target = fmaxf(p.top_p, 1e-9f) * z;
-    float lo = thr > -INFINITY ? thr : m - 88.f;
-    float hi = nextafterf(m, INFINITY);
-    for (int it = 0; it < 64; it++) {
-      float mid = 0.5f * (lo + hi);
-      if (mid <= lo || mid >= hi) break;
-      if (mass_at_least(row, V, p.inv_temp, m, mid, scratch) >= target)
-        lo = mid;
-      else
-        hi = mid;
-    }
-    // Snap to the smallest candidate value >= lo.
-    float low = INFINITY;
-    for (int i = threadIdx.x; i < V; i += blockDim.x) {
-      float v = row[i] * p.inv_temp;
-      if (v >= lo) low = fminf(low, v);
-    }
-    low = -block_max(-low, scratch);
-    thr = fmaxf(thr, low);
-  }
-  if (use_m) thr = fmaxf(thr, m + logf(p.min_p));
-  if (threadIdx.x == 0) threshold[blockIdx.x] = thr;
-}
 
 __device__ __forceinline__ void better(float& bv, int& bi, float ov, int oi) {  // the lowest index wins ties
   if (ov > bv || (ov == bv && oi < bi)) {
@@ -145,71 +49,187 @@ __device__ __forceinline__ void better(float& bv, int& bi, float ov, int oi) {  
   }
 }
 
-// Best (value, index) of a block of kPickThreads threads; valid in thread 0.
-constexpr int kPickThreads = 256;
-__device__ void block_best(float& bv, int& bi) {
-  __shared__ float sv[kPickThreads / 32];
-  __shared__ int si[kPickThreads / 32];
+// What the CTAs of a row's cluster exchange: each leaves its part, and after one cluster barrier every one reads all of them, in the order of the ranks.
+// Two places are used in turn: a CTA writes a place again only behind the barrier after the one that its readers passed.
+struct RowShared {
+  float warp_part[kWarpsOfRow][16];
+  int warp_index[kWarpsOfRow];
+  float part[2][16];
+  float part_index[2];   // (bits of whole numbers)
+  float total[16];
+  float bins[16][kThreads];   // a thread's sixteen sums of a pass
+};
+
+// f(i, value) for this CTA's values of the row: four neighbours an access and sixteen requested at a time where the row starts on 16 bytes.
+template <class F>
+__device__ __forceinline__ void each_value(const float* __restrict__ row, int begin, int end, F f) {
+  constexpr int U = 4;
+  if (((uintptr_t)(row + begin) & 15) == 0) {
+    const int quads = (end - begin) / 4;
+    const float4* src = (const float4*)(row + begin);
+    for (int q0 = threadIdx.x; q0 < quads; q0 += U * kThreads) {
+      float4 v[U];
+#pragma unroll
+      for (int u = 0; u < U; u++)
+        if (q0 + u * kThreads < quads) v[u] = src[q0 + u * kThreads];
+#pragma unroll
+      for (int u = 0; u < U; u++) {
+        const int i = begin + 4 * (q0 + u * kThreads);
+        if (q0 + u * kThreads < quads) f(i, v[u].x), f(i + 1, v[u].y), f(i + 2, v[u].z), f(i + 3, v[u].w);
+      }
+    }
+    begin += 4 * quads;
+  }
+#pragma unroll 4
+  for (int i = begin + threadIdx.x; i < end; i += kThreads) f(i, row[i]);
+}
+
+// The sums over the cluster of sixteen values of every thread, in sh.total for all threads; `turn` is 0 and 1 from call to call.
+__device__ __forceinline__ void cluster_sums(float (&s)[16], RowShared& sh, int ctas, int turn) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 16; o > 1; o >>= 1) {   // lanes halve the values between them: lane (l4 l3 l2 l1 l0) ends with value l4 l3 l2 l1
+    const bool up = lane & o;
+#pragma unroll
+    for (int i = 0; i < o / 2; i++) {
+      const float give = up ? s[i] : s[i + o / 2], keep = up ? s[i + o / 2] : s[i];
+      s[i] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+    }
+  }
+  s[0] += __shfl_xor_sync(0xffffffffu, s[0], 1);
+  if (!(lane & 1)) sh.warp_part[warp][lane >> 1] = s[0];
+  __syncthreads();
+  if (threadIdx.x < 16) {
+    float t = 0.f;
+#pragma unroll
+    for (int w = 0; w < kWarpsOfRow; w++) t += sh.warp_part[w][threadIdx.x];
+    if (ctas > 1) sh.part[turn][threadIdx.x] = t;
+    else sh.total[threadIdx.x] = t;
+  }
+  if (ctas > 1) {
+    __syncwarp();
+    ib::cluster_sync();
+    if (threadIdx.x < 16) {
+      float t = 0.f;
+      for (int c = 0; c < ctas; c++) t += ib::peer_ld(&sh.part[turn][threadIdx.x], c);
+      sh.total[threadIdx.x] = t;
+    }
+  }
+  __syncthreads();
+}
+
+// The best (value, index) of the cluster, in the first warp of every CTA.
+__device__ __forceinline__ void cluster_best(float& bv, int& bi, RowShared& sh, int ctas, int turn) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) better(bv, bi, __shfl_xor_sync(0xffffffffu, bv, o), __shfl_xor_sync(0xffffffffu, bi, o));
-  if (lane == 0) {
-    sv[warp] = bv;
-    si[warp] = bi;
-  }
+  if (lane == 0) sh.warp_part[warp][0] = bv, sh.warp_index[warp] = bi;
   __syncthreads();
   if (warp == 0) {
-    bv = lane < kPickThreads / 32 ? sv[lane] : -INFINITY;
-    bi = lane < kPickThreads / 32 ? si[lane] : 0x7fffffff;
+    bv = lane < kWarpsOfRow ? sh.warp_part[lane][0] : -INFINITY;
+    bi = lane < kWarpsOfRow ? sh.warp_index[lane] : 0x7fffffff;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) better(bv, bi, __shfl_xor_sync(0xffffffffu, bv, o), __shfl_xor_sync(0xffffffffu, bi, o));
+    if (lane == 0) sh.part[turn][0] = bv, sh.part_index[turn] = __int_as_float(bi);
   }
+  __syncwarp();
+  if (ctas == 1) return;
+  ib::cluster_sync();
+  if (warp == 0)
+    for (int c = 0; c < ctas; c++) better(bv, bi, ib::peer_ld(&sh.part[turn][0], c), __float_as_int(ib::peer_ld(&sh.part_index[turn], c)));
 }
 
-// Stage 2, grid (chunks, rows): the best candidate of one chunk of the vocabulary.
-__global__ void __launch_bounds__(kPickThreads) sample_pick_kernel(const float* __restrict__ logits, int V, const RowParams* __restrict__ params,
-                                                                   const float* __restrict__ threshold, float* __restrict__ part_v,
-                                                                   int* __restrict__ part_i, int chunk) {
+// The largest key t of lo .. hi - 1 with at least `target` of weight in the values of key t and above (lo when there is none), the weight being a count or
+// the mass e^(v - m). A pass looks at the sixteen parts of the interval that is left; what lies above it is known from the passes before.
+// FRACTION: target is a share of the weight of lo and above.
+template <bool MASS, bool FRACTION>
+__device__ __forceinline__ unsigned search(const float* row, int begin, int end, float inv_temp, float m, unsigned lo, unsigned long long hi, float target, RowShared& sh, int ctas,
+                                           int& turn) {
+  float above = 0.f;   // the weight of hi and above
+  bool first = true;
+  while (lo + 1ull < hi) {
+    const int bits = 64 - __clzll((long long)(hi - lo - 1)), shift = bits > 4 ? bits - 4 : 0;
+#pragma unroll
+    for (int j = 0; j < 16; j++) sh.bins[j][threadIdx.x] = 0.f;
+    each_value(row, begin, end, [&](int, float x) {
+      const float v = x * inv_temp;
+      const unsigned key = order_key(v);
+      if (key < lo || key >= hi) return;
+      sh.bins[(key - lo) >> shift][threadIdx.x] += MASS ? expf(v - m) : 1.f;
+    });
+    float s[16];   // of part j and above
+#pragma unroll
+    for (int j = 15; j >= 0; j--) s[j] = sh.bins[j][threadIdx.x] + (j < 15 ? s[j + 1] : 0.f);
+    cluster_sums(s, sh, ctas, turn);
+    turn ^= 1;
+    if (FRACTION && first) target *= sh.total[0];
+    first = false;
+    int best = 0;
+    float next = above;
+#pragma unroll
+    for (int j = 1; j < 16; j++)
+      if (above + sh.total[j] >= target) best = j;
+    if (best < 15) next = above + sh.total[best + 1];
+    hi = min(hi, (unsigned long long)lo + ((unsigned long long)(best + 1) << shift));
+    lo += (unsigned)best << shift;
+    above = next;
+  }
+  return lo;
+}
+
+// One row. All of a greedy row is one pass over its logits; a threshold is eight passes of four bits each over logits that stay in L2, and what a pass costs
+// is its reductions, not its reads. A row of 151,936 took 945 us with top-p, 185 with top-k and 850 with both, by one CTA and a pass for every step of a
+// bisection, and a greedy one 13 us in three kernels: 54, 48, 77 and 9 us so (64 rows: 955, 196, 906 and 20 against 113, 102, 156 and 12).
+// With `status` the step's status word is copied to tokens[rows], so the host gets it in the transfer that brings the tokens.
+__global__ void __launch_bounds__(kThreads, 3) sample_kernel(const float* __restrict__ logits, int V, const RowParams* __restrict__ params, int* __restrict__ tokens,
+                                                          const unsigned* __restrict__ status) {
+  __shared__ RowShared sh;
   ib::pdl_launch_dependents();
   ib::pdl_wait();
-  const int r = blockIdx.y;
+  const int r = blockIdx.y, ctas = gridDim.x, rank = blockIdx.x;
   const float* row = logits + (size_t)r * V;
   const RowParams p = params[r];
   const bool sampling = p.inv_temp > 0.f;
-  const float thr = threshold[r];
-  const int begin = blockIdx.x * chunk, end = min(V, begin + chunk);
-  float bv = -INFINITY;
-  int bi = 0x7fffffff;
-  for (int i = begin + threadIdx.x; i < end; i += kPickThreads) {
-    float v = row[i];
-    if (sampling) {
-      v *= p.inv_temp;
-      if (v < thr) continue;
-      v += gumbel(p.seed, p.step, (unsigned)i);
+  const int share = ((V + ctas - 1) / ctas + 3) & ~3, begin = min(V, rank * share), end = min(V, begin + share);
+  int turn = 0;
+  float thr = -INFINITY;
+  const bool use_k = p.top_k > 0 && p.top_k < V, use_p = p.top_p < 1.f, use_m = p.min_p > 0.f;
+  if (sampling && (use_k || use_p || use_m)) {   // (the same for all CTAs of the row)
+    float m = -INFINITY;
+    if (use_p || use_m) {
+      int none = 0;
+      each_value(row, begin, end, [&](int, float x) { m = fmaxf(m, x * p.inv_temp); });
+      cluster_best(m, none, sh, ctas, turn);
+      turn ^= 1;
+      if (threadIdx.x == 0) sh.total[0] = m;
+      __syncthreads();
+      m = sh.total[0];
     }
-    better(bv, bi, v, i);
+    if (use_k) thr = order_value(search<false, false>(row, begin, end, p.inv_temp, m, 0u, 1ull << 32, (float)p.top_k, sh, ctas, turn));
+    if (use_p) {   // the largest threshold whose candidates (also above the top-k threshold) hold mass >= top_p * total
+      const float lo = thr > -INFINITY ? thr : m - 88.f;
+      thr = fmaxf(thr, order_value(search<true, true>(row, begin, end, p.inv_temp, m, order_key(lo), order_key(nextafterf(m, INFINITY)), fmaxf(p.top_p, 1e-9f), sh, ctas, turn)));
+    }
+    if (use_m) thr = fmaxf(thr, m + logf(p.min_p));
   }
-  block_best(bv, bi);
-  if (threadIdx.x == 0) {
-    part_v[r * gridDim.x + blockIdx.x] = bv;
-    part_i[r * gridDim.x + blockIdx.x] = bi;
-  }
-}
-
-// Stage 3, one warp per row: the best of the chunks.
-// With `status` the step's status word is copied to tokens[gridDim.x], so the host gets it in the transfer that brings the tokens.
-__global__ void sample_final_kernel(const float* __restrict__ part_v, const int* __restrict__ part_i, int chunks, int* __restrict__ tokens,
-                                    const unsigned* __restrict__ status) {
-  ib::pdl_launch_dependents();
-  ib::pdl_wait();
-  const int r = blockIdx.x;
   float bv = -INFINITY;
   int bi = 0x7fffffff;
-  for (int c = threadIdx.x; c < chunks; c += 32) better(bv, bi, part_v[r * chunks + c], part_i[r * chunks + c]);
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) better(bv, bi, __shfl_xor_sync(0xffffffffu, bv, o), __shfl_xor_sync(0xffffffffu, bi, o));
-  if (threadIdx.x == 0) tokens[r] = bi == 0x7fffffff ? 0 : bi;
-  if (status && r == 0 && threadIdx.x == 0) tokens[gridDim.x] = (int)*status;
+  if (sampling)
+    each_value(row, begin, end, [&](int i, float x) {
+      const float v = x * p.inv_temp;
+      if (!(v < thr)) better(bv, bi, v + gumbel(p.seed, p.step, (unsigned)i), i);
+    });
+  else
+    each_value(row, begin, end, [&](int i, float x) { better(bv, bi, x, i); });
+  cluster_best(bv, bi, sh, ctas, turn);
+  if (rank == 0 && threadIdx.x == 0) {
+    tokens[r] = bi == 0x7fffffff ? 0 : bi;
+    if (status && r == 0) tokens[gridDim.y] = (int)*status;
+  }
+  if (ctas > 1) {   // nobody leaves while its part may still be read
+    __syncwarp();
+    ib::cluster_sync();
+  }
 }
 
 // After a decode step: feed every row's sampled token back as its next input, move its position on
@@ -272,26 +292,22 @@ extern "C" int ib_advance_rows(const int* sampled, int* token_in, int* positions
   return 0;
 }
 
-// chunks of the vocabulary per row in stage 2
-extern "C" int ib_sample_chunks(int V) { return V <= 4096 ? 1 : (V + 4095) / 4096 > 64 ? 64 : (V + 4095) / 4096; }
-
 // logits float32 [rows, V], params [rows] of six words -> tokens int32 [rows].
-// scratch: float32 [rows * (1 + 2 * ib_sample_chunks(V))] (threshold, then per-chunk best values and indices).
 // status: null, or the device status word, whose value is then stored in tokens[rows] (tokens has rows + 1 entries).
-extern "C" int ib_sample_rows(const float* logits, int rows, int V, const void* params, int* tokens, float* scratch, const unsigned* status,
-                              cudaStream_t stream) {
+extern "C" int ib_sample_rows(const float* logits, int rows, int V, const void* params, int* tokens, const unsigned* status, cudaStream_t stream) {
   if (rows == 0) return 0;
   IB_CHECK_ARG(rows > 0 && rows <= 65535 && V > 0, "sample_rows: bad sizes rows=%d V=%d", rows, V);
-  const int chunks = ib_sample_chunks(V);
-  const int chunk = (V + chunks - 1) / chunks;
-  float* threshold = scratch;
-  float* part_v = scratch + rows;
-  int* part_i = (int*)(part_v + (size_t)rows * chunks);
-  ib::launch(sample_threshold_kernel, rows, kThreads, 0, stream, logits, V, (const RowParams*)params, threshold);
-  IB_CHECK_LAUNCH("sample_rows threshold");
-  ib::launch(sample_pick_kernel, dim3(chunks, rows), kPickThreads, 0, stream, logits, V, (const RowParams*)params, threshold, part_v, part_i, chunk);
-  IB_CHECK_LAUNCH("sample_rows pick");
-  ib::launch(sample_final_kernel, rows, 32, 0, stream, part_v, part_i, chunks, tokens, status);
-  IB_CHECK_LAUNCH("sample_rows final");
+  static int sm_count = 0;
+  if (!sm_count) {
+    int dev = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
+  }
+  // As many CTAs a row as leave each 4,096 values and the device two CTAs an SM: 64 rows of 151,936 with top-p 219 us on 1 CTA a row, 131 on 2, 113 on 4,
+  // 145 on 8 (two rounds of CTAs); 64 of 32,768 60 | 48 | 46 | 74; one row of 151,936 54 on 8.
+  int ctas = 1;
+  while (ctas < kMaxCtas && ctas * kCtaValues < V && (long long)rows * 2 * ctas <= 2 * sm_count) ctas *= 2;
+  ib::launch_cluster(sample_kernel, dim3(ctas, rows), dim3(ctas), kThreads, 0, stream, logits, V, (const RowParams*)params, tokens, status);
+  IB_CHECK_LAUNCH("sample_rows");
   return 0;
 }

@@ -84,7 +84,7 @@ _SIGNATURES = {
     "ib_qk_norm_rope_kv": [_p, _i, _ll, _p, _p, _f, _p, _p, _i, _p, _p, _p, _i, C.POINTER(KvView), _i, _i, _i, _p, _p, _i, _i, _i, _i, _i, _i, _i, _p],
     "ib_attention_generic": [_p, _i, C.POINTER(KvView), _p, _p, _i, _f, _p, _i, _i, _p, _i, _i, _f, _i, _i, _p, _p, _i, _ll, _i, _f, _i, _i, _p, _p],
     "ib_gemm_simt": [_p, _i, _p, _i, _p, _i, _i, _i, _p],
-    "ib_sample_rows": [_p, _i, _i, _p, _p, _p, _p, _p],
+    "ib_sample_rows": [_p, _i, _i, _p, _p, _p, _p],
     "ib_advance_rows": [_p, _p, _p, _p, _p, _p, _p, _i, _i, _p, _p],
     "ib_fetch_ints": [_p, _p, _i, _p],
 }
@@ -131,7 +131,7 @@ def register(name: str, argtypes: list) -> None:
 launches = 0   # kernels launched so far through `call`
 
 
-KERNELS_PER_CALL = {"ib_sample_rows": 3, "ib_attention_decode": 2, "ib_attention_decode_stream": 2, "ib_attention_decode_fused": 2}
+KERNELS_PER_CALL = {"ib_attention_decode": 2, "ib_attention_decode_stream": 2, "ib_attention_decode_fused": 2}
 
 
 class _Notes(threading.local):
