@@ -196,7 +196,7 @@ def measure_decode_device(engine, batch: int, steps: int, warmup: int, clocks=No
     if clocks is not None:
         clocks.mark_end()
     ms = e0.elapsed_time(e1) / steps
-    launches = engine.executor.graph_for(batch, alone=False).launches
+    launches = engine.executor.graph_for(batch, alone=False).launches[False]
     for rid in ids:
         engine.cache.release(rid)
     engine.rt.check_status()

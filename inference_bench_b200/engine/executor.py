@@ -24,11 +24,13 @@ RUN_AHEAD_MAX = 64
 
 
 class _DecodeGraph:
-    """The captured decode step for `rows` rows and the static buffers it reads and writes. alone: a step that the host waits for (`run`); it fetches its
-    inputs from the pinned block and leaves its tokens there itself. Otherwise the inputs are copied in front of it (`launch`, `run_ahead`)."""
+    """The captured decode step for `rows` rows and the static buffers it reads and writes. It has two forms, each captured when it is first needed, over the
+    same buffers and memory pool, so that a step of either form finds what the step before left on the device. alone: a step that the host waits for
+    (`run`); it fetches its inputs from the pinned block and leaves its tokens there itself. Otherwise the inputs are copied in front of it (`launch`,
+    `run_ahead`)."""
 
-    def __init__(self, runner: ModelRunner, rows: int, alone: bool):
-        self.runner, self.rows, self.alone = runner, rows, alone
+    def __init__(self, runner: ModelRunner, rows: int):
+        self.runner, self.rows = runner, rows
         cache, rt = runner.cache, runner.rt
         B, W = rows, cache.table_width
         n_groups = len(cache.groups)
@@ -58,14 +60,17 @@ class _DecodeGraph:
         self.tokens = self.result[:B]
         self.h_out = torch.zeros(B + 1, dtype=torch.int32).pin_memory()
         self.np_out = self.h_out.numpy()
-        # for steps launched without waiting (two may be in flight): a staging copy of the inputs, a place for the tokens and an event each
-        self.stages = [torch.zeros(self.n_ints, dtype=torch.int32).pin_memory() for _ in range(2)]
-        self.h_outs = [torch.zeros(B + 1, dtype=torch.int32).pin_memory() for _ in range(2)]
-        self.events = [torch.cuda.Event() for _ in range(2)]
+        # for steps launched without waiting (two may be in flight): a staging copy of the inputs, a place for the tokens and an event each (`capture`)
+        self.stages: list[torch.Tensor] = []
+        self.h_outs: list[torch.Tensor] = []
+        self.events: list[torch.cuda.Event] = []
         self.pending = [False, False]
         self.turn = 0
-        self.logits: Optional[torch.Tensor] = None
-        self.graph: Optional[torch.cuda.CUDAGraph] = None
+        self.logits: Optional[torch.Tensor] = None   # of the step replayed last
+        # by form: the captured step, its logits, the kernels in one replay
+        self.graphs: dict[bool, torch.cuda.CUDAGraph] = {}
+        self.logits_of: dict[bool, torch.Tensor] = {}
+        self.launches: dict[bool, int] = {}
         self._pad_all()
 
     def _pad_all(self) -> None:
@@ -78,31 +83,44 @@ class _DecodeGraph:
         for g, t in enumerate(self.h_tables):
             t[:] = cache.scratch_page(g)
 
-    def _forward(self) -> None:
+    def _forward(self, alone: bool) -> torch.Tensor:
         self.ctx.memo = {}
-        self.logits = self.runner.decoder.forward(self.ctx)
-        ops.sample_rows(self.logits, self.d_params, self.result, self.runner.rt.status)
+        logits = self.runner.decoder.forward(self.ctx)
+        ops.sample_rows(logits, self.d_params, self.result, self.runner.rt.status)
         c = self.ctx
-        ops.advance_rows(self.tokens, c.token_ids, c.positions, c.seg_pos0, self.d_params, self.history, self.d_count, self.h_out if self.alone else None)
+        ops.advance_rows(self.tokens, c.token_ids, c.positions, c.seg_pos0, self.d_params, self.history, self.d_count, self.h_out if alone else None)
+        return logits
 
-    def capture(self) -> None:
+    def capture(self, alone: bool) -> None:
+        """Capture one form. The second form runs nothing on the device (a step of the first may have left tokens there) and takes its memory from the first's
+        pool: a replay's intermediates are dead when it ends, and replays follow one another on one stream."""
         self.runner.rt.activate()
-        ops.fetch_ints(self.host, self.dev)
-        stream = torch.cuda.Stream(device=self.runner.rt.device)
-        stream.wait_stream(torch.cuda.current_stream())
-        with torch.cuda.stream(stream):
-            for _ in range(2):   # warm-up outside the capture: lazy kernel attributes, allocator
-                self._forward()
-        torch.cuda.current_stream().wait_stream(stream)
+        if not self.graphs:
+            ops.fetch_ints(self.host, self.dev)
+            stream = torch.cuda.Stream(device=self.runner.rt.device)
+            stream.wait_stream(torch.cuda.current_stream())
+            with torch.cuda.stream(stream):
+                for _ in range(2):   # warm-up outside the capture: lazy kernel attributes, allocator
+                    self._forward(alone)
+            torch.cuda.current_stream().wait_stream(stream)
+        if not alone and not self.stages:
+            self.stages = [torch.zeros(self.n_ints, dtype=torch.int32).pin_memory() for _ in range(2)]
+            self.h_outs = [torch.zeros(self.rows + 1, dtype=torch.int32).pin_memory() for _ in range(2)]
+            self.events = [torch.cuda.Event() for _ in range(2)]
         torch.cuda.synchronize()
         from ..kernels import lib
         before = lib.launches
-        self.graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(self.graph):
-            if self.alone:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, pool=next(iter(self.graphs.values())).pool() if self.graphs else None):
+            if alone:
                 ops.fetch_ints(self.host, self.dev)
-            self._forward()
-        self.launches = lib.launches - before    # kernels in one replay
+            self.logits_of[alone] = self._forward(alone)
+        self.graphs[alone] = graph
+        self.launches[alone] = lib.launches - before
+
+    def _replay(self, alone: bool) -> None:
+        self.graphs[alone].replay()
+        self.logits = self.logits_of[alone]
 
     def run_ahead(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], steps: int) -> list[list[int]]:
         """`steps` decode steps with no host work in between: every step's sampled tokens are the next
@@ -114,7 +132,7 @@ class _DecodeGraph:
         self._fill(entries, sampling, reqs, self.runner.cache.rows(reqs))
         self.dev.copy_(self.host, non_blocking=True)
         for _ in range(steps):
-            self.graph.replay()
+            self._replay(False)
         self.h_history.copy_(self.history, non_blocking=True)
         self.h_out.copy_(self.result, non_blocking=True)
         torch.cuda.current_stream(self.runner.rt.device).synchronize()
@@ -124,7 +142,7 @@ class _DecodeGraph:
     def run(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], reqs: list, rows) -> list[int]:
         """reqs, rows: the entries' requests and their slots (`CacheManager.rows`)."""
         self._fill(entries, sampling, reqs, rows)
-        self.graph.replay()
+        self._replay(True)
         torch.cuda.current_stream(self.runner.rt.device).synchronize()
         out = self.np_out.tolist()
         self.runner.rt.raise_for(out[self.rows])
@@ -144,7 +162,7 @@ class _DecodeGraph:
             self.dev[self.rows:].copy_(stage[self.rows:], non_blocking=True)
         else:
             self.dev.copy_(stage, non_blocking=True)
-        self.graph.replay()
+        self._replay(False)
         self.h_outs[slot].copy_(self.result, non_blocking=True)
         self.events[slot].record()
         self.pending[slot] = True
@@ -180,21 +198,22 @@ class GpuExecutor:
         self.runner = runner
         self.sampler = Sampler(runner.rt.device)
         self.use_graphs, self.max_graph_rows = use_graphs, max_graph_rows
-        self._graphs: dict[tuple[int, bool], _DecodeGraph] = {}
+        self._graphs: dict[int, _DecodeGraph] = {}
         self.last_logits: Optional[torch.Tensor] = None
         self.steps = 0
         self.h2d_bytes = 0
         self.d2h_bytes = 0
 
     def graph_for(self, n_rows: int, alone: bool = True) -> _DecodeGraph:
-        """The captured step for this many rows, in the form of `execute` or that of `launch_decode` and `decode_ahead`."""
+        """The captured step for this many rows, with the form of `execute` or that of `launch_decode` and `decode_ahead` captured."""
         rows = 1
         while rows < n_rows:
             rows *= 2
-        g = self._graphs.get((rows, alone))
+        g = self._graphs.get(rows)
         if g is None:
-            g = self._graphs[rows, alone] = _DecodeGraph(self.runner, rows, alone)
-            g.capture()
+            g = self._graphs[rows] = _DecodeGraph(self.runner, rows)
+        if alone not in g.graphs:
+            g.capture(alone)
         return g
 
     def decode_ahead(self, entries: list[StepEntry], sampling: list[tuple[SamplingParams, int]], steps: int) -> list[list[int]]:

@@ -75,3 +75,31 @@ def test_a_bad_token_is_reported():
     with pytest.raises(DeviceStatusError):
         ex.execute([StepEntry(0, [1], [0])], [(GREEDY, 1)])
     assert isinstance(ex.execute([StepEntry(0, [1], [0])], [(GREEDY, 2)])[0], int)
+
+
+@pytest.mark.parametrize("batch", [1, 3])
+def test_tokens_left_by_one_form_feed_the_other(batch):
+    """Steps that feed on the tokens left on the device, each behind a step that the host waited for, give the tokens that waiting for every step gives."""
+    from inference_bench_b200.engine.executor import GpuExecutor
+    from inference_bench_b200.engine.step import StepEntry
+    from inference_bench_b200.sampling.params import SamplingParams
+    got = []
+    for mixed in (False, True):
+        r = _runner(256, 640, 4, 2, 64, 0, 16)
+        ex, tokens = GpuExecutor(r), []
+        for i in range(batch):
+            r.cache.admit(i)
+            r.step([StepEntry(i, list(range(5 + 7 * i)), [])])
+        last = [9 + i for i in range(batch)]
+        for step in range(6):
+            sampling = [(SamplingParams(temperature=1.5, seed=3 + i), step) for i in range(batch)]
+            if mixed and step % 2:
+                last = ex.collect(ex.launch_decode([StepEntry(i, [0], [0]) for i in range(batch)], sampling, feed=True))
+            else:
+                last = ex.execute([StepEntry(i, [t], [0]) for i, t in enumerate(last)], sampling)
+            tokens.append(last)
+        got.append(tokens)
+    assert got[0] == got[1]
+    assert len(set(sum(got[0], []))) > 1
+    g = ex.graph_for(batch)   # two captured forms over one set of buffers and one pool
+    assert set(g.graphs) == {True, False} and len({x.pool() for x in g.graphs.values()}) == 1
