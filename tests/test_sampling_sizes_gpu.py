@@ -43,3 +43,32 @@ def test_ties_and_masked_values(V):
     toks = torch.empty(len(rows), dtype=torch.int32, device=DEV)
     ops.sample_rows(torch.stack([x for x, _ in rows]).to(DEV), params, toks)
     assert toks.cpu().tolist() == [P.sample_token(x, p.temperature, p.seed, 2, p.top_k, p.top_p, p.min_p) for x, p in rows]
+
+
+# rows at counts that give a row's cluster eight, four, two CTAs and one; vocabularies whose rows start on 16 bytes and ones whose rows do not
+@pytest.mark.parametrize("V", [20000, 20003, 33001])
+def test_a_row_does_not_depend_on_the_rows_beside_it(V):
+    """Sharp cuts: unlike values of group A first, then many values alike, group B, which top-p takes in or leaves out by the last bits of A's mass."""
+    from inference_bench_b200.kernels import ops
+    from inference_bench_b200.sampling.params import SamplingParams
+    g = torch.Generator().manual_seed(V)
+    logits = torch.full((V,), -30.0)
+    order = torch.randperm(V, generator=g)
+    a, b = order[:V // 4], order[V // 4:V - 100]
+    logits[a] = torch.rand(len(a), generator=g) * 2
+    logits[b] = -0.5
+    mass = torch.exp(logits.double() - logits.max().double())
+    edge = float(mass[a].sum() / mass.sum())
+    rows = [SamplingParams(temperature=1.0, seed=i, top_p=edge * (1 + k * 2.0**-24)).row(3) for i, k in enumerate(range(-20, 20))]
+    alone = []
+    for r in rows:
+        t = torch.empty(1, dtype=torch.int32, device=DEV)
+        ops.sample_rows(logits[None].to(DEV), torch.tensor([r], dtype=torch.int32, device=DEV), t)
+        alone.append(t.item())
+    in_b = torch.isin(torch.tensor(alone), b)
+    assert in_b.any() and not in_b.all()   # the cut lies among these rows
+    for count in (40, 80, 160):
+        t = torch.empty(count, dtype=torch.int32, device=DEV)
+        params = torch.tensor((rows * 4)[:count], dtype=torch.int32, device=DEV)
+        ops.sample_rows(logits.expand(count, V).contiguous().to(DEV), params, t)
+        assert t.tolist() == (alone * 4)[:count], f"{count} rows"
