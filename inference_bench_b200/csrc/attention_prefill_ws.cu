@@ -439,7 +439,10 @@ __global__ void __launch_bounds__(kThreads, 2)
     ib::cluster_sync();
     constexpr int QPR = HD / 4, U = 2;
     const int share = (rows + slices - 1) / slices, r0 = slice * share, n_own = max(min(rows - r0, share), 0);
-    float* const f_s = (float*)(sm + SM::oQ + BM * 8);   // [share][kMaxSlices]: the factors of a row's slices, -1 for one in which it saw no key
+    // [share][kMaxSlices]: the factors of a row's slices, -1 for one in which it saw no key (no maximum and a sum of zero; where every score is NaN there is
+    // no maximum either, but the sum is NaN, which is then the factor). What is NaN in a slice is NaN in the result, as in a row that is not cut.
+    float* const f_s = (float*)(sm + SM::oQ + BM * 8);
+    auto unseen = [](float2 s) { return s.x == -INFINITY && s.y == 0.f; };
     if (tid < n_own) {
       float2 ml[kMaxSlices];
       float M = -INFINITY, l = 0.f;
@@ -449,12 +452,12 @@ __global__ void __launch_bounds__(kThreads, 2)
       for (int i = 0; i < kMaxSlices; i++) M = fmaxf(M, ml[i].x);
 #pragma unroll
       for (int i = 0; i < kMaxSlices; i++)
-        if (ml[i].x != -INFINITY) l = fmaf(ml[i].y, ex2(ml[i].x - M), l);
+        if (!unseen(ml[i])) l = fmaf(ml[i].y, ex2(ml[i].x - M), l);
       if (sink) l += ex2((tail.sink_values ? tail.sink_values[h] * 1.4426950408889634f : 0.f) - M);
       const float inv = (l > 0.f ? 1.f / l : 0.f) * ib::tail_factor(tail, t0 + r0 + tid, h);
       f_s[tid * (kMaxSlices + 1) + kMaxSlices] = inv;
 #pragma unroll
-      for (int i = 0; i < kMaxSlices; i++) f_s[tid * (kMaxSlices + 1) + i] = ml[i].x == -INFINITY ? -1.f : ex2(ml[i].x - M);
+      for (int i = 0; i < kMaxSlices; i++) f_s[tid * (kMaxSlices + 1) + i] = unseen(ml[i]) ? -1.f : ml[i].x == -INFINITY ? ml[i].y : ex2(ml[i].x - M);
     }
     __syncthreads();
     for (int idx0 = tid; idx0 < n_own * QPR; idx0 += U * kThreads) {
@@ -475,7 +478,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 #pragma unroll
         for (int i = 0; i < kMaxSlices; i++) {
           const float f = fr[i];
-          if (f >= 0.f && i < slices) a.x = fmaf(o[u][i].x, f, a.x), a.y = fmaf(o[u][i].y, f, a.y), a.z = fmaf(o[u][i].z, f, a.z), a.w = fmaf(o[u][i].w, f, a.w);
+          if (!(f < 0.f) && i < slices) a.x = fmaf(o[u][i].x, f, a.x), a.y = fmaf(o[u][i].y, f, a.y), a.z = fmaf(o[u][i].z, f, a.z), a.w = fmaf(o[u][i].w, f, a.w);
         }
         const float inv = fr[kMaxSlices];
         uint2 v;

@@ -46,3 +46,42 @@ def test_sliced_portions(hd, heads, kvh, page, shapes, window, keep):
     ops.attention_generic(q, view, pos, seg, window, scale, other, heads, rt.status, **kw)
     rt.check_status()
     assert (out.double() - other.double()).abs().max() <= 2e-2 * top
+
+
+@pytest.mark.parametrize("hd,heads,kvh,page,shape", [(128, 4, 2, 64, (1100, 61)), (64, 8, 4, 16, (700, 100)), (128, 32, 8, 64, (1300, 250))])   # 8, 4 and 2 slices
+def test_what_is_not_finite_stays_so(hd, heads, kvh, page, shape):
+    """A query row of NaN, a key that gives infinite scores, a value that is infinite: the rows that see them are not finite, the others keep their bits."""
+    from inference_bench_b200.engine.context import Segment, build_context
+    from inference_bench_b200.engine.runtime import Runtime
+    from inference_bench_b200.kernels import attention
+    from inference_bench_b200.kernels.ops import KvLayerView
+    L, n = shape
+    rt, pages = Runtime(DEV), -(-L // page)
+    g = torch.Generator().manual_seed(hd)
+    pool = torch.randn((1, pages, 2, kvh, page, hd), generator=g).to(torch.bfloat16)
+    q = torch.randn((n, heads * hd), generator=g).to(torch.bfloat16)
+    table = torch.arange(pages, dtype=torch.int32, device=DEV)[None]
+    ctx = build_context(rt, [Segment(0, 0, L - n, [0] * n)])
+    run = lambda q, pool: attention.paged_attention(ctx, q.to(DEV), KvLayerView(pool.to(DEV), 0, table), heads, None, 1 / math.sqrt(hd)).view(n, heads, hd).cpu()
+    clean = run(q, pool)
+    assert torch.isfinite(clean).all()
+    bad = q.clone()
+    bad[7, :hd] = float("nan")   # a row of the first head
+    got = run(bad, pool)
+    assert torch.isnan(got[7, 0]).all()
+    got[7, 0] = clean[7, 0]
+    assert torch.equal(got, clean)
+    group, key = heads // kvh, L - n // 2   # seen by the rows behind the middle only, in the last slice
+    for at in (3, key):   # (a key in the first slice, and that one)
+        bad = pool.clone()
+        bad[0, at // page, 0, 0, at % page, 5] = float("inf")   # scores of plus or minus infinity
+        got, sees = run(q, bad), torch.arange(L - n, L) >= at
+        plus = (q.view(n, heads, hd)[:, :group, 5].float() > 0) & sees[:, None]
+        assert torch.isnan(got[:, :group][plus]).all() and torch.equal(got[:, group:], clean[:, group:])
+        assert torch.isfinite(got[:, :group][~plus & sees[:, None]]).all()
+        bad = pool.clone()
+        bad[0, at // page, 1, 0, at % page, 9] = float("inf")
+        got = run(q, bad)
+        assert not torch.isfinite(got[sees][:, :group, 9]).any()
+        same = [c for c in range(hd) if c != 9]
+        assert torch.equal(got[:, :group][..., same], clean[:, :group][..., same]) and torch.equal(got[:, group:], clean[:, group:])
