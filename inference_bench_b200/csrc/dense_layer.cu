@@ -75,7 +75,14 @@ struct IbDenseLayer {
   int delta_parts;
 };
 
-// Returns the number of kernels launched, or -1 with the error's text set.
+// A launch, unless one before it was refused: the layer then ends, with the text of that one's error.
+#define IB_LAYER_RUN(launch, kernels) \
+  do {                                \
+    if ((launch) != 0) return -1;     \
+    n += (kernels);                   \
+  } while (0)
+
+// Returns the number of kernels launched, or -1 with the error's text set: nothing is launched behind a kernel that was refused.
 extern "C" int ib_dense_layer(const IbDenseStep* s, const IbDenseLayer* l) {
   const int T = s->T, H = s->hidden, Q = s->heads * s->head_dim, R = Q + 2 * s->kv_heads * s->head_dim;
   if (T <= 0 || (s->n_dec > 0 && !s->part_o) || s->n_dec + s->n_tiles <= 0) {
@@ -83,41 +90,40 @@ extern "C" int ib_dense_layer(const IbDenseStep* s, const IbDenseLayer* l) {
     return -1;
   }
   int n = 0;
-  bool bad = false;
-  auto run = [&](int code, int kernels = 1) { bad = bad || code != 0, n += kernels; };
   auto product = [&](const IbDenseProduct& p, const void* in, const void* w, int N, int K) {
-    if (p.kind == 2) run(ib_gemm_tcgen05_2cta_add(in, w, s->x, T, N, K, s->status, s->stream));
-    else if (p.kind == 1) run(ib_gemm_tcgen05_2cta(in, w, s->partial, T, N, K, s->status, s->stream));
-    else run(ib_gemm_tcgen05(in, w, s->partial, T, N, K, p.bn, p.splits, p.wide, s->status, s->stream));
+    if (p.kind == 2) return ib_gemm_tcgen05_2cta_add(in, w, s->x, T, N, K, s->status, s->stream);
+    if (p.kind == 1) return ib_gemm_tcgen05_2cta(in, w, s->partial, T, N, K, s->status, s->stream);
+    return ib_gemm_tcgen05(in, w, s->partial, T, N, K, p.bn, p.splits, p.wide, s->status, s->stream);
   };
   auto norm = [&](const float* delta, int parts, const float* w, float eps) {
-    run(ib_add_rmsnorm(s->x, delta, delta ? parts : 0, delta ? (long long)T * H : 0, w, s->h, IB_BF16, nullptr, T, H, eps, 1, s->stream));
+    return ib_add_rmsnorm(s->x, delta, delta ? parts : 0, delta ? (long long)T * H : 0, w, s->h, IB_BF16, nullptr, T, H, eps, 1, s->stream);
   };
-  norm(l->delta, l->delta_parts, l->norm, s->norm_eps);
+  IB_LAYER_RUN(norm(l->delta, l->delta_parts, l->norm, s->norm_eps), 1);
   if (s->qkv.kind == 3) {
-    run(ib_gemm_qkv_tcgen05_2cta(s->h, l->w_qkv, T, H, l->q_norm, l->k_norm, s->qk_eps, s->cos_t, s->sin_t, s->positions, s->seg_of_token, s->q, l->kv, 1, s->heads, s->status, s->stream));
+    IB_LAYER_RUN(ib_gemm_qkv_tcgen05_2cta(s->h, l->w_qkv, T, H, l->q_norm, l->k_norm, s->qk_eps, s->cos_t, s->sin_t, s->positions, s->seg_of_token, s->q, l->kv, 1, s->heads,
+                                          s->status, s->stream), 1);
   } else {
-    product(s->qkv, s->h, l->w_qkv, R, H);
-    run(ib_qk_norm_rope_kv(s->partial, s->qkv.kind == 1 ? 1 : s->qkv.splits, (long long)T * R, l->q_norm, l->k_norm, s->qk_eps, s->cos_t, s->sin_t, s->rot_half, s->positions,
-                           s->seg_of_token, s->q, IB_BF16, l->kv, 1, T, s->heads, s->status, nullptr, s->head_dim, s->head_dim, 0, 0, 0, 0, 0, s->stream));
+    IB_LAYER_RUN(product(s->qkv, s->h, l->w_qkv, R, H), 1);
+    IB_LAYER_RUN(ib_qk_norm_rope_kv(s->partial, s->qkv.kind == 1 ? 1 : s->qkv.splits, (long long)T * R, l->q_norm, l->k_norm, s->qk_eps, s->cos_t, s->sin_t, s->rot_half,
+                                    s->positions, s->seg_of_token, s->q, IB_BF16, l->kv, 1, T, s->heads, s->status, nullptr, s->head_dim, s->head_dim, 0, 0, 0, 0, 0, s->stream), 1);
   }
   if (s->n_dec)
-    run(ib_attention_decode_stream(s->q, l->kv, s->dec_tokens, s->n_dec, s->positions, s->seg_of_token, s->window, s->scale, s->part_o, s->part_ml, s->o, s->heads, s->max_slices,
-                                   s->tiles_per_slice, s->kv_map, l->kv_row0, s->status, s->stream), 2);
+    IB_LAYER_RUN(ib_attention_decode_stream(s->q, l->kv, s->dec_tokens, s->n_dec, s->positions, s->seg_of_token, s->window, s->scale, s->part_o, s->part_ml, s->o, s->heads,
+                                            s->max_slices, s->tiles_per_slice, s->kv_map, l->kv_row0, s->status, s->stream), 2);
   if (s->n_tiles)
-    run(ib_attention_prefill_ws(s->q, l->kv, s->tile_seg, s->tile_row0, s->n_tiles, s->seg_start, s->seg_pos0, s->window, s->scale, s->o, s->heads, s->kv_map, l->kv_row0, s->tile_keys,
-                                s->status, s->stream));
-  product(s->out, s->o, l->w_out, H, Q);
-  norm(s->out.kind == 2 ? nullptr : s->partial, s->out.kind == 1 ? 1 : s->out.splits, l->ff_norm, s->ff_norm_eps);
+    IB_LAYER_RUN(ib_attention_prefill_ws(s->q, l->kv, s->tile_seg, s->tile_row0, s->n_tiles, s->seg_start, s->seg_pos0, s->window, s->scale, s->o, s->heads, s->kv_map, l->kv_row0,
+                                         s->tile_keys, s->status, s->stream), 1);
+  IB_LAYER_RUN(product(s->out, s->o, l->w_out, H, Q), 1);
+  IB_LAYER_RUN(norm(s->out.kind == 2 ? nullptr : s->partial, s->out.kind == 1 ? 1 : s->out.splits, l->ff_norm, s->ff_norm_eps), 1);
   const IbDenseProduct& g = s->gate_up;
   if (g.kind == 3 && g.bn == 0) {
-    run(ib_gemm_swiglu_tcgen05_2cta(s->h, l->w_gate_up, s->act, T, s->inter, H, nullptr, 0.f, s->status, s->stream));
+    IB_LAYER_RUN(ib_gemm_swiglu_tcgen05_2cta(s->h, l->w_gate_up, s->act, T, s->inter, H, nullptr, 0.f, s->status, s->stream), 1);
   } else if (g.kind == 3) {
-    run(ib_gemm_swiglu_tcgen05(s->h, l->w_gate_up, s->act, T, s->inter, H, g.bn, g.wide, nullptr, 0.f, s->status, s->stream));
+    IB_LAYER_RUN(ib_gemm_swiglu_tcgen05(s->h, l->w_gate_up, s->act, T, s->inter, H, g.bn, g.wide, nullptr, 0.f, s->status, s->stream), 1);
   } else {
-    product(g, s->h, l->w_gate_up, 2 * s->inter, H);
-    run(ib_silu_mul(s->partial, g.kind == 1 ? 1 : g.splits, (long long)T * 2 * s->inter, s->act, IB_BF16, T, s->inter, nullptr, 0.f, s->stream));
+    IB_LAYER_RUN(product(g, s->h, l->w_gate_up, 2 * s->inter, H), 1);
+    IB_LAYER_RUN(ib_silu_mul(s->partial, g.kind == 1 ? 1 : g.splits, (long long)T * 2 * s->inter, s->act, IB_BF16, T, s->inter, nullptr, 0.f, s->stream), 1);
   }
-  product(s->down, s->act, l->w_down, H, s->inter);
-  return bad ? -1 : n;
+  IB_LAYER_RUN(product(s->down, s->act, l->w_down, H, s->inter), 1);
+  return n;
 }

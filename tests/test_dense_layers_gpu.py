@@ -72,3 +72,22 @@ def test_other_kernels_asked_for_run(options, monkeypatch):
     r = _runner(256, 640, 4, 2, 64, 0, 16, RuntimeOptions(**options))
     r.cache.admit(0)
     assert torch.isfinite(r.step([StepEntry(0, list(range(40)), [39])])).all()
+
+
+def test_a_refused_kernel_ends_the_layer(monkeypatch):
+    """Nothing is launched behind a product that was refused: the request's pages and the count of kernels stay as they were before it."""
+    from inference_bench_b200.engine.step import StepEntry
+    from inference_bench_b200.kernels import gemm_tcgen05 as G, lib
+    r = _runner(256, 640, 4, 2, 64, 0, 16)
+    r.cache.admit(0)
+    r.step([StepEntry(0, list(range(40)), [39])])
+    before = [g.tensor.clone() for g in r.cache.groups]
+    form = G.product_form
+    monkeypatch.setattr(G, "product_form", lambda rt, T, n, k, allow_split=True, add=False: form(rt, T, n, k, allow_split, add) if add else ("single", 17, 1, False))
+    with pytest.raises(lib.KernelError, match="token tile 17"):
+        r.step([StepEntry(0, list(range(50)), [49])])
+    monkeypatch.undo()
+    torch.cuda.synchronize()
+    assert all(torch.equal(a, g.tensor) for a, g in zip(before, r.cache.groups))
+    assert r.cache.length(0) == 40
+    assert torch.isfinite(r.step([StepEntry(0, list(range(50)), [49])])).all()
