@@ -27,8 +27,13 @@ constexpr int BK = 64;
 constexpr int UMMA_K = 16;
 constexpr int kThreads = 192;
 // EPI_ADD adds where the stream lies, in L2: a read, an addition and a store by the epilogue's threads took 4 to 6 us more than a store alone, since a
-// tile's last trip to memory has nothing behind it (1,003 tokens of 4,096 x 4,096: 41.0 us, 34.8 now; 2,048 of 1,024 x 2,048: 28.7 and 24.6). The sums
-// are the same bits but for results below 2^-126, which become zero.
+// tile's last trip to memory has nothing behind it (1,003 tokens of 4,096 x 4,096: 41.0 us, 34.8 now; 2,048 of 1,024 x 2,048: 28.7 and 24.6). Such an
+// addition takes numbers below 2^-126 for zero, in the stream and in the sum. With a product of 2^-100 and more neither can matter: a number below 2^-126 in the
+// stream is less than half of the product's last place, and a sum of the product (a multiple of 2^-123) and a number of at least 2^-102 (a multiple of 2^-125) is
+// zero or at least 2^-125. Where a thread has a smaller
+// product among its 32 it adds them itself, so the sums are the bits of an IEEE addition.
+// (What the look at the 32 costs, warm: 1,003 tokens of 4,096 x 4,096 42.4 -> 43.0 us, 2,048 of 1,024 x 2,048 19.8 -> 20.1, 300 of 1,024 x 3,072 22.1 -> 23.6.)
+constexpr float kAddInL2 = 0x1p-100f;
 constexpr int EPI_STORE = 0, EPI_SWIGLU = 1, EPI_ADD = 2;   // float32 out; bfloat16 silu(gate) * up; float32 out += product
 constexpr int EPI_QKV = 3;   // the q/k/v projection finished in the epilogue: per-head norm, rotation, queries out, keys and values into the cache
 constexpr int EPI_CLAMPED = 6;   // EPI_SWIGLU with clamped halves (ib::clamped_glu): the limit in QkvEpi::act_pq[0], the slope in QkvEpi::act_slope
@@ -448,6 +453,17 @@ __global__ void __launch_bounds__(kThreads, 1)
             sm100::tmem_ld_32x32b_x32(lane_addr + b * MT * BN + m * BN + c0, r);
             sm100::tmem_ld_wait();
             if (n < N) {
+              if constexpr (EPI == EPI_ADD) {
+                float least = INFINITY;
+#pragma unroll
+                for (int c = 0; c < 32; c++) least = fminf(least, t0 + c0 + c < t_end ? fabsf(__uint_as_float(r[c])) : INFINITY);
+                if (least < kAddInL2) {
+#pragma unroll
+                  for (int c = 0; c < 32; c++)
+                    if (t0 + c0 + c < t_end) dst[(size_t)(t0 + c0 + c) * N + n] += __uint_as_float(r[c]);
+                  continue;
+                }
+              }
 #pragma unroll
               for (int c = 0; c < 32; c++) {
                 const int t = t0 + c0 + c;

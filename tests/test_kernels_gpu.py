@@ -764,3 +764,29 @@ def test_sample_rows_matches_plain():
     want = [P.sample_token(logits[i], p.temperature, p.seed, steps[i], p.top_k, p.top_p, p.min_p) for i, p in enumerate(params)]
     assert toks.cpu().tolist() == want
     assert want[0] == 17 and want[7] == int(logits[7].argmax())
+
+
+@pytest.mark.parametrize("T,N,K", [(256, 256, 64), (300, 520, 72)])
+def test_sums_added_to_the_stream_are_ieee_sums(T, N, K):
+    """Products of every size down to numbers below 2^-126, zeros, infinities and NaN, added to a stream with the same: the bits of an addition in float32."""
+    from inference_bench_b200.kernels import gemm_tcgen05 as G
+    status, g = torch.zeros(1, dtype=torch.int32, device=DEV), _g(T + N)
+    x = torch.randn((T, K), generator=g)
+    w = torch.randn((N, K), generator=g) * 2.0 ** torch.randint(-126, 3, (N, 1), generator=g).float()   # rows of the product between 2^-126 and 2^3
+    x[5] = 0.0
+    w[7] = 0.0
+    x, w = x.to(torch.bfloat16).to(DEV), w.to(torch.bfloat16).to(DEV)
+    product = torch.empty((T, N), device=DEV)
+    G.gemm_pair(x, w, product, status)
+    near = lambda f: product.cpu() * f
+    streams = [torch.randn((T, N), generator=g) * 2.0 ** torch.randint(-149, 3, (T, N), generator=g).float(),   # (some below 2^-126)
+               near(-1.0), near(-1.0 + 2.0 ** -20), near(-0.75), torch.full((T, N), 1e-40), torch.full((T, N), -0.0)]
+    odd = torch.randn((T, N), generator=g)
+    odd[::3], odd[1::3, ::2] = float("inf"), float("nan")
+    for old in streams + [odd]:
+        out = old.to(DEV)
+        G.gemm_pair(x, w, out, status, add=True)
+        want = old + product.cpu()
+        assert torch.equal(torch.isnan(out.cpu()), torch.isnan(want))
+        assert torch.equal(out.cpu().view(torch.int32)[~torch.isnan(want)], want.view(torch.int32)[~torch.isnan(want)])
+    assert int(status[0]) == 0
