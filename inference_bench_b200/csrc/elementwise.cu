@@ -316,9 +316,13 @@ __device__ __forceinline__ O silu_mul_one(float g, float u, const float* limit, 
   return ib::from_f32<O>(limit ? ib::clamped_glu<false>(g, u, limit[0], slope) : (g / (1.f + expf(-g))) * u);
 }
 
-// Four values a thread (I a multiple of four, rows on 16 bytes), the partial sums of both halves requested four at a time and added in order: a trip to
-// memory where there were as many as partial sums. 777 tokens of 3,072 float32 values: 18.4 us with one value a thread, 12.3 now; 300 of 12,288: 24.5 and
+// Four values a thread (I a multiple of four, rows on 16 bytes), the partial sums of both halves requested together (the first
+// five, then four at a time) and added in order: a trip to memory where there were as many as partial sums. 777 tokens of 3,072 float32 values: 18.4 us with one value a thread, 12.3 now; 300 of 12,288: 24.5 and
 // 16.4; 64 tokens of 3,072 in four partial sums 10.2 and 8.2 (timed with the caches cold).
+// From 2^18 partial sums on: with fewer the four exponentials and divisions in a row of a thread show (warm, us, one value a thread | four: 8 tokens of 3,072 1.5 |
+// 1.9, 300 of 768 2.0 | 2.2, of 1,408 2.9 | 2.6; in four partial sums 8 of 3,072 2.2 | 2.0, 64 of 1,408 2.7 | 2.2, in five 8 of 3,072 1.9 | 2.3).
+constexpr long long kSiluWide = 1 << 18;
+
 template <typename O>
 __global__ void __launch_bounds__(128) silu_mul_vec_kernel(const float* __restrict__ gu, int P, size_t stride, O* __restrict__ act, int I, const float* __restrict__ limit, float slope) {
   ib::pdl_launch_dependents();
@@ -326,15 +330,23 @@ __global__ void __launch_bounds__(128) silu_mul_vec_kernel(const float* __restri
   const int t = blockIdx.y, i = (blockIdx.x * 128 + threadIdx.x) * 4;
   if (i >= I) return;
   const float* row = gu + (size_t)t * 2 * I + i;
-  float4 g = *(const float4*)row, u = *(const float4*)(row + I);
-  for (int p0 = 1; p0 < P; p0 += 4) {
-    float4 a[4], b[4];
+  float4 g, u, a[5], b[5];
+  auto request = [&](int p0, int n) {
 #pragma unroll
-    for (int p = 0; p < 4; p++)
-      if (p0 + p < P) a[p] = *(const float4*)(row + (p0 + p) * stride), b[p] = *(const float4*)(row + (p0 + p) * stride + I);
+    for (int p = 0; p < 5; p++)
+      if (p < n && p0 + p < P) a[p] = *(const float4*)(row + (p0 + p) * stride), b[p] = *(const float4*)(row + (p0 + p) * stride + I);
+  };
+  auto add = [&](int p0, int first, int n) {
 #pragma unroll
-    for (int p = 0; p < 4; p++)
-      if (p0 + p < P) g.x += a[p].x, g.y += a[p].y, g.z += a[p].z, g.w += a[p].w, u.x += b[p].x, u.y += b[p].y, u.z += b[p].z, u.w += b[p].w;
+    for (int p = 0; p < 5; p++)
+      if (p >= first && p < n && p0 + p < P) g.x += a[p].x, g.y += a[p].y, g.z += a[p].z, g.w += a[p].w, u.x += b[p].x, u.y += b[p].y, u.z += b[p].z, u.w += b[p].w;
+  };
+  request(0, 5);
+  g = a[0], u = b[0];
+  add(0, 1, 5);
+  for (int p0 = 5; p0 < P; p0 += 4) {
+    request(p0, 4);
+    add(p0, 0, 4);
   }
   alignas(16) O v[4] = {silu_mul_one<O>(g.x, u.x, limit, slope), silu_mul_one<O>(g.y, u.y, limit, slope), silu_mul_one<O>(g.z, u.z, limit, slope), silu_mul_one<O>(g.w, u.w, limit, slope)};
   O* to = act + (size_t)t * I + i;
@@ -547,7 +559,7 @@ extern "C" int ib_silu_mul(const float* gu, int P, long long stride, void* act, 
   if (T == 0) return 0;
   IB_CHECK_ARG(T > 0 && I > 0 && P >= 1, "silu_mul: bad sizes T=%d I=%d P=%d", T, I, P);
   IB_CHECK_ARG(T <= 65535, "silu_mul: T=%d rows exceed the grid limit 65535", T);
-  if (I % 4 == 0 && stride % 4 == 0 && (((uintptr_t)gu | (uintptr_t)act) & 15) == 0 && (act_dtype == IB_F32 || act_dtype == IB_BF16)) {
+  if ((long long)T * I * P >= kSiluWide && I % 4 == 0 && stride % 4 == 0 && (((uintptr_t)gu | (uintptr_t)act) & 15) == 0 && (act_dtype == IB_F32 || act_dtype == IB_BF16)) {
     const dim3 vec((I / 4 + 127) / 128, T);
     if (act_dtype == IB_F32) ib::launch(silu_mul_vec_kernel<float>, vec, 128, 0, stream, gu, P, (size_t)stride, (float*)act, I, limit, slope);
     else ib::launch(silu_mul_vec_kernel<__nv_bfloat16>, vec, 128, 0, stream, gu, P, (size_t)stride, (__nv_bfloat16*)act, I, limit, slope);
