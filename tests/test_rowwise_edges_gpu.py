@@ -27,6 +27,15 @@ def test_silu_mul(T, I, P, dtype):
     assert ((act[:T].double() - want).abs() <= bound).all() and (act[T:] == 7.0).all()
 
 
+# from 2^18 partial sums on a thread has four neighbours: inner sizes that end inside a CTA's 512, at it and behind it; partial sums around the five that are
+# requested together and the four behind them
+@pytest.mark.parametrize("T,I", [(2100, 132), (520, 508), (512, 512), (300, 1028), (90, 3072), (700, 510)])
+@pytest.mark.parametrize("P", [1, 2, 5, 6, 10])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_silu_mul_of_many(T, I, P, dtype):
+    test_silu_mul(T, I, P, dtype)
+
+
 @pytest.mark.parametrize("H", [8, 504, 520, 4096, 4104, 12, 7])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_embed(status, H, dtype):  # noqa: F811
