@@ -345,15 +345,19 @@ def grouped_pairs(rows: int, groups: int, inter: int, sm_count: int = FITTED_SM_
 
 
 def pair_tile(rows: int, groups: int, inter: int, gated: bool = True, sm_count: int = FITTED_SM_COUNT) -> int:
-    """Rows of a token tile of that form. 256: an expert's share is mostly one tile, loaded and multiplied as far as it goes, so that its matrix passes through
-    the SMs once (gate and up of 64 experts, 192 rows each: 156 us against 174). 128 where gate and up rows cannot be taken sixteen at a time, and
-    where large shares make fewer than four rounds of the wide tiles, whose last is then nearly empty (16 experts of 1,024 x 1,024, 512 rows each:
-    82 us against 90)."""
+    """Rows of a token tile of that form. 256 around 112 to 256 rows an expert: its share is then mostly one tile, loaded and multiplied as far as it goes, so that
+    its matrix passes through the SMs once. 128 above, where the last wide tile is mostly nearly empty and costs almost a whole one, and below, where a share
+    fits the narrow tile and its four blocks of matrix rows keep more of a matrix in flight; but for matrices that the narrow form's blocks of 256 gate
+    rows pad by more than a twelfth, or of which it has fewer tiles than there are pairs; and where gate and up rows cannot be taken sixteen at a time.
+    Both products, tokens drawn evenly over the experts, 128 | 256 in us: 128 experts of 1,536 x 4,096, 32 rows each 788 | 811, 96 834 | 899, 128 907 | 893,
+    160 1,135 | 936; 8 of 14,336 x 4,096, 64 rows 486 | 510, 160 623 | 569, 300 889 | 1,098, 512 1,548 | 1,845; 64 of 1,408 x 2,048, 64 rows 229 | 223, 160 262
+    | 242, 300 395 | 446, 512 567 | 637, 700 770 | 717; 32 of 2,880 x 2,880, 300 rows 590 | 684, 700 1,041 | 981, 768 1,141 | 1,231; 16 of 1,024 x 1,024, 64
+    rows 63 | 55. Experts of unlike shares (a factor of two between them) move the figures above 256 towards 128."""
     avg = -(-rows // groups)
-    if gated and inter % 16:
+    if gated and inter % 16 or avg > PAIR_WIDE_TILE:
         return PAIR_TILE
-    rounds = groups * -(-avg // PAIR_WIDE_TILE) * -(-inter // 128) / (sm_count // 2)
-    return PAIR_TILE if avg > PAIR_WIDE_TILE and rounds < 4 else PAIR_WIDE_TILE
+    blocks = -(-inter // 256)
+    return PAIR_WIDE_TILE if avg >= 112 or 12 * 256 * blocks > 13 * inter or groups * blocks < sm_count // 2 else PAIR_TILE
 
 
 def gemm_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bn: int, offsets: torch.Tensor, tiles: torch.Tensor, status: torch.Tensor, pair: bool = False) -> None:

@@ -52,3 +52,11 @@ def test_the_tile_is_chosen_by_sizes():
     assert [G.grouped_pairs(r, 4, 256) for r in (4 * 127, 4 * 128)] == [False, True] and not G.grouped_pairs(1 << 20, 257, 1408)
     assert G.pair_tile(12288, 64, 1408) == 256 and G.pair_tile(12288, 64, 1400) == 128 and G.pair_tile(12288, 64, 1400, gated=False) == 256
     assert G.pair_tile(16 * 512, 16, 1024) == 128 and G.pair_tile(16 * 256, 16, 1024) == 256
+
+
+def test_the_tile_of_small_and_large_shares():
+    from inference_bench_b200.kernels import gemm_tcgen05 as G
+    of = lambda avg, n, inter: G.pair_tile(avg * n, n, inter)
+    assert [of(a, 128, 1536) for a in (32, 111, 112, 256, 257, 300, 512, 700)] == [128, 128, 256, 256, 128, 128, 128, 128]
+    assert [of(a, 64, 1408) for a in (32, 192, 257)] == [256, 256, 128]   # (5.5 blocks of 256 gate rows are 6)
+    assert [of(64, 16, 1024), of(64, 32, 1024), of(64, 32, 2880)] == [256, 128, 128]
