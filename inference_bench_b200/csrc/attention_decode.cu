@@ -10,6 +10,7 @@
 // Reference design: crates/kir/src/cuda/attention/decode.rs, combine.rs (split-KV with packed GQA rows).
 #include <cuda.h>
 
+#include "entries.h"
 #include "kv_view.cuh"
 #include "mma_tiles.cuh"
 #include "sm100.cuh"

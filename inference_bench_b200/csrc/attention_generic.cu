@@ -11,6 +11,7 @@
 //    (mask: crates/kir/src/cuda/attention/flash_mma.rs:193).
 #include <type_traits>
 
+#include "entries.h"
 #include "kv_view.cuh"
 
 namespace {

@@ -25,6 +25,7 @@
 
 #include <algorithm>
 
+#include "entries.h"
 #include "kv_view.cuh"
 #include "mma_tiles.cuh"
 #include "sm100.cuh"

@@ -5,27 +5,7 @@
 // about 15 us, a launch takes 3, and the kernel itself 3 to 10. The forms of the products and the buffers are worked out once a step
 // (kernels/dense.py); a layer then costs its launches. 100 tokens in two layers of the 0.6B sizes: 514 to 277 us of host a step (with the step's arrays
 // in one transfer), 61 tokens behind 900 in eight layers 883 to 445, as long as its kernels.
-#include "kv_view.cuh"
-
-extern "C" {
-int ib_add_rmsnorm(float* x, const float* delta, int P, long long delta_stride, const float* w, void* out, int out_dtype, const int* rows, int n_rows, int H, float eps, int write_x,
-                   cudaStream_t stream);
-int ib_silu_mul(const float* gu, int P, long long stride, void* act, int act_dtype, int T, int I, const float* limit, float slope, cudaStream_t stream);
-int ib_qk_norm_rope_kv(const float* qkv, int P, long long stride_p, const float* q_norm_w, const float* k_norm_w, float eps, const float* cos_t, const float* sin_t, int rot_half,
-                       const int* positions, const int* seg_of_token, void* q_out, int act_dtype, const IbKvView* kv, int write_kv, int T, int heads, unsigned* status,
-                       const float* bias, int qk_dim, int v_dim, int row, int q_col, int k_col, int v_col, int unit_norm_after, cudaStream_t stream);
-int ib_attention_prefill_ws(const void* q, const IbKvView* kv, const int* tile_seg, const int* tile_row0, int n_tiles, const int* seg_start, const int* seg_pos0, int window, float scale,
-                            void* out, int heads, const void* kv_map, long long view_row0, int max_keys, unsigned* status, cudaStream_t stream);
-int ib_attention_decode_stream(const void* q, const IbKvView* kv, const int* dec_tokens, int n_dec, const int* positions, const int* seg_of_token, int window, float scale, float* part_o,
-                               float* part_ml, void* out, int heads, int max_slices, int tiles_per_slice, const void* kv_map, long long view_row0, unsigned* status, cudaStream_t stream);
-int ib_gemm_tcgen05(const void* x, const void* w, float* out, int T, int N, int K, int bn, int splits, int wide, unsigned* status, cudaStream_t stream);
-int ib_gemm_swiglu_tcgen05(const void* x, const void* w, void* act, int T, int I, int K, int bn, int half, const float* limit, float slope, unsigned* status, cudaStream_t stream);
-int ib_gemm_tcgen05_2cta(const void* x, const void* w, float* out, int T, int N, int K, unsigned* status, cudaStream_t stream);
-int ib_gemm_tcgen05_2cta_add(const void* x, const void* w, float* out, int T, int N, int K, unsigned* status, cudaStream_t stream);
-int ib_gemm_swiglu_tcgen05_2cta(const void* x, const void* w, void* act, int T, int I, int K, const float* limit, float slope, unsigned* status, cudaStream_t stream);
-int ib_gemm_qkv_tcgen05_2cta(const void* x, const void* w, int T, int K, const float* q_norm_w, const float* k_norm_w, float eps, const float* cos_t, const float* sin_t,
-                             const int* positions, const int* seg_of_token, void* q_out, const IbKvView* kv, int write_kv, int heads, unsigned* status, cudaStream_t stream);
-}
+#include "entries.h"
 
 // How a product runs. kind 0: the single-CTA kernel, `splits` partial sums of tiles of bn tokens; 1: CTA pairs, one sum; 2: CTA pairs, added to the
 // residual stream; 3: with the epilogue that finishes it (q/k/v: norm, rotation and cache write on CTA pairs; gate/up: the activation, on CTA pairs where
@@ -126,4 +106,10 @@ extern "C" int ib_dense_layer(const IbDenseStep* s, const IbDenseLayer* l) {
   }
   IB_LAYER_RUN(product(s->down, s->act, l->w_down, H, s->inter), 1);
   return n;
+}
+
+// The sizes of IbDenseStep and IbDenseLayer, for a caller that mirrors them in another language.
+extern "C" int ib_dense_sizes(int* step, int* layer) {
+  *step = (int)sizeof(IbDenseStep), *layer = (int)sizeof(IbDenseLayer);
+  return 0;
 }

@@ -9,6 +9,7 @@
 #include <type_traits>
 
 #include "common.cuh"
+#include "entries.h"
 
 static thread_local char g_error[512] = "";
 extern "C" const char* ib_last_error() { return g_error; }

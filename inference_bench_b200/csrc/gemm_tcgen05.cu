@@ -17,6 +17,7 @@
 // with the ACT epilogue for gate/up (core.rs:199-213).
 #include <cuda.h>
 
+#include "entries.h"
 #include "sm100.cuh"
 #include "tma_host.cuh"
 

@@ -16,6 +16,7 @@
 
 #include <cuda_bf16.h>
 
+#include "entries.h"
 #include "kv_view.cuh"
 #include "sm100.cuh"
 #include "tma_host.cuh"

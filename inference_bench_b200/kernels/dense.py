@@ -8,6 +8,7 @@ same arguments, so the same bits; the buffers belong to the step, and everything
 from __future__ import annotations
 
 import ctypes as C
+import functools
 from typing import Optional
 
 import torch
@@ -40,6 +41,17 @@ class DenseLayer(C.Structure):
 
 
 L.register("ib_dense_layer", [C.POINTER(DenseStep), C.POINTER(DenseLayer)])
+L.register("ib_dense_sizes", [C.POINTER(_i), C.POINTER(_i)])
+
+
+@functools.lru_cache(maxsize=1)
+def _check_mirrors() -> None:
+    """The library and the structures above are of one make."""
+    step, layer = _i(), _i()
+    L.load().ib_dense_sizes(C.byref(step), C.byref(layer))
+    if (step.value, layer.value) != (C.sizeof(DenseStep), C.sizeof(DenseLayer)):
+        raise L.KernelError(f"csrc/dense_layer.cu has structures of {step.value} and {layer.value} bytes, kernels/dense.py of {C.sizeof(DenseStep)} and {C.sizeof(DenseLayer)}")
+
 
 # Steps of more tokens go layer by layer through the parts: their kernels take longer than the host, and one buffer for a whole layer's intermediates is
 # harder for the allocator to find than its pieces (contexts of 8 requests built in steps of 8,192 tokens: 42 ms, 54 with it). 2,048 tokens, the default
@@ -65,6 +77,7 @@ class DenseLayers:
     """A step's dense layers of one key (`PreNormBlock.repeat_key`). `fits` tells whether the key's sizes are ones the kernels take."""
 
     def __init__(self, ctx, block, cache, x: torch.Tensor):
+        _check_mirrors()
         m, f, rt, T = block.mixer, block.feed_forward, ctx.rt, ctx.n_tokens
         H, I, hd, opt = m.hidden, f.intermediate, m.head_dim, rt.options
         Q, R = m.heads * hd, (m.heads + 2 * m.kv_heads) * hd
