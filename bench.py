@@ -342,8 +342,8 @@ def run_ours(args) -> dict:
             from inference_bench_b200.kernels import lib as L
             real, report["without"] = L.call, {}
             try:
-                for kind in args.leave_out.split(","):
-                    names = set(sum((LEAVE_OUT[k] for k in kind.split("+")), []))
+                for kind in ["nothing"] + args.leave_out.split(","):   # (to subtract from: the same calls one by one, with all of them made)
+                    names = set(sum((LEAVE_OUT[k] for k in kind.split("+") if k != "nothing"), []))
                     L.call = lambda name, *a, _n=names: None if name in _n else real(name, *a)
                     report["without"][kind] = measure_prefill(engine, args.steps, warm, after)
             finally:

@@ -59,6 +59,7 @@ def _check_mirrors() -> None:
 MAX_TOKENS = 2560
 
 KIND = {"single": 0, "pair": 1, "add": 2}
+EPILOGUE = 3   # finished by the product's own epilogue
 
 
 def _product(form: tuple) -> Product:
@@ -67,10 +68,10 @@ def _product(form: tuple) -> Product:
 
 def takes(ctx, cache) -> bool:
     """Whether this step's dense layers can go this way at all (their own sizes are asked in `DenseLayers`): a bfloat16 step with prompt portions on the
-    kernels that TMA feeds, and nobody who looks at the calls one by one."""
+    kernels that TMA feeds, outside a layer whose calls are being noted."""
     opt = ctx.rt.options
     return (ctx.n_tokens <= MAX_TOKENS and ctx.rt.mode == "bfloat16" and ctx.rt.gemm != "simt" and not ctx.fixed_shape and ctx.n_segments != ctx.n_tokens and opt.prefill_attention != "tcgen05"
-            and opt.decode_attention != "split" and not L.watched() and cache.tma()[0] is not None)
+            and opt.decode_attention != "split" and L.notes.calls is None and cache.tma()[0] is not None)
 
 
 class DenseLayers:
@@ -91,13 +92,13 @@ class DenseLayers:
         work = A._work_lists(ctx)
         rot_half = 0 if cos is None else cos.shape[1]
         if hd == 128 and rot_half in (0, 64) and G.qkv_in_epilogue(rt, T, R, H):
-            qkv = Product(3, 0, 0, 0)
+            qkv = Product(EPILOGUE, 0, 0, 0)
         else:
             qkv = _product(G.product_form(rt, T, R, H))
         out, down = _product(G.product_form(rt, T, H, Q, add=True)), _product(G.product_form(rt, T, H, I, add=True))
         if opt.swiglu_epilogue and G.swiglu_supported(T, H, I):
             bn, half = G.swiglu_form(T, I, opt.pair_min_tokens)
-            gate_up = Product(3, bn, 0, 1 if half else 0)
+            gate_up = Product(EPILOGUE, bn, 0, 1 if half else 0)
         else:
             gate_up = _product(G.product_form(rt, T, 2 * I, H))
         max_slices = tps = 0
@@ -139,7 +140,51 @@ class DenseLayers:
         l.k_norm = None if m.k_norm is None else m.k_norm.data_ptr()
         l.kv = C.addressof(cache.c_view())
         l.kv_row0, l.delta, l.delta_parts = cache.tma()[1], delta, parts
-        L.call_counted("ib_dense_layer", self._ref, self._layer_ref)
+        if L.watched():
+            self._one_by_one(C.byref(cache.c_view()))
+        else:
+            L.call_counted("ib_dense_layer", self._ref, self._layer_ref)
+
+    def _one_by_one(self, kv) -> None:
+        """The launches of `ib_dense_layer`, each through `call`, for somebody who looks at the calls: the same kernels on the same buffers."""
+        s, l = self.step, self.layer
+        T, H, I, Q = s.T, s.hidden, s.inter, s.heads * s.head_dim
+        R, end = Q + 2 * s.kv_heads * s.head_dim, (s.status, s.stream)
+
+        def product(p: Product, x, w, n: int, k: int) -> None:
+            if p.kind == KIND["add"]:
+                L.call("ib_gemm_tcgen05_2cta_add", x, w, s.x, T, n, k, *end)
+            elif p.kind == KIND["pair"]:
+                L.call("ib_gemm_tcgen05_2cta", x, w, s.partial, T, n, k, *end)
+            else:
+                L.call("ib_gemm_tcgen05", x, w, s.partial, T, n, k, p.bn, p.splits, p.wide, *end)
+
+        def norm(delta, parts: int, w, eps: float) -> None:
+            L.call("ib_add_rmsnorm", s.x, delta, parts if delta else 0, T * H if delta else 0, w, s.h, L.BF16, None, T, H, eps, 1, s.stream)
+
+        norm(l.delta, l.delta_parts, l.norm, s.norm_eps)
+        if s.qkv.kind == EPILOGUE:
+            L.call("ib_gemm_qkv_tcgen05_2cta", s.h, l.w_qkv, T, H, l.q_norm, l.k_norm, s.qk_eps, s.cos_t, s.sin_t, s.positions, s.seg_of_token, s.q, kv, 1, s.heads, *end)
+        else:
+            product(s.qkv, s.h, l.w_qkv, R, H)
+            L.call("ib_qk_norm_rope_kv", s.partial, s.qkv.splits, T * R, l.q_norm, l.k_norm, s.qk_eps, s.cos_t, s.sin_t, s.rot_half, s.positions, s.seg_of_token, s.q, L.BF16, kv, 1,
+                   T, s.heads, s.status, None, s.head_dim, s.head_dim, 0, 0, 0, 0, 0, s.stream)
+        if s.n_dec:
+            L.call("ib_attention_decode_stream", s.q, kv, s.dec_tokens, s.n_dec, s.positions, s.seg_of_token, s.window, s.scale, s.part_o, s.part_ml, s.o, s.heads, s.max_slices,
+                   s.tiles_per_slice, s.kv_map, l.kv_row0, *end)
+        if s.n_tiles:
+            L.call("ib_attention_prefill_ws", s.q, kv, s.tile_seg, s.tile_row0, s.n_tiles, s.seg_start, s.seg_pos0, s.window, s.scale, s.o, s.heads, s.kv_map, l.kv_row0, s.tile_keys,
+                   *end)
+        product(s.out, s.o, l.w_out, H, Q)
+        norm(None if s.out.kind == KIND["add"] else s.partial, s.out.splits, l.ff_norm, s.ff_norm_eps)
+        if s.gate_up.kind == EPILOGUE and s.gate_up.bn == 0:
+            L.call("ib_gemm_swiglu_tcgen05_2cta", s.h, l.w_gate_up, s.act, T, I, H, None, 0.0, *end)
+        elif s.gate_up.kind == EPILOGUE:
+            L.call("ib_gemm_swiglu_tcgen05", s.h, l.w_gate_up, s.act, T, I, H, s.gate_up.bn, s.gate_up.wide, None, 0.0, *end)
+        else:
+            product(s.gate_up, s.h, l.w_gate_up, 2 * I, H)
+            L.call("ib_silu_mul", s.partial, s.gate_up.splits, T * 2 * I, s.act, L.BF16, T, I, None, 0.0, s.stream)
+        product(s.down, s.act, l.w_down, H, I)
 
     def pending(self) -> Optional[torch.Tensor]:
         """What the last layer left to add, as the parts hand it on."""

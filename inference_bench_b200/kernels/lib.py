@@ -174,5 +174,5 @@ _own_call = call
 
 
 def watched() -> bool:
-    """Whether somebody looks at this thread's calls one by one: notes them, or has put a function of its own in the place of `call`."""
-    return call is not _own_call or notes.calls is not None
+    """Whether somebody looks at the calls one by one, by a function of their own in the place of `call`."""
+    return call is not _own_call

@@ -35,31 +35,39 @@ STEPS = [[2], [15, 1, 1], [17, 16], [31, 1, 33], [63, 1, 1], [65], [127, 1, 1], 
 
 @pytest.mark.parametrize("sizes", [(256, 640, 4, 2, 64, 0, 16), (256, 640, 2, 2, 128, 70, 8), (1024, 3072, 16, 8, 128, 0, 64), (320, 9728, 4, 1, 128, 0, 128)])
 def test_the_same_bits_as_the_parts(sizes, monkeypatch):
+    """Three ways: one call a layer, the same launches one by one for somebody who looks at them, and the parts."""
     from inference_bench_b200.engine.step import StepEntry
-    from inference_bench_b200.kernels import lib
-    outs, counts, native = [], [], []
-    for watch in (False, True):
+    from inference_bench_b200.kernels import dense, lib
+    from inference_bench_b200.parts.standard import PreNormBlock
+    outs, counts, native, by_parts = [], [], [], []
+    forward = PreNormBlock.forward
+    monkeypatch.setattr(PreNormBlock, "forward", lambda self, ctx, *a: (by_parts.append(ctx.n_tokens), forward(self, ctx, *a))[1])
+    for way in ("native", "watched", "parts"):
         names = []
-        if watch:   # somebody looks at every call: the parts run
+        if way == "native":
+            counted = lib.call_counted
+            monkeypatch.setattr(lib, "call_counted", lambda name, *a: (native.append(name), counted(name, *a))[1])
+        elif way == "watched":
             real = lib.call
             monkeypatch.setattr(lib, "call", lambda name, *a: (names.append(name), real(name, *a))[1])
         else:
-            counted = lib.call_counted
-            monkeypatch.setattr(lib, "call_counted", lambda name, *a: (native.append(name), counted(name, *a))[1])
+            monkeypatch.setattr(dense, "MAX_TOKENS", 0)
         r, g = _runner(*sizes), torch.Generator().manual_seed(3)
         for i in range(3):
             r.cache.admit(i)
         got = []
+        del by_parts[:]
         for lens in STEPS:
             entries = [StepEntry(i, torch.randint(0, 333, (n,), generator=g).tolist(), [0, n - 1]) for i, n in enumerate(lens)]
             before = lib.launches
             got.append(r.step(entries).clone())
             counts.append(lib.launches - before)
         outs.append(got + [gr.tensor.clone() for gr in r.cache.groups])
-        assert not watch or "ib_attention_prefill_ws" in names
-    assert native.count("ib_dense_layer") == 3 * 11   # every step but the one of single tokens and the one of 2,561
-    assert counts[:len(STEPS)] == counts[len(STEPS):]
-    assert all(torch.equal(a, b) for a, b in zip(*outs))
+        assert way != "watched" or "ib_attention_prefill_ws" in names
+        assert way == "parts" or set(by_parts) == {3, 2561}   # every step but the one of single tokens and the one of 2,561
+    assert native.count("ib_dense_layer") == 3 * 11
+    assert counts[:len(STEPS)] == counts[len(STEPS):2 * len(STEPS)] == counts[2 * len(STEPS):]
+    assert all(torch.equal(a, b) and torch.equal(a, c) for a, b, c in zip(*outs))
 
 
 @pytest.mark.parametrize("options", [dict(prefill_attention="tcgen05"), dict(decode_attention="split"), dict(gemm="simt")])
