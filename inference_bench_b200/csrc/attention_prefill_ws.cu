@@ -579,6 +579,11 @@ extern "C" int ib_attention_prefill_ws_capped(const void* q, const IbKvView* kv,
   return ib_set_error("attention_prefill_ws: head_dim %d has no tensor-core kernel (64 and 128 have)", kv->head_dim);
 }
 
+// Into how many slices a step's keys are cut on a device of sm_count SMs (arguments as below).
+extern "C" int ib_attention_prefill_slices(int heads, int n_tiles, int max_keys, int window, int keep, int sm_count) {
+  return slices_for((long long)heads * n_tiles, max_keys, window, keep, sm_count);
+}
+
 extern "C" int ib_attention_prefill_ws(const void* q, const IbKvView* kv, const int* tile_seg, const int* tile_row0, int n_tiles,
                                        const int* seg_start, const int* seg_pos0, int window, float scale, void* out, int heads,
                                        const void* kv_map, long long view_row0, int max_keys, unsigned* status, cudaStream_t stream) {

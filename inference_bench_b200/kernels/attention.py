@@ -56,6 +56,7 @@ L.register("ib_attention_decode_fused", [L._p, L._i, L._ll, L._p, L._p, L._f, L.
                                          L._p, L._i, L._i, L._i, L._p, L._ll, L._p, L._p])
 L.register("ib_attention_prefill_tc", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._p])
 L.register("ib_attention_prefill_ws", [L._p, C.POINTER(L.KvView), L._p, L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._i, L._p, L._ll, L._i, L._p, L._p])
+L.register("ib_attention_prefill_slices", [L._i, L._i, L._i, L._i, L._i, L._i])
 # the same with capped scores and a sink (softcap, sink before the status word)
 # (softcap, sink, the output's tail or null, the kept first positions, then the status word)
 L.register("ib_attention_decode_capped", [L._p, C.POINTER(L.KvView), L._p, L._i, L._p, L._p, L._i, L._f, L._p, L._p, L._p, L._i, L._i, L._i, L._f, L._i, C.POINTER(L.AttnTail),

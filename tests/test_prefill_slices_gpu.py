@@ -12,15 +12,24 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-@pytest.mark.parametrize("hd,heads,kvh,page,shapes", [
-    (128, 4, 2, 64, [(1100, 61)]),                          # 8 slices of 18 tiles, one query tile that is half full
-    (64, 6, 3, 8, [(1025, 128), (70, 2), (3, 3)]),          # 8 slices: segments of 17, 2 and 1 key tiles; eight pages a tile
-    (128, 16, 8, 16, [(700, 100), (641, 129)]),             # 4 slices of 11 tiles, a query tile of one row
-    (128, 32, 8, 192, [(1300, 256), (130, 130)]),           # 2 slices at two CTAs an SM: 128 CTAs, tiles of causal keys only beside long ones
-    (64, 2, 1, 128, [(4500, 2), (2500, 300)]),
+def _slices(heads, shapes, window=None, keep=0):
+    """The number of slices on a device of 148 SMs."""
+    from inference_bench_b200.kernels import attention, lib
+    starts = [sum(n for _, n in shapes[:i]) for i in range(len(shapes))]
+    _, _, seg, _, keys = attention.work_lists([n for _, n in shapes], starts, [L - n for L, n in shapes])
+    return lib.load().ib_attention_prefill_slices(heads, len(seg), keys, window or 0, keep, 148)
+
+
+@pytest.mark.parametrize("hd,heads,kvh,page,shapes,slices", [
+    (128, 4, 2, 64, [(1100, 61)], 8),                       # 8 slices of 18 tiles, one query tile that is half full
+    (64, 6, 3, 8, [(1025, 128), (70, 2), (3, 3)], 8),       # 8 slices: segments of 17, 2 and 1 key tiles; eight pages a tile
+    (128, 8, 4, 16, [(700, 100), (641, 129)], 4),           # 4 slices of 11 tiles, a query tile of one row
+    (128, 32, 8, 192, [(1300, 256), (130, 130)], 2),        # 2 slices at two CTAs an SM: 128 CTAs, tiles of causal keys only beside long ones
+    (64, 2, 1, 128, [(4500, 2), (2500, 300)], 8),
 ])
 @pytest.mark.parametrize("window,keep", [(None, 0), (1000, 0), (1030, 70)])
-def test_sliced_portions(hd, heads, kvh, page, shapes, window, keep):
+def test_sliced_portions(hd, heads, kvh, page, shapes, slices, window, keep):
+    assert _slices(heads, shapes) == slices and _slices(heads, shapes, window, keep) > 1
     from inference_bench_b200.engine.context import Segment, build_context
     from inference_bench_b200.engine.runtime import Runtime
     from inference_bench_b200.kernels import attention, ops
@@ -48,14 +57,15 @@ def test_sliced_portions(hd, heads, kvh, page, shapes, window, keep):
     assert (out.double() - other.double()).abs().max() <= 2e-2 * top
 
 
-@pytest.mark.parametrize("hd,heads,kvh,page,shape", [(128, 4, 2, 64, (1100, 61)), (64, 8, 4, 16, (700, 100)), (128, 32, 8, 64, (1300, 250))])   # 8, 4 and 2 slices
-def test_what_is_not_finite_stays_so(hd, heads, kvh, page, shape):
+@pytest.mark.parametrize("hd,heads,kvh,page,shape,slices", [(128, 4, 2, 64, (1100, 61), 8), (64, 8, 4, 16, (700, 100), 4), (128, 32, 8, 64, (1300, 300), 2)])
+def test_what_is_not_finite_stays_so(hd, heads, kvh, page, shape, slices):
     """A query row of NaN, a key that gives infinite scores, a value that is infinite: the rows that see them are not finite, the others keep their bits."""
     from inference_bench_b200.engine.context import Segment, build_context
     from inference_bench_b200.engine.runtime import Runtime
     from inference_bench_b200.kernels import attention
     from inference_bench_b200.kernels.ops import KvLayerView
     L, n = shape
+    assert _slices(heads, [shape]) == slices
     rt, pages = Runtime(DEV), -(-L // page)
     g = torch.Generator().manual_seed(hd)
     pool = torch.randn((1, pages, 2, kvh, page, hd), generator=g).to(torch.bfloat16)
