@@ -494,7 +494,7 @@ __global__ void __launch_bounds__(kThreads, 2)
 }
 
 // Into how many slices the keys of a query tile are cut: a short portion behind a long context has few query tiles, each a chain of key tiles
-// of 0.6 us; the merge takes 4 us more. 61 tokens behind 900 in eight layers of the 0.6B sizes: 588 -> 535 us a step, behind 3,000 785 -> 560. A row: CTAs of the cluster, the fewest key tiles (of the tile that sees the most) with one CTA an SM
+// of 0.6 us; the merge takes 4 us more. 61 tokens behind 900 in eight layers of the 0.6B sizes: 433 -> 387 us on the device, behind 3,000 639 -> 419. A row: CTAs of the cluster, the fewest key tiles (of the tile that sees the most) with one CTA an SM
 // and with two. Measured alone (us, 1 | 2 | 4 | 8 slices; query tiles x heads, most key tiles): 16 CTAs of 16 tiles 20.5 | 18.5 | 16.4 | 16.4, of 32
 // 32.8 | 25.6 | 18.4 | 17.5; 16 of 10 16.4 | 16.4 | 14.4 | 16.4, of 5 12.3 | 14.3 | 14.3 | 13.2; 32 of 47 46.0 | 32.8 | 23.6 | 22.6, of 126 107 | 64 |
 // 41 | 35; 48 of 10 16.6 | 19.4 | 18.4 | 28.7; 64 of 17 23.5 | 21.4 | 20.5 | 31.7, of 8 15.4 | 17.3 | 19.2; 128 of 16 23.5 | 21.4 | 31.7, of 24 29.6 |

@@ -53,9 +53,10 @@ def _check_mirrors() -> None:
         raise L.KernelError(f"csrc/dense_layer.cu has structures of {step.value} and {layer.value} bytes, kernels/dense.py of {C.sizeof(DenseStep)} and {C.sizeof(DenseLayer)}")
 
 
-# Steps of more tokens go layer by layer through the parts: their kernels take longer than the host, and one buffer for a whole layer's intermediates is
-# harder for the allocator to find than its pieces (contexts of 8 requests built in steps of 8,192 tokens: 42 ms, 54 with it). 2,048 tokens, the default
-# portion, beside up to 512 decoded ones go this way.
+# Steps of more tokens go layer by layer through the parts: their kernels take longer than the host, so nothing is gained (2,048 tokens in three layers of the
+# 8B sizes already take 2,160 us either way), and one buffer for a whole layer's intermediates is harder for the allocator to find than its pieces (contexts of
+# 8 requests built in steps of 8,192 tokens: 42 ms, 54 with it). Where between the two the line lies matters little; 2,048 tokens, the default portion,
+# beside up to 512 decoded ones go this way.
 MAX_TOKENS = 2560
 
 KIND = {"single": 0, "pair": 1, "add": 2}

@@ -64,10 +64,12 @@ def choose(T: int, N: int, K: int, allow_split: bool = True, sm_count: int = FIT
     return bn, splits, False
 
 
-# Cost model for 129 to 2,048 tokens, fitted to timings of every variant below on the layer shapes of Qwen3-0.6B, 8B,
+# Cost model for more than 128 tokens, fitted to timings of every variant below on the layer shapes of Qwen3-0.6B, 8B,
 # 14B and 32B at 160 to 1,536 tokens (the variant it picks is within 5 % of the fastest on all of them, 0.2 % on
 # average). A variant's time is waves of CTAs (or CTA pairs) times the longer of a CTA's MMA time and its copy time,
-# plus a fixed cost, plus the traffic of split-K partial sums. Units: FLOP/us, bytes/us, us.
+# plus a fixed cost, plus the traffic of split-K partial sums. Units: FLOP/us, bytes/us, us. From `pair_always_tokens` tokens on it is asked for products that
+# give fewer tiles than there are CTA pairs only (`_fills_pairs`); over 15 such matrices of 8 to 2,304 columns at 2,048 to 8,192 tokens its choice was
+# never slower than the pairs, and 0.84 of their time on average.
 _MID = dict(rate=4.015e6, cap=250e3, t0=4.36, partial_bw=3.455e6, pair_rate=5.446e6, hbm=8.0e6, pair_cap=188e3,
             speed={(256, True): 1.0, (256, False): 0.982, (128, True): 0.895, (128, False): 0.956})
 
@@ -89,7 +91,7 @@ def single_variants(T: int, N: int, K: int, sm_count: int = FITTED_SM_COUNT, all
 
 @functools.lru_cache(maxsize=4096)
 def plan_costs(T: int, N: int, K: int, sm_count: int = FITTED_SM_COUNT, allow_split: bool = True) -> tuple:
-    """(expected us of the CTA-pair kernel, expected us of the best single-CTA form, that form) for 129 <= T < 2048.
+    """(expected us of the CTA-pair kernel, expected us of the best single-CTA form, that form) for more than 128 tokens.
     allow_split=False leaves out the forms that cut the k-range (for a caller that wants one finished product)."""
     m = _MID
     tiles = -(-N // 256) * -(-T // 256)
@@ -110,7 +112,7 @@ def plan_costs(T: int, N: int, K: int, sm_count: int = FITTED_SM_COUNT, allow_sp
 
 
 def plan(T: int, N: int, K: int, sm_count: int = FITTED_SM_COUNT, allow_split: bool = True) -> tuple:
-    """For 129 <= T < 2048: ("pair",) or ("single", tokens per CTA, k-splits, wide), whichever the cost model
+    """For more than 128 tokens: ("pair",) or ("single", tokens per CTA, k-splits, wide), whichever the cost model
     expects to be faster. Depends on the sizes (and the device's SM count) only."""
     pair, single, form = plan_costs(T, N, K, sm_count, allow_split)
     return ("pair",) if pair <= single else ("single",) + form
@@ -256,7 +258,7 @@ def swiglu_form(T: int, inter: int, pair_min_tokens: int = 129) -> tuple[int, bo
     if T >= pair_min_tokens or (T > 32 and -(-inter // 256) >= PAIR_SWIGLU_MIN_TILES):
         return 0, False
     bn = 64 if T <= 64 else (128 if T <= 128 else 256)
-    return bn, bn in (16, 32)
+    return bn, False
 
 
 def gemm_swiglu(x: torch.Tensor, w_gate_up: torch.Tensor, act: torch.Tensor, status: torch.Tensor, bn: int | None = None, pair_min_tokens: int = 129,

@@ -8,7 +8,7 @@ pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
 
 
-def _runner(hidden, inter, heads, kv_heads, head_dim, window, page, options=None):
+def _runner(hidden, inter, heads, kv_heads, head_dim, window, page, options=None, layers=3, change=lambda plan: plan):
     from inference_bench_b200.cache.manager import CacheManager
     from inference_bench_b200.config.runtime_options import RuntimeOptions
     from inference_bench_b200.engine.model import plan_from_config
@@ -16,13 +16,13 @@ def _runner(hidden, inter, heads, kv_heads, head_dim, window, page, options=None
     from inference_bench_b200.engine.step import ModelRunner
     from inference_bench_b200.parts.decoder import Decoder
     from inference_bench_b200.weights.random_init import random_weights
-    cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", vocab_size=333, hidden_size=hidden, intermediate_size=inter, num_hidden_layers=3, num_attention_heads=heads,
+    cfg = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", vocab_size=333, hidden_size=hidden, intermediate_size=inter, num_hidden_layers=layers, num_attention_heads=heads,
                num_key_value_heads=kv_heads, head_dim=head_dim, rms_norm_eps=1e-6, rope_theta=1e6, tie_word_embeddings=True, max_position_embeddings=8192, hidden_act="silu",
                attention_bias=False, torch_dtype="bfloat16")
     if window:
-        cfg.update(use_sliding_window=True, sliding_window=window, max_window_layers=0, layer_types=["full_attention", "sliding_attention", "full_attention"])
+        cfg.update(use_sliding_window=True, sliding_window=window, max_window_layers=0, layer_types=["full_attention", "sliding_attention"] * (layers // 2) + ["full_attention"] * (layers % 2))
     rt = Runtime(DEV, "bfloat16", options=options or RuntimeOptions())
-    decoder = Decoder(plan_from_config(cfg)[1])
+    decoder = Decoder(change(plan_from_config(cfg)[1]))
     decoder.bind({k: v.to(DEV) for k, v in random_weights(decoder.weight_specs(), 5, std=0.05).items()}, rt)
     cache = CacheManager(decoder.cache_needs(), page, 12000 // page, 8, 6000, device=rt.device, dtype=rt.act_dtype, sources=decoder.cache_sources())
     return ModelRunner(decoder, cache, rt)
@@ -99,3 +99,27 @@ def test_a_refused_kernel_ends_the_layer(monkeypatch):
     assert all(torch.equal(a, g.tensor) for a, g in zip(before, r.cache.groups))
     assert r.cache.length(0) == 40
     assert torch.isfinite(r.step([StepEntry(0, list(range(50)), [49])])).all()
+
+
+def test_layers_of_two_keys_around_other_arrangements(monkeypatch):
+    """Full and windowed layers before, between and behind layers with another norm (which the parts run): the same bits as by parts alone."""
+    from dataclasses import replace
+    from inference_bench_b200.engine.step import StepEntry
+    from inference_bench_b200.kernels import dense, lib
+
+    def other(plan):   # layers 1 and 4 of six
+        norm = lambda spec: replace(spec, kind="layernorm")
+        return replace(plan, layers=tuple(replace(lp, mixer_norm=norm(lp.mixer_norm), feed_forward_norm=norm(lp.feed_forward_norm)) if i in (1, 4) else lp
+                                          for i, lp in enumerate(plan.layers)))
+    outs, native, counted = [], [], lib.call_counted
+    monkeypatch.setattr(lib, "call_counted", lambda name, *a: (native.append(name), counted(name, *a))[1])
+    for way in ("native", "parts"):
+        if way == "parts":
+            monkeypatch.setattr(dense, "MAX_TOKENS", 0)
+        r, g = _runner(256, 640, 4, 2, 64, 70, 16, layers=6, change=other), torch.Generator().manual_seed(7)
+        for i in range(2):
+            r.cache.admit(i)
+        got = [r.step([StepEntry(i, torch.randint(0, 333, (n,), generator=g).tolist(), [0, n - 1]) for i, n in enumerate(lens)]).clone() for lens in ([90, 33], [1, 40], [200, 1])]
+        outs.append(got + [gr.tensor.clone() for gr in r.cache.groups])
+    assert len(native) == 3 * 4
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
