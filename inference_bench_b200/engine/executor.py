@@ -8,6 +8,8 @@ slot, and the graph holds the whole model, the sampling kernel included.
 """
 from __future__ import annotations
 
+import contextlib
+import gc
 from typing import Optional
 
 import numpy as np
@@ -21,6 +23,19 @@ from .step import ModelRunner, StepEntry
 
 
 RUN_AHEAD_MAX = 64
+
+
+@contextlib.contextmanager
+def _no_collection():
+    """A capture is lost when the garbage collector destroys another graph meanwhile (of an engine that is no longer used, say): the driver allows no such call
+    while a stream is capturing. What is garbage now is collected afterwards."""
+    on = gc.isenabled()
+    gc.disable()
+    try:
+        yield
+    finally:
+        if on:
+            gc.enable()
 
 
 class _DecodeGraph:
@@ -111,7 +126,7 @@ class _DecodeGraph:
         from ..kernels import lib
         before = lib.launches
         graph = torch.cuda.CUDAGraph()
-        with torch.cuda.graph(graph, pool=next(iter(self.graphs.values())).pool() if self.graphs else None):
+        with _no_collection(), torch.cuda.graph(graph, pool=next(iter(self.graphs.values())).pool() if self.graphs else None):
             if alone:
                 ops.fetch_ints(self.host, self.dev)
             self.logits_of[alone] = self._forward(alone)

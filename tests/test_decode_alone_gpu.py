@@ -103,3 +103,33 @@ def test_tokens_left_by_one_form_feed_the_other(batch):
     assert len(set(sum(got[0], []))) > 1
     g = ex.graph_for(batch)   # two captured forms over one set of buffers and one pool
     assert set(g.graphs) == {True, False} and len({x.pool() for x in g.graphs.values()}) == 1
+
+
+def test_a_capture_outlives_a_garbage_collection():
+    """Another graph becomes garbage in a cycle while a step is captured, and enough objects are made for the collector to run."""
+    import gc
+    from inference_bench_b200.engine.executor import GpuExecutor
+    from inference_bench_b200.engine.step import StepEntry
+    from inference_bench_b200.sampling.params import GREEDY
+    x = torch.zeros(8, device=DEV)
+    other = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(other):
+        x.add_(1)
+    held = [other]
+    held.append(held)
+    del other
+    r = _runner(256, 640, 4, 2, 64, 0, 16)
+    ex, forward = GpuExecutor(r), r.decoder.forward
+
+    def dropping(ctx):
+        nonlocal held
+        if torch.cuda.is_current_stream_capturing():
+            held = None
+            made = [[] for _ in range(5000)]
+            assert not gc.isenabled() and len(made) == 5000
+        return forward(ctx)
+    r.decoder.forward = dropping
+    r.cache.admit(0)
+    first = ex.execute([StepEntry(0, [1], [0])], [(GREEDY, 0)])
+    assert held is None and gc.isenabled()
+    assert ex.execute([StepEntry(0, first, [0])], [(GREEDY, 1)])
