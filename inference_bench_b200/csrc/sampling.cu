@@ -12,7 +12,7 @@
 namespace {
 
 constexpr int kThreads = 512, kWarpsOfRow = kThreads / 32;
-constexpr int kCtasOfSm = 3;         // CTAs that share an SM
+constexpr int kCtasOfSm = 3;         // CTAs that may share an SM
 constexpr int kMaxParts = 8;         // of a row: its vocabulary is cut into 1, 2, 4 or 8 parts, which its cluster's CTAs share
 constexpr int kPartValues = 4096;    // the least number of values in a part
 
@@ -204,13 +204,15 @@ __device__ __forceinline__ unsigned search(const float* row, int V, int share, i
 }
 
 // One row. All of a greedy row is one pass over its logits; a threshold is eight passes of four bits each over logits that stay in L2, and what a pass costs
-// is its reductions, not its reads. A row of 151,936 took 945 us with top-p, 185 with top-k and 850 with both, by one CTA and a pass for every step of a
-// bisection, and a greedy one 13 us in three kernels: 54, 48, 77 and 9 us so (64 rows: 955, 196, 906 and 20 against 135, 103, 175 and 12). Where a CTA has
-// several parts of a row their masses are summed one after the other: 64 rows with top-p took 113 us in an order that followed the number of CTAs, and the
+// is its reductions, not its reads. A row of 151,936 took 929 us with top-p, 222 with top-k and 885 with both and min-p, by one CTA and a pass for every step of a
+// bisection, and a greedy one 17 us in three kernels: 51, 45, 71 and 12 us so (64 rows: 1,000, 240, 941 and 36 against 129, 92, 166 and 18; caches cold). Where a
+// CTA has several parts of a row their masses are summed one after the other: 64 rows with top-p took 113 us in an order that followed the number of CTAs, and the
 // token of a row could then change with the number of rows.
 // With `status` the step's status word is copied to tokens[rows], so the host gets it in the transfer that brings the tokens.
-__global__ void __launch_bounds__(kThreads, kCtasOfSm) sample_kernel(const float* __restrict__ logits, int V, int share, int own, const RowParams* __restrict__ params,
-                                                             int* __restrict__ tokens, const unsigned* __restrict__ status) {
+// PER_SM: how many CTAs share an SM, by the registers a thread may have.
+template <int PER_SM>
+__global__ void __launch_bounds__(kThreads, PER_SM) sample_kernel(const float* __restrict__ logits, int V, int share, int own, const RowParams* __restrict__ params,
+                                                                  int* __restrict__ tokens, const unsigned* __restrict__ status) {
   __shared__ RowShared sh;
   ib::pdl_launch_dependents();
   ib::pdl_wait();
@@ -326,24 +328,45 @@ extern "C" int ib_advance_rows(const int* sampled, int* token_in, int* positions
   return 0;
 }
 
+namespace {
+
+// How many rows of 1 << lg CTAs the device runs at once (a cluster's CTAs lie in one group of SMs, so this is less than the CTAs that fit).
+template <int PER_SM>
+int rows_at_once(int lg) {
+  static int known[4] = {};
+  if (!known[lg]) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(1u << lg, 65535);
+    cfg.blockDim = kThreads;
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 1u << lg, attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, sample_kernel<PER_SM>, &cfg) != cudaSuccess) cudaGetLastError(), n = 0;
+    known[lg] = n > 0 ? n : 1;
+  }
+  return known[lg];
+}
+
+}  // namespace
+
 // logits float32 [rows, V], params [rows] of six words -> tokens int32 [rows].
 // status: null, or the device status word, whose value is then stored in tokens[rows] (tokens has rows + 1 entries).
 extern "C" int ib_sample_rows(const float* logits, int rows, int V, const void* params, int* tokens, const unsigned* status, cudaStream_t stream) {
   if (rows == 0) return 0;
   IB_CHECK_ARG(rows > 0 && rows <= 65535 && V > 0, "sample_rows: bad sizes rows=%d V=%d", rows, V);
-  static int sm_count = 0;
-  if (!sm_count) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev);
-  }
-  // The parts follow from the vocabulary alone. The CTAs that share them: as many as leave the device kCtasOfSm an SM, so that
-  // all run at once: 64 rows of 151,936 with top-p take 311 us on 1 CTA a row, 182 on 2, 143 on 4, 177 on 8; 160 rows 463 | 345 | 307 | 355; 128 rows of
-  // 32,768 114 | 105 | 120 | 159; 38 rows of 151,936 307 | 178 | 137 | 112.
-  int parts = 1, ctas = 1;
+  // The parts follow from the vocabulary alone. The CTAs that share them: as many as leave all rows running at once, three CTAs an SM: 64 rows of 151,936 with
+  // top-p take 311 us on 1 CTA a row, 182 on 2, 143 on 4, 177 on 8; 160 rows 463 | 345 | 307 | 355; 128 rows of 32,768 114 | 105 | 120 | 159; 38 rows of 151,936
+  // 307 | 178 | 137 | 112. And no more CTAs an SM than that takes: where three fit, some SMs are given three and others one. 64 rows of 151,936, logits in L2,
+  // three | two an SM: drawn without a filter 44 | 32 us, top-k 129 | 85, top-p 172 | 122; 128 rows 86 | 62, 220 | 141, 309 | 212.
+  int parts = 1, lg = 0;
   while (parts < kMaxParts && 2 * parts * kPartValues <= V) parts *= 2;
-  while (ctas < parts && (long long)rows * 2 * ctas <= kCtasOfSm * sm_count) ctas *= 2;
-  ib::launch_cluster(sample_kernel, dim3(ctas, rows), dim3(ctas), kThreads, 0, stream, logits, V, ((V + parts - 1) / parts + 3) & ~3, parts / ctas, (const RowParams*)params, tokens, status);
+  while (1 << lg < parts && rows <= rows_at_once<kCtasOfSm>(lg + 1)) lg++;
+  const int ctas = 1 << lg;
+  ib::launch_cluster(rows <= rows_at_once<2>(lg) ? sample_kernel<2> : sample_kernel<kCtasOfSm>, dim3(ctas, rows), dim3(ctas), kThreads, 0, stream, logits, V,
+                     ((V + parts - 1) / parts + 3) & ~3, parts / ctas, (const RowParams*)params, tokens, status);
   IB_CHECK_LAUNCH("sample_rows");
   return 0;
 }
