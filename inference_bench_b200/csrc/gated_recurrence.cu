@@ -1021,10 +1021,12 @@ extern "C" int ib_recurrence_chunks_finish(const int* long_segs, int n_long, con
   if (n_long == 0 || n_chunks == 0) return 0;
   IB_CHECK_ARG(n_long > 0 && n_chunks > 0 && heads > 0 && heads <= 65535 && D > 0 && V > 0, "recurrence_chunks_finish: bad sizes");
   // The kernels before hold up to 179 KB of shared memory a CTA. With a small share of their own these two made every SM that had one of those CTAs change its
-  // split first, 10 us where the kernels take 40: 400 tokens of 2 heads of 128 x 128, all three kernels, 52.7 -> 39.7 us, 200 of 4 heads 52.2 -> 39.5.
+  // split first, 10 us where the kernels take 40: 400 tokens of 2 heads of 128 x 128, all three kernels, 52.7 -> 40.2 us, 200 of 4 heads 52.3 -> 39.6. They ask for
+  // the 164 KB that gated_chunk_kernel gets; with all of it, and less left as cache, 2,048 tokens of 16 heads were 1 % slower.
   static const cudaError_t split = [] {
-    const cudaError_t e = cudaFuncSetAttribute(chunk_carry_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
-    return e == cudaSuccess ? cudaFuncSetAttribute(chunk_apply_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared) : e;
+    constexpr int percent = 164 * 100 / 228 + 1;
+    const cudaError_t e = cudaFuncSetAttribute(chunk_carry_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent);
+    return e == cudaSuccess ? cudaFuncSetAttribute(chunk_apply_kernel, cudaFuncAttributePreferredSharedMemoryCarveout, percent) : e;
   }();
   IB_CHECK_ARG(split == cudaSuccess, "recurrence_chunks_finish: cannot set the split of shared memory: %s", cudaGetErrorString(split));
   ib::launch(chunk_carry_kernel, dim3((unsigned)n_long, (unsigned)heads, (unsigned)min((D * V + 255) / 256, 64)), 256, 0, stream, long_segs, seg_slot, state,
