@@ -33,7 +33,8 @@ constexpr int kThreads = 192;
 // stream is less than half of the product's last place, and a sum of the product (a multiple of 2^-123) and a number of at least 2^-102 (a multiple of 2^-125) is
 // zero or at least 2^-125. Where a thread has a smaller
 // product among its 32 it adds them itself, so the sums are the bits of an IEEE addition.
-// (What the look at the 32 costs, warm: 1,003 tokens of 4,096 x 4,096 42.4 -> 43.0 us, 2,048 of 1,024 x 2,048 19.8 -> 20.1, 300 of 1,024 x 3,072 22.1 -> 23.6.)
+// (Whole 32s are looked at and added without a test a token, which pays for the look: warm, additions of every product in L2 | now, 300 tokens of 1,024 x 3,072
+// 21.7 | 21.6 us, 2,048 of 4,096 x 4,096 53.1 | 52.7, of 4,096 x 12,288 141.1 | 140.3.)
 constexpr float kAddInL2 = 0x1p-100f;
 constexpr int EPI_STORE = 0, EPI_SWIGLU = 1, EPI_ADD = 2;   // float32 out; bfloat16 silu(gate) * up; float32 out += product
 constexpr int EPI_QKV = 3;   // the q/k/v projection finished in the epilogue: per-head norm, rotation, queries out, keys and values into the cache
@@ -453,18 +454,34 @@ __global__ void __launch_bounds__(kThreads, 1)
             uint32_t r[32];
             sm100::tmem_ld_32x32b_x32(lane_addr + b * MT * BN + m * BN + c0, r);
             sm100::tmem_ld_wait();
-            if (n < N) {
-              if constexpr (EPI == EPI_ADD) {
-                float least = INFINITY;
+            if constexpr (EPI == EPI_ADD) {
+              const bool whole = t0 + c0 + 32 <= t_end;
+              float least = INFINITY;
+              if (whole) {
+#pragma unroll
+                for (int c = 0; c < 32; c += 2) least = fminf(fminf(least, fabsf(__uint_as_float(r[c]))), fabsf(__uint_as_float(r[c + 1])));
+              } else {
 #pragma unroll
                 for (int c = 0; c < 32; c++) least = fminf(least, t0 + c0 + c < t_end ? fabsf(__uint_as_float(r[c])) : INFINITY);
+              }
+              // every element belongs to one thread of one launch: one addition, the same sum in every run
+              auto add = [&](int t, uint32_t v) { asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + (size_t)t * N + n), "f"(__uint_as_float(v)) : "memory"); };
+              if (n < N) {
                 if (least < kAddInL2) {
 #pragma unroll
                   for (int c = 0; c < 32; c++)
                     if (t0 + c0 + c < t_end) dst[(size_t)(t0 + c0 + c) * N + n] += __uint_as_float(r[c]);
-                  continue;
+                } else if (whole) {
+#pragma unroll
+                  for (int c = 0; c < 32; c++) add(t0 + c0 + c, r[c]);
+                } else {
+#pragma unroll
+                  for (int c = 0; c < 32; c++)
+                    if (t0 + c0 + c < t_end) add(t0 + c0 + c, r[c]);
                 }
               }
+              __syncwarp();   // (the next load from tensor memory is the whole warp's)
+            } else if (n < N) {
 #pragma unroll
               for (int c = 0; c < 32; c++) {
                 const int t = t0 + c0 + c;
@@ -473,8 +490,6 @@ __global__ void __launch_bounds__(kThreads, 1)
                     dst_act[(size_t)t * N + n] = __float2bfloat16_rn(ib::xielu(__uint_as_float(r[c]), ap, an));
                   else if constexpr (EPI == EPI_RELU2)
                     dst_act[(size_t)t * N + n] = __float2bfloat16_rn(ib::relu2(__uint_as_float(r[c])));
-                  else if constexpr (EPI == EPI_ADD)   // every element belongs to one thread of one launch: one addition, the same sum in every run
-                    asm volatile("red.global.add.f32 [%0], %1;" ::"l"(dst + (size_t)t * N + n), "f"(__uint_as_float(r[c])) : "memory");
                   else
                     dst[(size_t)t * N + n] = __uint_as_float(r[c]);
                 }
